@@ -98,6 +98,7 @@ class PagedCache:
                         dtype=getattr(torch, need.state_dtype), device=self.device)
             else:
                 raise ValueError(f"unknown cache need {need.kind!r}")
+        self._state_units = [state.unsqueeze(0) for state in self.states.values()]   # [1, requests, ...] each
         host = build.host()
         self.manager = host.CacheManager(
             [host.GroupConfig(page_tokens, g.need.window or 0, g.num_pages, g.need.chunk or 0, g.need.keep) for g in self.groups],
@@ -137,19 +138,18 @@ class PagedCache:
         source_slot, target_slot, copies = self.manager.fork(parent, child)
         if self.device.type != "cuda":
             return
-        for group in self.groups:
-            pairs = [(source, target) for g, source, target in copies if g == group.index]
-            if pairs and group.pool is not None:
-                ops.copy_units(group.pool, torch.tensor(pairs, dtype=torch.int32, device=self.device))
-        if self.states:
-            slots = torch.tensor([[source_slot, target_slot]], dtype=torch.int32, device=self.device)
-            for state in self.states.values():
-                ops.copy_units(state.unsqueeze(0), slots)
+        ops.copy_units_by_host([(self.groups[g].pool, source, target) for g, source, target in copies
+                                if self.groups[g].pool is not None]
+                               + [(state, source_slot, target_slot) for state in self._state_units])
 
     # ------------------------------------------------------------- step views
     def zero_state(self, slot: int) -> None:
-        for state in self.states.values():
-            state[slot].zero_()
+        if self._state_units and self.device.type == "cuda":
+            from .. import ops
+            ops.copy_units_by_host([(state, None, slot) for state in self._state_units])   # one launch for all of them
+        else:
+            for state in self.states.values():
+                state[slot].zero_()
 
     def view(self, entry: int, write: bool, tables: Dict[int, torch.Tensor],
              slots: Dict[int, torch.Tensor]) -> CacheView:

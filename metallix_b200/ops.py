@@ -33,6 +33,7 @@ _SIGNATURES = {
     "mxb_add_summands_rmsnorm": [_P, _P, _I, _P, _I, _P, _I, _I, _F, _P],
     "mxb_add": [_P, _P, _I, _L, _L, _P],
     "mxb_copy_units": [_P, _I, _I, _L, _P, _I, _P, _P],
+    "mxb_copy_spans": [_P, _I, _P],
     "mxb_qk_norm_rope_cache": [_P, _P, _P, _L, _L, _L, _P, _P, _P, _P, _P, _P, _P, _P,
                                _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _P],
     "mxb_paged_attention_tile": [_P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
@@ -1233,6 +1234,24 @@ def copy_units(pool: torch.Tensor, pairs: torch.Tensor) -> None:
     unit_bytes = pool[0, 0].numel() * pool.element_size()
     _call("mxb_copy_units", pool.data_ptr(), entries, units, unit_bytes, pairs.data_ptr(), pairs.shape[0],
           status_word(pool.device).data_ptr(), _stream())
+
+
+def copy_units_by_host(copies) -> None:
+    """``copies``: [(pool, source, target)]: pool[:, target] = pool[:, source] of contiguous pools ``[entries, units, ...]``
+    on one device, ``source`` None for zeros; all in one launch, the unit numbers known to the host. No target may be
+    another copy's source."""
+    spans = []
+    for pool, source, target in copies:
+        _need(pool.is_cuda and pool.is_contiguous() and pool.dim() >= 2, "pool must be a contiguous device tensor")
+        entries, units = pool.shape[0], pool.shape[1]
+        _need(0 <= target < units and (source is None or 0 <= source < units), f"unit outside the pool's {units}")
+        if source == target or pool.numel() == 0:
+            continue
+        base, stride = pool.data_ptr(), pool.stride(0) * pool.element_size()
+        size = stride // units
+        spans += (base + target * size, 0 if source is None else base + source * size, size, stride, entries)
+    if spans:
+        _call("mxb_copy_spans", (ctypes.c_longlong * len(spans))(*spans), len(spans) // 5, _stream())
 
 
 # ------------------------------------------------- q/k norm, rotation, cache

@@ -1111,3 +1111,21 @@ def test_copy_units(shape, dtype):
     assert torch.equal(pool, expected)
     with pytest.raises(ops.KernelError, match="outside the page pool"):
         ops.check_status(pool.device)
+
+
+@pytest.mark.parametrize("unit", [1, 20, 16384, 16384 + 16, 3 * 16384 + 4])   # bytes: below, at and across a block's piece
+def test_copy_units_by_host(unit):
+    """Several pools in one launch (more than one launch's list holds), copies and zeros; other units untouched."""
+    from metallix_b200 import ops
+    pools = [torch.randint(-100, 100, (1 + index % 3, 4, unit), dtype=torch.int8, device="cuda") for index in range(35)]
+    expected = [pool.clone() for pool in pools]
+    copies = []
+    for index, (pool, want) in enumerate(zip(pools, expected)):
+        source, target = (None, 3) if index % 4 == 1 else (index % 3, 3)
+        want[:, target] = 0 if source is None else want[:, source]
+        copies.append((pool, source, target))
+    ops.copy_units_by_host(copies + [(pools[0], 1, 1)])
+    for pool, want in zip(pools, expected):
+        assert torch.equal(pool, want)
+    with pytest.raises(ops.KernelError):
+        ops.copy_units_by_host([(pools[0], 0, 4)])
