@@ -46,16 +46,20 @@ constexpr int kFaValueWarp = kFaThreads / 32 - 1;
 constexpr int kFaTmemColumns = 512;
 constexpr int kFaHalfBytes = 128 * kTmaColumns * 2;  // a [128 x 64] bfloat16 operand block: 16 KiB
 
-template <int HD> struct FaConfig {
-  static constexpr int kHalves = HD / kTmaColumns;
-  static constexpr int kTileBytes = kHalves * kFaHalfBytes;    // Q, a K stage or a V stage
-  static constexpr int kKeyStages = HD == 64 ? 4 : 3;          // at most; one block per SM either way
-  static constexpr int kValueStages = HD == 64 ? 4 : 2;
+// HDK: how many values of a query and a key take part; HDV: how many values of a head's output a block makes.
+template <int HDK, int HDV> struct FaConfig {
+  static constexpr int kKeyHalves = HDK / kTmaColumns, kValueHalves = HDV / kTmaColumns;
+  static constexpr int kKeyBytes = kKeyHalves * kFaHalfBytes;      // Q or a K stage
+  static constexpr int kValueBytes = kValueHalves * kFaHalfBytes;  // a V stage
+  static constexpr int kKeyStages = HDK == 64 ? 4 : (HDK == 128 ? 3 : (HDK == 192 ? 2 : 1));   // at most; one block per SM either way
+  static constexpr int kValueStages = HDV == 64 ? 4 : 2;
   static constexpr int kSmallBytes = 512 + 2 * kFaParts * kFaRows * 4;  // barriers and the exchange of maxima, after the tiles
   // Wanted: the tiles of every stage, the small area and room to align to 1024 bytes.
-  static constexpr int kSharedBytes = (1 + kKeyStages + kValueStages) * kTileBytes + kSmallBytes + 1024;
+  static constexpr int kSharedBytes = (1 + kKeyStages) * kKeyBytes + kValueStages * kValueBytes + kSmallBytes + 1024;
   static constexpr int kScoreColumns = kFaKeys;                // two buffers of 128 columns
-  static constexpr int kOutputBase = 2 * kFaKeys;              // then two buffers of HD columns
+  static constexpr int kOutputBase = 2 * kFaKeys;              // then two buffers of HDV columns
+  // Whether a softmax weight meets the values as two bfloat16 parts, itself and what its rounding left, instead of one.
+  static constexpr bool kSplitWeights = HDK > 128;
 };
 
 __device__ __forceinline__ float fa_exp2(float x) {
@@ -69,35 +73,43 @@ __device__ __forceinline__ uint32_t fa_pack(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&pair);
 }
 
-template <int HD, bool BIASED>   // BIASED: built apart, its registers and instructions are no unbiased call's
+// Heads of 256 values. Two score and two output buffers of a whole head would be 768 columns of tensor memory, so a
+// block makes 128 values of the output (the scores are made again for the other 128, a third of the whole work, and not
+// at all where the caller says that the values end there), and 192 values of queries and keys are brought where no more
+// are in use. The general kernel, which took these heads before, multiplies float32 weights with the values; so here a
+// weight is two bfloat16 parts, 16 bits of it, and V meets both. 2,048 tokens,
+// 32 heads of 192 / 128 values: 99 us, 30.9 ms in the general kernel.
+template <int HDK, int HDV, bool BIASED>   // BIASED: built apart, its registers and instructions are no unbiased call's
 __global__ void __launch_bounds__(kFaThreads, 1)
 flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_cache,
                              __nv_bfloat16* __restrict__ out, const int* __restrict__ block_tables, int max_pages,
                              const int* __restrict__ tile_request, const int* __restrict__ tile_start,
                              const int* __restrict__ tile_length, const int* __restrict__ positions, int heads,
-                             int kv_heads, int page_tokens, int num_pages, int window, int chunk, int keep, float scale, float softcap,
-                             int shared_bytes, float* __restrict__ partial, const __nv_bfloat16* __restrict__ gate,
+                             int kv_heads, int groups, int page_tokens, int num_pages, int window, int chunk, int keep,
+                             float scale, float softcap, int shared_bytes, float* __restrict__ partial, const __nv_bfloat16* __restrict__ gate,
                              long long gate_stride, int has_sink, float sink_log2, const float* __restrict__ sink_heads,
                              ScoreBias bias, int bias_bytes, int* status) {
-  using Config = FaConfig<HD>;
-  constexpr int MAX_STAGES = Config::kKeyStages;
-  constexpr int HALVES = Config::kHalves;
+  using Config = FaConfig<HDK, HDV>;
+  constexpr int head_dim = HDK > 128 ? 256 : HDK;         // of a row of queries, keys, values or output
+  const int value_groups = HDK > 128 ? groups : 1;        // blocks per head, each with HDV values of the output
+  constexpr int MAX_KEY_STAGES = Config::kKeyStages;
+  constexpr int MAX_STAGES = MAX_KEY_STAGES > Config::kValueStages ? MAX_KEY_STAGES : Config::kValueStages;   // of barriers
   // All shared memory is dynamic: the block gets `shared_bytes` (up to the
   // device's limit) and uses as many key stages as fit behind the 1024-byte
   // boundary the swizzled tiles need.
   extern __shared__ unsigned char fa_shared_raw[];
   const int slack = (1024 - (shared_address(fa_shared_raw) & 1023)) & 1023;
   const int VS = Config::kValueStages;
-  const int fitting = (shared_bytes - slack - Config::kSmallBytes - bias_bytes) / Config::kTileBytes - 1 - VS;
-  const int KS = fitting < MAX_STAGES ? fitting : MAX_STAGES;
+  const int fitting = (shared_bytes - slack - Config::kSmallBytes - bias_bytes - VS * Config::kValueBytes) / Config::kKeyBytes - 1;
+  const int KS = fitting < MAX_KEY_STAGES ? fitting : MAX_KEY_STAGES;
   if (KS < 1) {  // the launcher asks for more than that
     if (threadIdx.x == 0) atomicOr(status, kStatusWaitTimeout);
     return;
   }
   unsigned char* q_tile = fa_shared_raw + slack;
-  unsigned char* k_tiles = q_tile + Config::kTileBytes;
-  unsigned char* v_tiles = k_tiles + KS * Config::kTileBytes;
-  unsigned char* small = v_tiles + VS * Config::kTileBytes;
+  unsigned char* k_tiles = q_tile + Config::kKeyBytes;
+  unsigned char* v_tiles = k_tiles + KS * Config::kKeyBytes;
+  unsigned char* small = v_tiles + VS * Config::kValueBytes;
   uint64_t* q_full = reinterpret_cast<uint64_t*>(small);
   uint64_t* k_full = q_full + 1;
   uint64_t* k_empty = k_full + MAX_STAGES;
@@ -116,7 +128,8 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
   float* near_bias = reinterpret_cast<float*>(small + Config::kSmallBytes);
   static_assert((1 + 4 * MAX_STAGES + 8 + 4 + 1) * 8 + 8 <= 512, "the barriers do not fit their area");
 
-  const int head = blockIdx.x, tile = blockIdx.y;  // heads of one tile run side by side and share its keys in L2
+  // heads of one tile run side by side and share its keys in L2
+  const int head = blockIdx.x / value_groups, group = blockIdx.x % value_groups, tile = blockIdx.y;
   const int kv = head / (heads / kv_heads);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = tile_start[tile], n = tile_length[tile];
@@ -176,14 +189,17 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     uint64_t* empty = values ? v_empty : k_empty;
     unsigned char* tiles = values ? v_tiles : k_tiles;
     const int* table = block_tables + static_cast<size_t>(tile_request[tile]) * max_pages;
+    const int halves = values ? Config::kValueHalves : Config::kKeyHalves;
+    const uint32_t tile_bytes = values ? Config::kValueBytes : Config::kKeyBytes;
     if (!values && lane == 0) {
-      barrier_arrive_expect(q_full, Config::kTileBytes);
-      for (int half = 0; half < HALVES; ++half)
-        tma_load_2d(q_tile + half * kFaHalfBytes, &map_q, head * HD + half * kTmaColumns, t0, q_full);
+      barrier_arrive_expect(q_full, Config::kKeyBytes);
+      for (int half = 0; half < Config::kKeyHalves; ++half)
+        tma_load_2d(q_tile + half * kFaHalfBytes, &map_q, head * head_dim + half * kTmaColumns, t0, q_full);
     }
     const int pages_per_tile = kFaKeys / page_tokens;
-    const int copies = pages_per_tile * HALVES;  // every page, every 64-value half
-    const int slot = lane / HALVES, half = lane % HALVES;  // copies <= 32: one per lane
+    const int copies = pages_per_tile * halves;  // every page, every 64-value half
+    const int slot = lane / halves, half = lane % halves;  // copies <= 32: one per lane
+    const int column = (values ? group * HDV : 0) + half * kTmaColumns;
     const uint32_t offset = half * kFaHalfBytes + slot * page_tokens * (kTmaColumns * 2);
     // Pages no row of the tile can see are not looked up: their box starts
     // beyond the cache's last row, where the copy engine writes zeros. A
@@ -218,17 +234,17 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       uint64_t* landing = tail ? v_tail : &full[stage];
       // K as soon as the scores that read this stage last are done, V when the P V product is.
       if (!barrier_wait(&empty[stage], ((i / stages) & 1) ^ 1, status)) { failed = 1; break; }
-      if (lane == 0) barrier_arrive_expect(landing, Config::kTileBytes);
+      if (lane == 0) barrier_arrive_expect(landing, tile_bytes);
       __syncwarp();
-      unsigned char* stage_tile = tiles + stage * Config::kTileBytes;
+      unsigned char* stage_tile = tiles + stage * tile_bytes;
       if (lane < copies)
-        tma_load_2d(stage_tile + offset, &map_cache, half * kTmaColumns, box_row, landing);
+        tma_load_2d(stage_tile + offset, &map_cache, column, box_row, landing);
       if (tail) {
         if (!barrier_wait(v_tail, 0, status)) { failed = 1; break; }
         // a key's 64 values of one half are 128 bytes, swizzled among themselves
-        for (int c = lane; c < (zero_to - zero_from) * HALVES * 8; c += 32)
-          *reinterpret_cast<uint4*>(stage_tile + ((c >> 3) % HALVES) * kFaHalfBytes +
-                                    (zero_from + c / (HALVES * 8)) * (kTmaColumns * 2) + (c & 7) * 16) =
+        for (int c = lane; c < (zero_to - zero_from) * Config::kValueHalves * 8; c += 32)
+          *reinterpret_cast<uint4*>(stage_tile + ((c >> 3) % Config::kValueHalves) * kFaHalfBytes +
+                                    (zero_from + c / (Config::kValueHalves * 8)) * (kTmaColumns * 2) + (c & 7) * 16) =
               make_uint4(0u, 0u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // before the tensor core reads them
         __syncwarp();
@@ -240,7 +256,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     // ---- one thread issues every MMA
     if (lane == 0) {
       constexpr uint32_t idesc_s = tc_instruction_descriptor(kFaRows, kFaKeys);
-      constexpr uint32_t idesc_o = tc_instruction_descriptor_b_mn(kFaRows, HD);
+      constexpr uint32_t idesc_o = tc_instruction_descriptor_b_mn(kFaRows, HDV);
       // This one thread is the block's pacemaker: what it does per key tile
       // (three waits, sixteen MMAs, four commits) is kept short. The
       // descriptors of the operands are made once; a stage or a step along k
@@ -254,10 +270,10 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         const int stage = i % KS;
         if (!barrier_wait(&k_full[stage], (i / KS) & 1, status)) return false;
         tc_fence_after_sync();
-        const uint64_t k_stage = k_desc + static_cast<uint64_t>(stage) * (Config::kTileBytes >> 4);
+        const uint64_t k_stage = k_desc + static_cast<uint64_t>(stage) * (Config::kKeyBytes >> 4);
         const uint32_t tmem_s = tmem_base + (i & 1) * Config::kScoreColumns;
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
+        for (int kk = 0; kk < HDK / 16; ++kk) {
           const uint64_t offset = ((kk / 4) * kFaHalfBytes + (kk % 4) * 32) >> 4;
           tc_mma(tmem_s, q_desc + offset, k_stage + offset, idesc_s, kk > 0 ? 1u : 0u);
         }
@@ -272,14 +288,17 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         // it before it arrived for P of tile i - 1, let alone of tile i.
         if (!barrier_wait(&p_full[buffer], (i >> 1) & 1, status)) return false;
         tc_fence_after_sync();
-        const uint64_t v_stage = v_desc + static_cast<uint64_t>(stage) * (Config::kTileBytes >> 4);
+        const uint64_t v_stage = v_desc + static_cast<uint64_t>(stage) * (Config::kValueBytes >> 4);
         const uint32_t tmem_p = tmem_base + buffer * Config::kScoreColumns;
-        const uint32_t tmem_o = tmem_base + Config::kOutputBase + buffer * HD;
+        const uint32_t tmem_o = tmem_base + Config::kOutputBase + buffer * HDV;
 #pragma unroll
         for (int kk = 0; kk < kFaKeys / 16; ++kk) {  // 16 keys per instruction: two 8-row groups of V, 8 columns of P
           // P of the keys' quarter q lies over the first half of that quarter's score columns.
           tc_mma_ts(tmem_o, tmem_p + (kk / 2) * (kFaKeys / kFaParts) + (kk % 2) * 8, v_stage + kk * (2048 >> 4),
                     idesc_o, kk > 0 ? 1u : 0u);
+          if constexpr (Config::kSplitWeights)   // what the rounding of P left lies over the quarter's second half
+            tc_mma_ts(tmem_o, tmem_p + (kk / 2) * (kFaKeys / kFaParts) + kFaKeys / kFaParts / 2 + (kk % 2) * 8,
+                      v_stage + kk * (2048 >> 4), idesc_o, 1u);
         }
         tc_commit(&v_empty[stage]);
         tc_commit(&o_full[buffer]);
@@ -295,8 +314,8 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
   } else {
     // ---- softmax and accumulation: four threads per query row. Warps w,
     // w + 4, w + 8 and w + 12 reach the same 32 lanes of tensor memory; each
-    // takes 32 keys of a tile and HD / 4 values of the output.
-    constexpr int PART_KEYS = kFaKeys / kFaParts, PART_HD = HD / kFaParts;
+    // takes 32 keys of a tile and a quarter of the block's values of the output.
+    constexpr int PART_KEYS = kFaKeys / kFaParts, PART_HD = HDV / kFaParts;
     static_assert(PART_KEYS == 32 && (PART_HD == 16 || PART_HD == 32), "the tensor-memory loads below take 16 or 32 columns");
     const int lane_base = (warp & 3) * 32;
     const int part = (warp - 2) >> 2;
@@ -321,7 +340,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       if (!barrier_wait(&o_full[buffer], (i >> 1) & 1, status)) return false;
       tc_fence_after_sync();
       uint32_t o[PART_HD];
-      tc_load(tmem_lane + Config::kOutputBase + buffer * HD + part * PART_HD, o);
+      tc_load(tmem_lane + Config::kOutputBase + buffer * HDV + part * PART_HD, o);
       tc_fence_before_sync();   // the MMA thread reuses the buffer only behind this thread's next arrival for P
 #pragma unroll
       for (int j = 0; j < PART_HD; ++j) acc[j] = fmaf(acc[j], alpha, __uint_as_float(o[j]));
@@ -378,7 +397,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       const float ref = m_new == -INFINITY ? 0.0f : m_new;
       const float alpha = fa_exp2(m - ref);
       float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      uint32_t packed[PART_KEYS / 2];
+      uint32_t packed[PART_KEYS / 2], left[Config::kSplitWeights ? PART_KEYS / 2 : 1];
 #pragma unroll
       for (int j = 0; j < PART_KEYS; j += 2) {
         // A masked score is -inf here and gives exactly 0.
@@ -386,9 +405,12 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         const float p1 = fa_exp2(fmaf(s[j + 1], scale_log2, -ref));
         sum4[(j >> 1) & 3] += p0 + p1;
         packed[j >> 1] = fa_pack(p0, p1);
+        if constexpr (Config::kSplitWeights)
+          left[j >> 1] = fa_pack(p0 - __uint_as_float(packed[j >> 1] << 16), p1 - __uint_as_float(packed[j >> 1] & 0xffff0000u));
       }
       // P lies over the scores it came from: columns only this thread reads.
       tc_store_16(tmem_s, packed);
+      if constexpr (Config::kSplitWeights) tc_store_16(tmem_s + PART_KEYS / 2, left);
       tc_store_wait();
       tc_fence_before_sync();
       barrier_arrive(&p_full[buffer]);
@@ -409,20 +431,20 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         (row_max[key_tiles & 1][2][row] + row_max[key_tiles & 1][3][row]);
     if (!ok) failed = 1;
     if (ok && valid && partial != nullptr) {
-      // [token][head][share][HD values, maximum (in units of log 2), sum]
-      float* dst = partial + ((static_cast<size_t>(t0 + row) * heads + head) * shares + share) * (HD + 2);
+      // [token][head][group of values][share][HDV values, maximum (in units of log 2), sum]
+      float* dst = partial + (((static_cast<size_t>(t0 + row) * heads + head) * value_groups + group) * shares + share) * (HDV + 2);
 #pragma unroll
       for (int c = 0; c < PART_HD; c += 4)
         *reinterpret_cast<float2*>(dst + part * PART_HD + c) = make_float2(acc[c], acc[c + 1]),
         *reinterpret_cast<float2*>(dst + part * PART_HD + c + 2) = make_float2(acc[c + 2], acc[c + 3]);
-      if (part == 0) { dst[HD] = m; dst[HD + 1] = l; }
+      if (part == 0) { dst[HDV] = m; dst[HDV + 1] = l; }
     } else if (ok && valid) {
       // one more key, without a value, in the denominator: one score for all heads, or one per head
       if (has_sink) l += fa_exp2((sink_heads != nullptr ? sink_heads[head] * 1.4426950408889634f : sink_log2) - m);
       const float inv = 1.0f / l;
-      __nv_bfloat16* dst = out + (static_cast<size_t>(t0 + row) * heads + head) * HD + part * PART_HD;
+      __nv_bfloat16* dst = out + (static_cast<size_t>(t0 + row) * heads + head) * head_dim + group * HDV + part * PART_HD;
       if (gate != nullptr) {   // an output gate over the concatenated heads: acc * sigmoid(gate) / l
-        const __nv_bfloat16* g = gate + (t0 + row) * gate_stride + head * HD + part * PART_HD;
+        const __nv_bfloat16* g = gate + (t0 + row) * gate_stride + head * head_dim + group * HDV + part * PART_HD;
 #pragma unroll
         for (int c = 0; c < PART_HD; c += 8) {
           const uint4 raw = *reinterpret_cast<const uint4*>(g + c);
@@ -439,6 +461,12 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         *reinterpret_cast<uint4*>(dst + c) =
             make_uint4(fa_pack(acc[c] * inv, acc[c + 1] * inv), fa_pack(acc[c + 2] * inv, acc[c + 3] * inv),
                        fa_pack(acc[c + 4] * inv, acc[c + 5] * inv), fa_pack(acc[c + 6] * inv, acc[c + 7] * inv));
+      }
+      if constexpr (HDK > 128) {   // values that no block makes are zeros
+        const int made = value_groups * HDV;
+        if (group == 0)
+          for (int c = made + part * 8; c < head_dim; c += kFaParts * 8)
+            *reinterpret_cast<uint4*>(out + (static_cast<size_t>(t0 + row) * heads + head) * head_dim + c) = make_uint4(0u, 0u, 0u, 0u);
       }
     }
   }
@@ -463,23 +491,24 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
 constexpr int kMergeGroups = 32;
 constexpr int kMergeShares = 8;   // at most
 
-template <int HD>
-__global__ void __launch_bounds__(HD)
+template <int HDV>
+__global__ void __launch_bounds__(HDV)
 flash_prefill_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                            const int* __restrict__ tile_start, const int* __restrict__ tile_length, int heads,
-                           int shares, const __nv_bfloat16* __restrict__ gate, long long gate_stride, int has_sink,
+                           int head_dim, int value_groups, int shares, const __nv_bfloat16* __restrict__ gate, long long gate_stride, int has_sink,
                            float sink_log2, const float* __restrict__ sink_heads) {
-  const int head = blockIdx.x, tile = blockIdx.y, d = threadIdx.x;
+  const int head = blockIdx.x / value_groups, group = blockIdx.x % value_groups, tile = blockIdx.y;
+  const int d = group * HDV + threadIdx.x;   // of the head
   const int t0 = tile_start[tile], n = tile_length[tile];
   for (int row = blockIdx.z; row < n; row += kMergeGroups) {
-    const float* base = partial + (static_cast<size_t>(t0 + row) * heads + head) * shares * (HD + 2);
+    const float* base = partial + ((static_cast<size_t>(t0 + row) * heads + head) * value_groups + group) * shares * (HDV + 2);
     float maxima[kMergeShares], sums[kMergeShares], values[kMergeShares];
 #pragma unroll
     for (int s = 0; s < kMergeShares; ++s) {   // every load first, then the arithmetic
       const bool live = s < shares;
-      maxima[s] = live ? base[s * (HD + 2) + HD] : -INFINITY;
-      sums[s] = live ? base[s * (HD + 2) + HD + 1] : 0.0f;
-      values[s] = live ? base[s * (HD + 2) + d] : 0.0f;
+      maxima[s] = live ? base[s * (HDV + 2) + HDV] : -INFINITY;
+      sums[s] = live ? base[s * (HDV + 2) + HDV + 1] : 0.0f;
+      values[s] = live ? base[s * (HDV + 2) + threadIdx.x] : 0.0f;
     }
     float highest = -INFINITY;
 #pragma unroll
@@ -493,28 +522,32 @@ flash_prefill_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __r
     }
     // one more key, without a value, in the denominator: one score for all heads, or one per head
     if (has_sink) sum += fa_exp2((sink_heads != nullptr ? sink_heads[head] * 1.4426950408889634f : sink_log2) - highest);
-    if (gate != nullptr) value *= sigmoid_of(__bfloat162float(gate[(t0 + row) * gate_stride + head * HD + d]));
-    out[(static_cast<size_t>(t0 + row) * heads + head) * HD + d] = __float2bfloat16_rn(value / sum);
+    if (gate != nullptr) value *= sigmoid_of(__bfloat162float(gate[(t0 + row) * gate_stride + head * head_dim + d]));
+    __nv_bfloat16* dst = out + (static_cast<size_t>(t0 + row) * heads + head) * head_dim;
+    dst[d] = __float2bfloat16_rn(value / sum);
+    if (group == 0)   // values that no block makes are zeros
+      for (int c = value_groups * HDV + threadIdx.x; c < head_dim; c += HDV) dst[c] = __float2bfloat16_rn(0.0f);
   }
 }
 
-template <int HD>
+template <int HDK, int HDV>
 static int launch_flash_tc(const void* q, const void* cache, void* out, const int* block_tables, int max_pages,
                            const int* tile_request, const int* tile_start, const int* tile_length,
-                           const int* positions, int tokens, int tiles, int heads, int kv_heads, int page_tokens,
+                           const int* positions, int tokens, int tiles, int heads, int kv_heads, int head_dim,
+                           int value_groups, int page_tokens,
                            int num_pages, int window, int chunk, int keep, float scale, int key_shares, float* partial,
                            const void* gate, long long gate_stride, float softcap, int has_sink, float sink_score, const float* sink_heads,
                            ScoreBias bias, int* status, cudaStream_t stream) {
-  using Config = FaConfig<HD>;
+  using Config = FaConfig<HDK, HDV>;
   const float sink_log2 = sink_score * 1.4426950408889634f;
   CUtensorMap map_q, map_cache;
-  // q as [tokens, heads * HD]; the cache as [pages * 2 * kv_heads * page_tokens, HD].
+  // q as [tokens, heads * head_dim]; the cache as [pages * 2 * kv_heads * page_tokens, head_dim].
   const long long cache_rows = static_cast<long long>(num_pages) * 2 * kv_heads * page_tokens;
   if (cache_rows > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
-  if (!make_map(&map_q, q, tokens, heads * HD, static_cast<long long>(heads) * HD, kFaRows) ||
-      !make_map(&map_cache, cache, static_cast<int>(cache_rows), HD, HD, page_tokens))
+  if (!make_map(&map_q, q, tokens, heads * head_dim, static_cast<long long>(heads) * head_dim, kFaRows) ||
+      !make_map(&map_cache, cache, static_cast<int>(cache_rows), head_dim, head_dim, page_tokens))
     return static_cast<int>(cudaErrorInvalidValue);
-  auto kernel = bias.table != nullptr ? flash_prefill_tcgen05_kernel<HD, true> : flash_prefill_tcgen05_kernel<HD, false>;
+  auto kernel = bias.table != nullptr ? flash_prefill_tcgen05_kernel<HDK, HDV, true> : flash_prefill_tcgen05_kernel<HDK, HDV, false>;
   static int shared_limit = 0;
   if (shared_limit == 0) {
     int device = 0;
@@ -528,16 +561,16 @@ static int launch_flash_tc(const void* q, const void* cache, void* out, const in
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   const bool shared_out = key_shares > 1;
-  dim3 grid(heads, tiles, shared_out ? key_shares : 1);
+  dim3 grid(heads * value_groups, tiles, shared_out ? key_shares : 1);
   kernel<<<grid, kFaThreads, shared_bytes, stream>>>(
       map_q, map_cache, static_cast<__nv_bfloat16*>(out), block_tables, max_pages, tile_request, tile_start,
-      tile_length, positions, heads, kv_heads, page_tokens, num_pages, window, chunk, keep, scale, softcap, shared_bytes,
+      tile_length, positions, heads, kv_heads, value_groups, page_tokens, num_pages, window, chunk, keep, scale, softcap, shared_bytes,
       shared_out ? partial : nullptr, static_cast<const __nv_bfloat16*>(gate), gate_stride, has_sink, sink_log2, sink_heads,
       bias, bias_bytes, status);
   e = cudaGetLastError();
   if (e != cudaSuccess || !shared_out) return static_cast<int>(e);
-  flash_prefill_merge_kernel<HD><<<dim3(heads, tiles, kMergeGroups), HD, 0, stream>>>(
-      partial, static_cast<__nv_bfloat16*>(out), tile_start, tile_length, heads, key_shares,
+  flash_prefill_merge_kernel<HDV><<<dim3(heads * value_groups, tiles, kMergeGroups), HDV, 0, stream>>>(
+      partial, static_cast<__nv_bfloat16*>(out), tile_start, tile_length, heads, head_dim, value_groups, key_shares,
       static_cast<const __nv_bfloat16*>(gate), gate_stride, has_sink, sink_log2, sink_heads);
   return static_cast<int>(cudaGetLastError());
 }
@@ -546,26 +579,31 @@ static int launch_flash_tc(const void* q, const void* cache, void* out, const in
 
 using namespace mxb;
 
-// bfloat16, head_dim 64 or 128, pages of 8, 16, 32, 64 or 128 tokens (a page
-// must fill whole 8-row groups of the swizzled tile and divide a key tile).
+// bfloat16, head_dim 64, 128 or 256, pages of 8, 16, 32, 64 or 128 tokens (a page must fill whole 8-row groups of the
+// swizzled tile and divide a key tile; of 256 values a warp's 32 copies cover pages of 16 tokens and more).
 MXB_API int mxb_flash_prefill_tcgen05_supported(int head_dim, int heads, int kv_heads, int page_tokens, int dtype) {
   if (kv_heads <= 0 || heads % kv_heads != 0 || dtype != kBF16) return 0;
-  if (head_dim != 64 && head_dim != 128) return 0;
-  if (page_tokens < 8 || page_tokens > kFaKeys || kFaKeys % page_tokens != 0) return 0;
+  if (head_dim != 64 && head_dim != 128 && head_dim != 256) return 0;
+  if (page_tokens < (head_dim == 256 ? 16 : 8) || page_tokens > kFaKeys || kFaKeys % page_tokens != 0) return 0;
   return 1;
 }
 
 MXB_API int mxb_flash_prefill_tcgen05_tile() { return kFaRows; }
 
-// Query tiles of up to 128 tokens each; q and out are [tokens, heads, head_dim].
-// key_shares > 1: that many blocks share a query tile's keys; partial is
-// float32 scratch of tokens * heads * key_shares * (head_dim + 2) values.
+// How many values of a row of head_dim the partial results of a share take, with their maxima and sums.
+MXB_API int mxb_flash_prefill_tcgen05_partial(int head_dim) { return head_dim == 256 ? 2 * (128 + 2) : head_dim + 2; }
+
+// Query tiles of up to 128 tokens each; q and out are [tokens, heads, head_dim]. Of heads of 256 values, key_width and
+// value_width say how many are in use, the others being zeros: key_width of queries and keys, value_width of the cached
+// values (what they leave out of `out` is written as zeros).
+// key_shares > 1: that many blocks share a query tile's keys; partial is float32 scratch of tokens * heads * key_shares *
+// mxb_flash_prefill_tcgen05_partial(head_dim) values.
 MXB_API int mxb_flash_prefill_tcgen05(const void* q, const void* cache, void* out, const int* block_tables,
                                       int max_pages, const int* tile_request, const int* tile_start,
                                       const int* tile_length, const int* positions, int tokens, int tiles,
-                                      int heads, int kv_heads, int head_dim, int page_tokens, int num_pages,
-                                      int window, int chunk, int keep, float scale, int dtype, int key_shares, float* partial,
-                                      const void* gate, long long gate_stride, float softcap, int has_sink,
+                                      int heads, int kv_heads, int head_dim, int key_width, int value_width, int page_tokens,
+                                      int num_pages, int window, int chunk, int keep, float scale, int dtype, int key_shares,
+                                      float* partial, const void* gate, long long gate_stride, float softcap, int has_sink,
                                       float sink_score, const float* sink_heads, const float* bias_table, int bias_far,
                                       int* status, cudaStream_t stream) {
   if (tiles <= 0) return 0;
@@ -573,16 +611,18 @@ MXB_API int mxb_flash_prefill_tcgen05(const void* q, const void* cache, void* ou
     return static_cast<int>(cudaErrorInvalidValue);
   if (!mxb_flash_prefill_tcgen05_supported(head_dim, heads, kv_heads, page_tokens, dtype))
     return static_cast<int>(cudaErrorInvalidValue);
+  if (key_width <= 0 || key_width > head_dim || value_width <= 0 || value_width > head_dim)
+    return static_cast<int>(cudaErrorInvalidValue);
   if ((reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(cache) & 15) ||
       (reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(gate) & 15) || ((gate_stride * 2) & 15))
     return static_cast<int>(cudaErrorInvalidValue);
   if (bias_table != nullptr && bias_far < 0) return static_cast<int>(cudaErrorInvalidValue);
   const ScoreBias bias = {bias_table, bias_far};
-  if (head_dim == 64)
-    return launch_flash_tc<64>(q, cache, out, block_tables, max_pages, tile_request, tile_start, tile_length,
-                               positions, tokens, tiles, heads, kv_heads, page_tokens, num_pages, window, chunk, keep, scale,
-                               key_shares, partial, gate, gate_stride, softcap, has_sink, sink_score, sink_heads, bias, status, stream);
-  return launch_flash_tc<128>(q, cache, out, block_tables, max_pages, tile_request, tile_start, tile_length,
-                              positions, tokens, tiles, heads, kv_heads, page_tokens, num_pages, window, chunk, keep, scale,
-                              key_shares, partial, gate, gate_stride, softcap, has_sink, sink_score, sink_heads, bias, status, stream);
+  const auto launch = head_dim == 64    ? launch_flash_tc<64, 64>
+                      : head_dim == 128 ? launch_flash_tc<128, 128>
+                      : key_width <= 192 ? launch_flash_tc<192, 128> : launch_flash_tc<256, 128>;
+  const int value_groups = head_dim == 256 && value_width > 128 ? 2 : 1;
+  return launch(q, cache, out, block_tables, max_pages, tile_request, tile_start, tile_length, positions, tokens, tiles,
+                heads, kv_heads, head_dim, value_groups, page_tokens, num_pages, window, chunk, keep, scale, key_shares,
+                partial, gate, gate_stride, softcap, has_sink, sink_score, sink_heads, bias, status, stream);
 }

@@ -93,7 +93,8 @@ _SIGNATURES = {
                           _P, _P, _I, _P, _P],
     "mxb_flash_prefill_supported": [_I, _I, _I, _I],
     "mxb_flash_prefill_tile": [],
-    "mxb_flash_prefill_tcgen05": [_P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P,
+    "mxb_flash_prefill_tcgen05_partial": [_I],
+    "mxb_flash_prefill_tcgen05": [_P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P,
                                   _P, _L, _F, _I, _F, _P, _P, _I, _P, _P],
     "mxb_flash_prefill_tcgen05_supported": [_I, _I, _I, _I, _I],
     "mxb_flash_prefill_tcgen05_tile": [],
@@ -1475,7 +1476,8 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
                   tile_request: torch.Tensor, tile_start: torch.Tensor, tile_length: torch.Tensor,
                   positions: torch.Tensor, scale: float, window: int = 0, kernel: str = "auto",
                   longest_context: int = 0, chunk: int = 0, gate: Optional[torch.Tensor] = None,
-                  softcap: float = 0.0, sink=None, bias=None, keep: int = 0) -> torch.Tensor:
+                  softcap: float = 0.0, sink=None, bias=None, keep: int = 0, key_width: int = 0,
+                  value_width: int = 0) -> torch.Tensor:
     """Causal attention of prompt portions on the tensor cores (bfloat16,
     float32 softmax and accumulation); tiles hold up to 128 consecutive tokens
     of one request. ``kernel``: "tcgen05" (TMA, tensor memory), "mma" (the
@@ -1486,7 +1488,10 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
     pass c tanh(s / c) ahead of the softmax. ``sink``: the score of one more
     key that has no value and that every query sees. ``bias`` (float32
     ``[heads, far + 1]``): joins the scores by head and distance. ``keep``: the
-    first that many positions are seen beside the window or chunk."""
+    first that many positions are seen beside the window or chunk. ``key_width``
+    and ``value_width``: how many values of each head's keys and values are in
+    use (0: all of them), the others being zeros, which a head of 256 need not
+    be asked for."""
     _need(softcap >= 0.0, "the cap on the scores cannot be negative")
     _check(q, "q", (torch.bfloat16,), 3)
     _check(out, "out", (torch.bfloat16,), 3)
@@ -1513,15 +1518,18 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
         tcgen05 = False   # its epilogue reads the gate 16 bytes at a time
     _need(tcgen05 or kernel != "tcgen05",
           f"the tcgen05 prompt kernel does not take head_dim {head_dim} with pages of {page_tokens} tokens")
-    if tcgen05 and kernel != "mma":
+    if tcgen05 and (kernel != "mma" or head_dim == 256):
         _need(q.is_contiguous() and cache.is_contiguous(), "q and cache must be contiguous")
-        shares = flash_key_shares(tiles * heads, int(longest_context), int(window or 0), int(chunk or 0))
+        key_width, value_width = int(key_width) or head_dim, int(value_width) or head_dim
+        blocks = tiles * heads * (2 if head_dim == 256 and value_width > 128 else 1)
+        shares = flash_key_shares(blocks, int(longest_context), int(window or 0), int(chunk or 0))
         partial = None
         if shares > 1:
-            partial = torch.empty(tokens * heads * shares * (head_dim + 2), dtype=torch.float32, device=q.device)
+            partial = torch.empty(tokens * heads * shares * _fn("mxb_flash_prefill_tcgen05_partial")(head_dim),
+                                  dtype=torch.float32, device=q.device)
         _call("mxb_flash_prefill_tcgen05", q.data_ptr(), cache.data_ptr(), out.data_ptr(),
               block_tables.data_ptr(), block_tables.shape[1], tile_request.data_ptr(), tile_start.data_ptr(),
-              tile_length.data_ptr(), positions.data_ptr(), tokens, tiles, heads, kv_heads, head_dim,
+              tile_length.data_ptr(), positions.data_ptr(), tokens, tiles, heads, kv_heads, head_dim, key_width, value_width,
               page_tokens, num_pages, int(window or 0), int(chunk or 0), _kept(keep), float(scale), _CODES[q.dtype], shares, _ptr(partial),
               _ptr(gate), gate_stride, float(softcap), *_sink(sink, heads), *_score_bias(bias, heads),
               status_word(q.device).data_ptr(), _stream())

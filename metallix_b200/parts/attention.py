@@ -179,7 +179,7 @@ def tiles_of(ctx: StepContext) -> Dict[str, object]:
 def attend_cached(q_heads: torch.Tensor, cache: CacheView, ctx: StepContext, *, scale: float, window: int = 0,
                   chunk: int = 0, softcap: float = 0.0, gate: Optional[torch.Tensor] = None, gate_per_head: bool = False,
                   split_decode: bool = False, flash: bool = False, project=None, sink: Optional[float] = None,
-                  bias: Optional[torch.Tensor] = None, keep: int = 0):
+                  bias: Optional[torch.Tensor] = None, keep: int = 0, key_width: int = 0, value_width: int = 0):
     """Attention of a step's queries ``[tokens, heads, head_dim]`` over what the
     cache entry holds (this step's rows included), each kind of request on the
     kernel made for it: single tokens split along the keys, portions of prompts
@@ -188,8 +188,12 @@ def attend_cached(q_heads: torch.Tensor, cache: CacheView, ctx: StepContext, *, 
     kernel. Returns (``[tokens, heads, head_dim]``, False); with ``project`` (the
     output projection, a ``Linear``) a step of few single tokens may come back
     as (float32 ``[heads, tokens, hidden]`` summands, True), merged and
-    projected by one kernel."""
+    projected by one kernel. ``key_width`` / ``value_width``: how many values of
+    a head's keys and values are in use (0: all), the others being zeros."""
     tokens, heads, head_dim = q_heads.shape
+    # Heads of 256 values have a prompt kernel for some page sizes only, and it reads a gate 16 bytes at a time.
+    if head_dim == 256 and split_decode and not gate_per_head and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0)):
+        flash = ops.flash_prefill_tcgen05_supported(head_dim, heads, cache.pool.shape[2], cache.pool.shape[3], q_heads.dtype)
     tiles = tiles_of(ctx)
     multi_tiles = tiles["multi_tiles"]
     split = tiles["decode_rows"] and split_decode
@@ -215,7 +219,7 @@ def attend_cached(q_heads: torch.Tensor, cache: CacheView, ctx: StepContext, *, 
             ops.flash_prefill(q_heads, cache.pool, out, cache.block_tables, tiles["wide_request"],
                               tiles["wide_start"], tiles["wide_length"], ctx.positions, scale, window,
                               longest_context=tiles["longest_keys"], chunk=chunk, gate=gate, softcap=softcap,
-                              sink=sink, bias=bias, keep=keep)
+                              sink=sink, bias=bias, keep=keep, key_width=key_width, value_width=value_width)
         rest = None if split else slice(multi_tiles, None)   # single tokens not yet served
     else:
         rest = slice(0, multi_tiles) if split else slice(0, None)

@@ -200,7 +200,8 @@ class LatentAttention:
         ops.latent_heads(q, widened, rows, r, q_heads, cache.pool if write else None, cache.slots if write else None,
                          ctx.positions, cos, sin, paired, D, R, V)
         out, _ = attend_cached(q_heads, cache, ctx, scale=self.scale, window=self.window, split_decode=self.split_decode,
-                               flash=self.flash, sink=self.sink, gate=proj[:, :self.gate_rows] if self.gate_rows else None)
+                               flash=self.flash, sink=self.sink, gate=proj[:, :self.gate_rows] if self.gate_rows else None,
+                               key_width=D + R, value_width=V)
         return self.o.forward(out.view(tokens, H * hd))
 
     def weight_bytes(self) -> int:

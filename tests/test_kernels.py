@@ -459,7 +459,7 @@ def test_attention_does_not_depend_on_the_cut(ops):
 
 
 def run_flash(ops, q, k, v, lengths, page_tokens, scale, window=0, seed=0, kernel="mma", tile=128, chunk=0,
-              gate=None):
+              gate=None, widths={}):
     """A tensor-core prompt kernel ("mma": warp-level, "tcgen05": TMA and
     tensor memory) on requests whose last ``queries`` positions are the
     queries (bfloat16), cut into tiles of up to ``tile`` tokens."""
@@ -489,7 +489,7 @@ def run_flash(ops, q, k, v, lengths, page_tokens, scale, window=0, seed=0, kerne
     ops.flash_prefill(q_all, dev(host_cache, dtype), out, dev(tables, torch.int32),
                       dev([t[0] for t in tiles], torch.int32), dev([t[1] for t in tiles], torch.int32),
                       dev([t[2] for t in tiles], torch.int32), dev(positions, torch.int32), scale, window,
-                      kernel=kernel, chunk=chunk, gate=gate)
+                      kernel=kernel, chunk=chunk, gate=gate, **widths)
     ops.check_status("cuda")
     return out.cpu().double().numpy()
 
@@ -523,6 +523,34 @@ def test_flash_prefill(ops, heads, kv_heads, head_dim, page_tokens, kernel):
             cursor += queries
     assert not ops.flash_prefill_supported(head_dim, heads, kv_heads, torch.float32)
     assert not ops.flash_prefill_supported(48, 3, 1, dtype)
+
+
+@pytest.mark.parametrize("heads, kv_heads, page_tokens, key_width, value_width, shares",
+                         [(2, 1, 16, 0, 0, None), (4, 2, 32, 192, 128, None), (3, 3, 64, 130, 200, 3), (1, 1, 128, 256, 128, 2)])
+def test_flash_prefill_with_heads_of_256(ops, heads, kv_heads, page_tokens, key_width, value_width, shares):
+    """Weights meet the values as two bfloat16 parts (2^-17 of a weight is lost at most), so what an output of at most 4
+    is off is its own rounding, 2^-9 of it, and little else; a width leaves out zeros only."""
+    rng = np.random.default_rng(heads + page_tokens)
+    dtype = torch.bfloat16
+    lengths = [(200, 200), (130, 2), (65, 65), (500, 129), (3, 3), (700, 300)]
+    cut = lambda x, width: x * (np.arange(256) < (width or 256))
+    q = [rounded(cut(rng.normal(size=(n, heads, 256)), key_width), dtype) for n, _ in lengths]
+    k = [rounded(cut(rng.normal(size=(n, kv_heads, 256)), key_width), dtype) for n, _ in lengths]
+    v = [rounded(cut(np.clip(rng.normal(size=(n, kv_heads, 256)), -4.0, 4.0), value_width), dtype) for n, _ in lengths]
+    assert ops.flash_prefill_tcgen05_supported(256, heads, kv_heads, page_tokens, dtype)
+    assert not ops.flash_prefill_tcgen05_supported(256, heads, kv_heads, 8, dtype)
+    ops.KEY_SHARES = shares
+    try:
+        for window in (0, 50, 200):
+            out = run_flash(ops, q, k, v, lengths, page_tokens, 1.0 / 16, window=window, kernel="tcgen05",
+                            widths=dict(key_width=key_width, value_width=value_width))
+            cursor = 0
+            for r, (total, queries) in enumerate(lengths):
+                ref = plain.causal_gqa_attention(q[r], k[r], v[r], 1.0 / 16, window=window or None)[total - queries:]
+                assert np.abs(out[cursor:cursor + queries] - ref).max() < 4 * 2.0 ** -9 + 2e-4, (window, r)
+                cursor += queries
+    finally:
+        ops.KEY_SHARES = None
 
 
 @pytest.mark.parametrize("kernel", FLASH_KERNELS)
