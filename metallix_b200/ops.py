@@ -1500,7 +1500,8 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
     tokens, heads, head_dim = q.shape
     num_pages, two, kv_heads, page_tokens, cache_dim = cache.shape
     _need(two == 2 and cache_dim == head_dim, "cache must be [pages, 2, kv_heads, page_tokens, head_dim]")
-    _need(flash_prefill_supported(head_dim, heads, kv_heads, q.dtype),
+    tcgen05 = flash_prefill_tcgen05_supported(head_dim, heads, kv_heads, page_tokens, q.dtype)
+    _need(flash_prefill_supported(head_dim, heads, kv_heads, q.dtype) or (head_dim == 256 and tcgen05 and kernel != "mma"),
           f"the tensor-core prompt kernel does not take head_dim {head_dim} with {heads}/{kv_heads} heads")
     _check(block_tables, "block_tables", (torch.int32,), 2)
     for name, tensor in (("tile_request", tile_request), ("tile_start", tile_start),
@@ -1510,15 +1511,14 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
     _need(tile_start.numel() == tiles and tile_length.numel() == tiles, "tile lists differ in length")
     _need(positions.numel() == tokens, "one position per token")
     if kernel == "auto":
-        kernel = PROMPT_KERNEL
+        kernel = PROMPT_KERNEL if head_dim != 256 else "tcgen05"   # the only one that takes such heads
     _need(kernel in ("auto", "tcgen05", "mma"), f"unknown prompt-attention kernel {kernel!r}")
     gate_stride = _gate_stride(gate, q)
-    tcgen05 = flash_prefill_tcgen05_supported(head_dim, heads, kv_heads, page_tokens, q.dtype)
     if gate is not None and (gate.data_ptr() % 16 or (gate_stride * 2) % 16):
         tcgen05 = False   # its epilogue reads the gate 16 bytes at a time
     _need(tcgen05 or kernel != "tcgen05",
           f"the tcgen05 prompt kernel does not take head_dim {head_dim} with pages of {page_tokens} tokens")
-    if tcgen05 and (kernel != "mma" or head_dim == 256):
+    if tcgen05 and kernel != "mma":
         _need(q.is_contiguous() and cache.is_contiguous(), "q and cache must be contiguous")
         key_width, value_width = int(key_width) or head_dim, int(value_width) or head_dim
         blocks = tiles * heads * (2 if head_dim == 256 and value_width > 128 else 1)
