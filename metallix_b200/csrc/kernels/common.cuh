@@ -59,7 +59,7 @@ __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 33 floa
   return scratch[32];
 }
 
-inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+__host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Asks for the cache line of `p` without waiting for it: for what a kernel
 // will read behind its wait for the kernel ahead but that this kernel does not write.
