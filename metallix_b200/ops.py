@@ -70,6 +70,9 @@ _SIGNATURES = {
     "mxb_stream_mix": [_P, _P, _P, _L, _L, _F, _F, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P],
     "mxb_weighted_sum": [_P, _P, _P, _L, _L, _F, _F, _I, _I, _I, _P],
     "mxb_mlstm_state_values": [_I, _I, _I],
+    "mxb_mlstm_chunks_scratch": [_L, _I, _I, _I, _I, _I],
+    "mxb_mlstm_chunks": [_P, _L, _I, _I, _I, _I, _I, _P, _P, _F, _F, _P, _L, _I, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I,
+                         _P, _P, _P],
     "mxb_mlstm_scan": [_P, _L, _I, _I, _I, _I, _I, _P, _P, _F, _F, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I,
                        _I, _P, _P],
     "mxb_head_norm_gate": [_P, _P, _P, _L, _I, _P, _I, _I, _I, _I, _I, _F, _P],
@@ -902,9 +905,10 @@ def mlstm_scan(proj: torch.Tensor, offsets, i_bias: torch.Tensor, f_bias: torch.
     (float32 ``[slots, mlstm_state_values]``, advanced in place). Returns
     float32 ``[tokens, heads * vdim]``: each head's C^T q over its bounded
     normaliser, before the head norm. ``longest`` (the most tokens any row
-    brings, as the host knows it) chooses the form: from 8 tokens on the
-    rows are worked on in chunks of 16 tokens side by side, below that token
-    by token; the two agree to rounding."""
+    brings, as the host knows it) chooses the form: steps of some hundred
+    tokens take all chunks of 64 tokens at once, from 8 tokens on a row's
+    chunks of 16 tokens follow one another, below that its tokens; the forms
+    agree to rounding."""
     _need(proj.is_cuda and proj.dtype in _CODES and proj.dim() == 2 and proj.stride(1) == 1,
           "proj must be a CUDA [tokens, columns] tensor with unit column stride")
     _check(state, "state", (torch.float32,), 2)
@@ -922,6 +926,14 @@ def mlstm_scan(proj: torch.Tensor, offsets, i_bias: torch.Tensor, f_bias: torch.
     _need(cap > 0.0, "the cap on the gates must be positive")
     tokens = proj.shape[0]
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=proj.device)
+    scratch_kib = _fn("mxb_mlstm_chunks_scratch")(tokens, rows, int(longest), heads, dim, vdim)
+    if scratch_kib:
+        scratch = torch.empty(scratch_kib << 10, dtype=torch.uint8, device=proj.device)
+        _call("mxb_mlstm_chunks", proj.data_ptr(), proj.stride(0), q_off, k_off, v_off, i_off, f_off, i_bias.data_ptr(),
+              f_bias.data_ptr(), float(cap), float(dim) ** -0.5, state.data_ptr(), state.stride(0), state.shape[0],
+              row_start.data_ptr(), row_length.data_ptr(), request_slots.data_ptr(), out.data_ptr(), tokens, rows, heads,
+              dim, vdim, _CODES[proj.dtype], int(longest), scratch.data_ptr(), status_word(proj.device).data_ptr(), _stream())
+        return out
     _call("mxb_mlstm_scan", proj.data_ptr(), proj.stride(0), q_off, k_off, v_off, i_off, f_off, i_bias.data_ptr(),
           f_bias.data_ptr(), float(cap), float(dim) ** -0.5, state.data_ptr(), state.stride(0), state.shape[0],
           row_start.data_ptr(), row_length.data_ptr(), request_slots.data_ptr(), out.data_ptr(), rows, heads, dim,

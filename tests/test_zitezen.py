@@ -432,6 +432,60 @@ def test_matrix_memory_kernel(heads, dim, vdim, dtype, form):
 
 @gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, dim, vdim, lengths", [(2, 64, 128, [64, 1, 0, 65, 200]), (3, 20, 36, [63, 193]),
+                                                       (1, 256, 130, [1, 192, 129]), (2, 5, 3, [64, 63, 128, 127, 130]),
+                                                       (33, 256, 512, [1090])])
+def test_matrix_memory_over_all_chunks_at_once(dtype, heads, dim, vdim, lengths):
+    """Against the recurrence in 64 bits (some heads of it) and against the form that walks chunks of 16; the second
+    launch starts from the first one's state. The last shape needs more than one window of scratch."""
+    from metallix_b200 import ops
+    rng = np.random.default_rng(heads * dim + vdim)
+    cap, k_size, v_size = 7.0, heads * dim, heads * vdim
+    at = {"q": 3, "k": 3 + k_size, "v": 3 + 2 * k_size, "i": 3 + 2 * k_size + v_size}
+    at["f"] = at["i"] + heads
+    total = 2 * sum(lengths)
+    proj = rng.normal(size=(total, at["f"] + heads))
+    proj[:, at["i"]:] *= 6.0
+    proj = rounded(proj, dtype)
+    i_bias, f_bias = rng.normal(size=heads), rng.normal(size=heads) + 2.0
+    slots = list(range(len(lengths), 0, -1))
+    device_proj, outs, states = dev(proj, dtype), {}, {}
+    assert ops._fn("mxb_mlstm_chunks_scratch")(total, len(lengths), max(lengths), heads, dim, vdim)
+    for longest in (max(lengths), 8):
+        state = torch.zeros((len(lengths) + 2, ops.mlstm_state_values(heads, dim, vdim)), device="cuda")
+        state[0] = 3.0
+        cursor, parts = 0, []
+        for half in range(2):
+            starts = [cursor + sum(lengths[:row]) for row in range(len(lengths))]
+            cursor += sum(lengths)
+            got = ops.mlstm_scan(device_proj, (at["q"], at["k"], at["v"], at["i"], at["f"]), dev(i_bias), dev(f_bias), cap,
+                                 state, dev(starts, torch.int32), dev(lengths, torch.int32), dev(slots, torch.int32),
+                                 heads, dim, vdim, longest=longest)
+            parts.append(got[starts[0]:cursor])
+        ops.check_status("cuda")
+        outs[longest], states[longest] = torch.cat(parts).double().cpu().numpy(), state
+    (many, walked), (ahead, behind) = outs.values(), states.values()
+    assert np.abs(many - walked).max() < 2e-4 * max(1.0, np.abs(walked).max())
+    assert float((ahead - behind).abs().max()) < 2e-4 * max(1.0, float(behind.abs().max()))
+    assert float(ahead[0].min()) == 3.0
+    f32 = lambda a: dev(a).double().cpu().numpy()
+    for row, length in enumerate(lengths):
+        if not length:
+            continue
+        begin = sum(lengths[:row])
+        rows = np.concatenate([np.arange(s, s + length) for s in (begin, sum(lengths) + begin)])
+        x = proj[rows]
+        for h in range(min(heads, 2)):
+            log_i, log_f = plain.capped_gates(x[:, at["i"] + h] + f32(i_bias)[h], x[:, at["f"] + h] + f32(f_bias)[h], cap)
+            want, _ = plain.matrix_memory(x[:, at["q"] + h * dim:at["q"] + (h + 1) * dim] * dim ** -0.5,
+                                          x[:, at["k"] + h * dim:at["k"] + (h + 1) * dim],
+                                          x[:, at["v"] + h * vdim:at["v"] + (h + 1) * vdim], log_i, log_f)
+            error = np.abs(many[rows, h * vdim:(h + 1) * vdim] - want).max()
+            assert error < 2e-4 * max(1.0, np.abs(want).max()), (row, h)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rank, rot, heads, dim", [(20, 6, 4, 12), (48, 16, 2, 32), (12, 4, 3, 8), (96, 2, 1, 5)])
 def test_latent_rows_into_the_cache_and_rotated_query_parts(dtype, rank, rot, heads, dim):
     from metallix_b200 import ops
