@@ -60,6 +60,9 @@ _SIGNATURES = {
     "mxb_delta_rule_max_dim": [],
     "mxb_delta_rule": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I,
                        _I, _I, _P, _P],
+    "mxb_delta_prompt_scratch": [_L, _I, _I, _I, _I, _I],
+    "mxb_delta_prompt": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _L, _I, _I, _I,
+                         _I, _I, _I, _I, _P, _P, _P],
     "mxb_lightning_chunks_supported": [_P, _L, _I, _I, _I, _I, _I, _I],
     "mxb_lightning_steps_supported": [_P, _L, _I, _I, _P, _L, _I, _I],
     "mxb_lightning_steps": [_P, _L, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
@@ -1126,11 +1129,17 @@ def _matrix_state(mode: int, qkv, offsets, beta, step, step_bias, rate, skip, st
     _need(max(q_off + groups * dim, k_off + groups * dim, v_off + heads * vdim) <= qkv.shape[1],
           "the column offsets reach beyond qkv")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=qkv.device)
-    _call("mxb_delta_rule", qkv.data_ptr(), qkv.stride(0), q_off, k_off, v_off, _ptr(beta),
-          beta.stride(0) if beta is not None else 0, 0, _ptr(step), step.stride(0) if step is not None else 0, _ptr(step_bias),
-          rate.data_ptr(), _ptr(skip), mode, state.data_ptr(), state.stride(0),
-          state.shape[0], row_start.data_ptr(), row_length.data_ptr(), request_slots.data_ptr(), out.data_ptr(), rows,
-          heads, groups, dim, vdim, _CODES[qkv.dtype], int(longest), status_word(qkv.device).data_ptr(), _stream())
+    inputs = (qkv.data_ptr(), qkv.stride(0), q_off, k_off, v_off, _ptr(beta), beta.stride(0) if beta is not None else 0, 0,
+              _ptr(step), step.stride(0) if step is not None else 0, _ptr(step_bias), rate.data_ptr(), _ptr(skip), mode,
+              state.data_ptr(), state.stride(0), state.shape[0], row_start.data_ptr(), row_length.data_ptr(),
+              request_slots.data_ptr(), out.data_ptr())
+    sizes = (rows, heads, groups, dim, vdim, _CODES[qkv.dtype], int(longest))
+    scratch_kib = _fn("mxb_delta_prompt_scratch")(tokens, rows, int(longest), mode, heads, dim)
+    if scratch_kib:
+        scratch = torch.empty(scratch_kib << 10, dtype=torch.uint8, device=qkv.device)
+        _call("mxb_delta_prompt", *inputs, tokens, *sizes, scratch.data_ptr(), status_word(qkv.device).data_ptr(), _stream())
+        return out
+    _call("mxb_delta_rule", *inputs, *sizes, status_word(qkv.device).data_ptr(), _stream())
     return out
 
 

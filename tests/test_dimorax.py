@@ -469,6 +469,55 @@ def test_delta_rule_kernel(dtype, heads, groups, dim, vdim):
 
 
 @gpu
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, groups, dim, vdim, lengths", [(4, 2, 128, 128, [33, 1, 0, 40]), (2, 1, 64, 36, [32, 7, 8, 9]),
+                                                               (3, 3, 36, 5, [1, 65]), (2, 2, 101, 50, [50]),
+                                                               (512, 1, 40, 4, [31, 300, 270])])
+def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, groups, dim, vdim, lengths):
+    """Against the recurrences in 64 bits, two launches one behind the other; the last shape takes several windows. An
+    eight's sums have up to 128 + 8 terms, so a few times 2^-24 of the result's size is what float32 leaves."""
+    from metallix_b200 import ops
+    rng = np.random.default_rng(heads * dim + vdim + mode)
+    total, per, widths = 2 * sum(lengths), heads // groups, (groups * dim, groups * dim, heads * vdim)
+    qkv = torch.cat([torch.zeros(total, 3), torch.from_numpy(rng.normal(size=(total, sum(widths))))], 1).to("cuda", dtype)
+    beta, step = (torch.from_numpy(rng.normal(size=(total, n))).to("cuda", t)
+                  for n, t in ((heads, dtype), (heads * dim, torch.float32) if mode == 0 else (heads, dtype)))
+    bias, rate, skip = (torch.from_numpy(x).float().cuda() for x in (rng.normal(size=heads * dim if mode == 0 else heads) - 2.0,
+                                                                     rng.uniform(0.5, 4.0, heads), rng.normal(size=heads)))
+    state = torch.zeros((len(lengths) + 1, heads, vdim, dim), device="cuda")
+    state[0] = 3.0
+    slots, outs = list(range(len(lengths), 0, -1)), []
+    assert ops._fn("mxb_delta_prompt_scratch")(total, len(lengths), max(lengths), mode, heads, dim)
+    for half in range(2):
+        starts = [half * sum(lengths) + sum(lengths[:row]) for row in range(len(lengths))]
+        outs.append(ops._matrix_state(mode, qkv, (3, 3 + widths[0], 3 + 2 * widths[0]), None if mode == 2 else beta, step, bias, rate,
+                                      skip if mode == 2 else None, state, dev(starts, torch.int32), dev(lengths, torch.int32),
+                                      dev(slots, torch.int32), heads, groups, dim, vdim, max(lengths)))
+    ops.check_status("cuda")
+    assert float(state[0].min()) == 3.0
+    q, k, v = (x.double() for x in qkv[:, 3:].split(widths, 1))
+    q, k = (x.view(total, groups, dim).repeat_interleave(per, 1) for x in (q, k))
+    v, write = v.reshape(total, heads, vdim), torch.nn.functional.softplus(step.double() + bias.double())
+    decay = torch.exp(-rate.double()[:, None] * write.view(total, heads, -1))
+    if mode < 2:
+        unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+        q, k, write = unit(q) * dim ** -0.5, unit(k), torch.sigmoid(beta.double())
+    for row, length in enumerate(lengths):
+        S, begin = torch.zeros((heads, dim, vdim), dtype=torch.float64, device="cuda"), sum(lengths[:row])
+        want, have = [], torch.cat([outs[half][half * sum(lengths) + begin:][:length] for half in range(2)])
+        for t in [half * sum(lengths) + begin + i for half in range(2) for i in range(length)]:
+            S = S * decay[t][:, :, None]
+            seen = torch.einsum("hdv,hd->hv", S, k[t]) if mode < 2 else 0.0
+            S = S + k[t][:, :, None] * (write[t][:, None] * (v[t] - seen))[:, None, :]
+            want.append(torch.einsum("hdv,hd->hv", S, q[t]) + (skip.double()[:, None] * v[t] if mode == 2 else 0.0))
+        if length:
+            want = torch.stack(want).view(2 * length, -1)
+            assert float((have.double() - want).norm() / want.norm()) < 2e-6, row
+            assert float((state[slots[row]].double().transpose(1, 2) - S).norm() / S.norm()) < 2e-6, row
+
+
+@gpu
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("size", [72, 128, 2056])
 def test_the_sum_of_two_sublayers_and_both_norms(out_dtype, size):
