@@ -269,6 +269,119 @@ qk_norm_rope_cache_warp_kernel(
   reinterpret_cast<Values*>(dst + HALF)[sub] = out_hi;
 }
 
+// The same for rotations over part of a head or of neighbouring values: a lane holds V consecutive values of a head, so a
+// rotation partner is in the same lane (neighbouring values) or half / V lanes away (halves). The first kernel above,
+// which these took before, is a block and two barriers per head: 2,048 tokens of 32 + 16 heads of 128 with 64 rotated 86
+// us, MEASURED here.
+template <typename T, int HD>
+__global__ void __launch_bounds__(256)
+qk_norm_rope_cache_lanes_kernel(
+    const T* __restrict__ q_in, const T* __restrict__ k_in, const T* __restrict__ v_in,
+    long long q_stride, long long k_stride, long long v_stride, T* __restrict__ q_out,
+    T* __restrict__ cache, const int* __restrict__ slots, const int* __restrict__ positions,
+    const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary_dim,
+    int interleaved, int tokens, int heads, int kv_heads, int page_tokens, int num_pages, float eps,
+    const float* __restrict__ q_factors, int factor_positions, int* status) {
+  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  constexpr int LANES = HD / V, HEADS = 32 / LANES;   // lanes of a head, heads of a warp
+  static_assert(LANES >= 1 && LANES <= 32, "a head's lanes must divide a warp");
+  using Values = Pack<T, V>;
+  chain_release();
+  // Up to chain_wait(): only what no kernel of this step writes.
+  const int lane = threadIdx.x & 31, sub = lane % LANES;
+  const unsigned per_token = heads + 2 * kv_heads, total = static_cast<unsigned>(tokens) * per_token;
+  const unsigned item = (blockIdx.x * 8u + (threadIdx.x >> 5)) * HEADS + lane / LANES;
+  bool active = item < total;   // lanes without work stay to the end: the others exchange values with their warp
+  const int t = active ? static_cast<int>(item / per_token) : 0, h = active ? static_cast<int>(item % per_token) : 0;
+  const bool is_q = h < heads, is_k = !is_q && h < heads + kv_heads;
+  const int kv = is_q ? 0 : (is_k ? h - heads : h - heads - kv_heads);
+  const T* src = is_q ? q_in + t * q_stride + static_cast<long long>(h) * HD
+               : is_k ? k_in + t * k_stride + static_cast<long long>(kv) * HD
+                      : v_in + t * v_stride + static_cast<long long>(kv) * HD;
+  T* dst = nullptr;
+  if (is_q) {
+    if (q_out == nullptr) active = false;
+    else dst = q_out + (static_cast<size_t>(t) * heads + h) * HD;
+  } else if (slots == nullptr || cache == nullptr) {
+    active = false;
+  } else if (active) {
+    const int slot = slots[t], page = slot / page_tokens, row = slot - page * page_tokens;
+    if (slot < 0) {
+      active = false;
+    } else if (page >= num_pages) {
+      if (sub == 0) atomicOr(status, kStatusBadSlot);
+      active = false;
+    } else {
+      dst = cache + (((static_cast<size_t>(page) * 2 + (is_k ? 0 : 1)) * kv_heads + kv) * page_tokens + row) * HD;
+    }
+  }
+  const bool worked = is_q || is_k;   // values are stored as projected
+  const float* weight = is_q ? q_weight : k_weight;
+  const int half = rotary_dim >> 1, first = sub * V;   // the lane's first value of the head
+  const bool turns = active && worked && cos_table != nullptr && first < rotary_dim;
+  float gain[V], c[V], sn[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) { gain[j] = 1.0f; c[j] = 1.0f; sn[j] = 0.0f; }
+  if (active && worked && weight != nullptr)
+#pragma unroll
+    for (int j = 0; j < V; ++j) gain[j] = weight[first + j];
+  int pos = 0;
+  if (active && worked && cos_table != nullptr) {
+    pos = positions[t];
+    if (pos < 0 || pos >= table_positions) {
+      if (sub == 0) atomicOr(status, kStatusBadSlot);
+      pos = 0;
+    }
+  }
+  if (turns) {
+    const int from = interleaved ? first >> 1 : (first < half ? first : first - half);
+    const float *cs = cos_table + static_cast<size_t>(pos) * half + from, *ss = sin_table + static_cast<size_t>(pos) * half + from;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      c[j] = cs[interleaved ? j >> 1 : j];
+      sn[j] = ss[interleaved ? j >> 1 : j];
+    }
+  }
+  const float factor = active && is_q ? query_factor(q_factors, factor_positions, positions[t], sub == 0, status) : 1.0f;
+  chain_wait();
+  src = behind_wait(src);   // written by the kernel ahead of this one
+  Values in = {};
+  if (active) in = reinterpret_cast<const Values*>(src)[sub];
+  if (active && !worked) reinterpret_cast<Values*>(dst)[sub] = in;
+  float x[V], sum = 0.0f;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    x[j] = to_float(in.v[j]);
+    sum += x[j] * x[j];
+  }
+  if (q_weight != nullptr || k_weight != nullptr) {   // the same for the whole launch
+#pragma unroll
+    for (int offset = LANES / 2; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+    if (weight != nullptr) {
+      const float scale = rsqrtf(sum / static_cast<float>(HD) + eps);
+#pragma unroll
+      for (int j = 0; j < V; ++j) x[j] = x[j] * scale * gain[j];
+    }
+  }
+  if (cos_table != nullptr) {
+    float partner[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) partner[j] = interleaved ? x[j ^ 1] : __shfl_xor_sync(0xffffffffu, x[j], half / V);
+    if (turns)
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const bool lower = interleaved ? (j & 1) == 0 : first < half;
+        x[j] = lower ? x[j] * c[j] - partner[j] * sn[j] : x[j] * c[j] + partner[j] * sn[j];
+      }
+  }
+  if (!active || !worked) return;
+  Values out;
+#pragma unroll
+  for (int j = 0; j < V; ++j) out.v[j] = from_float<T>(x[j] * factor);
+  reinterpret_cast<Values*>(dst)[sub] = out;
+}
+
 // The norm over a token's whole projection: one RMS over all query heads'
 // values (weights [heads * head_dim]) and one over all key heads', then the
 // rotation head by head, q to q_out, k and v into the cache. One block per
@@ -498,6 +611,29 @@ MXB_API int mxb_qk_norm_rope_cache(
     }
 #undef WARP_LAUNCH
     return static_cast<int>(launch_status);
+  }
+  // Rotations that the kernel above does not take, where a lane's values are all turned or none and their partners lie a
+  // power of two of lanes away (or in the lane).
+  const int vector = 16 / element, half = rotary_dim >> 1;
+  if (vector_ok && cos_table != nullptr && half > 0 && half % vector == 0 && (interleaved || (half / vector & (half / vector - 1)) == 0) &&
+      (head_dim == 64 || head_dim == 128 || (head_dim == 256 && dtype == kBF16)) &&
+      static_cast<long long>(tokens) * (heads + 2 * kv_heads) < 0x7fffffffLL) {
+    const long long items = static_cast<long long>(tokens) * (heads + 2 * kv_heads);
+    const unsigned blocks = static_cast<unsigned>((items + 8 * (32 * vector / head_dim) - 1) / (8 * (32 * vector / head_dim)));
+    auto launch = [&](auto kernel, auto type) {
+      using T = decltype(type);
+      return static_cast<int>(launch_chained(kernel, dim3(blocks), dim3(256), 0, stream,
+          static_cast<const T*>(q_in), static_cast<const T*>(k_in), static_cast<const T*>(v_in), q_stride, k_stride, v_stride,
+          static_cast<T*>(q_out), static_cast<T*>(cache), slots, positions, q_weight, k_weight, cos_table, sin_table,
+          table_positions, rotary_dim, interleaved, tokens, heads, kv_heads, page_tokens, num_pages, eps, q_factors,
+          factor_positions, status));
+    };
+    if (dtype == kF32)
+      return head_dim == 64 ? launch(qk_norm_rope_cache_lanes_kernel<float, 64>, float())
+                            : launch(qk_norm_rope_cache_lanes_kernel<float, 128>, float());
+    return head_dim == 64    ? launch(qk_norm_rope_cache_lanes_kernel<__nv_bfloat16, 64>, __nv_bfloat16())
+           : head_dim == 128 ? launch(qk_norm_rope_cache_lanes_kernel<__nv_bfloat16, 128>, __nv_bfloat16())
+                             : launch(qk_norm_rope_cache_lanes_kernel<__nv_bfloat16, 256>, __nv_bfloat16());
   }
   int threads = 32;
   while (threads < head_dim && threads < 256) threads <<= 1;

@@ -133,6 +133,38 @@ def test_qk_norm_rope_cache(ops, dtype, heads, kv_heads, head_dim, rotary):
     assert np.array_equal(got[:, 1], expected[:, 1])  # values are stored as projected
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("head_dim, rotary, paired, normed", [(64, 16, False, True), (64, 32, False, False), (128, 64, False, True),
+                                                              (128, 48, True, True), (128, 128, True, False), (256, 128, False, True),
+                                                              (256, 256, True, True), (128, 96, False, True)])
+def test_partly_turned_heads_by_lanes_and_by_blocks(ops, dtype, head_dim, rotary, paired, normed):
+    """Rows on 16 bytes take the kernel of lanes (where the partner of a value lies well), the same rows one value
+    further the one of blocks: the same numbers up to the order of a norm's sum and one rounding of the result."""
+    rng = np.random.default_rng(head_dim + rotary)
+    tokens, heads, kv_heads, page_tokens, pages = 13, 5, 2, 4, 6
+    width, half = (heads + 2 * kv_heads) * head_dim, rotary // 2
+    angle = np.arange(100)[:, None] * 1e4 ** (-2.0 * np.arange(half) / rotary)[None, :]
+    qkv, positions = dev(rng.normal(size=(tokens, width)), dtype), dev(rng.integers(0, 100, size=tokens), torch.int32)
+    slots = dev(np.where(np.arange(tokens) == 3, -1, rng.permutation(pages * page_tokens)[:tokens]), torch.int32)
+    weights = [dev(1 + rng.uniform(-0.1, 0.1, size=head_dim)) if normed else None for _ in range(2)]
+    factors = dev(rng.uniform(0.5, 1.5, size=100))
+    results = []
+    for shift in (0, 1):
+        wide = torch.zeros((tokens, width + 8), dtype=dtype, device="cuda")
+        rows = wide[:, shift:shift + width]
+        rows.copy_(qkv)
+        q_out = torch.zeros(tokens, heads, head_dim, dtype=dtype, device="cuda")
+        cache = torch.zeros(pages, 2, kv_heads, page_tokens, head_dim, dtype=dtype, device="cuda")
+        ops.qk_norm_rope_cache(rows[:, :heads * head_dim], rows[:, heads * head_dim:(heads + kv_heads) * head_dim],
+                               rows[:, (heads + kv_heads) * head_dim:], q_out, cache, slots, positions, *weights,
+                               dev(np.cos(angle)), dev(np.sin(angle)), 1e-5, interleaved=paired, q_factors=factors)
+        ops.check_status("cuda")
+        results.append((q_out.float(), cache.float()))
+    for lanes, blocks in zip(*results):
+        assert float((lanes - blocks).abs().max()) <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * float(blocks.abs().max())
+    assert float(results[0][1].abs().max()) > 0.5
+
+
 def test_rotation_keeps_accuracy_at_far_positions(ops):
     """cos and sin come from a float64 table: at position 4000 a float32
     product of position and frequency would already be off by 1e-4."""
