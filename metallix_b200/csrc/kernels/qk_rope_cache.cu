@@ -271,8 +271,8 @@ qk_norm_rope_cache_warp_kernel(
 
 // The same for rotations over part of a head or of neighbouring values: a lane holds V consecutive values of a head, so a
 // rotation partner is in the same lane (neighbouring values) or half / V lanes away (halves). The first kernel above,
-// which these took before, is a block and two barriers per head: 2,048 tokens of 32 + 16 heads of 128 with 64 rotated 86
-// us, MEASURED here.
+// which these took before, is a block and two barriers per head: 2,048 tokens of 32 + 16 heads of 128 with 64 rotated took
+// 68 us there and 27 here, 2,401 of 16 + 16 with neighbours turned 57 and 23 (cold caches).
 template <typename T, int HD>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_cache_lanes_kernel(

@@ -445,6 +445,35 @@ def test_selective_scan_kernel(dtype, channels, states):
 
 
 @gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("channels, states, lengths", [(100, 16, [192, 1, 0, 65]), (33, 7, [300, 64, 63]), (8, 1, [193, 128])])
+def test_selective_scan_in_chunks(dtype, channels, states, lengths):
+    """Rows in chunks of 64 tokens side by side against one walk per row, two launches one behind the other: float32 to
+    rounding, bfloat16 outputs to one rounding of theirs; slow decays, so that a state ahead of a chunk counts in it."""
+    from metallix_b200 import ops
+    rng = np.random.default_rng(channels + states)
+    total, slots = sum(lengths), list(range(len(lengths), 0, -1))
+    a, bias = dev(-np.exp(rng.normal(size=(channels, states)) * 0.5)), dev(rng.normal(size=channels) * 0.3 - 5.0)
+    skip, starts = dev(rng.normal(size=channels)), [sum(lengths[:row]) for row in range(len(lengths))]
+    inputs = [(dev(rng.normal(size=(total, 2 * channels)), dtype), dev(rng.normal(size=(total, channels))),
+               dev(rng.normal(size=(total, 2 * states)), dtype)) for _ in range(2)]
+    assert ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, max(lengths))
+    results = []
+    for longest in (max(lengths), 0):
+        state = torch.zeros((len(lengths) + 1, channels, states), device="cuda")
+        state[0] = 3.0
+        outs = [ops.selective_scan(both[:, :channels], step, bias, a, picked[:, :states], picked[:, states:], skip,
+                                   both[:, channels:], state, dev(starts, torch.int32), dev(lengths, torch.int32),
+                                   dev(slots, torch.int32), longest=longest) for both, step, picked in inputs]
+        ops.check_status("cuda")
+        results.append((torch.cat(outs).float(), state))
+    (out, state), (walked, behind) = results
+    assert float((state - behind).abs().max()) < 2e-6 * float(behind[1:].abs().max()) and float(state[0].min()) == 3.0
+    limit = 5e-6 if dtype == torch.float32 else 2.0 ** -8
+    assert float(((out - walked).abs() / (walked.abs() + 0.05 * walked.abs().max())).max()) < limit
+
+
+@gpu
 @pytest.mark.parametrize("outputs, real, top", [(6, 5, 2), (5, 3, 3), (7, 7, 1), (2, 2, 2), (4, 1, 2), (40, 33, 6), (300, 290, 8)])
 def test_router_choice_by_corrected_scores_weights_by_scores(outputs, real, top):
     """Softmax over all outputs, identity experts included; the correction
