@@ -459,6 +459,122 @@ walk_kernel(WalkArgs a) {
   __syncthreads();
 }
 
+// A step of single tokens: bound by reading and writing the states. A warp has (LANES = 16) eight columns of a (request,
+// head), four columns and eight channels a thread as above; every load, the state's and the token's, is on its way at
+// once and no thread waits for another warp (delta_rule.cu: a trip to memory for the row's length, one for its slot, one
+// for the state with 32 bytes a thread, two barriers). 16 requests, 32 heads of 128 x 128, a decay per channel: 48 -> 22 us,
+// per head 41 -> 20, the dual with 128 heads of 128 x 64 54 -> 30 (their states' bytes take 10, 10 and 20); 64 requests
+// 137 -> 55; one request 10 either way.
+template <typename T, int LANES, int MODE>
+__global__ void __launch_bounds__(128)
+step_kernel(WalkArgs a) {
+  constexpr bool LOOKS = MODE != kWalkDual;
+  const int row = blockIdx.x, head = blockIdx.y;
+  const int length = a.row_length[row], slot = a.request_slots[row];
+  const long long token = a.row_start[row];
+  if (length <= 0) return;
+  if (slot < 0 || slot >= a.num_slots) {
+    if (threadIdx.x == 0) atomicOr(a.status, kStatusBadSlot);
+    return;
+  }
+  const int part = threadIdx.x % LANES, d0 = part * kWalkPer;
+  const int column = (blockIdx.z * (128 / LANES) + threadIdx.x / LANES) * kWalkCols;
+  const bool has = d0 < a.dim;   // dim is a multiple of eight
+  float* home = a.state + static_cast<long long>(slot) * a.slot_stride + (static_cast<long long>(head) * a.vdim + column) * a.dim + d0;
+  float4 s[kWalkCols][2];
+#pragma unroll
+  for (int c = 0; c < kWalkCols; ++c)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      s[c][i] = has && column + c < a.vdim ? *reinterpret_cast<const float4*>(home + static_cast<long long>(c) * a.dim + 4 * i)
+                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  struct alignas(16) Eight { T v[16 / sizeof(T)]; };
+  constexpr int PIECES = kWalkPer * sizeof(T) / 16, EACH = 16 / sizeof(T);
+  const T* x = static_cast<const T*>(a.qkv) + token * a.ld;
+  const int group = head / (a.heads / a.groups);
+  Eight raw_q[PIECES] = {}, raw_k[PIECES] = {};
+  if (has)
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      raw_q[i] = *reinterpret_cast<const Eight*>(x + a.q_off + group * a.dim + d0 + i * EACH);
+      raw_k[i] = *reinterpret_cast<const Eight*>(x + a.k_off + group * a.dim + d0 + i * EACH);
+    }
+  T raw_v[kWalkCols];
+#pragma unroll
+  for (int c = 0; c < kWalkCols; ++c) raw_v[c] = x[a.v_off + head * a.vdim + min(column + c, a.vdim - 1)];
+  float pre[MODE == kWalkChannel ? kWalkPer : 1], bias[MODE == kWalkChannel ? kWalkPer : 1];
+  if (MODE == kWalkChannel) {
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) {
+      pre[i] = has ? static_cast<const float*>(a.step_pre)[token * a.lds + head * a.dim + d0 + i] : 0.0f;
+      bias[i] = has ? a.step_bias[head * a.dim + d0 + i] : 0.0f;
+    }
+  } else {
+    pre[0] = to_float(static_cast<const T*>(a.step_pre)[token * a.lds + head]);
+    bias[0] = a.step_bias[head];
+  }
+  const float rate = a.rate[head], skip = MODE == kWalkDual ? a.skip[head] : 0.0f;
+  float beta = LOOKS ? sigmoid_of(to_float(static_cast<const T*>(a.beta_pre)[token * a.ldb + a.b_off + head])) : 0.0f;
+
+  float q[kWalkPer], k[kWalkPer], g[kWalkPer], qq = 0.0f, kk = 0.0f, qk = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kWalkPer; ++i) {
+    q[i] = to_float(raw_q[i / EACH].v[i % EACH]);
+    k[i] = to_float(raw_k[i / EACH].v[i % EACH]);
+    qq = fmaf(q[i], q[i], qq);
+    kk = fmaf(k[i], k[i], kk);
+    qk = fmaf(q[i], k[i], qk);
+  }
+  auto over_lanes = [](float v) {
+#pragma unroll
+    for (int offset = 1; offset < LANES; offset <<= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);
+    return v;
+  };
+  qk = over_lanes(qk);
+  if (LOOKS) {
+    const float q_unit = rsqrtf(over_lanes(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(over_lanes(kk) + 1e-6f);
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) {
+      q[i] *= q_unit;
+      k[i] *= k_unit;
+    }
+    qk *= q_unit * k_unit;
+  }
+  if (MODE == kWalkChannel) {
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) g[i] = expf(-rate * walk_softplus(pre[MODE == kWalkChannel ? i : 0] + bias[MODE == kWalkChannel ? i : 0]));
+  } else {
+    const float step = walk_softplus(pre[0] + bias[0]), decay = expf(-rate * step);
+    if (!LOOKS) beta = step;
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) g[i] = decay;
+  }
+#pragma unroll
+  for (int c = 0; c < kWalkCols; ++c) {
+    float r[kWalkPer] = {s[c][0].x, s[c][0].y, s[c][0].z, s[c][0].w, s[c][1].x, s[c][1].y, s[c][1].z, s[c][1].w};
+    float k_dot = 0.0f, q_dot = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) {
+      r[i] *= g[i];
+      k_dot = fmaf(k[i], r[i], k_dot);
+      q_dot = fmaf(q[i], r[i], q_dot);
+    }
+    if (LOOKS) k_dot = over_lanes(k_dot);
+    q_dot = over_lanes(q_dot);
+    const float v = to_float(raw_v[c]), u = beta * (LOOKS ? v - k_dot : v);
+    if (column + c < a.vdim) {
+      if (has) {
+        float4* to = reinterpret_cast<float4*>(home + static_cast<long long>(c) * a.dim);
+        to[0] = make_float4(fmaf(k[0], u, r[0]), fmaf(k[1], u, r[1]), fmaf(k[2], u, r[2]), fmaf(k[3], u, r[3]));
+        to[1] = make_float4(fmaf(k[4], u, r[4]), fmaf(k[5], u, r[5]), fmaf(k[6], u, r[6]), fmaf(k[7], u, r[7]));
+      }
+      if (part == 0)
+        a.out[token * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim + column + c] =
+            fmaf(qk, u, q_dot) + (MODE == kWalkDual ? skip * v : 0.0f);
+    }
+  }
+}
+
 static int walk_lanes(int dim) { return dim <= 64 ? 8 : 16; }
 // Tokens of a window; its rows' eights are at most window / 8 + rows.
 static long long walk_window(long long tokens, int rows, int heads, int dim) {
@@ -525,6 +641,46 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
     if (mode == kWalkChannel) return run(type, lanes_of, std::integral_constant<int, kWalkChannel>());
     if (mode == kWalkHead) return run(type, lanes_of, std::integral_constant<int, kWalkHead>());
     return run(type, lanes_of, std::integral_constant<int, kWalkDual>());
+  };
+  auto by_lanes = [&](auto type) {
+    return lanes == 8 ? by_mode(type, std::integral_constant<int, 8>()) : by_mode(type, std::integral_constant<int, 16>());
+  };
+  return dtype == kF32 ? by_lanes(float()) : by_lanes(__nv_bfloat16());
+}
+
+// Whether mxb_delta_step takes a step: single tokens (longest 1), keys of 40, 48 ... 128 channels whose rows and states
+// start on 16 bytes. Other steps of single tokens stay with mxb_delta_rule.
+MXB_API int mxb_delta_step_supported(const void* qkv, long long ld, int q_off, int k_off, int mode, const float* state,
+                                     long long slot_stride, int heads, int dim, int dtype, int longest) {
+  const int each = dtype == kF32 ? 4 : 8;   // values of 16 bytes
+  return longest == 1 && mode >= kWalkChannel && mode <= kWalkDual && (dtype == kF32 || dtype == kBF16) && heads > 0 &&
+                 heads <= 65535 && dim > 32 && dim <= 128 && dim % kWalkPer == 0 && ld % each == 0 && q_off % each == 0 &&
+                 k_off % each == 0 && slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 &&
+                 (reinterpret_cast<uintptr_t>(state) & 15) == 0
+             ? 1 : 0;
+}
+
+MXB_API int mxb_delta_step(const void* qkv, long long ld, int q_off, int k_off, int v_off, const void* beta_pre,
+                           long long ldb, int b_off, const void* step_pre, long long lds, const float* step_bias,
+                           const float* rate, const float* skip, int mode, float* state, long long slot_stride, int num_slots,
+                           const int* row_start, const int* row_length, const int* request_slots, float* out, int rows,
+                           int heads, int groups, int dim, int vdim, int dtype, int longest, int* status, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (groups <= 0 || heads % groups != 0 || vdim <= 0 || (mode == kWalkDual) != (skip != nullptr) ||
+      !mxb_delta_step_supported(qkv, ld, q_off, k_off, mode, state, slot_stride, heads, dim, dtype, longest))
+    return static_cast<int>(cudaErrorInvalidValue);
+  const WalkArgs a = {qkv, ld, q_off, k_off, v_off, beta_pre, ldb, b_off, step_pre, lds, step_bias, rate, skip, state,
+                      slot_stride, num_slots, row_start, row_length, request_slots, out, rows, heads, groups, dim, vdim, status,
+                      nullptr, 0, 0, 0};
+  const int lanes = walk_lanes(dim);
+  const dim3 grid(rows, heads, ceil_div(vdim, 128 / lanes * kWalkCols));
+  auto by_mode = [&](auto type, auto lanes_of) {
+    using T = decltype(type);
+    constexpr int LANES = decltype(lanes_of)::value;
+    if (mode == kWalkChannel) step_kernel<T, LANES, kWalkChannel><<<grid, 128, 0, stream>>>(a);
+    else if (mode == kWalkHead) step_kernel<T, LANES, kWalkHead><<<grid, 128, 0, stream>>>(a);
+    else step_kernel<T, LANES, kWalkDual><<<grid, 128, 0, stream>>>(a);
+    return static_cast<int>(cudaGetLastError());
   };
   auto by_lanes = [&](auto type) {
     return lanes == 8 ? by_mode(type, std::integral_constant<int, 8>()) : by_mode(type, std::integral_constant<int, 16>());

@@ -23,6 +23,8 @@
 //
 //   S <- g_h S + k v^T;   o = S^T q
 //
+// Rows of 32 tokens and more, and single tokens, mostly take the kernels of delta_prompt.cu instead.
+//
 // Every value column of S goes its own way: column j needs only v_j and what
 // all columns share (qn, kn, g, beta). A block owns some of the columns of
 // one head of one request; 4 to 16 lanes share a column, each with its share

@@ -61,6 +61,9 @@ _SIGNATURES = {
     "mxb_delta_rule_max_dim": [],
     "mxb_delta_rule": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I,
                        _I, _I, _P, _P],
+    "mxb_delta_step_supported": [_P, _L, _I, _I, _I, _P, _L, _I, _I, _I, _I],
+    "mxb_delta_step": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I,
+                       _I, _I, _P, _P],
     "mxb_delta_prompt_scratch": [_L, _I, _I, _I, _I, _I],
     "mxb_delta_prompt": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _L, _I, _I, _I,
                          _I, _I, _I, _I, _P, _P, _P],
@@ -1144,7 +1147,9 @@ def _matrix_state(mode: int, qkv, offsets, beta, step, step_bias, rate, skip, st
         scratch = torch.empty(scratch_kib << 10, dtype=torch.uint8, device=qkv.device)
         _call("mxb_delta_prompt", *inputs, tokens, *sizes, scratch.data_ptr(), status_word(qkv.device).data_ptr(), _stream())
         return out
-    _call("mxb_delta_rule", *inputs, *sizes, status_word(qkv.device).data_ptr(), _stream())
+    single = _fn("mxb_delta_step_supported")(qkv.data_ptr(), qkv.stride(0), q_off, k_off, mode, state.data_ptr(), state.stride(0),
+                                             heads, dim, _CODES[qkv.dtype], int(longest))
+    _call("mxb_delta_step" if single else "mxb_delta_rule", *inputs, *sizes, status_word(qkv.device).data_ptr(), _stream())
     return out
 
 
@@ -1585,7 +1590,8 @@ def decode_split_keys() -> int:
 def set_decode_resident_blocks(blocks: int, many: int = 2048) -> None:
     """How many blocks of the bfloat16 decode attention the GPU holds at once
     (444: three on each of 148 SMs), and into how many blocks a step with more
-    (token, key/value head) pairs than that is cut (2,048). A pair gets that
+    than half as many (token, key/value head) pairs is cut (2,048, two tiles a
+    block at least). A pair gets that
     many blocks divided by the number of pairs, each walking over its 128-key
     tiles; where a block would be left fewer than two tiles, and with
     ``blocks`` 0, every tile has a block of its own. For comparisons and tests."""

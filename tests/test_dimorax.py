@@ -518,6 +518,35 @@ def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, gro
 
 
 @gpu
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (3, 1, 40, 33), (2, 2, 64, 70), (1, 1, 120, 1)])
+def test_matrix_state_recurrences_of_single_tokens(mode, dtype, heads, groups, dim, vdim):
+    """The kernel for steps of single tokens against the general one, a padding row among the rows and states that are not
+    zero: float32 sums of up to 128 terms in another order."""
+    from metallix_b200 import ops
+    rng = np.random.default_rng(heads * dim + vdim + mode)
+    lengths, slots, width = [1, 1, 0, 1], [3, 1, 0, 2], 2 * groups * dim + heads * vdim
+    qkv = torch.from_numpy(rng.normal(size=(3, -(-width // 8) * 8))).to("cuda", dtype)[:, :width]
+    beta, step = (torch.from_numpy(rng.normal(size=(3, n))).to("cuda", t)
+                  for n, t in ((heads, dtype), (heads * dim, torch.float32) if mode == 0 else (heads, dtype)))
+    bias, rate, skip = (torch.from_numpy(x).float().cuda() for x in (rng.normal(size=heads * dim if mode == 0 else heads) - 2.0,
+                                                                     rng.uniform(0.5, 4.0, heads), rng.normal(size=heads)))
+    states = [dev(rng.normal(size=(5, heads, vdim, dim)))]
+    states.append(states[0].clone())
+    assert ops._fn("mxb_delta_step_supported")(qkv.data_ptr(), qkv.stride(0), 0, groups * dim, mode, states[0].data_ptr(),
+                                               states[0].stride(0), heads, dim, ops._CODES[dtype], 1)
+    outs = [ops._matrix_state(mode, qkv, (0, groups * dim, 2 * groups * dim), None if mode == 2 else beta, step, bias, rate,
+                              skip if mode == 2 else None, state, dev([0, 1, 2, 2], torch.int32), dev(lengths, torch.int32),
+                              dev(slots, torch.int32), heads, groups, dim, vdim, longest)
+            for state, longest in zip(states, (1, 2))]
+    ops.check_status("cuda")
+    assert torch.equal(states[0][[0, 4]], states[1][[0, 4]])
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 1e-6
+    assert float((states[0] - states[1]).norm() / states[1].norm()) < 1e-6
+
+
+@gpu
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("size", [72, 128, 2056])
 def test_the_sum_of_two_sublayers_and_both_norms(out_dtype, size):
