@@ -1091,7 +1091,7 @@ static int launch_decode(const void* q, const void* cache, void* out, float* par
 }
 
 static int decode_resident_blocks = 444;   // blocks of the decode attention that fit the GPU at once (3 an SM); 0: always one block per tile
-static int decode_many_blocks = 2048;      // blocks of a step with more (token, key/value head) pairs than that
+static int decode_many_blocks = 2048;      // blocks of a step with more than half as many (token, key/value head) pairs
 
 template <int HD>
 static int launch_decode_mma(const void* q, const void* cache, void* out, float* partial,
@@ -1193,7 +1193,7 @@ MXB_API int mxb_paged_attention_split_keys() { return kSplitKeys; }
 
 // How many blocks of the bfloat16 decode attention the GPU holds at once (3
 // an SM with their 64 KB of keys and values), and how many blocks a step with
-// more (token, key/value head) pairs than that is cut into. 0: one block per
+// more than half as many (token, key/value head) pairs is cut into. 0: one block per
 // tile always.
 MXB_API int mxb_set_decode_resident_blocks(int blocks, int many) {
   if (blocks < 0 || many < blocks) return static_cast<int>(cudaErrorInvalidValue);

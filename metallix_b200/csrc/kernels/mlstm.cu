@@ -229,7 +229,7 @@ mlstm_scan_registers_kernel(const T* __restrict__ proj, long long ld, int q_off,
   if (threadIdx.x == 0) m_state[0] = m;
 }
 
-// Portions of prompts: the same recurrence, a chunk of up to 16 tokens at a time. With the chunk's first
+// Short portions of prompts (mlstm_chunks.cu takes longer ones): the same recurrence, a chunk of up to 16 tokens at a time. With the chunk's first
 // state (C0, n0, m0), F_t the sum of the log forget gates up to token t of the chunk and i_s the log input
 // gates, unrolling the recurrence gives, exactly,
 //   m_t = max(f_t + m_(t-1), i_t)                                     (a scalar walk over the chunk)

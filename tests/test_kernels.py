@@ -899,6 +899,20 @@ def test_gemm_simple_float32_is_true_32_bit(ops, m, n, k):
     assert torch.equal(one_row[0], out[3 if m > 3 else 0])   # a row does not depend on the batch
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1, 4), (8, 77, 1028), (9, 70, 20), (33, 3588, 36), (65, 7041, 52), (200, 4700, 132)])
+def test_float32_products_have_one_order_of_additions(ops, m, n, k):
+    """Every tile size (up to eight rows, 16 x 32, 32 x 64, 64 x 128 with remainders of each) against the same rows where
+    they do not start on 16 bytes, which takes the plain kernel: the same bits, and 64-bit sums to 1e-6."""
+    rng = np.random.default_rng(m + n + k)
+    a, w = dev(rng.normal(size=(m, k))), dev(rng.normal(size=(n, k)))
+    wide = torch.zeros((max(m, n), 2 * k + 3), device="cuda")
+    wide[:m, 1:k + 1], wide[:n, k + 2:2 * k + 2] = a, w
+    out = ops.gemm_simple(a, w)
+    assert torch.equal(out, ops.gemm_simple(wide[:m, 1:k + 1], wide[:n, k + 2:2 * k + 2]))
+    ref = a.double() @ w.double().t()
+    assert float((out - ref).norm() / ref.norm()) < 1e-6
+
+
 @pytest.mark.parametrize("backend", ["simple", "cublas", "auto", "tcgen05"])
 @pytest.mark.parametrize("m, n, k", [(1, 384, 96), (5, 200, 136), (64, 331, 80), (300, 448, 192),
                                      (129, 130, 72), (700, 1030, 520)])
