@@ -365,7 +365,7 @@ walk_kernel(WalkArgs a) {
             for (int e = 0; e < t; ++e) seen = fmaf(line[e], u[e][0], seen);
             rest -= seen;
           }
-          u[t][0] = b[t] * rest;
+          u[t][0] = t < tokens ? b[t] * rest : 0.0f;
         }
       }
       // ---- (q_t G_t) . S, each lane's tokens counted from those whose outputs it writes
@@ -427,7 +427,8 @@ walk_kernel(WalkArgs a) {
         const int mine = t ^ turned;
         float o = qd[t][0];
 #pragma unroll
-        for (int e = 0; e < kEight; ++e) o = fmaf(line[t][e], u[e][0], o);
+        for (int e = 0; e < kEight; ++e)   // chosen, not weighed with 0: a later token's infinity stays out of this one
+          o = e <= mine ? fmaf(line[t][e], u[e][0], o) : o;
         if (MODE == kWalkDual) o = fmaf(head_skip, to_float(value_own[t]), o);
         if (mine < tokens && column + own < a.vdim)
           a.out[(first + r * kEight + mine) * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim +

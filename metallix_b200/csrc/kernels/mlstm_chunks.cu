@@ -410,14 +410,29 @@ mlstm_outputs_kernel(ChunkArgs a, int from) {
     dot = fmaf(decay[t], warp_sum(dot), a.s.sums[in_window * kTokens + t]);
     if (lane == 0) below[t] = fmaxf(fabsf(dot), expf(-a.s.m[at * kTokens + t])) + 1.0e-6f;
   }
+  bool finite = true;
+  auto value = [&](int s, int v) { return v0 + v < vdim ? to_float(x0[s * a.ld + a.v_off + head * vdim + v0 + v]) : 0.0f; };
   float acc[8][8] = {};
+  tile_product<8, false, false>(acc, tiles, len, [&](int s, int t) { return P[s * kTokens + t]; }, [&](int s, int v) {
+    const float f = value(s, v);
+    finite = finite && fabsf(f) < INFINITY;
+    return f;
+  });
+  if (__syncthreads_or(!finite)) {   // 0 times what is not finite is no 0: a token takes only what is not behind it
+#pragma unroll 1
+    for (int s = 0; s < len; ++s)
+#pragma unroll
+      for (int x = 0; x < 8; ++x)
+#pragma unroll
+        for (int y = 0; y < 8; ++y) {
+          if (s == 0) acc[x][y] = 0.0f;
+          if (s <= tile_row(x)) acc[x][y] = fmaf(P[s * kTokens + tile_row(x)], value(s, tile_column(y)), acc[x][y]);
+        }
+  }
   tile_product<8, true, false>(
       acc, tiles, dim,
       [&](int d, int t) { return t < len ? decay[t] * (to_float(x0[t * a.ld + a.q_off + head * dim + d]) * a.q_scale) : 0.0f; },
       [&](int d, int v) { return v0 + v < vdim ? C[static_cast<size_t>(d) * vdim + v0 + v] : 0.0f; });
-  tile_product<8, false, false>(
-      acc, tiles, len, [&](int s, int t) { return P[s * kTokens + t]; },
-      [&](int s, int v) { return v0 + v < vdim ? to_float(x0[s * a.ld + a.v_off + head * vdim + v0 + v]) : 0.0f; });
 #pragma unroll
   for (int x = 0; x < 8; ++x) {
     const int t = tile_row(x);

@@ -518,6 +518,24 @@ def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, gro
 
 
 @gpu
+@pytest.mark.parametrize("mode", [0, 2])
+def test_matrix_state_recurrences_keep_later_values_out_of_earlier_outputs(mode):
+    from metallix_b200 import ops
+    heads, dim, vdim, tokens, late = 2, 64, 32, 40, 20
+    rng = np.random.default_rng(mode)
+    qkv, outs = dev(rng.normal(size=(tokens, heads * (2 * dim + vdim)))), []
+    gates, step = dev(rng.normal(size=(tokens, heads))), dev(rng.normal(size=(tokens, heads * dim if mode == 0 else heads)))
+    ones = torch.ones(heads, device="cuda")
+    for value in (1.0, float("inf")):
+        qkv[late, 2 * heads * dim:] = value
+        state, zero = torch.zeros((1, heads, vdim, dim), device="cuda"), dev([0], torch.int32)
+        outs.append(ops._matrix_state(mode, qkv, (0, heads * dim, 2 * heads * dim), gates if mode == 0 else None, step,
+                                      torch.zeros(step.shape[1], device="cuda"), ones, ones if mode == 2 else None, state, zero,
+                                      dev([tokens], torch.int32), zero, heads, heads, dim, vdim, tokens))
+    assert torch.equal(outs[0][:late], outs[1][:late]) and not bool(outs[1][late:].isfinite().all())
+
+
+@gpu
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (3, 1, 40, 33), (2, 2, 64, 70), (1, 1, 120, 1)])

@@ -485,6 +485,23 @@ def test_matrix_memory_over_all_chunks_at_once(dtype, heads, dim, vdim, lengths)
 
 
 @gpu
+def test_matrix_memory_keeps_later_values_out_of_earlier_outputs():
+    from metallix_b200 import ops
+    heads, dim, vdim, tokens, late = 2, 64, 40, 200, 150
+    proj = dev(np.random.default_rng(0).normal(size=(tokens, heads * (2 * dim + vdim + 2))))
+    width, outs = heads * dim, []
+    for value in (1.0, float("inf")):
+        proj[late, 2 * width:2 * width + heads * vdim] = value
+        state = torch.zeros((1, ops.mlstm_state_values(heads, dim, vdim)), device="cuda")
+        at = (0, width, 2 * width, 2 * width + heads * vdim, 2 * width + heads * vdim + heads)
+        zeros, one = torch.zeros(heads, device="cuda"), dev([0], torch.int32)
+        outs.append(ops.mlstm_scan(proj, at, zeros, zeros + 3.0, 10.0, state, one, dev([tokens], torch.int32), one, heads, dim, vdim,
+                                   longest=tokens))
+    plain_out, late_out = outs
+    assert float((plain_out[:late] - late_out[:late]).abs().max()) < 1e-4 and not bool(late_out[late:].isfinite().any())
+
+
+@gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rank, rot, heads, dim", [(20, 6, 4, 12), (48, 16, 2, 32), (12, 4, 3, 8), (96, 2, 1, 5)])
 def test_latent_rows_into_the_cache_and_rotated_query_parts(dtype, rank, rot, heads, dim):
