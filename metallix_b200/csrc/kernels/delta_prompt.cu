@@ -1,5 +1,5 @@
-// The matrix-state recurrences of delta_rule.cu (which states them) over portions of prompts: the delta rule with a decay
-// per channel or per head, and the state-space dual.
+// The delta rule with a decay per channel (delta_rule.cu states it) over portions of prompts, and the steps of single tokens
+// of all three recurrences there that keep a matrix per head.
 //
 // A token by itself is a chain of dependent steps (decay, a dot with the key over the lanes that share a column, the
 // write), and delta_rule.cu pays that chain per token. Here eight tokens pay it once. With S the state ahead of eight
@@ -7,14 +7,16 @@
 //   u_t = beta_t (v_t - (k_t G_t) . S - sum_(s < t) A_ts u_s),    A_ts = sum_d k_t k_s g_(s+1) ... g_t
 //   o_t = (q_t G_t) . S + sum_(s <= t) P_ts u_s,                  P_ts = sum_d q_t k_s g_(s+1) ... g_t
 //   S <- G_8 S + sum_s (k_s g_(s+1) ... g_8) u_s^T
-// (the dual: u_t = dt_t v_t and no look at S). What does not depend on S or on the column, the three kinds of products
-// with keys and queries, G_8, A and P, is made first, a block per (eight tokens, head), in the order in which the lanes
-// will read it. Then a block of four warps walks a head's 32 columns, four columns and eight channels a thread: all 16
+// What does not depend on S or on the column, the three kinds of products with keys and queries, G_8, A and P, is made
+// first, a block per (eight tokens, head), in the order in which the lanes will read it. Then a block of four warps walks a head's 32 columns, four columns and eight channels a thread: all 16
 // dots with S at once, their sums over the lanes together, a small triangular solve per column, one update of S. A fifth
 // warp keeps the next eights on their way, one bulk copy each. Float32 throughout, as there.
 // The walk is bound by its shared-memory reads and by what is left of the chain: 342 us for 1,777 tokens of 32 heads of 128
 // x 128 with a decay per channel, the records 73 us; delta_rule.cu took 917. Token by token with four columns a thread it
 // stayed at 480 to 530, whichever way the channels were shared out: the exchanges of every token were the chain.
+// One decay per head and the dual stay with delta_rule.cu over prompts too, although eight tokens at a time took 341 us there
+// for 725 (one row of 1,777 tokens, 32 heads), and the dual 314 for 853: their sums in another order moved the logits of a
+// decoder whose routers stand close to a tie behind them by up to 0.05 of their size, one token's row by 0.28.
 #include <type_traits>
 
 #include "async_copy.cuh"
@@ -87,7 +89,7 @@ struct WalkArgs {
 };
 
 // One block per (eight tokens, head), a warp a token.
-template <typename T, int LANES, int MODE>
+template <typename T, int LANES>
 __global__ void __launch_bounds__(32 * kEight)
 walk_records_kernel(WalkArgs a) {
   constexpr int WIDTH = LANES * kWalkPer, NL = WIDTH / 32;
@@ -127,7 +129,7 @@ walk_records_kernel(WalkArgs a) {
   float* record = a.records + (static_cast<size_t>(head) * a.eights + blockIdx.x) * walk_record(WIDTH);
   float *const A = record + 25 * WIDTH, *const P = A + kEight * kEight, *const beta = P + kEight * kEight;
   const float rate = a.rate[head];
-  float q[NL] = {}, k[NL] = {}, write = 0.0f, decay = 1.0f, qq = 0.0f, kk = 0.0f;
+  float q[NL] = {}, k[NL] = {}, write = 0.0f, qq = 0.0f, kk = 0.0f;
   if (live) {
     const int group = head / (a.heads / a.groups);
     const T* x = static_cast<const T*>(a.qkv) + token * a.ld;
@@ -139,30 +141,22 @@ walk_records_kernel(WalkArgs a) {
       qq = fmaf(q[i], q[i], qq);
       kk = fmaf(k[i], k[i], kk);
     }
-    if (MODE != kWalkDual) {
-      const float q_unit = rsqrtf(warp_sum(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(warp_sum(kk) + 1e-6f);
+    const float q_unit = rsqrtf(warp_sum(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(warp_sum(kk) + 1e-6f);
 #pragma unroll
-      for (int i = 0; i < NL; ++i) {
-        q[i] *= q_unit;
-        k[i] *= k_unit;
-      }
-      write = sigmoid_of(to_float(static_cast<const T*>(a.beta_pre)[token * a.ldb + a.b_off + head]));
+    for (int i = 0; i < NL; ++i) {
+      q[i] *= q_unit;
+      k[i] *= k_unit;
     }
-    if (MODE != kWalkChannel) {
-      const float step = walk_softplus(to_float(static_cast<const T*>(a.step_pre)[token * a.lds + head]) + a.step_bias[head]);
-      decay = expf(-rate * step);
-      if (MODE == kWalkDual) write = step;
-    }
+    write = sigmoid_of(to_float(static_cast<const T*>(a.beta_pre)[token * a.ldb + a.b_off + head]));
   }
 #pragma unroll
   for (int i = 0; i < NL; ++i) {
     const int d = lane + 32 * i;
     sq[warp][d] = q[i];
     sk[warp][d] = k[i];
-    sg[warp][d] = MODE != kWalkChannel ? decay
-                  : live && d < a.dim  ? expf(-rate * walk_softplus(static_cast<const float*>(a.step_pre)[token * a.lds + head * a.dim + d] +
-                                                                     a.step_bias[head * a.dim + d]))
-                                       : 1.0f;
+    sg[warp][d] = live && d < a.dim ? expf(-rate * walk_softplus(static_cast<const float*>(a.step_pre)[token * a.lds + head * a.dim + d] +
+                                                                 a.step_bias[head * a.dim + d]))
+                                    : 1.0f;
   }
   if (lane == 0) beta[warp] = write;
   __syncthreads();
@@ -205,13 +199,12 @@ walk_records_kernel(WalkArgs a) {
 // LANES lanes share four columns, eight channels each. Block (request, head, columns): blockDim.x - 32 threads with
 // columns and a warp that fetches. A thread counts its four columns from one of them on (column c of a lane is c ^ own),
 // and tokens of the outputs likewise, so that an exchange which halves what a lane adds up needs no choosing.
-template <typename T, int LANES, int MODE>
+template <typename T, int LANES>
 __global__ void __launch_bounds__(160)
 walk_kernel(WalkArgs a) {
   constexpr int WIDTH = LANES * kWalkPer, RECORD = walk_record(WIDTH), PAIRS = kWalkPer / 2;
   constexpr int SHARERS = LANES / 4;            // lanes that end with the same column
   constexpr int OWN = kEight / SHARERS;         // tokens of it whose output a lane writes
-  constexpr bool LOOKS = MODE != kWalkDual;
   extern __shared__ __align__(16) float stages[];   // [kWalkStages][RECORD]
   __shared__ __align__(8) uint64_t full[kWalkStages], empty[kWalkStages];
   __shared__ int s_ahead;
@@ -261,7 +254,6 @@ walk_kernel(WalkArgs a) {
     const int own = (part & (LANES / 2) ? 2 : 0) + (part & (LANES / 4) ? 1 : 0);   // the column this lane ends with
     const int turned = part % SHARERS * OWN;                                        // the first token whose output it writes
     const int column = (blockIdx.z * (workers / LANES) + threadIdx.x / LANES) * kWalkCols;
-    const float head_skip = MODE == kWalkDual ? a.skip[head] : 0.0f;
     float* home = a.state + static_cast<long long>(slot) * a.slot_stride +
                   (static_cast<long long>(head) * a.vdim + column) * a.dim + part * kWalkPer;
     const bool whole = a.dim % kWalkPer == 0 && a.slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
@@ -288,23 +280,17 @@ walk_kernel(WalkArgs a) {
     // This lane's column of a stage's tokens, a stage ahead. The values stay as they come until they are used, and no
     // branch stands around a load (places outside repeat others): either would make each load wait for the one before.
     const T* values = static_cast<const T*>(a.qkv) + first * a.ld + a.v_off + head * a.vdim + min(column + own, a.vdim - 1);
-    T next[kEight], next_own[MODE == kWalkDual ? OWN : 1];
+    T next[kEight];
     auto fetch = [&](int t0) {
 #pragma unroll
       for (int t = 0; t < kEight; ++t) next[t] = values[static_cast<long long>(min(t0 + t, count - 1)) * a.ld];
-      if (MODE == kWalkDual)
-#pragma unroll
-        for (int t = 0; t < OWN; ++t) next_own[t] = values[static_cast<long long>(min(t0 + (t ^ turned), count - 1)) * a.ld];
     };
     fetch(0);
     for (int r = 0; r < rounds; ++r) {
       const int stage = r % kWalkStages, tokens = min(kEight, count - r * kEight);
-      T value[kEight], value_own[MODE == kWalkDual ? OWN : 1];
+      T value[kEight];
 #pragma unroll
       for (int t = 0; t < kEight; ++t) value[t] = next[t];
-      if (MODE == kWalkDual)
-#pragma unroll
-        for (int t = 0; t < OWN; ++t) value_own[t] = next_own[t];
       if (!barrier_wait(&full[stage], (r / kWalkStages) & 1, a.status)) { ok = false; break; }
       fetch((r + 1) * kEight);   // on their way while this stage is walked
       const float* record = stages + stage * RECORD;
@@ -330,7 +316,7 @@ walk_kernel(WalkArgs a) {
       };
       // ---- (k_t G_t) . S of this lane's column, then what is written of every token
       float u[kEight][kWalkCols];
-      if (LOOKS) {
+      {
         float kd[kEight][kWalkCols];
 #pragma unroll
         for (int t = 0; t < kEight; ++t) dots(t, kd[t]);
@@ -356,16 +342,12 @@ walk_kernel(WalkArgs a) {
         *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(beta + 4);
 #pragma unroll
         for (int t = 0; t < kEight; ++t) {
-          float rest = to_float(value[t]);
-          if (LOOKS) {
-            float line[kEight], seen = u[t][0];
-            *reinterpret_cast<float4*>(line) = *reinterpret_cast<const float4*>(A + t * kEight);
-            *reinterpret_cast<float4*>(line + 4) = *reinterpret_cast<const float4*>(A + t * kEight + 4);
+          float line[kEight], seen = u[t][0];
+          *reinterpret_cast<float4*>(line) = *reinterpret_cast<const float4*>(A + t * kEight);
+          *reinterpret_cast<float4*>(line + 4) = *reinterpret_cast<const float4*>(A + t * kEight + 4);
 #pragma unroll
-            for (int e = 0; e < t; ++e) seen = fmaf(line[e], u[e][0], seen);
-            rest -= seen;
-          }
-          u[t][0] = t < tokens ? b[t] * rest : 0.0f;
+          for (int e = 0; e < t; ++e) seen = fmaf(line[e], u[e][0], seen);
+          u[t][0] = t < tokens ? b[t] * (to_float(value[t]) - seen) : 0.0f;
         }
       }
       // ---- (q_t G_t) . S, each lane's tokens counted from those whose outputs it writes
@@ -429,7 +411,6 @@ walk_kernel(WalkArgs a) {
 #pragma unroll
         for (int e = 0; e < kEight; ++e)   // chosen, not weighed with 0: a later token's infinity stays out of this one
           o = e <= mine ? fmaf(line[t][e], u[e][0], o) : o;
-        if (MODE == kWalkDual) o = fmaf(head_skip, to_float(value_own[t]), o);
         if (mine < tokens && column + own < a.vdim)
           a.out[(first + r * kEight + mine) * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim +
                 column + own] = o;
@@ -590,20 +571,19 @@ static long long walk_window(long long tokens, int rows, int heads, int dim) {
 using namespace mxb;
 
 // How many KiB of scratch mxb_delta_prompt needs for a step of `tokens` tokens whose longest row brings `longest` (0:
-// unknown); 0: the step does not take this way. It does from 32 tokens a
-// row on (us, delta_rule.cu first: one row of 24 tokens, 32 heads, 19 and 21, the dual 21 and 21; of 64 tokens 43 and 32,
-// the dual 41 and 34; 40 tokens beside 31 single ones 131 and 87; 100 beside 31, the dual, 189 and 185), with keys of 33 to
+// unknown); 0: the step does not take this way. It does with a decay per channel (mode 0) from 32 tokens a
+// row on (us, delta_rule.cu first: one row of 24 tokens, 32 heads, 19 and 21; of 64 tokens 43 and 32;
+// 40 tokens beside 31 single ones 131 and 87), with keys of 33 to
 // 128 channels: narrower ones leave lanes without channels, wider ones do not fit a thread's registers.
 MXB_API int mxb_delta_prompt_scratch(long long tokens, int rows, int longest, int mode, int heads, int dim) {
-  if (tokens <= 0 || rows <= 0 || longest < 32 || mode < kWalkChannel || mode > kWalkDual || heads <= 0 || heads > 65535 ||
-      dim <= 32 || dim > 128)
+  if (tokens <= 0 || rows <= 0 || longest < 32 || mode != kWalkChannel || heads <= 0 || heads > 65535 || dim <= 32 || dim > 128)
     return 0;
   const long long eights = walk_window(tokens, rows, heads, dim) / kEight + rows;
   const long long kib = (eights * 4 * heads * walk_record(walk_lanes(dim) * kWalkPer) + 1023) >> 10;
   return kib > 0x7fffffffLL ? 0 : static_cast<int>(kib);
 }
 
-// As mxb_delta_rule (modes 0 to 2), for steps that mxb_delta_prompt_scratch gives a size for; `scratch` lies on 16 bytes.
+// As mxb_delta_rule (mode 0), for steps that mxb_delta_prompt_scratch gives a size for; `scratch` lies on 16 bytes.
 MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off, int v_off, const void* beta_pre,
                              long long ldb, int b_off, const void* step_pre, long long lds, const float* step_bias,
                              const float* rate, const float* skip, int mode, float* state, long long slot_stride, int num_slots,
@@ -611,7 +591,7 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
                              long long tokens, int rows, int heads, int groups, int dim, int vdim, int dtype, int longest,
                              void* scratch, int* status, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (groups <= 0 || heads % groups != 0 || vdim <= 0 || (mode == kWalkDual) != (skip != nullptr) || scratch == nullptr ||
+  if (groups <= 0 || heads % groups != 0 || vdim <= 0 || skip != nullptr || scratch == nullptr ||
       (reinterpret_cast<uintptr_t>(scratch) & 15) || (dtype != kF32 && dtype != kBF16) ||
       mxb_delta_prompt_scratch(tokens, rows, longest, mode, heads, dim) == 0)
     return static_cast<int>(cudaErrorInvalidValue);
@@ -624,27 +604,22 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
   const int columns = static_cast<long long>(rows) * heads * ceil_div(vdim, 32) < 120 ? 16 : 32;
   const int threads = ceil_div(columns / kWalkCols * lanes, 32) * 32 + 32;
   const int of_block = (threads - 32) / lanes * kWalkCols;
-  auto run = [&](auto type, auto lanes_of, auto mode_of) {
+  auto run = [&](auto type, auto lanes_of) {
     using T = decltype(type);
-    constexpr int LANES = decltype(lanes_of)::value, MODE = decltype(mode_of)::value;
+    constexpr int LANES = decltype(lanes_of)::value;
     constexpr int shared = kWalkStages * walk_record(LANES * kWalkPer) * 4;
-    const cudaError_t e = cudaFuncSetAttribute(walk_kernel<T, LANES, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+    const cudaError_t e = cudaFuncSetAttribute(walk_kernel<T, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
     if (e != cudaSuccess) return static_cast<int>(e);
     for (a.from = 0; a.from < tokens; a.from += window) {
       a.to = a.from + window < tokens ? a.from + window : tokens;
       const int eights = static_cast<int>((a.to - a.from) / kEight + rows);
-      walk_records_kernel<T, LANES, MODE><<<dim3(eights, heads), 32 * kEight, 0, stream>>>(a);
-      walk_kernel<T, LANES, MODE><<<dim3(rows, heads, ceil_div(vdim, of_block)), threads, shared, stream>>>(a);
+      walk_records_kernel<T, LANES><<<dim3(eights, heads), 32 * kEight, 0, stream>>>(a);
+      walk_kernel<T, LANES><<<dim3(rows, heads, ceil_div(vdim, of_block)), threads, shared, stream>>>(a);
     }
     return static_cast<int>(cudaGetLastError());
   };
-  auto by_mode = [&](auto type, auto lanes_of) {
-    if (mode == kWalkChannel) return run(type, lanes_of, std::integral_constant<int, kWalkChannel>());
-    if (mode == kWalkHead) return run(type, lanes_of, std::integral_constant<int, kWalkHead>());
-    return run(type, lanes_of, std::integral_constant<int, kWalkDual>());
-  };
   auto by_lanes = [&](auto type) {
-    return lanes == 8 ? by_mode(type, std::integral_constant<int, 8>()) : by_mode(type, std::integral_constant<int, 16>());
+    return lanes == 8 ? run(type, std::integral_constant<int, 8>()) : run(type, std::integral_constant<int, 16>());
   };
   return dtype == kF32 ? by_lanes(float()) : by_lanes(__nv_bfloat16());
 }

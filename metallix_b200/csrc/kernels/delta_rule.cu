@@ -23,7 +23,8 @@
 //
 //   S <- g_h S + k v^T;   o = S^T q
 //
-// Rows of 32 tokens and more, and single tokens, mostly take the kernels of delta_prompt.cu instead.
+// With a decay per channel, rows of 32 tokens and more mostly take the kernels of delta_prompt.cu instead; so do steps of
+// single tokens of the first three.
 //
 // Every value column of S goes its own way: column j needs only v_j and what
 // all columns share (qn, kn, g, beta). A block owns some of the columns of

@@ -474,8 +474,9 @@ def test_delta_rule_kernel(dtype, heads, groups, dim, vdim):
 @pytest.mark.parametrize("heads, groups, dim, vdim, lengths", [(4, 2, 128, 128, [33, 1, 0, 40]), (2, 1, 64, 36, [32, 7, 8, 9]),
                                                                (3, 3, 36, 5, [1, 65]), (2, 2, 101, 50, [50]),
                                                                (512, 1, 40, 4, [31, 300, 270])])
-def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, groups, dim, vdim, lengths):
-    """Against the recurrences in 64 bits, two launches one behind the other; the last shape takes several windows. An
+def test_matrix_state_recurrences_over_prompts(mode, dtype, heads, groups, dim, vdim, lengths):
+    """Against the recurrences in 64 bits, two launches one behind the other; with a decay per channel eight tokens at a
+    time, which takes several windows for the last shape. An
     eight's sums have up to 128 + 8 terms, so a few times 2^-24 of the result's size is what float32 leaves."""
     from metallix_b200 import ops
     rng = np.random.default_rng(heads * dim + vdim + mode)
@@ -488,7 +489,7 @@ def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, gro
     state = torch.zeros((len(lengths) + 1, heads, vdim, dim), device="cuda")
     state[0] = 3.0
     slots, outs = list(range(len(lengths), 0, -1)), []
-    assert ops._fn("mxb_delta_prompt_scratch")(total, len(lengths), max(lengths), mode, heads, dim)
+    assert bool(ops._fn("mxb_delta_prompt_scratch")(total, len(lengths), max(lengths), mode, heads, dim)) == (mode == 0)
     for half in range(2):
         starts = [half * sum(lengths) + sum(lengths[:row]) for row in range(len(lengths))]
         outs.append(ops._matrix_state(mode, qkv, (3, 3 + widths[0], 3 + 2 * widths[0]), None if mode == 2 else beta, step, bias, rate,
@@ -515,6 +516,44 @@ def test_matrix_state_recurrences_eight_tokens_at_a_time(mode, dtype, heads, gro
             want = torch.stack(want).view(2 * length, -1)
             assert float((have.double() - want).norm() / want.norm()) < 2e-6, row
             assert float((state[slots[row]].double().transpose(1, 2) - S).norm() / S.norm()) < 2e-6, row
+
+
+def matrix_state_case(mode, dtype, heads, groups, dim, vdim, tokens):
+    """Random inputs of a matrix-state recurrence, and a function that walks row 0 of them through portions of the given
+    lengths: (outputs, state)."""
+    from metallix_b200 import ops
+    rng = np.random.default_rng(heads * dim + vdim + mode)
+    width = 2 * groups * dim + heads * vdim
+    qkv = torch.from_numpy(rng.normal(size=(tokens, -(-width // 8) * 8))).to("cuda", dtype)[:, :width]
+    beta, step = (torch.from_numpy(rng.normal(size=(tokens, n))).to("cuda", t)
+                  for n, t in ((heads, dtype), (heads * dim, torch.float32) if mode == 0 else (heads, dtype)))
+    bias, rate, skip = (torch.from_numpy(x).float().cuda() for x in (rng.normal(size=heads * dim if mode == 0 else heads) - 2.0,
+                                                                     rng.uniform(0.5, 4.0, heads), rng.normal(size=heads)))
+    start = dev(rng.normal(size=(2, heads, vdim, dim)))
+
+    def walk(portions):
+        state, outs, at = start.clone(), [], 0
+        for count in portions:
+            outs.append(ops._matrix_state(mode, qkv[at:at + count], (0, groups * dim, 2 * groups * dim),
+                                          None if mode == 2 else beta[at:at + count], step[at:at + count], bias, rate,
+                                          skip if mode == 2 else None, state, dev([0], torch.int32), dev([count], torch.int32),
+                                          dev([1], torch.int32), heads, groups, dim, vdim, count))
+            at += count
+        ops.check_status("cuda")
+        return torch.cat(outs), state
+    return walk
+
+
+@gpu
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (2, 1, 64, 36), (3, 3, 100, 50)])
+def test_one_decay_per_head_gives_the_same_bits_however_a_prompt_is_cut(mode, dtype, heads, groups, dim, vdim):
+    walk = matrix_state_case(mode, dtype, heads, groups, dim, vdim, 75)
+    out, state = walk([75])
+    for portions in ([40, 33, 2], [31, 9, 35]):
+        again, carried = walk(portions)
+        assert torch.equal(out, again) and torch.equal(state, carried), portions
 
 
 @gpu
