@@ -443,15 +443,17 @@ walk_kernel(WalkArgs a) {
 
 // A step of single tokens: bound by reading and writing the states. A warp has (LANES = 16) eight columns of a (request,
 // head), four columns and eight channels a thread as above; every load, the state's and the token's, is on its way at
-// once and no thread waits for another warp (delta_rule.cu: a trip to memory for the row's length, one for its slot, one
-// for the state with 32 bytes a thread, two barriers). 16 requests, 32 heads of 128 x 128, a decay per channel: 48 -> 22 us,
-// per head 41 -> 20, the dual with 128 heads of 128 x 64 54 -> 30 (their states' bytes take 10, 10 and 20); 64 requests
-// 137 -> 55; one request 10 either way.
+// once and no thread waits for another warp. Every sum has the terms and the order of delta_rule.cu, so that a token gets
+// the same bits alone as among others of its request (delta_rule.cu: a trip to memory for the row's length, one for its slot, one
+// for the state with 32 bytes a thread, two barriers). 16 requests, 32 heads of 128 x 128, a decay per channel: 47 -> 24 us,
+// per head 41 -> 20, the dual with 128 heads of 128 x 64 56 -> 32 (their states' bytes take 10, 10 and 20); 64 requests,
+// per head 137 -> 55.
 template <typename T, int LANES, int MODE>
 __global__ void __launch_bounds__(128)
 step_kernel(WalkArgs a) {
   constexpr bool LOOKS = MODE != kWalkDual;
-  const int row = blockIdx.x, head = blockIdx.y;
+  constexpr int NL = LANES * kWalkPer / 32;   // channels a lane adds to the norms: those that delta_rule.cu gives it
+  const int row = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
   const int length = a.row_length[row], slot = a.request_slots[row];
   const long long token = a.row_start[row];
   if (length <= 0) return;
@@ -481,6 +483,13 @@ step_kernel(WalkArgs a) {
       raw_q[i] = *reinterpret_cast<const Eight*>(x + a.q_off + group * a.dim + d0 + i * EACH);
       raw_k[i] = *reinterpret_cast<const Eight*>(x + a.k_off + group * a.dim + d0 + i * EACH);
     }
+  T norm_q[NL], norm_k[NL];
+#pragma unroll
+  for (int i = 0; i < NL; ++i) {
+    const int d = min(lane + 32 * i, a.dim - 1);
+    norm_q[i] = x[a.q_off + group * a.dim + d];
+    norm_k[i] = x[a.k_off + group * a.dim + d];
+  }
   T raw_v[kWalkCols];
 #pragma unroll
   for (int c = 0; c < kWalkCols; ++c) raw_v[c] = x[a.v_off + head * a.vdim + min(column + c, a.vdim - 1)];
@@ -503,25 +512,31 @@ step_kernel(WalkArgs a) {
   for (int i = 0; i < kWalkPer; ++i) {
     q[i] = to_float(raw_q[i / EACH].v[i % EACH]);
     k[i] = to_float(raw_k[i / EACH].v[i % EACH]);
-    qq = fmaf(q[i], q[i], qq);
-    kk = fmaf(k[i], k[i], kk);
-    qk = fmaf(q[i], k[i], qk);
   }
-  auto over_lanes = [](float v) {
 #pragma unroll
-    for (int offset = 1; offset < LANES; offset <<= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);
-    return v;
-  };
-  qk = over_lanes(qk);
+  for (int i = 0; i < NL; ++i) {
+    const bool there = lane + 32 * i < a.dim;
+    const float qd = there ? to_float(norm_q[i]) : 0.0f, kd = there ? to_float(norm_k[i]) : 0.0f;
+    qq = fmaf(qd, qd, qq);
+    kk = fmaf(kd, kd, kk);
+    qk = fmaf(qd, kd, qk);
+  }
+  qk = warp_sum(qk);
   if (LOOKS) {
-    const float q_unit = rsqrtf(over_lanes(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(over_lanes(kk) + 1e-6f);
+    const float q_unit = rsqrtf(warp_sum(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(warp_sum(kk) + 1e-6f);
 #pragma unroll
     for (int i = 0; i < kWalkPer; ++i) {
       q[i] *= q_unit;
       k[i] *= k_unit;
     }
-    qk *= q_unit * k_unit;
+    qk = qk * q_unit * k_unit;
   }
+  // over the lanes of a column: neighbours first where the column is looked at, the dual in the order of its exchanges
+  auto over_lanes = [](float v) {
+#pragma unroll
+    for (int step = 1; step < LANES; step <<= 1) v += __shfl_xor_sync(0xffffffffu, v, LOOKS ? step : LANES / 2 / step);
+    return v;
+  };
   if (MODE == kWalkChannel) {
 #pragma unroll
     for (int i = 0; i < kWalkPer; ++i) g[i] = expf(-rate * walk_softplus(pre[MODE == kWalkChannel ? i : 0] + bias[MODE == kWalkChannel ? i : 0]));
@@ -550,9 +565,10 @@ step_kernel(WalkArgs a) {
         to[0] = make_float4(fmaf(k[0], u, r[0]), fmaf(k[1], u, r[1]), fmaf(k[2], u, r[2]), fmaf(k[3], u, r[3]));
         to[1] = make_float4(fmaf(k[4], u, r[4]), fmaf(k[5], u, r[5]), fmaf(k[6], u, r[6]), fmaf(k[7], u, r[7]));
       }
+      float o = fmaf(qk, u, q_dot);
+      if (MODE == kWalkDual) o = fmaf(skip, v, o);
       if (part == 0)
-        a.out[token * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim + column + c] =
-            fmaf(qk, u, q_dot) + (MODE == kWalkDual ? skip * v : 0.0f);
+        a.out[token * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim + column + c] = o;
     }
   }
 }

@@ -545,6 +545,18 @@ def matrix_state_case(mode, dtype, heads, groups, dim, vdim, tokens):
 
 
 @gpu
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (3, 1, 40, 33), (2, 2, 64, 70), (1, 1, 120, 1)])
+def test_single_tokens_get_the_bits_of_a_portion(mode, dtype, heads, groups, dim, vdim):
+    walk = matrix_state_case(mode, dtype, heads, groups, dim, vdim, 21)
+    out, state = walk([21])
+    for portions in ([1] * 21, [1, 19, 1]):
+        again, carried = walk(portions)
+        assert torch.equal(out, again) and torch.equal(state, carried), portions
+
+
+@gpu
 @pytest.mark.parametrize("mode", [1, 2])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (2, 1, 64, 36), (3, 3, 100, 50)])
