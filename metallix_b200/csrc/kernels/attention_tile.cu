@@ -303,10 +303,13 @@ paged_attention_tile_kernel(const __grid_constant__ TileArgs args) {
 
 constexpr size_t kTileSharedMost = 227 * 1024;
 
+// Bytes of queries and weights of G heads, and of a tile of keys and values.
+static size_t tile_fixed(int head_dim, int G) { return sizeof(float) * G * kTileQueries * (row_pitch(head_dim) + kScorePitch); }
+static size_t tile_stage(int head_dim, int VQ) { return sizeof(float) * kTileKeys * (row_pitch(head_dim) + VQ * 32); }
+
 template <typename T, int G, int VQ>
 static int launch_tile(TileArgs args, cudaStream_t stream) {
-  const size_t fixed = sizeof(float) * G * kTileQueries * (row_pitch(args.head_dim) + kScorePitch);
-  const size_t stage = sizeof(float) * kTileKeys * (row_pitch(args.head_dim) + VQ * 32);
+  const size_t fixed = tile_fixed(args.head_dim, G), stage = tile_stage(args.head_dim, VQ);
   const long long blocks = static_cast<long long>(args.tiles) * (args.heads / G);
   if (blocks > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   // Two key tiles at a time where the blocks are too few to hide a tile's trip to memory behind one another (a decode
@@ -322,23 +325,26 @@ static int launch_tile(TileArgs args, cudaStream_t stream) {
   return static_cast<int>(cudaGetLastError());
 }
 
-// How many query heads share a block: as many as the key/value head has, up to what the registers hold (`most`), as
+// How many query heads share a block: as many as the key/value head has, up to what the registers hold (`most`) and to
+// what fits shared memory (four heads of more than 532 values whose outputs have 65 to 128 do not; one always does), as
 // long as two blocks an SM are left.
-static int shared_heads(const TileArgs& args, int most) {
+static int shared_heads(const TileArgs& args, int most, int VQ) {
   const int group = args.heads / args.kv_heads;
   for (int g = most; g > 1; g /= 2)
-    if (group % g == 0 && static_cast<long long>(args.tiles) * (args.heads / g) >= 296) return g;
+    if (group % g == 0 && static_cast<long long>(args.tiles) * (args.heads / g) >= 296 &&
+        tile_fixed(args.head_dim, g) + tile_stage(args.head_dim, VQ) <= kTileSharedMost)
+      return g;
   return 1;
 }
 
 template <typename T, int VQ>
 static int launch_heads(const TileArgs& args, cudaStream_t stream) {
   if constexpr (VQ <= 4) {
-    const int g = shared_heads(args, 4);
+    const int g = shared_heads(args, 4, VQ);
     if (g == 4) return launch_tile<T, 4, VQ>(args, stream);
     if (g == 2) return launch_tile<T, 2, VQ>(args, stream);
   } else if constexpr (VQ <= 8) {
-    if (shared_heads(args, 2) == 2) return launch_tile<T, 2, VQ>(args, stream);
+    if (shared_heads(args, 2, VQ) == 2) return launch_tile<T, 2, VQ>(args, stream);
   }
   return launch_tile<T, 1, VQ>(args, stream);
 }

@@ -256,6 +256,76 @@ def test_paged_attention_window(ops, dtype, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, kv_heads, head_dim, value_dim, planes, options", [
+    (8, 2, 32, 32, 2, {}), (4, 1, 64, 64, 2, {"window": 21, "sink": 4}), (4, 1, 128, 128, 2, {"gate": "value"}),
+    (4, 1, 50, 50, 2, {"chunk": 16, "keep": 3}), (6, 3, 104, 70, 2, {"softcap": 5.0, "gate": "head"}),
+    (2, 1, 256, 256, 2, {"sink": 2}), (4, 2, 192, 150, 1, {"window": 9}),
+    (4, 1, 576, 128, 1, {}), (4, 1, 560, 64, 1, {"sink": 4}), (4, 1, 568, 24, 1, {})])
+def test_query_heads_that_share_a_block(ops, dtype, heads, kv_heads, head_dim, value_dim, planes, options):
+    """Steps with so many tiles that two or four query heads share a block's keys, against the formulas in 64 bits and, bit
+    for bit, against launches of few tiles, where every head has a block of its own. Wide keys leave room for fewer heads."""
+    gen = torch.Generator(device="cuda").manual_seed(head_dim)
+    normal = lambda *shape: torch.randn(shape, generator=gen, device="cuda").to(dtype)
+    lengths = [(100, 39), (37, 37), (65, 1)] + [(1 + n % 40, 1 + n % min(3, 1 + n % 40)) for n in range(620 // (heads // 2))]
+    pages = [-(-total // 16) for total, _ in lengths]
+    order = torch.randperm(sum(pages), generator=gen, device="cuda")
+    cache = normal(sum(pages), planes, kv_heads, 16, head_dim)
+    tables = torch.full((len(lengths), max(pages)), -1, dtype=torch.int32, device="cuda")
+    tokens = sum(count for _, count in lengths)
+    q, scale, used = normal(tokens, heads, head_dim), head_dim ** -0.5, 0
+    gate = {"value": normal(tokens, heads * value_dim), "head": normal(tokens, heads), None: None}[options.get("gate")]
+    sink = normal(heads).float() if options.get("sink") else None
+    bias = normal(heads, options["bias"]).float() if options.get("bias") else None
+    window, chunk, keep, cap = (options.get(name, 0) for name in ("window", "chunk", "keep", "softcap"))
+    want = torch.empty((tokens, heads, value_dim), dtype=torch.float64, device="cuda")
+    request, start, length, positions, begin = [], [], [], [], 0
+    for r, (total, count) in enumerate(lengths):
+        mine = order[used:used + pages[r]]
+        used += pages[r]
+        tables[r, :pages[r]] = mine.int()
+        rows = cache[mine].double().permute(1, 2, 0, 3, 4).reshape(planes, kv_heads, -1, head_dim)[:, :, :total]
+        cache[mine[-1], :, :, total - 16 * (pages[r] - 1):] = float("nan")     # beyond the request's positions
+        p, j = torch.arange(total - count, total, device="cuda")[:, None], torch.arange(total, device="cuda")[None, :]
+        seen = j <= p
+        if window or chunk:
+            seen &= ((p - j < window) if window else (p // chunk == j // chunk)) | (j < keep)
+        for head in range(heads):
+            k, v = rows[0, head // (heads // kv_heads)], rows[planes - 1, head // (heads // kv_heads), :, :value_dim]
+            s = (q[begin:begin + count, head].double() @ k.t()) * scale
+            s = cap * torch.tanh(s / cap) if cap else s
+            if bias is not None:
+                s = s + bias[head].double()[(p - j).clamp(0, bias.shape[1] - 1)]
+            s = s.masked_fill(~seen, -float("inf"))
+            if sink is not None:
+                s = torch.cat([s, sink[head].double().expand(count, 1)], dim=1)
+            out = torch.softmax(s, dim=1)[:, :total] @ v
+            if gate is not None:
+                part = gate[begin:begin + count, head:head + 1] if options["gate"] == "head" else \
+                    gate[begin:begin + count, head * value_dim:(head + 1) * value_dim]
+                out = out * torch.sigmoid(part.double())
+            want[begin:begin + count, head] = out
+        for first in range(0, count, 16):
+            request.append(r)
+            start.append(begin + first)
+            length.append(min(16, count - first))
+        positions += range(total - count, total)
+        begin += count
+    lists = [torch.tensor(x, dtype=torch.int32, device="cuda") for x in (request, start, length)]
+    positions = torch.tensor(positions, dtype=torch.int32, device="cuda")
+    assert len(request) * heads // min(4, heads // kv_heads) >= 296
+    outs = []
+    for size in (len(request), 290 // heads):
+        outs.append(torch.full((tokens, heads, value_dim), 9.0, dtype=dtype, device="cuda"))
+        for at in range(0, len(request), size):
+            ops.paged_attention_tile(q, cache, outs[-1], tables, *(x[at:at + size] for x in lists), positions, scale, window, chunk,
+                                     gate=gate, softcap=cap, gate_per_head=options.get("gate") == "head", sink=sink, bias=bias,
+                                     keep=keep)
+    ops.check_status("cuda")
+    assert torch.equal(outs[0], outs[1])
+    assert float((outs[0].double() - want).abs().max()) < tol(dtype, 1e-5, 2e-2)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_one_far_key_among_hundreds(ops, dtype):
     """Random keys would average a lost key away. Here one key matches the
     query so strongly that the output must be that key's value: at the first
