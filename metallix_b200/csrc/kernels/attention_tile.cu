@@ -214,9 +214,10 @@ paged_attention_tile_kernel(const __grid_constant__ TileArgs args) {
       for (int j = 0; j < 4; ++j) {
         const int key = key0 + lane8 + 8 * j;
         visible[j] = row_valid && key_seen(key, my_pos, my_first, args.keep);
-        float dot = s[g][j] * args.scale;
-        if (args.softcap > 0.0f) dot = args.softcap * tanhf(dot / args.softcap);
-        if (args.bias.table != nullptr) dot += bias_at(args.bias.row(head0 + g), my_pos - key, args.bias.far);
+        // rounded as written: every form of the kernel has to leave the compiler the same choice of joint roundings
+        float dot = __fmul_rn(s[g][j], args.scale);
+        if (args.softcap > 0.0f) dot = __fmul_rn(args.softcap, tanhf(dot / args.softcap));
+        if (args.bias.table != nullptr) dot = __fadd_rn(dot, bias_at(args.bias.row(head0 + g), my_pos - key, args.bias.far));
         s[g][j] = visible[j] ? dot : kMinusHuge;
         tile_max = fmaxf(tile_max, s[g][j]);
       }
@@ -235,7 +236,7 @@ paged_attention_tile_kernel(const __grid_constant__ TileArgs args) {
       }
 #pragma unroll
       for (int offset = 1; offset < 8; offset <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, offset);
-      l[g] = l[g] * alpha[g] + psum;
+      l[g] = fmaf(l[g], alpha[g], psum);
       m[g] = m_new;
     }
     __syncwarp();  // a row's 8 threads sit in one warp
@@ -267,10 +268,10 @@ paged_attention_tile_kernel(const __grid_constant__ TileArgs args) {
       }
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        acc[g][j].x = acc[g][j].x * alpha[g] + sum[g].x;
-        acc[g][j].y = acc[g][j].y * alpha[g] + sum[g].y;
-        acc[g][j].z = acc[g][j].z * alpha[g] + sum[g].z;
-        acc[g][j].w = acc[g][j].w * alpha[g] + sum[g].w;
+        acc[g][j].x = fmaf(acc[g][j].x, alpha[g], sum[g].x);
+        acc[g][j].y = fmaf(acc[g][j].y, alpha[g], sum[g].y);
+        acc[g][j].z = fmaf(acc[g][j].z, alpha[g], sum[g].z);
+        acc[g][j].w = fmaf(acc[g][j].w, alpha[g], sum[g].w);
       }
     }
     __syncwarp();

@@ -258,6 +258,7 @@ def test_paged_attention_window(ops, dtype, window):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads, kv_heads, head_dim, value_dim, planes, options", [
     (8, 2, 32, 32, 2, {}), (4, 1, 64, 64, 2, {"window": 21, "sink": 4}), (4, 1, 128, 128, 2, {"gate": "value"}),
+    (4, 1, 128, 120, 2, {"bias": 6, "gate": "value"}), (8, 2, 32, 32, 2, {"bias": 9, "softcap": 6.0}),
     (4, 1, 50, 50, 2, {"chunk": 16, "keep": 3}), (6, 3, 104, 70, 2, {"softcap": 5.0, "gate": "head"}),
     (2, 1, 256, 256, 2, {"sink": 2}), (4, 2, 192, 150, 1, {"window": 9}),
     (4, 1, 576, 128, 1, {}), (4, 1, 560, 64, 1, {"sink": 4}), (4, 1, 568, 24, 1, {})])
