@@ -50,7 +50,8 @@ selective_scan_kernel(const T* __restrict__ x, long long ldx, const float* __res
   if (PART == kChunkAdds && last) return;   // nothing follows it
   const int n = last ? all - begin : kScanChunk;
   const int slot = request_slots[row];
-  if (slot < 0 || slot >= num_slots) {
+  // A row of more chunks than the caller said would reach beyond its part of the scratch: none of it is worked on.
+  if (slot < 0 || slot >= num_slots || (PART != kWholeRow && all > chunks * kScanChunk)) {
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, kStatusBadSlot);
     return;
   }
@@ -237,7 +238,7 @@ selective_scan_states_kernel(const float* __restrict__ a, const float* __restric
                              const float* __restrict__ chunk_steps, int channels, int states, int num_slots, int chunks) {
   const int row = blockIdx.y, n = row_length[row], slot = request_slots[row];
   const size_t values = static_cast<size_t>(channels) * states, e = blockIdx.x * size_t(256) + threadIdx.x;
-  if (n <= 0 || slot < 0 || slot >= num_slots || e >= values) return;
+  if (n <= 0 || n > chunks * kScanChunk || slot < 0 || slot >= num_slots || e >= values) return;
   const int used = ceil_div(n, kScanChunk);
   const float decay = a[e];
   float s = state[slot * values + e];
@@ -314,7 +315,8 @@ MXB_API int mxb_selective_scan_scratch(long long tokens, int rows, int channels,
 
 // x, z: [tokens, channels] (row strides ldx, ldz); step: float32 [tokens, channels] ahead of its bias and softplus;
 // a: float32 [channels, states] (negative); b, c: [tokens, states] with row stride ldbc; d: [channels];
-// out: [tokens, channels] contiguous. Up to 256 states. longest: the most tokens of a row (0 if not known).
+// out: [tokens, channels] contiguous. Up to 256 states. longest: the most tokens of a row (0 if not known); with scratch,
+// a row that brings more than `longest` rounded up to 64 sets the status word's bit for bad rows and is left out.
 // scratch: as many float32 values as mxb_selective_scan_scratch says, or null: every row in one walk.
 MXB_API int mxb_selective_scan(const void* x, long long ldx, const float* step, long long ld_step,
                                const float* step_bias, const float* a, const void* b, const void* c, long long ldbc,

@@ -445,6 +445,37 @@ def test_selective_scan_kernel(dtype, channels, states):
 
 
 @gpu
+@pytest.mark.parametrize("lengths", [[70, 500, 0, 1], [192, 333], [193]])
+def test_selective_scan_of_rows_longer_than_said(lengths):
+    """A row that brings more chunks than ``longest`` says would reach beyond its part of the scratch: it is reported and left
+    out, the other rows get what they get without it."""
+    from metallix_b200 import ops
+    channels, states, said = 40, 16, 192
+    rng = np.random.default_rng(sum(lengths))
+    total, starts = sum(lengths), [sum(lengths[:row]) for row in range(len(lengths))]
+    a, bias, skip = dev(-np.exp(rng.normal(size=(channels, states)))), dev(rng.normal(size=channels) - 4.0), dev(rng.normal(size=channels))
+    both, picked = dev(rng.normal(size=(total, 2 * channels)), torch.bfloat16), dev(rng.normal(size=(total, 2 * states)), torch.bfloat16)
+    step, results = dev(rng.normal(size=(total, channels))), []
+    assert ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, said)
+    for brought in (lengths, [n if n <= said else 0 for n in lengths]):
+        state = torch.full((len(lengths), channels, states), 2.0, device="cuda")
+        out = ops.selective_scan(both[:, :channels], step, bias, a, picked[:, :states], picked[:, states:], skip, both[:, channels:],
+                                 state, dev(starts, torch.int32), dev(brought, torch.int32), dev(range(len(lengths)), torch.int32),
+                                 longest=said)
+        if brought is lengths:
+            with pytest.raises(ops.KernelError, match="slot"):
+                ops.check_status("cuda")
+        ops.check_status("cuda")
+        results.append((out, state))
+    assert torch.equal(results[0][1], results[1][1])
+    for row, n in enumerate(lengths):
+        if n > said:
+            assert bool((results[0][1][row] == 2.0).all())
+        else:
+            assert torch.equal(results[0][0][starts[row]:starts[row] + n], results[1][0][starts[row]:starts[row] + n])
+
+
+@gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("channels, states, lengths", [(100, 16, [192, 1, 0, 65]), (33, 7, [300, 64, 63]), (8, 1, [193, 128])])
 def test_selective_scan_in_chunks(dtype, channels, states, lengths):
