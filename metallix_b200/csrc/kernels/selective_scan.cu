@@ -302,13 +302,18 @@ using namespace mxb;
 // row is not known or short, or has more than 16 states, or where the step is wide: the chunks cost twice the arithmetic,
 // which pays as long as a walk's chain of steps is what takes the time. The line lies at 6,000 (channel, token) pairs per
 // token of the longest row (us, whole rows first): 4,600 pairs (2,048 channels, rows of 1,201, 700 and 800 tokens) 445 and
-// 210, 2,140 (700 beside 31 single tokens) 245 and 122, 2,048 (one row of 256) 93 and 52; 8,192 (as many channels, one row
-// of 192) 78 and 85, 18,400 618 and 730.
+// 210, 2,140 (700 beside 31 single tokens) 245 and 122, 2,048 (one row of 256) 93 and 52; 6,144 (6,144 channels, one row of
+// 192) 78 and 60, 8,192 (4,096 channels, two rows) 80 and 85, 18,400 618 and 730. And a row costs some 12 tokens' work and
+// half a token's per chunk of the longest row however short it is, mostly its state's way to the scratch and back: beside
+// a row of 256, 2,048 channels, 31 single tokens 96 and 83, 63 98 and 108, 400 166 and 415; beside one of 1,024, 63 360 and 192.
+// The second line's numbers take the measured winners among 140 such steps and no loser.
 MXB_API int mxb_selective_scan_scratch(long long tokens, int rows, int channels, int states, int longest) {
   if (tokens <= 0 || rows <= 0 || channels <= 0 || states <= 0 || states > 4 * kScanLanes || longest < 3 * kScanChunk ||
       tokens * channels > 6000ll * longest)
     return 0;
-  const long long chunks = ceil_div(longest, kScanChunk), each = static_cast<long long>(channels) * (states + 1);
+  const long long chunks = ceil_div(longest, kScanChunk);
+  if (channels * (tokens + rows * (24 + chunks)) > 18000ll * longest - 1600000ll) return 0;
+  const long long each = static_cast<long long>(channels) * (states + 1);
   const long long values = chunks * rows * each;
   return chunks > 65535 || values * 4 > kScanScratch ? 0 : static_cast<int>(values);
 }

@@ -444,6 +444,15 @@ def test_selective_scan_kernel(dtype, channels, states):
             assert (gap > 20 * tolerance * (1.0 + np.abs(want[-1]))).mean() > 0.1
 
 
+@pytest.mark.parametrize("channels, lengths, chunks", [
+    (2048, [256] + [1] * 63, False), (2048, [256] + [1] * 400, False), (512, [192] + [1] * 127, False),
+    (2048, [512] + [1] * 127, False), (2048, [256] + [1] * 31, True), (2048, [700] + [1] * 31, True),
+    (2048, [1201, 700, 800], True), (1024, [192] * 4, True), (2048, [1024] + [1] * 63, True), (3072, [192] * 3, False)])
+def test_scan_takes_chunks_where_they_were_measured_to_win(channels, lengths, chunks):
+    from metallix_b200 import ops
+    assert bool(ops._fn("mxb_selective_scan_scratch")(sum(lengths), len(lengths), channels, 16, max(lengths))) == chunks
+
+
 @gpu
 @pytest.mark.parametrize("lengths", [[70, 500, 0, 1], [192, 333], [193]])
 def test_selective_scan_of_rows_longer_than_said(lengths):
