@@ -12,13 +12,16 @@
 // both precisions; x, B, C and z arrive in the compute type. Four lanes share
 // a channel, each owning every fourth state in registers; a request row's
 // tokens are walked in order, so what a position gets does not depend on how
-// the sequence was cut into steps. `state` is [slots, channels, states]
-// float32; a row of length 0 touches no slot.
+// the sequence was cut into steps (float32 always; bfloat16 where no step took
+// the chunks below, which agree with the walk to float32's rounding). `state` is
+// [slots, channels, states] float32; a row of length 0 touches no slot.
 //
-// Prompts: one walk per channel over 1,201 tokens is a chain of 1,201 steps on few warps (that row and two of 700 and 800
+// Prompts in bfloat16: one walk per channel over 1,201 tokens is a chain of 1,201 steps on few warps (that row and two of 700 and 800
 // with 2,048 channels: 445 us). So their rows are cut into chunks of 64 tokens that run side by side, twice: once from a state of
 // zeros for what a chunk adds and the sum of its step sizes, from which the state ahead of every chunk follows
 // (S <- exp(A sum) S + added), then from that state for the outputs: 210 us.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mxb {
@@ -277,7 +280,7 @@ static int launch_scan(const void* x, long long ldx, const float* step, long lon
       static_cast<const T*>(x), ldx, step, ld_step, step_bias, a, static_cast<const T*>(b), static_cast<const T*>(c), \
       ldbc, d, static_cast<const T*>(z), ldz, state, row_start, row_length, request_slots, static_cast<T*>(out),    \
       channels, states, num_slots, scratch, steps, chunks, status)
-  if constexpr (PER <= 4) {
+  if constexpr (PER <= 4 && std::is_same_v<T, __nv_bfloat16>) {
     if (scratch != nullptr) {
       chunks = ceil_div(longest, kScanChunk);
       steps = scratch + static_cast<size_t>(rows) * chunks * channels * states;
@@ -298,7 +301,8 @@ static int launch_scan(const void* x, long long ldx, const float* step, long lon
 
 using namespace mxb;
 
-// How many float32 values of scratch mxb_selective_scan wants, to walk a step's rows in chunks: none (0) where the longest
+// How many float32 values of scratch mxb_selective_scan wants, to walk a step's rows in chunks: none (0) in float32, whose
+// results are the same however a sequence is cut and whatever else a step brings, where the longest
 // row is not known or short, or has more than 16 states, or where the step is wide: the chunks cost twice the arithmetic,
 // which pays as long as a walk's chain of steps is what takes the time. The line lies at 6,000 (channel, token) pairs per
 // token of the longest row (us, whole rows first): 4,600 pairs (2,048 channels, rows of 1,201, 700 and 800 tokens) 445 and
@@ -307,8 +311,8 @@ using namespace mxb;
 // half a token's per chunk of the longest row however short it is, mostly its state's way to the scratch and back: beside
 // a row of 256, 2,048 channels, 31 single tokens 96 and 83, 63 98 and 108, 400 166 and 415; beside one of 1,024, 63 360 and 192.
 // The second line's numbers take the measured winners among 140 such steps and no loser.
-MXB_API int mxb_selective_scan_scratch(long long tokens, int rows, int channels, int states, int longest) {
-  if (tokens <= 0 || rows <= 0 || channels <= 0 || states <= 0 || states > 4 * kScanLanes || longest < 3 * kScanChunk ||
+MXB_API int mxb_selective_scan_scratch(long long tokens, int rows, int channels, int states, int longest, int dtype) {
+  if (dtype != kBF16 || tokens <= 0 || rows <= 0 || channels <= 0 || states <= 0 || states > 4 * kScanLanes || longest < 3 * kScanChunk ||
       tokens * channels > 6000ll * longest)
     return 0;
   const long long chunks = ceil_div(longest, kScanChunk);
@@ -331,7 +335,7 @@ MXB_API int mxb_selective_scan(const void* x, long long ldx, const float* step, 
                                cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (channels <= 0 || states <= 0 || states > 64 * kScanLanes) return static_cast<int>(cudaErrorInvalidValue);
-  if (scratch != nullptr && (states > 4 * kScanLanes || longest <= 0)) return static_cast<int>(cudaErrorInvalidValue);
+  if (scratch != nullptr && (dtype != kBF16 || states > 4 * kScanLanes || longest <= 0)) return static_cast<int>(cudaErrorInvalidValue);
   const int per = ceil_div(states, kScanLanes);
 #define ARGS x, ldx, step, ld_step, step_bias, a, b, c, ldbc, d, z, ldz, state, row_start, row_length, request_slots, \
              out, rows, channels, states, num_slots, longest, scratch, status, stream

@@ -41,7 +41,7 @@ _SIGNATURES = {
     "mxb_short_conv": [_P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "mxb_selective_scan": [_P, _L, _P, _L, _P, _P, _P, _P, _L, _P, _P, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I,
                            _P, _I, _P, _P],
-    "mxb_selective_scan_scratch": [_L, _I, _I, _I, _I],
+    "mxb_selective_scan_scratch": [_L, _I, _I, _I, _I, _I],
     "mxb_route_experts": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _L, _I, _I, _P],
     "mxb_expert_rows": [_P, _P, _P, _I, _I, _I, _P],
     "mxb_expert_rows_tile": [],
@@ -674,8 +674,9 @@ def selective_scan(x: torch.Tensor, step: torch.Tensor, step_bias: torch.Tensor,
     ``[tokens, channels]``; ``a`` float32 ``[channels, states]``; ``state``
     float32 ``[slots, channels, states]``, read and moved on. ``longest``: the
     most tokens of a row if known (1 picks the kernel for single tokens; from
-    192 on a narrow step's rows may run as chunks of 64 tokens side by side,
-    which agrees with one walk to rounding)."""
+    192 on a narrow bfloat16 step's rows may run as chunks of 64 tokens side by
+    side, which agrees with one walk to float32's rounding; no row may then
+    bring more than that)."""
     dtype = x.dtype
     for name, tensor in (("x", x), ("z", z), ("b", b), ("c", c)):
         _need(tensor.is_cuda and tensor.dtype == dtype and dtype in _CODES and tensor.dim() == 2
@@ -698,7 +699,7 @@ def selective_scan(x: torch.Tensor, step: torch.Tensor, step_bias: torch.Tensor,
     rows = row_start.numel()
     _need(row_length.numel() == rows and request_slots.numel() >= rows, "the step's row lists differ in length")
     out = torch.empty((tokens, channels), dtype=dtype, device=x.device)
-    values = _fn("mxb_selective_scan_scratch")(tokens, rows, channels, states, int(longest))
+    values = _fn("mxb_selective_scan_scratch")(tokens, rows, channels, states, int(longest), _CODES[dtype])
     scratch = torch.empty(values, dtype=torch.float32, device=x.device) if values else None
     _call("mxb_selective_scan", x.data_ptr(), x.stride(0), step.data_ptr(), step.stride(0), step_bias.data_ptr(),
           a.data_ptr(), b.data_ptr(), c.data_ptr(), b.stride(0), d.data_ptr(), z.data_ptr(), z.stride(0),

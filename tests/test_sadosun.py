@@ -444,13 +444,35 @@ def test_selective_scan_kernel(dtype, channels, states):
             assert (gap > 20 * tolerance * (1.0 + np.abs(want[-1]))).mean() > 0.1
 
 
+@gpu
+@pytest.mark.parametrize("states", [16, 5])
+def test_float32_scan_gives_the_same_bits_however_a_prompt_is_cut(states):
+    from metallix_b200 import ops
+    channels, tokens = 70, 400
+    rng = np.random.default_rng(states)
+    a, bias, skip = dev(-np.exp(rng.normal(size=(channels, states)))), dev(rng.normal(size=channels) - 4.0), dev(rng.normal(size=channels))
+    both, picked = dev(rng.normal(size=(tokens, 2 * channels))), dev(rng.normal(size=(tokens, 2 * states)))
+    step, one, results = dev(rng.normal(size=(tokens, channels))), dev([0], torch.int32), []
+    for portions in ([400], [200, 193, 7], [1, 399], [64] * 6 + [16]):
+        state, outs, at = torch.zeros((1, channels, states), device="cuda"), [], 0
+        for n in portions:
+            cut = slice(at, at + n)
+            outs.append(ops.selective_scan(both[cut, :channels], step[cut], bias, a, picked[cut, :states], picked[cut, states:], skip,
+                                           both[cut, channels:], state, one, dev([n], torch.int32), one, longest=n))
+            at += n
+        results.append((torch.cat(outs), state))
+    for out, state in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(state, results[0][1])
+
+
 @pytest.mark.parametrize("channels, lengths, chunks", [
     (2048, [256] + [1] * 63, False), (2048, [256] + [1] * 400, False), (512, [192] + [1] * 127, False),
     (2048, [512] + [1] * 127, False), (2048, [256] + [1] * 31, True), (2048, [700] + [1] * 31, True),
     (2048, [1201, 700, 800], True), (1024, [192] * 4, True), (2048, [1024] + [1] * 63, True), (3072, [192] * 3, False)])
 def test_scan_takes_chunks_where_they_were_measured_to_win(channels, lengths, chunks):
     from metallix_b200 import ops
-    assert bool(ops._fn("mxb_selective_scan_scratch")(sum(lengths), len(lengths), channels, 16, max(lengths))) == chunks
+    wanted = lambda dtype: ops._fn("mxb_selective_scan_scratch")(sum(lengths), len(lengths), channels, 16, max(lengths), ops._CODES[dtype])
+    assert bool(wanted(torch.bfloat16)) == chunks and not wanted(torch.float32)
 
 
 @gpu
@@ -465,7 +487,7 @@ def test_selective_scan_of_rows_longer_than_said(lengths):
     a, bias, skip = dev(-np.exp(rng.normal(size=(channels, states)))), dev(rng.normal(size=channels) - 4.0), dev(rng.normal(size=channels))
     both, picked = dev(rng.normal(size=(total, 2 * channels)), torch.bfloat16), dev(rng.normal(size=(total, 2 * states)), torch.bfloat16)
     step, results = dev(rng.normal(size=(total, channels))), []
-    assert ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, said)
+    assert ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, said, ops._CODES[torch.bfloat16])
     for brought in (lengths, [n if n <= said else 0 for n in lengths]):
         state = torch.full((len(lengths), channels, states), 2.0, device="cuda")
         out = ops.selective_scan(both[:, :channels], step, bias, a, picked[:, :states], picked[:, states:], skip, both[:, channels:],
@@ -488,8 +510,9 @@ def test_selective_scan_of_rows_longer_than_said(lengths):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("channels, states, lengths", [(100, 16, [192, 1, 0, 65]), (33, 7, [300, 64, 63]), (8, 1, [193, 128])])
 def test_selective_scan_in_chunks(dtype, channels, states, lengths):
-    """Rows in chunks of 64 tokens side by side against one walk per row, two launches one behind the other: float32 to
-    rounding, bfloat16 outputs to one rounding of theirs; slow decays, so that a state ahead of a chunk counts in it."""
+    """Rows in chunks of 64 tokens side by side (bfloat16) against one walk per row, two launches one behind the other: states
+    to float32's rounding, outputs to one rounding of theirs; slow decays, so that a state ahead of a chunk counts in it.
+    Float32 walks whole rows either way."""
     from metallix_b200 import ops
     rng = np.random.default_rng(channels + states)
     total, slots = sum(lengths), list(range(len(lengths), 0, -1))
@@ -497,7 +520,8 @@ def test_selective_scan_in_chunks(dtype, channels, states, lengths):
     skip, starts = dev(rng.normal(size=channels)), [sum(lengths[:row]) for row in range(len(lengths))]
     inputs = [(dev(rng.normal(size=(total, 2 * channels)), dtype), dev(rng.normal(size=(total, channels))),
                dev(rng.normal(size=(total, 2 * states)), dtype)) for _ in range(2)]
-    assert ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, max(lengths))
+    scratch = ops._fn("mxb_selective_scan_scratch")(total, len(lengths), channels, states, max(lengths), ops._CODES[dtype])
+    assert bool(scratch) == (dtype == torch.bfloat16)
     results = []
     for longest in (max(lengths), 0):
         state = torch.zeros((len(lengths) + 1, channels, states), device="cuda")
@@ -509,7 +533,7 @@ def test_selective_scan_in_chunks(dtype, channels, states, lengths):
         results.append((torch.cat(outs).float(), state))
     (out, state), (walked, behind) = results
     assert float((state - behind).abs().max()) < 2e-6 * float(behind[1:].abs().max()) and float(state[0].min()) == 3.0
-    limit = 5e-6 if dtype == torch.float32 else 2.0 ** -8
+    limit = 1e-30 if dtype == torch.float32 else 2.0 ** -8
     assert float(((out - walked).abs() / (walked.abs() + 0.05 * walked.abs().max())).max()) < limit
 
 
