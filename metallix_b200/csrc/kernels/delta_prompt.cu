@@ -1,4 +1,4 @@
-// The delta rule with a decay per channel (delta_rule.cu states it) over portions of prompts, and the steps of single tokens
+// The delta rule with a decay per channel (delta_rule.cu states it) over portions of prompts in bfloat16, and the steps of single tokens
 // of all three recurrences there that keep a matrix per head.
 //
 // A token by itself is a chain of dependent steps (decay, a dot with the key over the lanes that share a column, the
@@ -11,7 +11,8 @@
 // first, a block per (eight tokens, head), in the order in which the lanes will read it. Then a block of four warps walks a head's 32 columns, four columns and eight channels a thread: all 16
 // dots with S at once, their sums over the lanes together, a small triangular solve per column, one update of S. A fifth
 // warp keeps the next eights on their way, one bulk copy each. Float32 throughout, as there.
-// The walk is bound by its shared-memory reads and by what is left of the chain: 342 us for 1,777 tokens of 32 heads of 128
+// Its sums run in another order than token by token, so
+// float32, whose results are the same however a prompt is cut, stays there. The walk is bound by its shared-memory reads and by what is left of the chain: 342 us for 1,777 tokens of 32 heads of 128
 // x 128 with a decay per channel, the records 73 us; delta_rule.cu took 917. Token by token with four columns a thread it
 // stayed at 480 to 530, whichever way the channels were shared out: the exchanges of every token were the chain.
 // One decay per head and the dual stay with delta_rule.cu over prompts too, although eight tokens at a time took 341 us there
@@ -587,12 +588,12 @@ static long long walk_window(long long tokens, int rows, int heads, int dim) {
 using namespace mxb;
 
 // How many KiB of scratch mxb_delta_prompt needs for a step of `tokens` tokens whose longest row brings `longest` (0:
-// unknown); 0: the step does not take this way. It does with a decay per channel (mode 0) from 32 tokens a
+// unknown); 0: the step does not take this way. It does in bfloat16 with a decay per channel (mode 0) from 32 tokens a
 // row on (us, delta_rule.cu first: one row of 24 tokens, 32 heads, 19 and 21; of 64 tokens 43 and 32;
 // 40 tokens beside 31 single ones 131 and 87), with keys of 33 to
 // 128 channels: narrower ones leave lanes without channels, wider ones do not fit a thread's registers.
-MXB_API int mxb_delta_prompt_scratch(long long tokens, int rows, int longest, int mode, int heads, int dim) {
-  if (tokens <= 0 || rows <= 0 || longest < 32 || mode != kWalkChannel || heads <= 0 || heads > 65535 || dim <= 32 || dim > 128)
+MXB_API int mxb_delta_prompt_scratch(long long tokens, int rows, int longest, int mode, int heads, int dim, int dtype) {
+  if (dtype != kBF16 || tokens <= 0 || rows <= 0 || longest < 32 || mode != kWalkChannel || heads <= 0 || heads > 65535 || dim <= 32 || dim > 128)
     return 0;
   const long long eights = walk_window(tokens, rows, heads, dim) / kEight + rows;
   const long long kib = (eights * 4 * heads * walk_record(walk_lanes(dim) * kWalkPer) + 1023) >> 10;
@@ -608,8 +609,8 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
                              void* scratch, int* status, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (groups <= 0 || heads % groups != 0 || vdim <= 0 || skip != nullptr || scratch == nullptr ||
-      (reinterpret_cast<uintptr_t>(scratch) & 15) || (dtype != kF32 && dtype != kBF16) ||
-      mxb_delta_prompt_scratch(tokens, rows, longest, mode, heads, dim) == 0)
+      (reinterpret_cast<uintptr_t>(scratch) & 15) ||
+      mxb_delta_prompt_scratch(tokens, rows, longest, mode, heads, dim, dtype) == 0)
     return static_cast<int>(cudaErrorInvalidValue);
   const int lanes = walk_lanes(dim);
   const long long window = walk_window(tokens, rows, heads, dim);
@@ -620,8 +621,8 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
   const int columns = static_cast<long long>(rows) * heads * ceil_div(vdim, 32) < 120 ? 16 : 32;
   const int threads = ceil_div(columns / kWalkCols * lanes, 32) * 32 + 32;
   const int of_block = (threads - 32) / lanes * kWalkCols;
-  auto run = [&](auto type, auto lanes_of) {
-    using T = decltype(type);
+  auto run = [&](auto lanes_of) {
+    using T = __nv_bfloat16;
     constexpr int LANES = decltype(lanes_of)::value;
     constexpr int shared = kWalkStages * walk_record(LANES * kWalkPer) * 4;
     const cudaError_t e = cudaFuncSetAttribute(walk_kernel<T, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
@@ -634,10 +635,7 @@ MXB_API int mxb_delta_prompt(const void* qkv, long long ld, int q_off, int k_off
     }
     return static_cast<int>(cudaGetLastError());
   };
-  auto by_lanes = [&](auto type) {
-    return lanes == 8 ? run(type, std::integral_constant<int, 8>()) : run(type, std::integral_constant<int, 16>());
-  };
-  return dtype == kF32 ? by_lanes(float()) : by_lanes(__nv_bfloat16());
+  return lanes == 8 ? run(std::integral_constant<int, 8>()) : run(std::integral_constant<int, 16>());
 }
 
 // Whether mxb_delta_step takes a step: single tokens (longest 1), keys of 40, 48 ... 128 channels whose rows and states

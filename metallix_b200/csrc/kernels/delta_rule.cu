@@ -23,8 +23,8 @@
 //
 //   S <- g_h S + k v^T;   o = S^T q
 //
-// With a decay per channel, rows of 32 tokens and more mostly take the kernels of delta_prompt.cu instead; so do steps of
-// single tokens of the first three.
+// In bfloat16 with a decay per channel, rows of 32 tokens and more mostly take the kernels of delta_prompt.cu instead, whose
+// sums agree with these to float32's rounding; so do steps of single tokens of the first three, with the same bits.
 //
 // Every value column of S goes its own way: column j needs only v_j and what
 // all columns share (qn, kn, g, beta). A block owns some of the columns of

@@ -64,7 +64,7 @@ _SIGNATURES = {
     "mxb_delta_step_supported": [_P, _L, _I, _I, _I, _P, _L, _I, _I, _I, _I],
     "mxb_delta_step": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I,
                        _I, _I, _P, _P],
-    "mxb_delta_prompt_scratch": [_L, _I, _I, _I, _I, _I],
+    "mxb_delta_prompt_scratch": [_L, _I, _I, _I, _I, _I, _I],
     "mxb_delta_prompt": [_P, _L, _I, _I, _I, _P, _L, _I, _P, _L, _P, _P, _P, _I, _P, _L, _I, _P, _P, _P, _P, _L, _I, _I, _I,
                          _I, _I, _I, _I, _P, _P, _P],
     "mxb_lightning_chunks_supported": [_P, _L, _I, _I, _I, _I, _I, _I],
@@ -1143,7 +1143,7 @@ def _matrix_state(mode: int, qkv, offsets, beta, step, step_bias, rate, skip, st
               state.data_ptr(), state.stride(0), state.shape[0], row_start.data_ptr(), row_length.data_ptr(),
               request_slots.data_ptr(), out.data_ptr())
     sizes = (rows, heads, groups, dim, vdim, _CODES[qkv.dtype], int(longest))
-    scratch_kib = _fn("mxb_delta_prompt_scratch")(tokens, rows, int(longest), mode, heads, dim)
+    scratch_kib = _fn("mxb_delta_prompt_scratch")(tokens, rows, int(longest), mode, heads, dim, _CODES[qkv.dtype])
     if scratch_kib:
         scratch = torch.empty(scratch_kib << 10, dtype=torch.uint8, device=qkv.device)
         _call("mxb_delta_prompt", *inputs, tokens, *sizes, scratch.data_ptr(), status_word(qkv.device).data_ptr(), _stream())

@@ -475,8 +475,8 @@ def test_delta_rule_kernel(dtype, heads, groups, dim, vdim):
                                                                (3, 3, 36, 5, [1, 65]), (2, 2, 101, 50, [50]),
                                                                (512, 1, 40, 4, [31, 300, 270])])
 def test_matrix_state_recurrences_over_prompts(mode, dtype, heads, groups, dim, vdim, lengths):
-    """Against the recurrences in 64 bits, two launches one behind the other; with a decay per channel eight tokens at a
-    time, which takes several windows for the last shape. An
+    """Against the recurrences in 64 bits, two launches one behind the other; bfloat16 with a decay per channel eight
+    tokens at a time, which takes several windows for the last shape. An
     eight's sums have up to 128 + 8 terms, so a few times 2^-24 of the result's size is what float32 leaves."""
     from metallix_b200 import ops
     rng = np.random.default_rng(heads * dim + vdim + mode)
@@ -489,7 +489,8 @@ def test_matrix_state_recurrences_over_prompts(mode, dtype, heads, groups, dim, 
     state = torch.zeros((len(lengths) + 1, heads, vdim, dim), device="cuda")
     state[0] = 3.0
     slots, outs = list(range(len(lengths), 0, -1)), []
-    assert bool(ops._fn("mxb_delta_prompt_scratch")(total, len(lengths), max(lengths), mode, heads, dim)) == (mode == 0)
+    scratch = ops._fn("mxb_delta_prompt_scratch")(total, len(lengths), max(lengths), mode, heads, dim, ops._CODES[dtype])
+    assert bool(scratch) == (mode == 0 and dtype == torch.bfloat16)
     for half in range(2):
         starts = [half * sum(lengths) + sum(lengths[:row]) for row in range(len(lengths))]
         outs.append(ops._matrix_state(mode, qkv, (3, 3 + widths[0], 3 + 2 * widths[0]), None if mode == 2 else beta, step, bias, rate,
@@ -557,10 +558,11 @@ def test_single_tokens_get_the_bits_of_a_portion(mode, dtype, heads, groups, dim
 
 
 @gpu
-@pytest.mark.parametrize("mode", [1, 2])
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode, dtype", [(0, torch.float32), (1, torch.float32), (1, torch.bfloat16), (2, torch.float32),
+                                         (2, torch.bfloat16)])
 @pytest.mark.parametrize("heads, groups, dim, vdim", [(4, 2, 128, 128), (2, 1, 64, 36), (3, 3, 100, 50)])
-def test_one_decay_per_head_gives_the_same_bits_however_a_prompt_is_cut(mode, dtype, heads, groups, dim, vdim):
+def test_matrix_state_recurrences_give_the_same_bits_however_a_prompt_is_cut(mode, dtype, heads, groups, dim, vdim):
+    """All but bfloat16 with a decay per channel, which takes eight tokens at a time in longer rows."""
     walk = matrix_state_case(mode, dtype, heads, groups, dim, vdim, 75)
     out, state = walk([75])
     for portions in ([40, 33, 2], [31, 9, 35]):
@@ -574,8 +576,9 @@ def test_matrix_state_recurrences_keep_later_values_out_of_earlier_outputs(mode)
     from metallix_b200 import ops
     heads, dim, vdim, tokens, late = 2, 64, 32, 40, 20
     rng = np.random.default_rng(mode)
-    qkv, outs = dev(rng.normal(size=(tokens, heads * (2 * dim + vdim)))), []
-    gates, step = dev(rng.normal(size=(tokens, heads))), dev(rng.normal(size=(tokens, heads * dim if mode == 0 else heads)))
+    qkv, outs = dev(rng.normal(size=(tokens, heads * (2 * dim + vdim))), torch.bfloat16), []
+    gates = dev(rng.normal(size=(tokens, heads)), torch.bfloat16)
+    step = dev(rng.normal(size=(tokens, heads * dim))) if mode == 0 else dev(rng.normal(size=(tokens, heads)), torch.bfloat16)
     ones = torch.ones(heads, device="cuda")
     for value in (1.0, float("inf")):
         qkv[late, 2 * heads * dim:] = value
