@@ -588,13 +588,16 @@ static long long walk_window(long long tokens, int rows, int heads, int dim) {
 using namespace mxb;
 
 // How many KiB of scratch mxb_delta_prompt needs for a step of `tokens` tokens whose longest row brings `longest` (0:
-// unknown); 0: the step does not take this way. It does in bfloat16 with a decay per channel (mode 0) from 32 tokens a
-// row on (us, delta_rule.cu first: one row of 24 tokens, 32 heads, 19 and 21; of 64 tokens 43 and 32;
-// 40 tokens beside 31 single ones 131 and 87), with keys of 33 to
-// 128 channels: narrower ones leave lanes without channels, wider ones do not fit a thread's registers.
+// unknown); 0: the step does not take this way. It does in bfloat16 with a decay per channel (mode 0) where a row brings 64
+// tokens, or 32 and there is other work (us, delta_rule.cu first, heads of 128 x 128: 16 heads, one row of 24 tokens 17 and
+// 17, of 32 20 and 25, of 56 29 and 30, of 64 33 and 32, of 1,777 672 and 304; 8 heads, four rows of 32 26 and 26; 16 heads,
+// three 43 and 28; 24 heads, one row of 40 29 and 30, of 48 34 and 32; 32 heads, one row of 32 25 and 26, of 40 30 and 28;
+// beside 31 single tokens 131 and 89; 128 heads, eight rows of 512 7,383 and 3,025, whose records come in several
+// windows). Keys have 33 to 128 channels: narrower ones leave lanes without channels, wider ones do not fit a thread's registers.
 MXB_API int mxb_delta_prompt_scratch(long long tokens, int rows, int longest, int mode, int heads, int dim, int dtype) {
   if (dtype != kBF16 || tokens <= 0 || rows <= 0 || longest < 32 || mode != kWalkChannel || heads <= 0 || heads > 65535 || dim <= 32 || dim > 128)
     return 0;
+  if (longest < 64 && static_cast<long long>(heads) * rows < 40 && heads * tokens < 1152) return 0;
   const long long eights = walk_window(tokens, rows, heads, dim) / kEight + rows;
   const long long kib = (eights * 4 * heads * walk_record(walk_lanes(dim) * kWalkPer) + 1023) >> 10;
   return kib > 0x7fffffffLL ? 0 : static_cast<int>(kib);
