@@ -456,7 +456,6 @@ step_kernel(WalkArgs a) {
   constexpr int NL = LANES * kWalkPer / 32;   // channels a lane adds to the norms: those that delta_rule.cu gives it
   const int row = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
   const int length = a.row_length[row], slot = a.request_slots[row];
-  const long long token = a.row_start[row];
   if (length <= 0) return;
   if (slot < 0 || slot >= a.num_slots) {
     if (threadIdx.x == 0) atomicOr(a.status, kStatusBadSlot);
@@ -475,101 +474,108 @@ step_kernel(WalkArgs a) {
                                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   struct alignas(16) Eight { T v[16 / sizeof(T)]; };
   constexpr int PIECES = kWalkPer * sizeof(T) / 16, EACH = 16 / sizeof(T);
-  const T* x = static_cast<const T*>(a.qkv) + token * a.ld;
   const int group = head / (a.heads / a.groups);
-  Eight raw_q[PIECES] = {}, raw_k[PIECES] = {};
-  if (has)
+  const long long first = a.row_start[row];
+#pragma unroll 1
+  for (long long token = first; token < first + length; ++token) {   // once, unless a row is longer than the caller said
+    const T* x = static_cast<const T*>(a.qkv) + token * a.ld;
+    const bool last = token + 1 == first + length;
+    Eight raw_q[PIECES] = {}, raw_k[PIECES] = {};
+    if (has)
 #pragma unroll
-    for (int i = 0; i < PIECES; ++i) {
-      raw_q[i] = *reinterpret_cast<const Eight*>(x + a.q_off + group * a.dim + d0 + i * EACH);
-      raw_k[i] = *reinterpret_cast<const Eight*>(x + a.k_off + group * a.dim + d0 + i * EACH);
-    }
-  T norm_q[NL], norm_k[NL];
-#pragma unroll
-  for (int i = 0; i < NL; ++i) {
-    const int d = min(lane + 32 * i, a.dim - 1);
-    norm_q[i] = x[a.q_off + group * a.dim + d];
-    norm_k[i] = x[a.k_off + group * a.dim + d];
-  }
-  T raw_v[kWalkCols];
-#pragma unroll
-  for (int c = 0; c < kWalkCols; ++c) raw_v[c] = x[a.v_off + head * a.vdim + min(column + c, a.vdim - 1)];
-  float pre[MODE == kWalkChannel ? kWalkPer : 1], bias[MODE == kWalkChannel ? kWalkPer : 1];
-  if (MODE == kWalkChannel) {
-#pragma unroll
-    for (int i = 0; i < kWalkPer; ++i) {
-      pre[i] = has ? static_cast<const float*>(a.step_pre)[token * a.lds + head * a.dim + d0 + i] : 0.0f;
-      bias[i] = has ? a.step_bias[head * a.dim + d0 + i] : 0.0f;
-    }
-  } else {
-    pre[0] = to_float(static_cast<const T*>(a.step_pre)[token * a.lds + head]);
-    bias[0] = a.step_bias[head];
-  }
-  const float rate = a.rate[head], skip = MODE == kWalkDual ? a.skip[head] : 0.0f;
-  float beta = LOOKS ? sigmoid_of(to_float(static_cast<const T*>(a.beta_pre)[token * a.ldb + a.b_off + head])) : 0.0f;
-
-  float q[kWalkPer], k[kWalkPer], g[kWalkPer], qq = 0.0f, kk = 0.0f, qk = 0.0f;
-#pragma unroll
-  for (int i = 0; i < kWalkPer; ++i) {
-    q[i] = to_float(raw_q[i / EACH].v[i % EACH]);
-    k[i] = to_float(raw_k[i / EACH].v[i % EACH]);
-  }
-#pragma unroll
-  for (int i = 0; i < NL; ++i) {
-    const bool there = lane + 32 * i < a.dim;
-    const float qd = there ? to_float(norm_q[i]) : 0.0f, kd = there ? to_float(norm_k[i]) : 0.0f;
-    qq = fmaf(qd, qd, qq);
-    kk = fmaf(kd, kd, kk);
-    qk = fmaf(qd, kd, qk);
-  }
-  qk = warp_sum(qk);
-  if (LOOKS) {
-    const float q_unit = rsqrtf(warp_sum(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(warp_sum(kk) + 1e-6f);
-#pragma unroll
-    for (int i = 0; i < kWalkPer; ++i) {
-      q[i] *= q_unit;
-      k[i] *= k_unit;
-    }
-    qk = qk * q_unit * k_unit;
-  }
-  // over the lanes of a column: neighbours first where the column is looked at, the dual in the order of its exchanges
-  auto over_lanes = [](float v) {
-#pragma unroll
-    for (int step = 1; step < LANES; step <<= 1) v += __shfl_xor_sync(0xffffffffu, v, LOOKS ? step : LANES / 2 / step);
-    return v;
-  };
-  if (MODE == kWalkChannel) {
-#pragma unroll
-    for (int i = 0; i < kWalkPer; ++i) g[i] = expf(-rate * walk_softplus(pre[MODE == kWalkChannel ? i : 0] + bias[MODE == kWalkChannel ? i : 0]));
-  } else {
-    const float step = walk_softplus(pre[0] + bias[0]), decay = expf(-rate * step);
-    if (!LOOKS) beta = step;
-#pragma unroll
-    for (int i = 0; i < kWalkPer; ++i) g[i] = decay;
-  }
-#pragma unroll
-  for (int c = 0; c < kWalkCols; ++c) {
-    float r[kWalkPer] = {s[c][0].x, s[c][0].y, s[c][0].z, s[c][0].w, s[c][1].x, s[c][1].y, s[c][1].z, s[c][1].w};
-    float k_dot = 0.0f, q_dot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kWalkPer; ++i) {
-      r[i] *= g[i];
-      k_dot = fmaf(k[i], r[i], k_dot);
-      q_dot = fmaf(q[i], r[i], q_dot);
-    }
-    if (LOOKS) k_dot = over_lanes(k_dot);
-    q_dot = over_lanes(q_dot);
-    const float v = to_float(raw_v[c]), u = beta * (LOOKS ? v - k_dot : v);
-    if (column + c < a.vdim) {
-      if (has) {
-        float4* to = reinterpret_cast<float4*>(home + static_cast<long long>(c) * a.dim);
-        to[0] = make_float4(fmaf(k[0], u, r[0]), fmaf(k[1], u, r[1]), fmaf(k[2], u, r[2]), fmaf(k[3], u, r[3]));
-        to[1] = make_float4(fmaf(k[4], u, r[4]), fmaf(k[5], u, r[5]), fmaf(k[6], u, r[6]), fmaf(k[7], u, r[7]));
+      for (int i = 0; i < PIECES; ++i) {
+        raw_q[i] = *reinterpret_cast<const Eight*>(x + a.q_off + group * a.dim + d0 + i * EACH);
+        raw_k[i] = *reinterpret_cast<const Eight*>(x + a.k_off + group * a.dim + d0 + i * EACH);
       }
-      float o = fmaf(qk, u, q_dot);
-      if (MODE == kWalkDual) o = fmaf(skip, v, o);
-      if (part == 0)
-        a.out[token * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim + column + c] = o;
+    T norm_q[NL], norm_k[NL];
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const int d = min(lane + 32 * i, a.dim - 1);
+      norm_q[i] = x[a.q_off + group * a.dim + d];
+      norm_k[i] = x[a.k_off + group * a.dim + d];
+    }
+    T raw_v[kWalkCols];
+#pragma unroll
+    for (int c = 0; c < kWalkCols; ++c) raw_v[c] = x[a.v_off + head * a.vdim + min(column + c, a.vdim - 1)];
+    float pre[MODE == kWalkChannel ? kWalkPer : 1], bias[MODE == kWalkChannel ? kWalkPer : 1];
+    if (MODE == kWalkChannel) {
+#pragma unroll
+      for (int i = 0; i < kWalkPer; ++i) {
+        pre[i] = has ? static_cast<const float*>(a.step_pre)[token * a.lds + head * a.dim + d0 + i] : 0.0f;
+        bias[i] = has ? a.step_bias[head * a.dim + d0 + i] : 0.0f;
+      }
+    } else {
+      pre[0] = to_float(static_cast<const T*>(a.step_pre)[token * a.lds + head]);
+      bias[0] = a.step_bias[head];
+    }
+    const float rate = a.rate[head], skip = MODE == kWalkDual ? a.skip[head] : 0.0f;
+    float beta = LOOKS ? sigmoid_of(to_float(static_cast<const T*>(a.beta_pre)[token * a.ldb + a.b_off + head])) : 0.0f;
+
+    float q[kWalkPer], k[kWalkPer], g[kWalkPer], qq = 0.0f, kk = 0.0f, qk = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kWalkPer; ++i) {
+      q[i] = to_float(raw_q[i / EACH].v[i % EACH]);
+      k[i] = to_float(raw_k[i / EACH].v[i % EACH]);
+    }
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const bool there = lane + 32 * i < a.dim;
+      const float qd = there ? to_float(norm_q[i]) : 0.0f, kd = there ? to_float(norm_k[i]) : 0.0f;
+      qq = fmaf(qd, qd, qq);
+      kk = fmaf(kd, kd, kk);
+      qk = fmaf(qd, kd, qk);
+    }
+    qk = warp_sum(qk);
+    if (LOOKS) {
+      const float q_unit = rsqrtf(warp_sum(qq) + 1e-6f) * rsqrtf(static_cast<float>(a.dim)), k_unit = rsqrtf(warp_sum(kk) + 1e-6f);
+#pragma unroll
+      for (int i = 0; i < kWalkPer; ++i) {
+        q[i] *= q_unit;
+        k[i] *= k_unit;
+      }
+      qk = qk * q_unit * k_unit;
+    }
+    // over the lanes of a column: neighbours first where the column is looked at, the dual in the order of its exchanges
+    auto over_lanes = [](float v) {
+#pragma unroll
+      for (int step = 1; step < LANES; step <<= 1) v += __shfl_xor_sync(0xffffffffu, v, LOOKS ? step : LANES / 2 / step);
+      return v;
+    };
+    if (MODE == kWalkChannel) {
+#pragma unroll
+      for (int i = 0; i < kWalkPer; ++i) g[i] = expf(-rate * walk_softplus(pre[MODE == kWalkChannel ? i : 0] + bias[MODE == kWalkChannel ? i : 0]));
+    } else {
+      const float step = walk_softplus(pre[0] + bias[0]), decay = expf(-rate * step);
+      if (!LOOKS) beta = step;
+#pragma unroll
+      for (int i = 0; i < kWalkPer; ++i) g[i] = decay;
+    }
+#pragma unroll
+    for (int c = 0; c < kWalkCols; ++c) {
+      float r[kWalkPer] = {s[c][0].x, s[c][0].y, s[c][0].z, s[c][0].w, s[c][1].x, s[c][1].y, s[c][1].z, s[c][1].w};
+      float k_dot = 0.0f, q_dot = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kWalkPer; ++i) {
+        r[i] *= g[i];
+        k_dot = fmaf(k[i], r[i], k_dot);
+        q_dot = fmaf(q[i], r[i], q_dot);
+      }
+      if (LOOKS) k_dot = over_lanes(k_dot);
+      q_dot = over_lanes(q_dot);
+      const float v = to_float(raw_v[c]), u = beta * (LOOKS ? v - k_dot : v);
+      if (column + c < a.vdim) {
+        s[c][0] = make_float4(fmaf(k[0], u, r[0]), fmaf(k[1], u, r[1]), fmaf(k[2], u, r[2]), fmaf(k[3], u, r[3]));
+        s[c][1] = make_float4(fmaf(k[4], u, r[4]), fmaf(k[5], u, r[5]), fmaf(k[6], u, r[6]), fmaf(k[7], u, r[7]));
+        if (has && last) {
+          float4* to = reinterpret_cast<float4*>(home + static_cast<long long>(c) * a.dim);
+          to[0] = s[c][0];
+          to[1] = s[c][1];
+        }
+        float o = fmaf(qk, u, q_dot);
+        if (MODE == kWalkDual) o = fmaf(skip, v, o);
+        if (part == 0)
+          a.out[token * (static_cast<long long>(a.heads) * a.vdim) + static_cast<long long>(head) * a.vdim + column + c] = o;
+      }
     }
   }
 }

@@ -532,13 +532,13 @@ def matrix_state_case(mode, dtype, heads, groups, dim, vdim, tokens):
                                                                      rng.uniform(0.5, 4.0, heads), rng.normal(size=heads)))
     start = dev(rng.normal(size=(2, heads, vdim, dim)))
 
-    def walk(portions):
+    def walk(portions, said=0):
         state, outs, at = start.clone(), [], 0
         for count in portions:
             outs.append(ops._matrix_state(mode, qkv[at:at + count], (0, groups * dim, 2 * groups * dim),
                                           None if mode == 2 else beta[at:at + count], step[at:at + count], bias, rate,
                                           skip if mode == 2 else None, state, dev([0], torch.int32), dev([count], torch.int32),
-                                          dev([1], torch.int32), heads, groups, dim, vdim, count))
+                                          dev([1], torch.int32), heads, groups, dim, vdim, said or count))
             at += count
         ops.check_status("cuda")
         return torch.cat(outs), state
@@ -577,6 +577,16 @@ def test_the_walk_takes_eight_tokens_at_a_time_where_that_was_measured_to_win(he
     from metallix_b200 import ops
     wanted = ops._fn("mxb_delta_prompt_scratch")(sum(lengths), len(lengths), max(lengths), 0, heads, 128, ops._CODES[torch.bfloat16])
     assert bool(wanted) == eight
+
+
+@gpu
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_rows_longer_than_said_are_walked_to_their_end(mode):
+    """``longest`` only chooses a kernel: the one for single tokens walks longer rows too."""
+    walk = matrix_state_case(mode, torch.bfloat16, 4, 2, 64, 70, 5)
+    out, state = walk([5])
+    again, carried = walk([5], said=1)
+    assert torch.equal(out, again) and torch.equal(state, carried)
 
 
 @gpu
