@@ -315,7 +315,9 @@ MXB_API int mxb_gemm_simple(void* c, int c_dtype, const void* a, const void* w, 
     const float *x = static_cast<const float*>(a), *weight = static_cast<const float*>(w);
     if (m <= kFewRows) {
       const int shared = kFewStages * (kFewColumns + m) * kFewPitch * 4;
-      cudaError_t e = cudaFuncSetAttribute(gemm_float_few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+      // The limit is the function's, not the launch's: always the most, so that another thread's launch still fits it.
+      constexpr int most = kFewStages * (kFewColumns + kFewRows) * kFewPitch * 4;
+      cudaError_t e = cudaFuncSetAttribute(gemm_float_few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
       if (e != cudaSuccess) return static_cast<int>(e);
       gemm_float_few_rows_kernel<<<ceil_div(n, kFewColumns), kFewThreads, shared, stream>>>(to, x, weight, m, n, k, lda, ldw, ldc);
       return static_cast<int>(cudaGetLastError());

@@ -984,6 +984,29 @@ def test_float32_products_have_one_order_of_additions(ops, m, n, k):
     assert float((out - ref).norm() / ref.norm()) < 1e-6
 
 
+def test_float32_products_of_two_threads(ops):
+    """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
+    import threading
+    w, failures = dev(np.ones((64, 512))), []
+
+    def work(rows):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x = dev(np.ones((rows, 512)))
+                for _ in range(4000):
+                    out = ops.gemm_simple(x, w)
+                assert bool((out == 512.0).all())
+        except Exception as error:     # for the thread that waits
+            failures.append(error)
+
+    threads = [threading.Thread(target=work, args=(rows,)) for rows in (1, 8, 1, 8)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures
+
+
 @pytest.mark.parametrize("backend", ["simple", "cublas", "auto", "tcgen05"])
 @pytest.mark.parametrize("m, n, k", [(1, 384, 96), (5, 200, 136), (64, 331, 80), (300, 448, 192),
                                      (129, 130, 72), (700, 1030, 520)])
