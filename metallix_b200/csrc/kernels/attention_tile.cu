@@ -319,7 +319,8 @@ static int launch_tile(TileArgs args, cudaStream_t stream) {
   const size_t shared = fixed + args.stages * stage;
   auto kernel = paged_attention_tile_kernel<T, G, VQ>;
   if (shared > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
+    // The limit is the function's, not the launch's: always the most, so that another thread's launch still fits it.
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTileSharedMost));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   kernel<<<static_cast<unsigned>(blocks), kTileThreads, shared, stream>>>(args);

@@ -326,6 +326,32 @@ def test_query_heads_that_share_a_block(ops, dtype, heads, kv_heads, head_dim, v
     assert float((outs[0].double() - want).abs().max()) < tol(dtype, 1e-5, 2e-2)
 
 
+def test_general_attention_of_two_threads(ops):
+    """Two host threads, one with heads of 128 values, one with heads of 68: the same form with different amounts of shared
+    memory, neither launch meeting the other's limit."""
+    import threading
+    failures = []
+
+    def work(head_dim):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                q, out = (torch.ones((1, 2, head_dim), device="cuda") for _ in range(2))
+                cache, table = torch.ones((1, 2, 2, 16, head_dim), device="cuda"), dev([[0]], torch.int32)
+                zero, one = dev([0], torch.int32), dev([1], torch.int32)
+                for _ in range(3000):
+                    ops.paged_attention_tile(q, cache, out, table, zero, zero, one, zero, 0.1)
+                assert bool((out == 1.0).all())
+        except Exception as error:     # for the thread that waits
+            failures.append(error)
+
+    threads = [threading.Thread(target=work, args=(head_dim,)) for head_dim in (128, 68, 128, 68)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_one_far_key_among_hundreds(ops, dtype):
     """Random keys would average a lost key away. Here one key matches the
