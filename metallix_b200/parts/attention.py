@@ -188,12 +188,14 @@ def attend_cached(q_heads: torch.Tensor, cache: CacheView, ctx: StepContext, *, 
     kernel. Returns (``[tokens, heads, head_dim]``, False); with ``project`` (the
     output projection, a ``Linear``) a step of few single tokens may come back
     as (float32 ``[heads, tokens, hidden]`` summands, True), merged and
-    projected by one kernel. ``key_width`` / ``value_width``: how many values of
-    a head's keys and values are in use (0: all), the others being zeros."""
+    projected by one kernel. ``split_decode`` and ``flash`` say which of the first
+    two the caller lets its requests take. ``key_width`` / ``value_width``: how many
+    values of a head's keys and values are in use (0: all), the others being zeros."""
     tokens, heads, head_dim = q_heads.shape
-    # Heads of 256 values have a prompt kernel for some page sizes only, and it reads a gate 16 bytes at a time.
-    if head_dim == 256 and split_decode and not gate_per_head and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0)):
-        flash = ops.flash_prefill_tcgen05_supported(head_dim, heads, cache.pool.shape[2], cache.pool.shape[3], q_heads.dtype)
+    if flash and head_dim == 256:
+        # Such heads have a prompt kernel for some page sizes only; it reads a gate 16 bytes at a time.
+        flash = (not gate_per_head and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0))
+                 and ops.flash_prefill_tcgen05_supported(head_dim, heads, cache.pool.shape[2], cache.pool.shape[3], q_heads.dtype))
     tiles = tiles_of(ctx)
     multi_tiles = tiles["multi_tiles"]
     split = tiles["decode_rows"] and split_decode
@@ -409,8 +411,9 @@ class GQAttention:
         self.fused = norms_fuse and eps_agree and position_fuses and self.value_dim == self.head_dim
         self.split_decode = not self.general_only and ops.decode_attention_supported(
             self.head_dim, self.num_heads, self.num_kv_heads, self.dtype)
-        self.flash = not self.general_only and ops.flash_prefill_supported(
-            self.head_dim, self.num_heads, self.num_kv_heads, self.dtype)
+        # heads of 256 values: attend_cached asks whether the kernel takes the cache's pages
+        self.flash = not self.general_only and (ops.flash_prefill_supported(
+            self.head_dim, self.num_heads, self.num_kv_heads, self.dtype) or (self.split_decode and self.head_dim == 256))
 
     def cache_need(self) -> CacheNeed:
         return CacheNeed(kind="kv_pages", kv_heads=self.num_kv_heads, head_dim=self.row_dim,

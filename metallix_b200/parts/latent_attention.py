@@ -128,7 +128,7 @@ class LatentAttention:
                 self.o = Linear(padded.view(hidden, H * hd), runtime)
             self.uk = self.uk_t = self.uv = None
             self.split_decode = ops.decode_attention_supported(hd, H, H, self.dtype)
-            self.flash = ops.flash_prefill_supported(hd, H, H, self.dtype)
+            self.flash = ops.flash_prefill_supported(hd, H, H, self.dtype) or (self.split_decode and hd == 256)
 
     def cache_need(self) -> CacheNeed:
         if self.per_head:

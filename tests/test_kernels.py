@@ -682,6 +682,40 @@ def test_flash_prefill_with_heads_of_256(ops, heads, kv_heads, page_tokens, key_
         ops.KEY_SHARES = None
 
 
+def attend_256(monkeypatch, ops, flash, scale, tokens=40):
+    """``attend_cached`` over one request's prompt with two heads of 256 values: (its output, the formulas' in 64 bits,
+    whether the prompt kernel ran)."""
+    from metallix_b200.config.spec import CacheNeed
+    from metallix_b200.parts import attention
+    from metallix_b200.parts.registry import CacheView, StepContext
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn((tokens, 2, 256), generator=gen, device="cuda").bfloat16() for _ in range(3))
+    pages, ran = -(-tokens // 16), []
+    pool = torch.zeros((pages, 2, 2, 16, 256), dtype=torch.bfloat16, device="cuda")
+    for plane, rows in ((0, k), (1, v)):
+        padded = torch.zeros((pages * 16, 2, 256), dtype=torch.bfloat16, device="cuda")
+        padded[:tokens] = rows
+        pool[:, plane] = padded.view(pages, 16, 2, 256).transpose(1, 2)
+    whole = ops.flash_prefill
+    monkeypatch.setattr(ops, "flash_prefill", lambda *args, **options: (ran.append(1), whole(*args, **options))[1])
+    zeros = torch.zeros(tokens, dtype=torch.int32, device="cuda")
+    ctx = StepContext(torch.device("cuda"), torch.bfloat16, tokens, 1, torch.arange(tokens, dtype=torch.int32, device="cuda"), zeros,
+                      zeros[:1], [0, tokens], [0])
+    view = CacheView(need=CacheNeed("kv_pages", kv_heads=2, head_dim=256), pool=pool,
+                     block_tables=torch.arange(pages, dtype=torch.int32, device="cuda")[None], write=False)
+    out, _ = attention.attend_cached(q, view, ctx, scale=scale, split_decode=True, flash=flash)
+    ops.check_status("cuda")
+    s = torch.einsum("thd,jhd->htj", q.double(), k.double()) * scale
+    s = s.masked_fill(~torch.ones((tokens, tokens), dtype=torch.bool, device="cuda").tril(), -float("inf"))
+    return out.double(), torch.einsum("htj,jhd->thd", torch.softmax(s, -1), v.double()), bool(ran)
+
+
+@pytest.mark.parametrize("flash", [True, False])
+def test_the_caller_says_whether_heads_of_256_take_the_prompt_kernel(ops, monkeypatch, flash):
+    out, want, ran = attend_256(monkeypatch, ops, flash, 1.0 / 16)
+    assert ran == flash and float((out - want).abs().max()) < 2e-2
+
+
 @pytest.mark.parametrize("kernel", FLASH_KERNELS)
 def test_flash_prefill_one_far_key_and_cuts(ops, kernel):
     heads, kv_heads, head_dim, total = 4, 2, 128, 700
