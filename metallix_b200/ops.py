@@ -1550,6 +1550,7 @@ def flash_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block
         tcgen05 = False   # its epilogue reads the gate 16 bytes at a time
     _need(tcgen05 or kernel != "tcgen05",
           f"the tcgen05 prompt kernel does not take head_dim {head_dim} with pages of {page_tokens} tokens")
+    _need(head_dim != 256 or scale > 0.0, "the prompt kernel for heads of 256 values takes positive scales")
     if tcgen05 and kernel != "mma":
         _need(q.is_contiguous() and cache.is_contiguous(), "q and cache must be contiguous")
         key_width, value_width = int(key_width) or head_dim, int(value_width) or head_dim

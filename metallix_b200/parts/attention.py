@@ -193,8 +193,9 @@ def attend_cached(q_heads: torch.Tensor, cache: CacheView, ctx: StepContext, *, 
     values of a head's keys and values are in use (0: all), the others being zeros."""
     tokens, heads, head_dim = q_heads.shape
     if flash and head_dim == 256:
-        # Such heads have a prompt kernel for some page sizes only; it reads a gate 16 bytes at a time.
-        flash = (not gate_per_head and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0))
+        # Such heads have a prompt kernel for some page sizes only; it reads a gate 16 bytes at a time and takes a row's
+        # maximum ahead of the scaling.
+        flash = (scale > 0.0 and not gate_per_head and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0))
                  and ops.flash_prefill_tcgen05_supported(head_dim, heads, cache.pool.shape[2], cache.pool.shape[3], q_heads.dtype))
     tiles = tiles_of(ctx)
     multi_tiles = tiles["multi_tiles"]

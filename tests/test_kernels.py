@@ -716,6 +716,13 @@ def test_the_caller_says_whether_heads_of_256_take_the_prompt_kernel(ops, monkey
     assert ran == flash and float((out - want).abs().max()) < 2e-2
 
 
+@pytest.mark.parametrize("scale", [0.0, -1.0 / 16])
+def test_heads_of_256_with_a_scale_that_is_not_positive(ops, monkeypatch, scale):
+    """The prompt kernel's running maximum wants a positive scale; such steps stay with the general kernel."""
+    out, want, ran = attend_256(monkeypatch, ops, True, scale)
+    assert not ran and float((out - want).abs().max()) < 2e-2
+
+
 @pytest.mark.parametrize("kernel", FLASH_KERNELS)
 def test_flash_prefill_one_far_key_and_cuts(ops, kernel):
     heads, kv_heads, head_dim, total = 4, 2, 128, 700
