@@ -1091,7 +1091,8 @@ static int launch_decode(const void* q, const void* cache, void* out, float* par
 }
 
 static int decode_resident_blocks = 444;   // blocks of the decode attention that fit the GPU at once (3 an SM); 0: always one block per tile
-static int decode_many_blocks = 2048;      // blocks of a step with more than half as many (token, key/value head) pairs
+static int decode_many_blocks = 2048;      // blocks of a step with more (token, key/value head) pairs, or half as many and long contexts
+constexpr int kLongSplits = 32;            // tiles from which on contexts are long (an engine's bound is less than twice its longest context)
 
 template <int HD>
 static int launch_decode_mma(const void* q, const void* cache, void* out, float* partial,
@@ -1131,17 +1132,19 @@ static int launch_decode_mma(const void* q, const void* cache, void* out, float*
     // without a new block's start-up per tile, so a pair of (token, key/value
     // head) gets as few blocks as still fill the GPU: as many as keep the
     // whole grid resident at once when the pairs are few, else a few rounds'
-    // worth (with one block a pair the longest context paces the launch: 31
-    // requests x 8 key/value heads up to 1,500 keys 52 us with one, 46 with six).
+    // worth. Where one block a pair is all that would be resident and the
+    // contexts reach beyond 4,000 keys, which one block then walks alone, a few
+    // rounds are better too (32 requests x 8 key/value heads, the longest of
+    // 3,000 keys, 67 -> 56 us; below that bound most blocks of a short context
+    // would start for nothing: up to 250 keys 12 -> 18 us).
     // Where that would leave a block fewer than two tiles (few pairs,
     // short contexts) one block per tile is as good and simpler.
     const int pairs = rows * kv_heads;
     int slots = 0;
     if (decode_resident_blocks > 0 && pairs > 0) {
-      const bool few = 2 * pairs <= decode_resident_blocks;
-      const int target = few ? decode_resident_blocks : decode_many_blocks;
+      const bool resident = 2 * pairs <= decode_resident_blocks || (pairs <= decode_resident_blocks && max_splits < kLongSplits);
+      const int target = resident ? decode_resident_blocks : decode_many_blocks;
       slots = target / pairs > 0 ? target / pairs : 1;
-      if (!few && 2 * slots > max_splits) slots = max_splits / 2;
     }
     if (slots > 0 && 2 * slots <= max_splits) {
       auto kernel = project.bias.table != nullptr ? paged_attention_decode_resident_kernel<HD, true>
@@ -1193,8 +1196,8 @@ MXB_API int mxb_paged_attention_split_keys() { return kSplitKeys; }
 
 // How many blocks of the bfloat16 decode attention the GPU holds at once (3
 // an SM with their 64 KB of keys and values), and how many blocks a step with
-// more than half as many (token, key/value head) pairs is cut into. 0: one block per
-// tile always.
+// more (token, key/value head) pairs than that, or with more than half as many and
+// contexts of up to 4,096 keys or more, is cut into. 0: one block per tile always.
 MXB_API int mxb_set_decode_resident_blocks(int blocks, int many) {
   if (blocks < 0 || many < blocks) return static_cast<int>(cudaErrorInvalidValue);
   decode_resident_blocks = blocks;

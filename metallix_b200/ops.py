@@ -1592,8 +1592,8 @@ def decode_split_keys() -> int:
 def set_decode_resident_blocks(blocks: int, many: int = 2048) -> None:
     """How many blocks of the bfloat16 decode attention the GPU holds at once
     (444: three on each of 148 SMs), and into how many blocks a step with more
-    than half as many (token, key/value head) pairs is cut (2,048, two tiles a
-    block at least). A pair gets that
+    (token, key/value head) pairs than that is cut, or with more than half as
+    many and contexts of 4,096 keys or more (2,048). A pair gets that
     many blocks divided by the number of pairs, each walking over its 128-key
     tiles; where a block would be left fewer than two tiles, and with
     ``blocks`` 0, every tile has a block of its own. For comparisons and tests."""

@@ -840,13 +840,13 @@ def test_split_key_decode_attention(ops, dtype, heads, kv_heads, head_dim, page_
             assert np.abs(out[r] - ref).max() < tol(dtype, 5e-6, 2e-2), (window, r, total)
 
 
-@pytest.mark.parametrize("resident", [0, 444, 120, 12])
+@pytest.mark.parametrize("resident", [0, 444, 120, 12, 30])
 @pytest.mark.parametrize("heads, kv_heads, head_dim, page_tokens", [(6, 2, 64, 8), (4, 2, 128, 16), (16, 2, 128, 128)])
 def test_decode_attention_with_blocks_that_walk_over_tiles(ops, resident, heads, kv_heads, head_dim, page_tokens):
     """The bfloat16 kernel with one block per 128-key tile (0) and with as many
     blocks per (token, key/value head) as keep the grid resident, each walking
-    over its tiles (18 blocks of one to two tiles, 5 blocks of up to seven, and
-    a step cut into more blocks than are resident):
+    over its tiles (18 blocks of one to two tiles, 5 blocks of up to seven,
+    and steps cut into more blocks than are resident, of more pairs than that or of long contexts):
     the same attention. Lengths around the edges of tiles and of a block's
     rounds; a far key that only one block sees; windows that move the first
     tile."""
@@ -866,7 +866,8 @@ def test_decode_attention_with_blocks_that_walk_over_tiles(ops, resident, heads,
     scale = head_dim ** -0.5
     full_q = [np.concatenate([np.zeros((n - 1, heads, head_dim)), q[r]]) for r, n in enumerate(totals)]
     try:
-        ops.set_decode_resident_blocks(resident, 48 if resident == 12 else 2048)   # 12: 24 pairs exceed it, 48 / 24 = 2 blocks each
+        # 24 pairs: 12 is fewer, 48 / 24 = 2 blocks each; 30 is less than twice as many, 96 / 24 = 4 blocks each
+        ops.set_decode_resident_blocks(resident, {12: 48, 30: 96}.get(resident, 2048))
         for window in (0, 200, 1500):
             out = run_decode_attention(ops, dtype, full_q, k, v, totals, page_tokens, scale, window=window, pad_rows=2)
             for r, total in enumerate(totals):
