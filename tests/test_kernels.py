@@ -255,31 +255,28 @@ def test_paged_attention_window(ops, dtype, window):
         cursor += queries
 
 
-@pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("heads, kv_heads, head_dim, value_dim, planes, options", [
-    (8, 2, 32, 32, 2, {}), (4, 1, 64, 64, 2, {"window": 21, "sink": 4}), (4, 1, 128, 128, 2, {"gate": "value"}),
-    (4, 1, 128, 120, 2, {"bias": 6, "gate": "value"}), (8, 2, 32, 32, 2, {"bias": 9, "softcap": 6.0}),
-    (4, 1, 50, 50, 2, {"chunk": 16, "keep": 3}), (6, 3, 104, 70, 2, {"softcap": 5.0, "gate": "head"}),
-    (2, 1, 256, 256, 2, {"sink": 2}), (4, 2, 192, 150, 1, {"window": 9}),
-    (4, 1, 576, 128, 1, {}), (4, 1, 560, 64, 1, {"sink": 4}), (4, 1, 568, 24, 1, {})])
-def test_query_heads_that_share_a_block(ops, dtype, heads, kv_heads, head_dim, value_dim, planes, options):
-    """Steps with so many tiles that two or four query heads share a block's keys, against the formulas in 64 bits and, bit
-    for bit, against launches of few tiles, where every head has a block of its own. Wide keys leave room for fewer heads."""
+def attention_case(dtype, heads, kv_heads, head_dim, value_dim, planes, lengths, options, key_width=0):
+    """Requests whose last tokens are the queries, their pages in any order, NaN where no request wrote, and what the formulas
+    give in 64 bits: (arguments of the attention kernels by name, want). ``options``: window, chunk,
+    keep, softcap, a sink per head, a bias of that many distances, a gate per value or head."""
     gen = torch.Generator(device="cuda").manual_seed(head_dim)
     normal = lambda *shape: torch.randn(shape, generator=gen, device="cuda").to(dtype)
-    lengths = [(100, 39), (37, 37), (65, 1)] + [(1 + n % 40, 1 + n % min(3, 1 + n % 40)) for n in range(620 // (heads // 2))]
     pages = [-(-total // 16) for total, _ in lengths]
     order = torch.randperm(sum(pages), generator=gen, device="cuda")
     cache = normal(sum(pages), planes, kv_heads, 16, head_dim)
-    tables = torch.full((len(lengths), max(pages)), -1, dtype=torch.int32, device="cuda")
     tokens = sum(count for _, count in lengths)
-    q, scale, used = normal(tokens, heads, head_dim), head_dim ** -0.5, 0
+    q, scale, used, begin = normal(tokens, heads, head_dim), head_dim ** -0.5, 0, 0
+    if key_width:     # the values that are not in use are zeros
+        q[..., key_width:] = 0.0
+        cache[:, 0, ..., key_width:] = 0.0
+    if planes == 2:
+        cache[:, 1, ..., value_dim:] = 0.0
+    tables = torch.full((len(lengths), max(pages)), -1, dtype=torch.int32, device="cuda")
     gate = {"value": normal(tokens, heads * value_dim), "head": normal(tokens, heads), None: None}[options.get("gate")]
     sink = normal(heads).float() if options.get("sink") else None
     bias = normal(heads, options["bias"]).float() if options.get("bias") else None
     window, chunk, keep, cap = (options.get(name, 0) for name in ("window", "chunk", "keep", "softcap"))
-    want = torch.empty((tokens, heads, value_dim), dtype=torch.float64, device="cuda")
-    request, start, length, positions, begin = [], [], [], [], 0
+    want, positions = torch.empty((tokens, heads, value_dim), dtype=torch.float64, device="cuda"), []
     for r, (total, count) in enumerate(lengths):
         mine = order[used:used + pages[r]]
         used += pages[r]
@@ -305,22 +302,42 @@ def test_query_heads_that_share_a_block(ops, dtype, heads, kv_heads, head_dim, v
                     gate[begin:begin + count, head * value_dim:(head + 1) * value_dim]
                 out = out * torch.sigmoid(part.double())
             want[begin:begin + count, head] = out
-        for first in range(0, count, 16):
-            request.append(r)
-            start.append(begin + first)
-            length.append(min(16, count - first))
         positions += range(total - count, total)
         begin += count
-    lists = [torch.tensor(x, dtype=torch.int32, device="cuda") for x in (request, start, length)]
-    positions = torch.tensor(positions, dtype=torch.int32, device="cuda")
-    assert len(request) * heads // min(4, heads // kv_heads) >= 296
-    outs = []
-    for size in (len(request), 290 // heads):
-        outs.append(torch.full((tokens, heads, value_dim), 9.0, dtype=dtype, device="cuda"))
-        for at in range(0, len(request), size):
-            ops.paged_attention_tile(q, cache, outs[-1], tables, *(x[at:at + size] for x in lists), positions, scale, window, chunk,
-                                     gate=gate, softcap=cap, gate_per_head=options.get("gate") == "head", sink=sink, bias=bias,
-                                     keep=keep)
+    arguments = dict(q=q, cache=cache, block_tables=tables, positions=torch.tensor(positions, dtype=torch.int32, device="cuda"),
+                     scale=scale, window=window, chunk=chunk, keep=keep, softcap=cap, gate=gate, sink=sink, bias=bias)
+    return arguments, want
+
+
+def query_tiles(lengths, size):
+    """(request, first token, tokens) of every tile of up to ``size`` query tokens, as three device lists."""
+    tiles, begin = [], 0
+    for r, (_, count) in enumerate(lengths):
+        tiles += [(r, begin + first, min(size, count - first)) for first in range(0, count, size)]
+        begin += count
+    return [torch.tensor(x, dtype=torch.int32, device="cuda") for x in zip(*tiles)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, kv_heads, head_dim, value_dim, planes, options", [
+    (8, 2, 32, 32, 2, {}), (4, 1, 64, 64, 2, {"window": 21, "sink": 4}), (4, 1, 128, 128, 2, {"gate": "value"}),
+    (4, 1, 128, 120, 2, {"bias": 6, "gate": "value"}), (8, 2, 32, 32, 2, {"bias": 9, "softcap": 6.0}),
+    (4, 1, 50, 50, 2, {"chunk": 16, "keep": 3}), (6, 3, 104, 70, 2, {"softcap": 5.0, "gate": "head"}),
+    (2, 1, 256, 256, 2, {"sink": 2}), (4, 2, 192, 150, 1, {"window": 9}),
+    (4, 1, 576, 128, 1, {}), (4, 1, 560, 64, 1, {"sink": 4}), (4, 1, 568, 24, 1, {})])
+def test_query_heads_that_share_a_block(ops, dtype, heads, kv_heads, head_dim, value_dim, planes, options):
+    """Steps with so many tiles that two or four query heads share a block's keys, against the formulas in 64 bits and, bit
+    for bit, against launches of few tiles, where every head has a block of its own. Wide keys leave room for fewer heads."""
+    lengths = [(100, 39), (37, 37), (65, 1)] + [(1 + n % 40, 1 + n % min(3, 1 + n % 40)) for n in range(620 // (heads // 2))]
+    given, want = attention_case(dtype, heads, kv_heads, head_dim, value_dim, planes, lengths, options)
+    lists, outs = query_tiles(lengths, 16), []
+    assert lists[0].numel() * heads // min(4, heads // kv_heads) >= 296
+    for size in (lists[0].numel(), 290 // heads):
+        outs.append(torch.full(want.shape, 9.0, dtype=dtype, device="cuda"))
+        for at in range(0, lists[0].numel(), size):
+            request, start, length = (x[at:at + size] for x in lists)
+            ops.paged_attention_tile(out=outs[-1], tile_request=request, tile_start=start, tile_length=length,
+                                     gate_per_head=options.get("gate") == "head", **given)
     ops.check_status("cuda")
     assert torch.equal(outs[0], outs[1])
     assert float((outs[0].double() - want).abs().max()) < tol(dtype, 1e-5, 2e-2)
@@ -680,6 +697,34 @@ def test_flash_prefill_with_heads_of_256(ops, heads, kv_heads, page_tokens, key_
                 cursor += queries
     finally:
         ops.KEY_SHARES = None
+
+
+@pytest.mark.parametrize("shares", [1, 3])
+@pytest.mark.parametrize("heads, kv_heads, key_width, value_width, options", [
+    (4, 2, 256, 256, {"gate": "value", "softcap": 5.0}), (4, 1, 192, 128, {"sink": 4}), (2, 2, 256, 130, {"bias": 40, "gate": "value"}),
+    (4, 4, 150, 100, {"bias": 300, "softcap": 8.0}), (2, 1, 192, 256, {"chunk": 48, "keep": 5, "sink": 2}),
+    (2, 2, 256, 128, {"window": 70, "keep": 20, "gate": "value", "sink": 2, "bias": 9})])
+def test_options_of_the_prompt_kernel_for_heads_of_256(ops, heads, kv_heads, key_width, value_width, options, shares):
+    """Each option against the formulas in 64 bits, one block a query tile and three that share its keys. An output is off by
+    its own rounding, at most 2^-9 of the power of two above it, and by 2^-17 of a weight times a value of some 4."""
+    lengths = [(200, 200), (130, 2), (65, 65), (500, 129), (3, 3), (700, 300)]
+    given, want = attention_case(torch.bfloat16, heads, kv_heads, 256, value_width, 2, lengths, options, key_width)
+    if given["gate"] is not None:      # a row of the gate is as wide as the heads
+        wide = torch.zeros((want.shape[0], heads, 256), dtype=torch.bfloat16, device="cuda")
+        wide[..., :value_width] = given["gate"].view(want.shape[0], heads, value_width)
+        given["gate"] = wide.view(want.shape[0], heads * 256)
+    request, start, length = query_tiles(lengths, 128)
+    out = torch.full_like(given["q"], float("nan"))
+    ops.KEY_SHARES = shares
+    try:
+        ops.flash_prefill(out=out, tile_request=request, tile_start=start, tile_length=length, kernel="tcgen05",
+                          key_width=key_width, value_width=value_width, **given)
+    finally:
+        ops.KEY_SHARES = None
+    ops.check_status("cuda")
+    bound = 2.0 ** (np.ceil(np.log2(float(want.abs().max()))) - 9) + 2e-4
+    assert float((out[..., :value_width].double() - want).abs().max()) < bound
+    assert not bool(out[..., value_width:].any())
 
 
 def attend_256(monkeypatch, ops, flash, scale, tokens=40):
