@@ -481,12 +481,25 @@ static ChunkScratch chunk_scratch(unsigned char* base, long long tokens, int row
 using namespace mxb;
 
 // How many KiB of scratch mxb_mlstm_chunks needs for a step of `tokens` tokens whose longest row brings `longest`; 0: the
-// step does not take this way. It does where a row brings 192 tokens, or 64 in a step of 512 or more: this way costs about
-// the same for a few chunks as for one (8 heads of 128 x 512, us, the walk of mlstm.cu first: one row of 64 tokens 46 and
-// 99, of 128 84 and 101, of 256 158 and 101; eight rows of 64 264 and 159; one of 64 beside 31 single tokens 260 and 323;
-// 8 heads of 64 x 128, one row of 512 tokens 207 and 77).
+// step does not take this way. It costs some 90 us, little for a chunk and as much for a row of one token as for a whole
+// chunk; mlstm.cu's walk costs 0.4 to 0.6 us per token of the longest row, or the whole step's work where that is more. So
+// it is taken where a row is long (a row of 256 tokens; of 192 where the step's work is much) and the rows beside it are few
+// for that, and where a step brings 512 tokens in rows of 32 and more and much work. us, the walk first, heads x dim x vdim:
+//   one row of 192 tokens      8 x 128 x 512  122 and 120   8 x 64 x 256   83 and  97   4 x 64 x 128   81 and  91
+//   of 256                                    159 and 122                 108 and  97                 105 and  93
+//   of 2,048                                1,205 and 450                 802 and 198                 787 and 108
+//   192, 63 single tokens                     587 and 654                 260 and 243                 113 and 149
+//   512, 127 single tokens                  1,306 and 1,248               584 and 417                 265 and 237
+//   512, 255 single tokens                  2,162 and 2,311               932 and 755                 348 and 456
+//   four rows of 128                          294 and 155                 109 and  98                  57 and  95
+//   sixteen of 128                          1,017 and 486                 365 and 204                 108 and 112
+//   eight of 64                               265 and 167                 110 and 104                  33 and  99
+//   four of 64, 300 single tokens           2,169 and 2,692               872 and 843                 222 and 509
 MXB_API int mxb_mlstm_chunks_scratch(long long tokens, int rows, int longest, int heads, int dim, int vdim) {
-  if (rows <= 0 || tokens <= 0 || longest < 64 || (longest < 192 && tokens < 512)) return 0;
+  const bool much = tokens * heads * dim * vdim > 1ll << 26;
+  const bool few_beside_long = (longest >= 256 || (longest >= 192 && much)) && 3ll * rows <= longest - 128;
+  const bool many = longest >= 64 && tokens >= 512 && tokens >= 32ll * rows && much;
+  if (rows <= 0 || tokens <= 0 || !(few_beside_long || many)) return 0;
   if (heads <= 0 || heads > 65535 || dim <= 0 || dim > 256 || vdim <= 0 || vdim > 65536) return 0;
   size_t bytes = 0;
   chunk_scratch(nullptr, tokens, rows, longest, heads, dim, vdim, &bytes);
