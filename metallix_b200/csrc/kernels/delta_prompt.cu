@@ -1,5 +1,5 @@
-// The delta rule with a decay per channel (delta_rule.cu states it) over portions of prompts in bfloat16, and the steps of single tokens
-// of all three recurrences there that keep a matrix per head.
+// The delta rule with a decay per channel (delta_rule.cu states it) over portions of prompts in bfloat16, and the steps of
+// single tokens of all three recurrences there that keep a matrix per head.
 //
 // A token by itself is a chain of dependent steps (decay, a dot with the key over the lanes that share a column, the
 // write), and delta_rule.cu pays that chain per token. Here eight tokens pay it once. With S the state ahead of eight
@@ -8,13 +8,14 @@
 //   o_t = (q_t G_t) . S + sum_(s <= t) P_ts u_s,                  P_ts = sum_d q_t k_s g_(s+1) ... g_t
 //   S <- G_8 S + sum_s (k_s g_(s+1) ... g_8) u_s^T
 // What does not depend on S or on the column, the three kinds of products with keys and queries, G_8, A and P, is made
-// first, a block per (eight tokens, head), in the order in which the lanes will read it. Then a block of four warps walks a head's 32 columns, four columns and eight channels a thread: all 16
-// dots with S at once, their sums over the lanes together, a small triangular solve per column, one update of S. A fifth
-// warp keeps the next eights on their way, one bulk copy each. Float32 throughout, as there.
-// Its sums run in another order than token by token, so
-// float32, whose results are the same however a prompt is cut, stays there. The walk is bound by its shared-memory reads and by what is left of the chain: 342 us for 1,777 tokens of 32 heads of 128
-// x 128 with a decay per channel, the records 73 us; delta_rule.cu took 917. Token by token with four columns a thread it
-// stayed at 480 to 530, whichever way the channels were shared out: the exchanges of every token were the chain.
+// first, a block per (eight tokens, head), in the order in which the lanes will read it. Then a block of four warps walks
+// a head's 32 columns, four columns and eight channels a thread: all 16 dots with S at once, their sums over the lanes
+// together, a small triangular solve per column, one update of S. A fifth warp keeps the next eights on their way, one bulk
+// copy each. Float32 throughout, as there. The sums run in another order than token by token, so a float32 step, whose
+// results are the same however a prompt is cut, stays there.
+// The walk is bound by its shared-memory reads and by what is left of the chain: 353 us with its records for 1,777 tokens
+// of 32 heads of 128 x 128; delta_rule.cu takes 919. Token by token with four columns a thread it stayed at 480 to 530,
+// whichever way the channels were shared out: the exchanges of every token were the chain.
 // One decay per head and the dual stay with delta_rule.cu over prompts too, although eight tokens at a time took 341 us there
 // for 725 (one row of 1,777 tokens, 32 heads), and the dual 314 for 853: their sums in another order moved the logits of a
 // decoder whose routers stand close to a tie behind them by up to 0.05 of their size, one token's row by 0.28.

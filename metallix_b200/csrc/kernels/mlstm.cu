@@ -12,9 +12,9 @@
 //
 // One block owns a slice of 32 value columns of one head of one request and
 // walks that request's tokens of the step in order, its slice of C in shared
-// memory; a decode step and a portion of a prompt are the same kernel, and a
-// position's output does not depend on how the tokens were cut into steps
-// (the state that is carried is exact). Each slice keeps n and m for itself
+// memory: a decode step or a few tokens. Longer portions take the chunks below
+// or those of mlstm_chunks.cu; the forms carry the same float32 state and agree
+// to float32's rounding. Each slice keeps n and m for itself
 // (they are a few values), so that no block reads what another one writes.
 // State of one slot: per head [C: D * V][n: slices * D][m: slices]. Key widths up to 256 run a form that
 // keeps C in registers and fetches a token ahead; wider ones the form with C in shared memory.

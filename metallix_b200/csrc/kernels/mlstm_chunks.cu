@@ -12,8 +12,8 @@
 //   3. pass     C <- e^(F_L + m0 - m_L) C + S over the chunks, value by value; S is replaced by the C ahead of its chunk.
 //   4. outputs  per chunk, head and 128 columns: [e^(F_t + m0 - m_t) q_t | P_t] times [C ; V], over the normaliser.
 // 2 and 4 are products of 64 x 128 tiles, 64 outputs a thread, and take nearly all the time: bound by the multiply-adds
-// and the shared-memory reads they need. 2,048 tokens, 8 heads of 128 x 512: 1,196 us in mlstm.cu, 398 here (outputs 206,
-// parts 117, pass 32).
+// and the shared-memory reads they need. 2,048 tokens, 8 heads of 128 x 512: 1,205 us in mlstm.cu, 450 here
+// (outputs 206, parts 117, pass 32 with a warm L2 and without the outputs' check for what is not finite, some 25).
 // What a window of chunks needs of scratch is bounded; longer steps go window by window, the state carried in its slot.
 #include <type_traits>
 

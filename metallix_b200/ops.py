@@ -917,10 +917,10 @@ def mlstm_scan(proj: torch.Tensor, offsets, i_bias: torch.Tensor, f_bias: torch.
     (float32 ``[slots, mlstm_state_values]``, advanced in place). Returns
     float32 ``[tokens, heads * vdim]``: each head's C^T q over its bounded
     normaliser, before the head norm. ``longest`` (the most tokens any row
-    brings, as the host knows it) chooses the form: steps of some hundred
-    tokens take all chunks of 64 tokens at once, from 8 tokens on a row's
-    chunks of 16 tokens follow one another, below that its tokens; the forms
-    agree to rounding."""
+    brings, as the host knows it) chooses the form with the numbers of rows and
+    tokens: long rows, or much work, take all chunks of 64 tokens at once, from 8
+    tokens on a row's chunks of 16 tokens follow one another, below that its
+    tokens; the forms agree to rounding."""
     _need(proj.is_cuda and proj.dtype in _CODES and proj.dim() == 2 and proj.stride(1) == 1,
           "proj must be a CUDA [tokens, columns] tensor with unit column stride")
     _check(state, "state", (torch.float32,), 2)

@@ -17,10 +17,11 @@ multiplied by a weight and by sigmoid(a Wg^T), and projected by Wo. The six
 projections are one product whose output stays float32, since the gates, the
 state and everything that meets them are float32 in both precisions.
 
-A step's tokens of one request are walked in order by one kernel, whether the
-step brings one token or a portion of a prompt; what is carried between steps
-is the exact state, so a position's output does not depend on how the prompt
-was cut.
+A step's tokens of one request are taken in order: token by token where the step
+brings few, in chunks of 16 one behind the other or of 64 side by side where it
+brings more (``ops.mlstm_scan``). What is carried between steps is the float32
+state of every form, so how a prompt was cut, and what else a step brought,
+moves a position's output by float32's rounding and no more.
 """
 from __future__ import annotations
 
