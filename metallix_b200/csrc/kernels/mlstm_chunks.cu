@@ -12,8 +12,7 @@
 //   3. pass     C <- e^(F_L + m0 - m_L) C + S over the chunks, value by value; S is replaced by the C ahead of its chunk.
 //   4. outputs  per chunk, head and 128 columns: [e^(F_t + m0 - m_t) q_t | P_t] times [C ; V], over the normaliser.
 // 2 and 4 are products of 64 x 128 tiles, 64 outputs a thread, and take nearly all the time: bound by the multiply-adds
-// and the shared-memory reads they need. 2,048 tokens, 8 heads of 128 x 512: 1,205 us in mlstm.cu, 450 here
-// (outputs 206, parts 117, pass 32 with a warm L2 and without the outputs' check for what is not finite, some 25).
+// and the shared-memory reads they need. 2,048 tokens, 8 heads of 128 x 512: 1,205 us in mlstm.cu, 348 here.
 // What a window of chunks needs of scratch is bounded; longer steps go window by window, the state carried in its slot.
 #include <type_traits>
 
@@ -177,48 +176,82 @@ mlstm_gates_kernel(ChunkArgs a) {
   for (int slice = threadIdx.x; slice < slices; slice += kGateWarps * 32) m_state[slice] = s_m0[kGateWarps];
 }
 
+// Four neighbours of a row of the projection's output, or of scratch; QUADS: they lie on a boundary that takes one load.
+template <bool QUADS>
+__device__ __forceinline__ float4 four_of(const float* p, int count) {
+  if (QUADS) return count > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  return make_float4(count > 0 ? p[0] : 0.0f, count > 1 ? p[1] : 0.0f, count > 2 ? p[2] : 0.0f, count > 3 ? p[3] : 0.0f);
+}
+template <bool QUADS>
+__device__ __forceinline__ float4 four_of(const __nv_bfloat16* p, int count) {
+  if (QUADS) {
+    if (count <= 0) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                       __uint_as_float(raw.y & 0xffff0000u));
+  }
+  return make_float4(count > 0 ? to_float(p[0]) : 0.0f, count > 1 ? to_float(p[1]) : 0.0f, count > 2 ? to_float(p[2]) : 0.0f,
+                     count > 3 ? to_float(p[3]) : 0.0f);
+}
+template <bool QUADS>
+__device__ __forceinline__ void put_four(float* to, int count, const float* four) {
+  if (QUADS) {
+    if (count > 0) *reinterpret_cast<float4*>(to) = make_float4(four[0], four[1], four[2], four[3]);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i < count) to[i] = four[i];
+}
+__device__ __forceinline__ float4 times(float4 x, float f) { return make_float4(f * x.x, f * x.y, f * x.z, f * x.w); }
+
 // acc[8][N] += sum over k < count of A[k][row] B[k][column]: a tile of 64 x 16 N outputs by 8 x 16 threads. load_a(k,
-// row) and load_b(k, column) give the operands (0 beyond what they have); A_ALONG_K: neighbouring k of A lie side by side
-// in memory (else neighbouring rows), B_ALONG_K likewise.
+// row) and load_b(k, column) give four neighbours of the operands (0 beyond what they have): of k from there on where
+// A_ALONG_K (B_ALONG_K), else of rows (columns). Loads of one value each took as long as the
+// multiply-adds: 2,048 tokens, 8 heads of 128 x 512, the whole recurrence 476 us, 348 with four a load.
 template <int N, bool A_ALONG_K, bool B_ALONG_K, typename LoadA, typename LoadB>
 __device__ __forceinline__ void tile_product(float (&acc)[8][N], float* shared, int count, LoadA load_a, LoadB load_b) {
   constexpr int BN = 16 * N, PITCH_A = kTokens + 4, PITCH_B = BN + 4;
-  constexpr int A_EACH = kTokens * kStep / kTileThreads, B_EACH = BN * kStep / kTileThreads;
+  constexpr int A_EACH = kTokens * kStep / 4 / kTileThreads, B_EACH = BN * kStep / 4 / kTileThreads;
   float* sA = shared;                          // [2][kStep][PITCH_A]
   float* sB = shared + 2 * kStep * PITCH_A;    // [2][kStep][PITCH_B]
   const int tid = threadIdx.x;
   const int ty = (tid >> 6) * 4 + ((tid >> 3) & 3), tx = ((tid >> 5) & 1) * 8 + (tid & 7);
-  float next_a[A_EACH], next_b[B_EACH];
+  float4 next_a[A_EACH], next_b[B_EACH];
   auto place = [](int e, int rows, bool along_k, int& k, int& row) {
-    k = along_k ? e % kStep : e / rows;
-    row = along_k ? e / kStep : e % rows;
+    k = along_k ? e % (kStep / 4) * 4 : e / (rows / 4);
+    row = along_k ? e / (kStep / 4) : e % (rows / 4) * 4;
   };
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int x = 0; x < A_EACH; ++x) {
       int k, row;
       place(tid + x * kTileThreads, kTokens, A_ALONG_K, k, row);
-      next_a[x] = k0 + k < count ? load_a(k0 + k, row) : 0.0f;
+      next_a[x] = k0 + k < count ? load_a(k0 + k, row) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 #pragma unroll
     for (int x = 0; x < B_EACH; ++x) {
       int k, row;
       place(tid + x * kTileThreads, BN, B_ALONG_K, k, row);
-      next_b[x] = k0 + k < count ? load_b(k0 + k, row) : 0.0f;
+      next_b[x] = k0 + k < count ? load_b(k0 + k, row) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+  };
+  auto put = [](float* at, int pitch, bool along_k, float4 four) {
+    if (along_k) at[0] = four.x, at[pitch] = four.y, at[2 * pitch] = four.z, at[3 * pitch] = four.w;
+    else *reinterpret_cast<float4*>(at) = four;
   };
   auto store = [&](int stage) {
 #pragma unroll
     for (int x = 0; x < A_EACH; ++x) {
       int k, row;
       place(tid + x * kTileThreads, kTokens, A_ALONG_K, k, row);
-      sA[(stage * kStep + k) * PITCH_A + row] = next_a[x];
+      put(sA + (stage * kStep + k) * PITCH_A + row, PITCH_A, A_ALONG_K, next_a[x]);
     }
 #pragma unroll
     for (int x = 0; x < B_EACH; ++x) {
       int k, row;
       place(tid + x * kTileThreads, BN, B_ALONG_K, k, row);
-      sB[(stage * kStep + k) * PITCH_B + row] = next_b[x];
+      put(sB + (stage * kStep + k) * PITCH_B + row, PITCH_B, B_ALONG_K, next_b[x]);
     }
   };
   const int stages = (count + kStep - 1) / kStep;
@@ -258,7 +291,7 @@ __device__ __forceinline__ int tile_column(int y) {
 }
 
 // Block (chunk of the window, head, piece): the pieces are S in tiles of 64 of its rows x 128 columns, then P.
-template <typename T>
+template <typename T, bool QUADS>
 __global__ void __launch_bounds__(kTileThreads, 3)
 mlstm_parts_kernel(ChunkArgs a, int from) {
   __shared__ __align__(16) float tiles[tile_shared<8>()];
@@ -286,17 +319,15 @@ mlstm_parts_kernel(ChunkArgs a, int from) {
     float acc[8][8] = {};
     tile_product<8, false, false>(
         acc, tiles, len,
-        [&](int s, int d) { return d0 + d < dim ? take[s] * to_float(x0[s * a.ld + a.k_off + head * dim + d0 + d]) : 0.0f; },
-        [&](int s, int v) { return v0 + v < vdim ? to_float(x0[s * a.ld + a.v_off + head * vdim + v0 + v]) : 0.0f; });
+        [&](int s, int d) { return times(four_of<QUADS>(x0 + s * a.ld + a.k_off + head * dim + d0 + d, dim - d0 - d), take[s]); },
+        [&](int s, int v) { return four_of<QUADS>(x0 + s * a.ld + a.v_off + head * vdim + v0 + v, vdim - v0 - v); });
     float* S = a.s.S + in_window * (static_cast<size_t>(dim) * vdim + dim);
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
       const int d = d0 + tile_row(x);
 #pragma unroll
-      for (int y = 0; y < 8; ++y) {
-        const int v = v0 + tile_column(y);
-        if (d < dim && v < vdim) S[static_cast<size_t>(d) * vdim + v] = acc[x][y];
-      }
+      for (int y = 0; y < 8; y += 4)
+        if (d < dim) put_four<QUADS>(S + static_cast<size_t>(d) * vdim + v0 + tile_column(y), vdim - v0 - tile_column(y), acc[x] + y);
     }
     if (v0 == 0 && threadIdx.x < kTokens && d0 + threadIdx.x < dim) {
       const int d = d0 + threadIdx.x;
@@ -309,8 +340,8 @@ mlstm_parts_kernel(ChunkArgs a, int from) {
   float acc[8][4] = {};   // rows s, columns t
   tile_product<4, true, true>(
       acc, tiles, dim,
-      [&](int d, int s) { return s < len ? to_float(x0[s * a.ld + a.k_off + head * dim + d]) : 0.0f; },
-      [&](int d, int t) { return t < len ? to_float(x0[t * a.ld + a.q_off + head * dim + d]) * a.q_scale : 0.0f; });
+      [&](int d, int s) { return four_of<QUADS>(x0 + s * a.ld + a.k_off + head * dim + d, s < len ? dim - d : 0); },
+      [&](int d, int t) { return times(four_of<QUADS>(x0 + t * a.ld + a.q_off + head * dim + d, t < len ? dim - d : 0), a.q_scale); });
   float* P = a.s.P + in_window * kTokens * kTokens;
   float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -382,7 +413,7 @@ mlstm_pass_kernel(ChunkArgs a, int from) {
   if (row >= 0) put(row, c);
 }
 
-template <typename T>
+template <typename T, bool QUADS>
 __global__ void __launch_bounds__(kTileThreads, 3)
 mlstm_outputs_kernel(ChunkArgs a, int from) {
   __shared__ __align__(16) float tiles[tile_shared<8>()];
@@ -413,9 +444,11 @@ mlstm_outputs_kernel(ChunkArgs a, int from) {
   bool finite = true;
   auto value = [&](int s, int v) { return v0 + v < vdim ? to_float(x0[s * a.ld + a.v_off + head * vdim + v0 + v]) : 0.0f; };
   float acc[8][8] = {};
-  tile_product<8, false, false>(acc, tiles, len, [&](int s, int t) { return P[s * kTokens + t]; }, [&](int s, int v) {
-    const float f = value(s, v);
-    finite = finite && fabsf(f) < INFINITY;
+  tile_product<8, false, false>(acc, tiles, len, [&](int s, int t) { return *reinterpret_cast<const float4*>(P + s * kTokens + t); },
+                                [&](int s, int v) {
+    const float4 f = four_of<QUADS>(x0 + s * a.ld + a.v_off + head * vdim + v0 + v, vdim - v0 - v);
+    finite = finite && fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))) < INFINITY && f.x == f.x && f.y == f.y &&
+             f.z == f.z && f.w == f.w;
     return f;
   });
   if (__syncthreads_or(!finite)) {   // 0 times what is not finite is no 0: a token takes only what is not behind it
@@ -431,17 +464,20 @@ mlstm_outputs_kernel(ChunkArgs a, int from) {
   }
   tile_product<8, true, false>(
       acc, tiles, dim,
-      [&](int d, int t) { return t < len ? decay[t] * (to_float(x0[t * a.ld + a.q_off + head * dim + d]) * a.q_scale) : 0.0f; },
-      [&](int d, int v) { return v0 + v < vdim ? C[static_cast<size_t>(d) * vdim + v0 + v] : 0.0f; });
+      [&](int d, int t) {
+        return times(times(four_of<QUADS>(x0 + t * a.ld + a.q_off + head * dim + d, t < len ? dim - d : 0), a.q_scale), decay[t]);
+      },
+      [&](int d, int v) { return four_of<QUADS>(C + static_cast<size_t>(d) * vdim + v0 + v, vdim - v0 - v); });
 #pragma unroll
   for (int x = 0; x < 8; ++x) {
     const int t = tile_row(x);
     if (t >= len) continue;
     float* out = a.out + (static_cast<long long>(first + t) * a.heads + head) * vdim;
 #pragma unroll
-    for (int y = 0; y < 8; ++y) {
+    for (int y = 0; y < 8; y += 4) {
       const int v = v0 + tile_column(y);
-      if (v < vdim) out[v] = acc[x][y] / below[t];
+      const float four[4] = {acc[x][y] / below[t], acc[x][y + 1] / below[t], acc[x][y + 2] / below[t], acc[x][y + 3] / below[t]};
+      put_four<QUADS>(out + v, vdim - v, four);
     }
   }
 }
@@ -520,17 +556,21 @@ MXB_API int mxb_mlstm_chunks(const void* proj, long long ld, int q_off, int k_of
                        num_slots, row_start, row_length, request_slots, out, rows, heads, dim, vdim, status,
                        chunk_scratch(static_cast<unsigned char*>(scratch), tokens, rows, longest, heads, dim, vdim, &bytes)};
   const int across = ceil_div(vdim, kColumns), pieces = across * ceil_div(dim, kTokens) + 1;
-  auto run = [&](auto type) {
+  auto run = [&](auto type, auto quads) {
     using T = decltype(type);
+    constexpr bool QUADS = decltype(quads)::value;
     mlstm_gates_kernel<T><<<dim3(rows, heads), kGateWarps * 32, 0, stream>>>(a);
     for (int from = 0; from < a.s.chunks; from += a.s.window) {
       const int here = a.s.chunks - from < a.s.window ? a.s.chunks - from : a.s.window;
-      mlstm_parts_kernel<T><<<dim3(here, heads, pieces), kTileThreads, 0, stream>>>(a, from);
+      mlstm_parts_kernel<T, QUADS><<<dim3(here, heads, pieces), kTileThreads, 0, stream>>>(a, from);
       mlstm_pass_kernel<<<dim3(ceil_div(dim * vdim + dim, 256), heads), 256, 0, stream>>>(a, from);
-      mlstm_outputs_kernel<T><<<dim3(here, heads, across), kTileThreads, 0, stream>>>(a, from);
+      mlstm_outputs_kernel<T, QUADS><<<dim3(here, heads, across), kTileThreads, 0, stream>>>(a, from);
     }
   };
-  if (dtype == kF32) run(float());
-  else run(__nv_bfloat16());
+  // Four values a load where every head's part of a row starts on such a boundary.
+  const bool quads = dim % 4 == 0 && vdim % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && ld % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(proj) & (dtype == kF32 ? 15 : 7)) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  if (dtype == kF32) quads ? run(float(), std::true_type()) : run(float(), std::false_type());
+  else quads ? run(__nv_bfloat16(), std::true_type()) : run(__nv_bfloat16(), std::false_type());
   return static_cast<int>(cudaGetLastError());
 }

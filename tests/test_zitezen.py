@@ -501,6 +501,25 @@ def test_all_chunks_at_once_where_that_was_measured_to_win(layout, lengths, chun
 
 
 @gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, dim, vdim", [(2, 64, 40), (1, 20, 132), (2, 18, 50)])
+def test_matrix_memory_reads_four_values_at_a_time_or_one(dtype, heads, dim, vdim):
+    """The same bits, state included, where the projection's rows start a value off the boundary that wide loads need."""
+    from metallix_b200 import ops
+    lengths, width, results = [300, 65, 1], heads * dim, []
+    given = torch.randn(sum(lengths), 2 * width + heads * vdim + 2 * heads, generator=torch.Generator().manual_seed(dim)).to(dtype).cuda()
+    at = (0, width, 2 * width, 2 * width + heads * vdim, 2 * width + heads * vdim + heads)
+    for shift in (0, 1):
+        wide = torch.zeros((given.shape[0], (given.shape[1] + 15) // 8 * 8), dtype=dtype, device="cuda")
+        proj = wide[:, shift:shift + given.shape[1]]
+        proj.copy_(given)
+        state, zeros = torch.zeros((3, ops.mlstm_state_values(heads, dim, vdim)), device="cuda"), torch.zeros(heads, device="cuda")
+        results.append((ops.mlstm_scan(proj, at, zeros, zeros + 3.0, 10.0, state, dev([0, 300, 365], torch.int32), dev(lengths, torch.int32),
+                                       dev([0, 1, 2], torch.int32), heads, dim, vdim, longest=300), state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@gpu
 def test_matrix_memory_keeps_later_values_out_of_earlier_outputs():
     from metallix_b200 import ops
     heads, dim, vdim, tokens, late = 2, 64, 40, 300, 150
