@@ -255,63 +255,68 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
   } else if (warp == 1) {
     // ---- one thread issues every MMA
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = tc_instruction_descriptor(kFaRows, kFaKeys);
-      constexpr uint32_t idesc_o = tc_instruction_descriptor_b_mn(kFaRows, HDV);
-      // This one thread is the block's pacemaker: what it does per key tile
-      // (three waits, sixteen MMAs, four commits) is kept short. The
-      // descriptors of the operands are made once; a stage or a step along k
-      // only adds to their address field (16-byte units, no carry: shared
-      // memory ends below 256 KiB).
-      const uint64_t q_desc = tc_smem_descriptor(shared_address(q_tile));
-      const uint64_t k_desc = tc_smem_descriptor(shared_address(k_tiles));
-      const uint64_t v_desc = tc_smem_descriptor_mn(shared_address(v_tiles), kFaHalfBytes);
-      bool ok = barrier_wait(q_full, 0, status);
-      auto scores = [&](int i) {  // S_i = Q K_i^T
-        const int stage = i % KS;
-        if (!barrier_wait(&k_full[stage], (i / KS) & 1, status)) return false;
-        tc_fence_after_sync();
-        const uint64_t k_stage = k_desc + static_cast<uint64_t>(stage) * (Config::kKeyBytes >> 4);
+    constexpr uint32_t idesc_s = tc_instruction_descriptor(kFaRows, kFaKeys);
+    constexpr uint32_t idesc_o = tc_instruction_descriptor_b_mn(kFaRows, HDV);
+    // This one thread is the block's pacemaker: what it does per key tile
+    // (three waits, sixteen MMAs, four commits) is kept short. The
+    // descriptors of the operands are made once; a stage or a step along k
+    // only adds to their address field (16-byte units, no carry: shared
+    // memory ends below 256 KiB).
+    const uint64_t q_desc = tc_smem_descriptor(shared_address(q_tile));
+    const uint64_t k_desc = tc_smem_descriptor(shared_address(k_tiles));
+    const uint64_t v_desc = tc_smem_descriptor_mn(shared_address(v_tiles), kFaHalfBytes);
+    int k_stage = 0, v_stage = 0;
+    uint32_t k_parity = 0, v_parity = 0;
+    bool ok = barrier_wait(q_full, 0, status);
+    auto scores = [&](int i) {  // S_i = Q K_i^T
+      if (!barrier_wait(&k_full[k_stage], k_parity, status)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        const uint64_t k_at = k_desc + k_stage * (Config::kKeyBytes >> 4);
         const uint32_t tmem_s = tmem_base + (i & 1) * Config::kScoreColumns;
 #pragma unroll
         for (int kk = 0; kk < HDK / 16; ++kk) {
-          const uint64_t offset = ((kk / 4) * kFaHalfBytes + (kk % 4) * 32) >> 4;
-          tc_mma(tmem_s, q_desc + offset, k_stage + offset, idesc_s, kk > 0 ? 1u : 0u);
+          constexpr int block = kFaHalfBytes >> 4;
+          tc_mma(tmem_s, q_desc + kk / 4 * block + kk % 4 * 2, k_at + kk / 4 * block + kk % 4 * 2, idesc_s, kk > 0 ? 1u : 0u);
         }
-        tc_commit(&k_empty[stage]);
         tc_commit(&s_full[i & 1]);
-        return true;
-      };
-      auto outputs = [&](int i) {  // O_tile_i = P_i V_i
-        const int stage = i % VS, buffer = i & 1;
-        if (!barrier_wait(&v_full[stage], (i / VS) & 1, status)) return false;
-        // The output buffer is free: every softmax thread took tile i - 2 out of
-        // it before it arrived for P of tile i - 1, let alone of tile i.
-        if (!barrier_wait(&p_full[buffer], (i >> 1) & 1, status)) return false;
-        tc_fence_after_sync();
-        const uint64_t v_stage = v_desc + static_cast<uint64_t>(stage) * (Config::kValueBytes >> 4);
+        tc_commit(&k_empty[k_stage]);
+      }
+      if (++k_stage == KS) k_stage = 0, k_parity ^= 1;
+      return true;
+    };
+    auto outputs = [&](int i) {  // O_tile_i = P_i V_i
+      const int buffer = i & 1;
+      if (!barrier_wait(&v_full[v_stage], v_parity, status)) return false;
+      // The output buffer is free: every softmax thread took tile i - 2 out of
+      // it before it arrived for P of tile i - 1, let alone of tile i.
+      if (!barrier_wait(&p_full[buffer], (i >> 1) & 1, status)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        const uint64_t v_at = v_desc + v_stage * (Config::kValueBytes >> 4);
         const uint32_t tmem_p = tmem_base + buffer * Config::kScoreColumns;
         const uint32_t tmem_o = tmem_base + Config::kOutputBase + buffer * HDV;
 #pragma unroll
         for (int kk = 0; kk < kFaKeys / 16; ++kk) {  // 16 keys per instruction: two 8-row groups of V, 8 columns of P
           // P of the keys' quarter q lies over the first half of that quarter's score columns.
-          tc_mma_ts(tmem_o, tmem_p + (kk / 2) * (kFaKeys / kFaParts) + (kk % 2) * 8, v_stage + kk * (2048 >> 4),
+          tc_mma_ts(tmem_o, tmem_p + (kk / 2) * (kFaKeys / kFaParts) + (kk % 2) * 8, v_at + kk * (2048 >> 4),
                     idesc_o, kk > 0 ? 1u : 0u);
           if constexpr (Config::kSplitWeights)   // what the rounding of P left lies over the quarter's second half
             tc_mma_ts(tmem_o, tmem_p + (kk / 2) * (kFaKeys / kFaParts) + kFaKeys / kFaParts / 2 + (kk % 2) * 8,
-                      v_stage + kk * (2048 >> 4), idesc_o, 1u);
+                      v_at + kk * (2048 >> 4), idesc_o, 1u);
         }
-        tc_commit(&v_empty[stage]);
         tc_commit(&o_full[buffer]);
-        return true;
-      };
-      ok = ok && (key_tiles == 0 || scores(0));
-      for (int i = 0; i < key_tiles && ok && !failed; ++i) {
-        if (i + 1 < key_tiles) ok = scores(i + 1);
-        ok = ok && outputs(i);
+        tc_commit(&v_empty[v_stage]);
       }
-      if (!ok) failed = 1;
+      if (++v_stage == VS) v_stage = 0, v_parity ^= 1;
+      return true;
+    };
+    ok = ok && (key_tiles == 0 || scores(0));
+    for (int i = 0; i < key_tiles && ok && !failed; ++i) {
+      if (i + 1 < key_tiles) ok = scores(i + 1);
+      ok = ok && outputs(i);
     }
+    if (!ok) failed = 1;
   } else {
     // ---- softmax and accumulation: four threads per query row. Warps w,
     // w + 4, w + 8 and w + 12 reach the same 32 lanes of tensor memory; each

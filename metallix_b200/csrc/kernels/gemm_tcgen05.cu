@@ -6,7 +6,8 @@
 //
 // One block computes one 128 x BN tile. Warp 0 feeds the pipeline (one lane
 // issues the TMA loads), warp 1 owns tensor memory and issues the MMAs, warps
-// 2..5 run the epilogue: plain store (bfloat16 or float32), or SwiGLU, where
+// 2..9 (two per 32 rows, 32 columns in turn; with four warps gelu's arithmetic
+// took longer than the products of 1,024 k) run the epilogue: plain store (bfloat16 or float32), or SwiGLU, where
 // the B tile is made of 128 gate rows and the 128 up rows of the same columns
 // and the block writes silu(gate) * up, so gate and up never reach memory
 // (the reference does this as two products and three element-wise passes,
@@ -14,17 +15,16 @@
 //
 // Every wait on a barrier is bounded: if it runs out, the status word gets a
 // bit, the block stops issuing work, frees its tensor memory and leaves.
-#include "tcgen05.cuh"
+#include "tc_epilogue.cuh"
 
 namespace mxb {
 
 constexpr int kTcM = 128;     // rows of a tile
 constexpr int kTcK = 64;      // k per stage: 64 bfloat16 = one 128-byte swizzle row
-constexpr int kTcThreads = 192;
-
-enum TcEpilogue : int { kTcStoreBf16 = 0, kTcStoreF32 = 1, kTcSwiGLU = 2, kTcReluSquared = 3, kTcGeGLU = 4, kTcClampedGLU = 5, kTcGelu = 6 };
-// the epilogues that take a tile of gate rows beside a tile of up rows: act(gate) * up (silu, or the tanh form of gelu), or the product of clamped halves
-__host__ __device__ constexpr bool tc_gated(int epilogue) { return epilogue == kTcSwiGLU || epilogue == kTcGeGLU || epilogue == kTcClampedGLU; }
+constexpr int kTcEpilogueWarps = 8;
+constexpr int kTcThreads = 64 + 32 * kTcEpilogueWarps;
+constexpr int kTcBand = 16;   // row tiles that meet all of W before the next ones do
+constexpr int kTcListed = 2048;   // row tiles of a grouped product whose bands fit the list in shared memory
 
 template <int BN, int STAGES_> struct TcConfig {
   static constexpr int kStageBytes = (kTcM + BN) * kTcK * 2;
@@ -38,8 +38,12 @@ template <int BN, int STAGES_> struct TcConfig {
 // The kernel is persistent: a block walks over tiles (tile, tile + gridDim.x,
 // ...), with two accumulators in tensor memory, so the epilogue of one tile
 // runs while the MMAs of the next fill the other accumulator and the TMA
-// loads run ahead of both. Tiles are numbered with the row tile fastest:
-// blocks working side by side share a tile of W.
+// loads run ahead of both. Tiles are numbered band by band: up to kTcBand row
+// tiles of one matrix, and within a band with the row tile fastest, so that
+// blocks working side by side share tiles of W and of A. With the row tiles of
+// all groups fastest the whole of A passed through L2 once per tile of W's
+// rows: 3,300 tokens, two of 12 experts and one shared, 6144 x 4096 with gelu
+// 537 us, 431 band by band; 4096 x 6144 661 and 492; 16 tokens 163 and 142.
 //
 // Grouped form (tile_group given): W holds several matrices of group_rows
 // rows each, one below the other, and row tile i of A is multiplied by matrix
@@ -63,12 +67,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __shared__ __align__(8) uint64_t accumulator_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
+  __shared__ uint16_t run_start[kTcListed], run_length[kTcListed];   // grouped: per row tile the first one of its run of one group; by that, how many
 
   unsigned char* tiles = tc_shared_raw + ((1024 - (shared_address(tc_shared_raw) & 1023)) & 1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (m + kTcM - 1) / kTcM;
   const int n_tiles = (n + OUT_COLUMNS - 1) / OUT_COLUMNS;
   const int total_tiles = m_tiles * n_tiles;
+  const bool by_group = tile_group != nullptr && m_tiles <= kTcListed;
   const int k_blocks = (k + kTcK - 1) / kTcK;
 
   if (threadIdx.x == 0) {
@@ -88,27 +94,56 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                  ::"r"(shared_address(&tmem_base_slot)), "r"(2 * BN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
+  if (warp == 2 && by_group) {
+    int carried = -1, carried_start = 0;   // of the 32 row tiles before: the last one's group, its run's beginning
+    for (int base = 0; base < m_tiles; base += 32) {
+      const int i = base + lane;
+      const int group = i < m_tiles ? tile_group[i] : -1;
+      int before = __shfl_up_sync(0xffffffffu, group, 1);
+      if (lane == 0) before = carried;
+      const uint32_t begins = __ballot_sync(0xffffffffu, group != before) & (0xffffffffu >> (31 - lane));
+      const int start = begins != 0 ? base + 31 - __clz(begins) : carried_start;
+      if (i < m_tiles) run_start[i] = static_cast<uint16_t>(start);
+      carried = __shfl_sync(0xffffffffu, group, 31);
+      carried_start = __shfl_sync(0xffffffffu, start, 31);
+    }
+    __syncwarp();
+    for (int i = lane; i < m_tiles; i += 32)
+      if (i + 1 == m_tiles || run_start[i + 1] != run_start[i]) run_length[run_start[i]] = static_cast<uint16_t>(i + 1 - run_start[i]);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem_base = tmem_base_slot;
+  // Row tile and tile of W's rows of a tile number.
+  auto place = [&](int tile, int& m_tile, int& n_tile) {
+    const int at = tile / n_tiles;   // some row tile of its band
+    const int run = by_group ? run_start[at] : 0, length = by_group ? run_length[run] : m_tiles;
+    const int bands = (length + kTcBand - 1) / kTcBand, per = (length + bands - 1) / bands;
+    const int band = (at - run) / per * per;
+    const int count = per < length - band ? per : length - band;
+    const int within = tile - (run + band) * n_tiles;
+    m_tile = run + band + within % count;
+    n_tile = within / count;
+  };
 
   if (warp == 0) {
     // ---- producer: TMA loads of the A and B tiles of every k block of every tile
-    if (lane == 0) {
-      int step = 0;  // k blocks issued so far, over all tiles
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-        const int m0 = (tile % m_tiles) * kTcM;
-        int n0 = (tile / m_tiles) * OUT_COLUMNS;
-        if (tile_group != nullptr) {
-          const int group = tile_group[tile % m_tiles];
-          if (group < 0) continue;
-          n0 += group * group_rows;   // the rows of this group's matrix
-        }
-        for (int kb = 0; kb < k_blocks; ++kb, ++step) {
-          const int stage = step % STAGES;
-          const uint32_t parity = (step / STAGES) & 1;
-          if (!barrier_wait(&empty_barrier[stage], parity ^ 1, status)) { failed = 1; break; }
+    int stage = 0;
+    uint32_t parity = 1;
+    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+      int m_tile, n_tile;
+      place(tile, m_tile, n_tile);
+      const int m0 = m_tile * kTcM;
+      int n0 = n_tile * OUT_COLUMNS;
+      if (tile_group != nullptr) {
+        const int group = tile_group[m_tile];
+        if (group < 0) continue;
+        n0 += group * group_rows;   // the rows of this group's matrix
+      }
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!barrier_wait(&empty_barrier[stage], parity, status)) { failed = 1; break; }
+        if (elect_one()) {
           unsigned char* a_tile = tiles + stage * Config::kStageBytes;
           unsigned char* b_tile = a_tile + kTcM * kTcK * 2;
           barrier_arrive_expect(&full_barrier[stage], Config::kStageBytes);
@@ -120,46 +155,49 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tma_load_2d(b_tile, &map_b, kb * kTcK, n0, &full_barrier[stage]);
           }
         }
+        if (++stage == STAGES) stage = 0, parity ^= 1;
       }
     }
   } else if (warp == 1) {
     // ---- one thread issues every MMA; completion frees the stage
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc_instruction_descriptor(kTcM, BN);
-      int step = 0, local = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-        if (tile_group != nullptr && tile_group[tile % m_tiles] < 0) continue;
-        const int buffer = local & 1;
-        // The epilogue must have drained this accumulator (two tiles ago).
-        if (!barrier_wait(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t tmem_d = tmem_base + buffer * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++step) {
-          const int stage = step % STAGES;
-          const uint32_t parity = (step / STAGES) & 1;
-          if (!barrier_wait(&full_barrier[stage], parity, status)) { failed = 1; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const uint32_t a_address = shared_address(tiles + stage * Config::kStageBytes);
-          const uint32_t b_address = a_address + kTcM * kTcK * 2;
+    constexpr uint32_t idesc = tc_instruction_descriptor(kTcM, BN);
+    const uint64_t a_desc = tc_smem_descriptor(shared_address(tiles));
+    int stage = 0, local = 0;
+    uint32_t parity = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+      int m_tile, n_tile;
+      place(tile, m_tile, n_tile);
+      if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
+      const int buffer = local & 1;
+      // The epilogue must have drained this accumulator (two tiles ago).
+      if (!barrier_wait(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
+      tc_fence_after_sync();
+      const uint32_t tmem_d = tmem_base + buffer * BN;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!barrier_wait(&full_barrier[stage], parity, status)) { failed = 1; break; }
+        tc_fence_after_sync();
+        if (elect_one()) {
+          const uint64_t a_stage = a_desc + stage * (Config::kStageBytes >> 4), b_stage = a_stage + (kTcM * kTcK * 2 >> 4);
 #pragma unroll
-          for (int kk = 0; kk < kTcK / 16; ++kk) {  // 16 k per instruction: 32 bytes further along the swizzled row
-            tc_mma(tmem_d, tc_smem_descriptor(a_address + kk * 32), tc_smem_descriptor(b_address + kk * 32),
-                   idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < kTcK / 16; ++kk)   // 16 k per instruction: 32 bytes further along the swizzled row
+            tc_mma(tmem_d, a_stage + kk * 2, b_stage + kk * 2, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&empty_barrier[stage]);
+          if (kb + 1 == k_blocks) tc_commit(&accumulator_full[buffer]);   // arrives when this tile's accumulator is final
         }
-        tc_commit(&accumulator_full[buffer]);  // arrives when this tile's accumulator is final
-        ++local;
+        if (++stage == STAGES) stage = 0, parity ^= 1;
       }
+      ++local;
     }
   } else {
     // ---- epilogue: warp w reads the 32 accumulator rows (lanes) (w % 4) * 32 ...
-    const int lane_base = (warp & 3) * 32;
+    const int lane_base = (warp & 3) * 32, half = (warp - 2) >> 2;
     int local = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-      if (tile_group != nullptr && tile_group[tile % m_tiles] < 0) continue;
+      int m_tile, n_tile;
+      place(tile, m_tile, n_tile);
+      if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
       const int buffer = local & 1;
-      const int m0 = (tile % m_tiles) * kTcM, n0 = (tile / m_tiles) * OUT_COLUMNS;
+      const int m0 = m_tile * kTcM, n0 = n_tile * OUT_COLUMNS;
       if (!barrier_wait(&accumulator_full[buffer], (local >> 1) & 1, status)) { failed = 1; break; }
       if (failed) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -167,65 +205,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const float scale = EPI == kTcGelu && row_scale != nullptr && row < m ? row_scale[row] : 1.0f;
       const uint32_t tmem_row = tmem_base + buffer * BN + (static_cast<uint32_t>(lane_base) << 16);
 #pragma unroll 1
-      for (int c = 0; c < OUT_COLUMNS; c += 32) {
-        uint32_t acc[32];
-        tc_load_32(tmem_row + c, acc);
-        float values[32];
-        if (tc_gated(EPI)) {
-          uint32_t up[32];
-          tc_load_32(tmem_row + BN / 2 + c, up);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            // gate and up take the rounding to bfloat16 they would get on their way through memory
-            const float gate = to_float(from_float<__nv_bfloat16>(__uint_as_float(acc[i])));
-            const float u = to_float(from_float<__nv_bfloat16>(__uint_as_float(up[i])));
-            values[i] = gated_product(gate, u, EPI == kTcGeGLU ? kActGeluTanh : (EPI == kTcClampedGLU ? kActClamped : kActSilu), limit);  // rounded to bfloat16 anyway
-          }
-        } else if (EPI == kTcReluSquared) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float u = fmaxf(__uint_as_float(acc[i]), 0.0f);
-            values[i] = u * u;
-          }
-        } else if (EPI == kTcGelu) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) values[i] = gelu_of(scale * __uint_as_float(acc[i]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) values[i] = __uint_as_float(acc[i]);
-        }
-        if (row < m) {
-          const int column = n0 + c;
-          if (EPI == kTcStoreF32) {
-            float* dst = static_cast<float*>(out) + static_cast<long long>(row) * ldo + column;
-            if (column + 32 <= n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 4)
-                *reinterpret_cast<float4*>(dst + i) = make_float4(values[i], values[i + 1], values[i + 2], values[i + 3]);
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (column + i < n) dst[i] = values[i];
-            }
-          } else {
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + static_cast<long long>(row) * ldo + column;
-            if (column + 32 <= n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                uint32_t packed[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  __nv_bfloat162 pair = __floats2bfloat162_rn(values[i + 2 * j], values[i + 2 * j + 1]);
-                  packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-                }
-                *reinterpret_cast<uint4*>(dst + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (column + i < n) dst[i] = from_float<__nv_bfloat16>(values[i]);
-            }
-          }
-        }
-      }
+      for (int c = half * 32; c < OUT_COLUMNS; c += 64)
+        tc_epilogue<EPI, 32>(tmem_row + c, tmem_row + BN / 2 + c, out, row, row < m, n0 + c, n, ldo, limit, scale);
       // This thread has read all it needs of the accumulator: hand it back.
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       barrier_arrive(&accumulator_empty[buffer]);

@@ -1,0 +1,75 @@
+// What the tcgen05 products do with finished columns of the accumulator, one thread per row.
+#pragma once
+
+#include "tcgen05.cuh"
+
+namespace mxb {
+
+enum TcEpilogue : int { kTcStoreBf16 = 0, kTcStoreF32 = 1, kTcSwiGLU = 2, kTcReluSquared = 3, kTcGeGLU = 4, kTcClampedGLU = 5, kTcGelu = 6 };
+// the epilogues that take a tile of gate rows beside a tile of up rows: act(gate) * up (silu, or the tanh form of gelu), or the product of clamped halves
+__host__ __device__ constexpr bool tc_gated(int epilogue) { return epilogue == kTcSwiGLU || epilogue == kTcGeGLU || epilogue == kTcClampedGLU; }
+
+// WIDE (16 or 32) columns of row `row` from `column` on, from tensor memory at `taddr` (a gated epilogue's up columns at
+// `taddr_up`) through the epilogue to `out`; columns from n on are left out, and the row altogether unless `stored`. All
+// lanes of a warp call it.
+template <int EPI, int WIDE>
+__device__ __forceinline__ void tc_epilogue(uint32_t taddr, uint32_t taddr_up, void* out, int row, bool stored, int column,
+                                            int n, long long ldo, float limit, float scale) {
+  uint32_t acc[WIDE];
+  tc_load(taddr, acc);
+  float values[WIDE];
+  if (tc_gated(EPI)) {
+    uint32_t up[WIDE];
+    tc_load(taddr_up, up);
+#pragma unroll
+    for (int i = 0; i < WIDE; ++i) {
+      // gate and up take the rounding to bfloat16 they would get on their way through memory
+      const float gate = to_float(from_float<__nv_bfloat16>(__uint_as_float(acc[i])));
+      const float u = to_float(from_float<__nv_bfloat16>(__uint_as_float(up[i])));
+      values[i] = gated_product(gate, u, EPI == kTcGeGLU ? kActGeluTanh : (EPI == kTcClampedGLU ? kActClamped : kActSilu), limit);  // rounded to bfloat16 anyway
+    }
+  } else if (EPI == kTcReluSquared) {
+#pragma unroll
+    for (int i = 0; i < WIDE; ++i) {
+      const float u = fmaxf(__uint_as_float(acc[i]), 0.0f);
+      values[i] = u * u;
+    }
+  } else if (EPI == kTcGelu) {
+#pragma unroll
+    for (int i = 0; i < WIDE; ++i) values[i] = gelu_of(scale * __uint_as_float(acc[i]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < WIDE; ++i) values[i] = __uint_as_float(acc[i]);
+  }
+  if (!stored) return;
+  if (EPI == kTcStoreF32) {
+    float* dst = static_cast<float*>(out) + static_cast<long long>(row) * ldo + column;
+    if (column + WIDE <= n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < WIDE; i += 4)
+        *reinterpret_cast<float4*>(dst + i) = make_float4(values[i], values[i + 1], values[i + 2], values[i + 3]);
+    } else {
+      for (int i = 0; i < WIDE; ++i)
+        if (column + i < n) dst[i] = values[i];
+    }
+  } else {
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + static_cast<long long>(row) * ldo + column;
+    if (column + WIDE <= n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < WIDE; i += 8) {
+        uint32_t packed[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          __nv_bfloat162 pair = __floats2bfloat162_rn(values[i + 2 * j], values[i + 2 * j + 1]);
+          packed[j] = *reinterpret_cast<uint32_t*>(&pair);
+        }
+        *reinterpret_cast<uint4*>(dst + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      }
+    } else {
+      for (int i = 0; i < WIDE; ++i)
+        if (column + i < n) dst[i] = from_float<__nv_bfloat16>(values[i]);
+    }
+  }
+}
+
+}  // namespace mxb

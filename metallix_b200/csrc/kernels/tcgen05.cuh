@@ -23,6 +23,23 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
                  "r"(x), "r"(y) : "memory");
 }
 
+// True in one lane of a warp that is there as a whole, the same one every time. Who issues TMA loads and MMAs is chosen with
+// it around a few instructions, inside loops that the whole warp walks: behind a branch on the lane number the compiler
+// moves every operand of an MMA through vector registers. A block of 64 k (wait, four MMAs, commit) took 660 cycles of the
+// issuing thread that way, whatever the tile's width, and 514 (N = 256, whose MMAs take 512) or 380 (N = 128) this way, with
+// descriptors made once to which a block only adds.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(chosen));
+  return chosen != 0;
+}
+
 // Shared-memory matrix descriptor of a K-major tile with the 128-byte swizzle:
 // rows of 128 bytes, groups of 8 rows 1024 bytes apart.
 __device__ __forceinline__ uint64_t tc_smem_descriptor(uint32_t address) {

@@ -1220,6 +1220,24 @@ def test_tcgen05_swiglu_epilogue(ops, m, inter, k):
     assert np.abs(out.cpu().double().numpy() - ref).max() < 3e-2 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("counts, n, k", [([300, 2181, 0, 1], 300, 72), ([4100], 520, 64), ([129] * 40, 40, 136)])
+def test_grouped_products_walk_bands_of_row_tiles(ops, counts, n, k):
+    """Runs of one tile, of several and of more than a band's, tiles left out between and behind them: each group's rows have
+    the bits of its own product."""
+    from metallix_b200 import tensor_core
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    tiles = [[e] * -(-count // 128) + [-1] * (e % 2) for e, count in enumerate(counts)]
+    a = torch.randn(128 * sum(map(len, tiles)), k, generator=gen, device="cuda").bfloat16()
+    w = torch.randn(len(counts) * n, k, generator=gen, device="cuda").bfloat16()
+    out = tensor_core.gemm_grouped(a, w, dev(sum(tiles, []), torch.int32), len(counts), tensor_core.STORE_F32)
+    begin = 0
+    for e, count in enumerate(counts):
+        if count:
+            assert torch.equal(out[begin:begin + count], tensor_core.gemm(a[begin:begin + count], w[e * n:(e + 1) * n], torch.float32))
+        begin += 128 * len(tiles[e])
+    ops.check_status("cuda")
+
+
 def test_tcgen05_refuses_what_it_cannot_take(ops):
     from metallix_b200 import tensor_core
     a, w = dev(np.zeros((4, 100)), torch.bfloat16), dev(np.zeros((8, 100)), torch.bfloat16)
