@@ -229,6 +229,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
 // ------------------------------------------------------------------ host side
 int g_tc_bn = 0, g_tc_deep = -1;  // tuning overrides: tile width, deep (1) or shallow (0) pipeline
+int g_tc_rows = -1;               // rows up to which the kernel for few rows is taken, -1: kTcFewRows
+static int tc_rows_limit() { return g_tc_rows < 0 ? kTcFewRows : g_tc_rows; }
 
 template <int BN, int EPI, int STAGES_>
 static int launch_tc_staged(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n, int k,
@@ -283,6 +285,9 @@ MXB_API int mxb_gemm_tcgen05(void* out, const void* a, const void* w, int m, int
   if (!mxb_gemm_tcgen05_supported(m, n, k, lda, ldw)) return static_cast<int>(cudaErrorInvalidValue);
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return static_cast<int>(cudaErrorInvalidValue);
   const int w_rows = tc_gated(epilogue) ? 2 * n : n;
+  if (epilogue == kTcReluSquared) return static_cast<int>(cudaErrorInvalidValue);   // of grouped products
+  if (g_tc_bn == 0 && m <= tc_rows_limit())
+    return launch_tc_rows({out, a, w, m, n, k, w_rows, lda, ldw, ldo, nullptr, 0, m, limit, nullptr, status}, epilogue, stream);
   // Narrow outputs take narrower tiles so that the grid still covers the GPU.
   const int m_tiles = (m + kTcM - 1) / kTcM;
   int bn = 256;
@@ -341,7 +346,7 @@ MXB_API int mxb_gemm_tcgen05(void* out, const void* a, const void* w, int m, int
 // [2 * n, k], its gate rows and then its up rows (group_rows = 2 n), and out is
 // bfloat16 silu(gate) * up; 6 bfloat16 gelu(row_scale[row] * c), row_scale being float32 [m] or null (1).
 MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, const int* tile_group, int m, int n,
-                                     int k, int groups, int group_rows, long long lda, long long ldw, long long ldo,
+                                     int k, int groups, int group_rows, int tile_rows, long long lda, long long ldw, long long ldo,
                                      int epilogue, const float* row_scale, int* status, cudaStream_t stream) {
   if (!mxb_gemm_tcgen05_supported(m, n, k, lda, ldw) || groups < 1 || n > group_rows || tile_group == nullptr)
     return static_cast<int>(cudaErrorInvalidValue);
@@ -349,6 +354,10 @@ MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, co
   const long long w_rows = static_cast<long long>(groups) * group_rows;
   if (w_rows > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   if (epilogue == kTcSwiGLU && group_rows != 2 * n) return static_cast<int>(cudaErrorInvalidValue);
+  if (tile_rows < 1 || tile_rows > kTcM) return static_cast<int>(cudaErrorInvalidValue);
+  if (tile_rows <= tc_rows_limit() && !(tc_gated(epilogue) && epilogue != kTcSwiGLU))
+    return launch_tc_rows({out, a, w, m, n, k, static_cast<int>(w_rows), lda, ldw, ldo, tile_group, group_rows, tile_rows, 0.0f, row_scale,
+                           status}, epilogue, stream);
   // a gated tile of width bn holds bn / 2 gate and bn / 2 up rows
   const int bn = epilogue == kTcSwiGLU ? (n > 64 ? 256 : (n > 32 ? 128 : 64)) : (n > 128 ? 256 : (n > 64 ? 128 : 64));
   CUtensorMap map_a, map_b;
@@ -370,6 +379,7 @@ MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, co
 
 // Tuning hook: force the tile width (64, 128, 256; 0 = choose) and the
 // pipeline depth (1 deep, 0 shallow, -1 = choose).
+MXB_API void mxb_gemm_tcgen05_tune_rows(int rows) { mxb::g_tc_rows = rows; }
 MXB_API void mxb_gemm_tcgen05_tune(int bn, int deep) {
   mxb::g_tc_bn = bn;
   mxb::g_tc_deep = deep;

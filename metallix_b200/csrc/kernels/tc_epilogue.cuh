@@ -72,4 +72,22 @@ __device__ __forceinline__ void tc_epilogue(uint32_t taddr, uint32_t taddr_up, v
   }
 }
 
+// A product's operands, as mxb_gemm_tcgen05 and its grouped form hand them on.
+struct TcProduct {
+  void* out;
+  const void* a;
+  const void* w;
+  int m, n, k, w_rows;
+  long long lda, ldw, ldo;
+  const int* tile_group;   // null: one matrix
+  int group_rows, tile_rows;
+  float limit;
+  const float* row_scale;
+  int* status;
+};
+
+// Products of few rows, bound by reading W (gemm_tcgen05_rows.cu).
+constexpr int kTcFewRows = 64;
+int launch_tc_rows(const TcProduct& p, int epilogue, cudaStream_t stream);
+
 }  // namespace mxb

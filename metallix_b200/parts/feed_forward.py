@@ -58,6 +58,11 @@ class SwiGLU:
             raise ValueError("the clamped activation needs a positive limit")
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
+        if self.gate_up.dtype == torch.bfloat16 and self.gate_up.backend == "auto" and ops.gemm_rows_takes(x, self.gate_up.weight, swiglu=True):
+            from .. import tensor_core
+            if tensor_core.supports(x, self.gate_up.weight, torch.bfloat16):
+                # A decode step of wide layers: gate, up and the activation in one pass over the weights on the tensor cores.
+                return self.down.forward(tensor_core.gemm_swiglu(x, self.gate_up.weight, activation=self.activation, limit=self.limit))
         few = ops.SKINNY_ROWS if x.shape[1] <= ops.STREAM_K else ops.SKINNY_ROWS // 2   # as ops.gemm_bf16
         if (x.shape[0] <= few and self.gate_up.backend in ("auto", "skinny")
                 and ops.gemm_skinny_takes(x, self.gate_up.weight, swiglu=True)):
@@ -239,9 +244,10 @@ class RoutedExperts:
             else:
                 gathered = ops.expert_gather_rows(x, position, rows)
             epilogue = {"swiglu": tensor_core.SWIGLU, "gelu": tensor_core.GELU, "relu_squared": tensor_core.RELU_SQUARED}
+            used = min(128, x.shape[0])     # of a tile's rows: a token takes an expert once
             act = tensor_core.gemm_grouped(gathered, self.up.weight, tile_group, self.stacked, epilogue[self.activation],
-                                           row_scale=row_scale)
-            out = tensor_core.gemm_grouped(act, self.down.weight, tile_group, self.stacked, tensor_core.STORE_F32)
+                                           row_scale=row_scale, tile_rows=used)
+            out = tensor_core.gemm_grouped(act, self.down.weight, tile_group, self.stacked, tensor_core.STORE_F32, tile_rows=used)
             return ops.expert_combine_rows(out, position, None if self.weigh_input else weights, on_identity, x)
         return ops.experts_routed(x, self.up.weight, self.down.weight, chosen, weights, self.stacked,
                                   self.intermediate_size, activation=self.activation, weigh_input=self.weigh_input)

@@ -78,7 +78,7 @@ def gemm_gelu(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 
 def gemm_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, groups: int, epilogue: int,
-                 row_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 row_scale: Optional[torch.Tensor] = None, tile_rows: int = 128) -> torch.Tensor:
     """Row tile i of a ``[m, k]`` (128 rows a tile, m a whole number of them)
     times matrix tile_group[i] of w ``[groups * n, k]`` transposed; tiles with a
     negative entry are left out, and their rows of the result are not written.
@@ -86,12 +86,15 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, gro
     (bfloat16 gelu(row_scale[row] c) in its exact form, ``row_scale`` float32
     ``[m]`` or None for 1) or
     SWIGLU (every matrix of w holds its gate rows and then as many up rows;
-    the result is bfloat16 silu(gate) * up, half as wide as a matrix has rows)."""
+    the result is bfloat16 silu(gate) * up, half as wide as a matrix has rows).
+    ``tile_rows``: how many rows of a tile are in use, from its first one on;
+    what the result has in the others is not to be read."""
     reason = why_not(a, w, torch.bfloat16)
     if reason:
         raise ops.KernelError("the tcgen05 kernel does not take this call: " + reason)
     ops._need(w.shape[0] % groups == 0 and a.shape[0] % 128 == 0 and tile_group.dtype == torch.int32
               and tile_group.numel() >= a.shape[0] // 128, "the groups do not fit")
+    ops._need(1 <= tile_rows <= 128, "a tile has 1 to 128 rows in use")
     m, group_rows = a.shape[0], w.shape[0] // groups
     ops._need(epilogue != SWIGLU or group_rows % 2 == 0, "gate and up rows must pair up")
     if row_scale is not None:
@@ -100,6 +103,6 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, gro
     n = group_rows // 2 if epilogue == SWIGLU else group_rows
     out = torch.empty((m, n), dtype=torch.float32 if epilogue == STORE_F32 else torch.bfloat16, device=a.device)
     ops._call("mxb_gemm_tcgen05_grouped", out.data_ptr(), a.data_ptr(), w.data_ptr(), tile_group.data_ptr(), m, n,
-              a.shape[1], groups, group_rows, a.stride(0), w.stride(0), out.stride(0), epilogue,
+              a.shape[1], groups, group_rows, int(tile_rows), a.stride(0), w.stride(0), out.stride(0), epilogue,
               ops._ptr(row_scale), ops.status_word(a.device).data_ptr(), ops._stream())
     return out

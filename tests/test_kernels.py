@@ -1238,6 +1238,35 @@ def test_grouped_products_walk_bands_of_row_tiles(ops, counts, n, k):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1, 8), (7, 300, 72), (8, 4096, 264), (33, 520, 136), (64, 40000, 128), (64, 130, 2000)])
+def test_products_of_few_rows_on_the_tensor_cores(ops, m, n, k):
+    """Every width of tile, one round of blocks and several: a row's bits are those it has among 130."""
+    from metallix_b200 import tensor_core
+    rng = np.random.default_rng(m + n)
+    a, w = dev(rng.normal(size=(130, k)), torch.bfloat16), dev(rng.normal(size=(2 * n, k)) * k ** -0.5, torch.bfloat16)
+    for call in (lambda x: tensor_core.gemm(x, w[:n]), lambda x: tensor_core.gemm(x, w[:n], torch.float32), lambda x: tensor_core.gemm_gelu(x, w[:n]),
+                 lambda x: tensor_core.gemm_swiglu(x, w), lambda x: tensor_core.gemm_swiglu(x, w, activation="clamped", limit=1.0)):
+        assert torch.equal(call(a[:m]), call(a)[:m])
+    ops.check_status("cuda")
+
+
+@pytest.mark.parametrize("counts, n, k", [([3, 0, 1, 64, 1, 29], 512, 128), ([7] * 13, 40, 256), ([0, 5, 0], 300, 72)])
+def test_few_rows_of_many_experts(ops, counts, n, k):
+    """Tiles of which some rows are in use, the others not even loaded: the bits of the product that takes all of them."""
+    from metallix_b200 import tensor_core
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    groups, used = len(counts), [i for i, count in enumerate(counts) if count]
+    rows = torch.cat([torch.arange(counts[e]) + 128 * i for i, e in enumerate(used)]).cuda()
+    a = torch.full((128 * (len(used) + 2), k), float("nan"), dtype=torch.bfloat16, device="cuda")
+    a[rows] = torch.randn(rows.numel(), k, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(groups * 2 * n, k, generator=gen, device="cuda") * k ** -0.5).bfloat16()
+    tiles = dev(used + [-1, -1], torch.int32)
+    for epilogue in (tensor_core.STORE_BF16, tensor_core.STORE_F32, tensor_core.SWIGLU, tensor_core.RELU_SQUARED, tensor_core.GELU):
+        few = tensor_core.gemm_grouped(a, w, tiles, groups, epilogue, tile_rows=max(counts))
+        assert torch.equal(few[rows], tensor_core.gemm_grouped(a, w, tiles, groups, epilogue)[rows])
+    ops.check_status("cuda")
+
+
 def test_tcgen05_refuses_what_it_cannot_take(ops):
     from metallix_b200 import tensor_core
     a, w = dev(np.zeros((4, 100)), torch.bfloat16), dev(np.zeros((8, 100)), torch.bfloat16)
