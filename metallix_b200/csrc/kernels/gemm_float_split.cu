@@ -1,0 +1,331 @@
+// C[M, N] = A[M, K] * W[N, K]^T of float32 operands on the fifth-generation tensor cores, with float32's precision.
+//
+// A float32 number is the sum of three bfloat16 numbers, x = x1 + x2 + x3, each the rounding of what the ones before
+// left: 8 bits each, 24 together. Of the nine products of two such numbers six are made: x1 y1, x1 y2, x2 y1, x2 y2, x1 y3
+// and x3 y1; what is left out is at most 2^-24 of |x y|, and 2^-27 on average. Products of bfloat16 are exact; what
+// limits the result is how they are added up. The tensor core cuts sums off where it aligns them, so x1 y1 is summed
+// over 64 k at a time and these sums are added up in registers, rounded to nearest; the five small products have an
+// accumulator of their own, whose errors are 2^-8 of the large one's. Against 64 bits the result is closer than a
+// float32 sum in ascending k: 1.0e-7 and 5.7e-7 at k = 1,024, 1.2e-7 and 9.9e-7 at 3,072 (normal numbers; positive ones 1.0e-7 and 4.9e-7).
+//
+// What bounds it: the tensor core, 6 x 64 cycles per 16 k of a 128 x 128 tile. The operands are read as float32 and
+// split by eight warps (5.5 instructions a value) on their way to shared memory: no pass over W beforehand and no room for
+// it. 917 rows (us, against the CUDA cores' kernel): 4096 x 1024 72 and 212, 6144 x 1024 109 and 261, 1024 x 2048 45 and 129, 1024 x
+// 3072 63 and 188: 106 TFLOP/s of float32, 640 of the tensor core's. Without the splitters' arithmetic it took 50 us for the
+// first of these, without their loads 55: a load has one step to arrive in, and they are volatile because the compiler moved
+// them down to their use (100 us).
+//
+// A number that is not finite, or too near the largest, has no such parts (infinity minus infinity), and leaves an output that is
+// not finite: such outputs are made again by one thread each, in float32 and ascending k, as the general product makes them.
+//
+// Every wait on a barrier is bounded: if it runs out, the status word gets a bit and the block stops, frees its tensor
+// memory and leaves.
+#include <cfloat>
+
+#include "tcgen05.cuh"
+
+namespace mxb {
+
+constexpr int kSplitTile = 128;          // rows of A and of W a tile
+constexpr int kSplitStep = 32;           // k that are handed over at once, half a 128-byte row of bfloat16
+constexpr int kSplitChunk = 64;          // k that the tensor core sums up
+constexpr int kSplitSlots = 4;           // steps in shared memory: two stages of 64 k, each in halves
+constexpr int kSplitPlaneBytes = kSplitTile * kSplitChunk * 2;
+constexpr int kSplitStageBytes = 6 * kSplitPlaneBytes;   // three parts of A, three of W
+constexpr int kSplitSharedBytes = 2 * kSplitStageBytes + 1024;
+constexpr int kSplitAdders = 8, kSplitSplitters = 8;     // warps
+constexpr int kSplitThreads = 32 * (4 + kSplitAdders + kSplitSplitters);   // warpgroups: one that issues, two and two
+constexpr int kSplitTmemColumns = 512;   // large sums twice, then small sums twice
+
+__device__ __forceinline__ float plain_dot(const float* __restrict__ a, const float* __restrict__ w, int k) {
+  float sum = 0.0f;
+  for (int i = 0; i < k; ++i) sum = fmaf(a[i], w[i], sum);
+  return sum;
+}
+
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= FLT_MAX; }
+
+// Two numbers' leading bfloat16 parts, packed; the numbers become what that left.
+__device__ __forceinline__ uint32_t split_pair(float& x, float& y) {
+  const __nv_bfloat162 pair = __floats2bfloat162_rn(x, y);
+  const uint32_t packed = *reinterpret_cast<const uint32_t*>(&pair);
+  x -= __uint_as_float(packed << 16);
+  y -= __uint_as_float(packed & 0xffff0000u);
+  return packed;
+}
+
+__global__ void __launch_bounds__(kSplitThreads, 1)
+gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w, int m, int n, int k,
+                        long long lda, long long ldw, long long ldc, int splits, float* __restrict__ scratch, int* status) {
+  extern __shared__ unsigned char split_shared_raw[];
+  __shared__ __align__(8) uint64_t step_full[kSplitSlots], step_empty[kSplitSlots];
+  __shared__ __align__(8) uint64_t large_full[2], large_empty[2], small_empty[2];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int failed_slot;
+  volatile int& failed = failed_slot;
+  unsigned char* stages = split_shared_raw + ((1024 - (shared_address(split_shared_raw) & 1023)) & 1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m_tiles = ceil_div(m, kSplitTile), n_tiles = ceil_div(n, kSplitTile);
+  const int chunks = ceil_div(k, kSplitChunk);
+  const int units = m_tiles * n_tiles * splits;   // (tile, part of k), the row tile fastest
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSplitSlots; ++s) {
+      barrier_init(&step_full[s], kSplitSplitters);
+      barrier_init(&step_empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      barrier_init(&large_full[b], 1);
+      barrier_init(&large_empty[b], kSplitAdders);
+      barrier_init(&small_empty[b], kSplitAdders);
+    }
+    barrier_init_fence();
+    failed = 0;
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                 ::"r"(shared_address(&tmem_base_slot)), "r"(kSplitTmemColumns) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+  auto first_chunk = [&](int split) { return static_cast<int>(static_cast<long long>(split) * chunks / splits); };
+
+  // 640 threads start with 96 registers each; the adders' 64 sums want more and the issuing warps need few.
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");
+    // ---- one thread issues every MMA
+    if (warp == 0) {
+      constexpr uint32_t idesc = tc_instruction_descriptor(kSplitTile, kSplitTile);
+      const uint64_t desc = tc_smem_descriptor(shared_address(stages));
+      int step = 0, chunk_count = 0, local = 0;
+      bool ok = true;
+      for (int unit = blockIdx.x; unit < units && ok && !failed; unit += gridDim.x, ++local) {
+        const int split = unit / m_tiles % splits;
+        const int begin = first_chunk(split), end = first_chunk(split + 1);
+        const uint32_t tmem_small = tmem_base + 2 * kSplitTile + (local & 1) * kSplitTile;
+        ok = barrier_wait(&small_empty[local & 1], ((local >> 1) & 1) ^ 1, status);
+        for (int chunk = begin; chunk < end && ok; ++chunk, ++chunk_count) {
+          const int buffer = chunk_count & 1;
+          ok = barrier_wait(&large_empty[buffer], ((chunk_count >> 1) & 1) ^ 1, status);
+          const uint32_t tmem_large = tmem_base + buffer * kSplitTile;
+#pragma unroll
+          for (int half = 0; half < 2; ++half, ++step) {
+            const int slot = step % kSplitSlots;
+            ok = ok && barrier_wait(&step_full[slot], (step / kSplitSlots) & 1, status);
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (elect_one()) {
+              const uint64_t at = desc + (((slot >> 1) * kSplitStageBytes + half * kSplitStep * 2) >> 4);
+              constexpr uint64_t plane = kSplitPlaneBytes >> 4;
+#pragma unroll
+              for (int kk = 0; kk < kSplitStep / 16; ++kk) {
+                const uint64_t x = at + kk * 2, y = x + 3 * plane;
+                tc_mma(tmem_small, x, y + 2 * plane, idesc, chunk > begin || half > 0 || kk > 0 ? 1u : 0u);
+                tc_mma(tmem_small, x + 2 * plane, y, idesc, 1u);
+                tc_mma(tmem_small, x + plane, y + plane, idesc, 1u);
+                tc_mma(tmem_small, x, y + plane, idesc, 1u);
+                tc_mma(tmem_small, x + plane, y, idesc, 1u);
+                tc_mma(tmem_large, x, y, idesc, half > 0 || kk > 0 ? 1u : 0u);
+              }
+              tc_commit(&step_empty[slot]);
+              if (half == 1) tc_commit(&large_full[buffer]);   // the last one of a tile covers its small sums too
+            }
+          }
+        }
+      }
+      if (!ok) failed = 1;
+    }
+  } else if (warp < 4 + kSplitAdders) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");   // 128 x 32 + 256 x 112 + 256 x 112 = 640 x 96 at most
+    // ---- adders: two warps per 32 rows, 64 columns each
+    const int lane_base = (warp & 3) * 32, columns = ((warp - 4) >> 2) * 64;
+    const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + columns;
+    int chunk_count = 0, local = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local) {
+      const int split = unit / m_tiles % splits;
+      const int begin = first_chunk(split), end = first_chunk(split + 1);
+      float acc[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
+      for (int chunk = begin; chunk < end; ++chunk, ++chunk_count) {
+        const int buffer = chunk_count & 1;
+        if (!barrier_wait(&large_full[buffer], (chunk_count >> 1) & 1, status) || failed) { ok = false; break; }
+        tc_fence_after_sync();
+#pragma unroll
+        for (int part = 0; part < 4; ++part) {
+          uint32_t sum[16];
+          tc_load_16(tmem_lane + buffer * kSplitTile + part * 16, sum);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(sum[i]);
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) barrier_arrive(&large_empty[buffer]);
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int part = 0; part < 4; ++part) {
+        uint32_t sum[16];
+        tc_load_16(tmem_lane + 2 * kSplitTile + (local & 1) * kSplitTile + part * 16, sum);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(sum[i]);
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) barrier_arrive(&small_empty[local & 1]);
+      const int row = unit % m_tiles * kSplitTile + lane_base + lane;
+      const int column = unit / m_tiles / splits * kSplitTile + columns;
+      if (row >= m) continue;
+      float* to = splits > 1 ? scratch + (static_cast<long long>(split) * m + row) * n + column : c + row * ldc + column;
+      if (column + 64 <= n && (reinterpret_cast<uintptr_t>(to) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (column + i < n) to[i] = acc[i];
+      }
+      if (splits == 1) {
+        float worst = 0.0f;   // stays finite, or becomes NaN
+#pragma unroll
+        for (int i = 0; i < 64; ++i) worst += 0.0f * acc[i];
+        if (worst != 0.0f)
+          for (int i = 0; i < 64 && column + i < n; ++i)
+            if (!is_finite(to[i])) to[i] = plain_dot(a + row * lda, w + (column + i) * ldw, k);
+      }
+    }
+    if (!ok) failed = 1;
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");
+    // ---- splitters: float32 from memory, a step ahead in registers, to three bfloat16 tiles each in shared memory
+    const int t = threadIdx.x - 32 * (4 + kSplitAdders);
+    // Eight lanes bring a row's 128 bytes. A half-warp's two rows are four apart, so that the swizzle puts their 64 bytes a
+    // part into different banks.
+    const int quad = t & 7, eight = t >> 3;
+    const int row_in = (eight & ~7) | ((eight & 1) << 2) | ((eight >> 1) & 3);   // of 32 rows a pass
+    float4 next[8];
+    const float* rows[8];   // of A and of W that this thread brings; rows behind the last one bring that one again
+    int unit = blockIdx.x, at = 0, last = 0;   // the step that is fetched next
+    auto open = [&]() {
+      const int split = unit / m_tiles % splits;
+      at = first_chunk(split) * 2, last = first_chunk(split + 1) * 2;
+      const int rows_a = unit % m_tiles * kSplitTile + row_in, rows_w = unit / m_tiles / splits * kSplitTile + row_in;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        rows[i] = a + min(rows_a + i * 32, m - 1) * lda;
+        rows[4 + i] = w + min(rows_w + i * 32, n - 1) * ldw;
+      }
+    };
+    auto fetch = [&](int i) {   // volatile: a load that the compiler moves down to its use is waited for there
+      const float* from = rows[i] + min(at * kSplitStep + quad * 4, k - 4);
+      float4 v;
+      asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(from));
+      return v;
+    };
+    bool more = unit < units;
+    if (more) {
+      open();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) next[i] = fetch(i);
+    }
+    int step = 0;
+    bool ok = true;
+    while (more && ok && !failed) {
+      const bool beyond = at * kSplitStep + quad * 4 >= k;   // what was fetched lies behind the end of k
+      if (++at == last) {
+        unit += gridDim.x;
+        more = unit < units;
+        if (more) open();
+      }
+      const int slot = step % kSplitSlots;
+      ok = barrier_wait(&step_empty[slot], ((step / kSplitSlots) & 1) ^ 1, status);
+      if (!ok) break;
+      unsigned char* stage = stages + (slot >> 1) * kSplitStageBytes;
+      const int piece = (slot & 1) * 4 + (quad >> 1);   // of 16 bytes in the row of 128
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float4 now = next[i];
+        if (more) next[i] = fetch(i);   // has this step's time to arrive
+        if (beyond) now = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const int row = (i & 3) * 32 + row_in;
+        unsigned char* to = stage + (i < 4 ? 0 : 3) * kSplitPlaneBytes + row * 128 + ((piece ^ (row & 7)) << 4) + (quad & 1) * 8;
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+          const uint32_t low = split_pair(now.x, now.y), high = split_pair(now.z, now.w);
+          *reinterpret_cast<uint2*>(to + part * kSplitPlaneBytes) = make_uint2(low, high);
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // before the tensor core reads them
+      __syncwarp();
+      if (lane == 0) barrier_arrive(&step_full[slot]);
+      ++step;
+    }
+    if (!ok) failed = 1;
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kSplitTmemColumns) : "memory");
+}
+
+// The parts of k, in order.
+__global__ void __launch_bounds__(256)
+gemm_float_parts_kernel(float* __restrict__ c, const float* __restrict__ scratch, const float* __restrict__ a,
+                        const float* __restrict__ w, int m, int n, int k, long long lda, long long ldw, long long ldc, int splits) {
+  const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x, all = static_cast<size_t>(m) * n;
+  if (i >= all) return;
+  float sum = scratch[i];
+  for (int s = 1; s < splits; ++s) sum += scratch[s * all + i];
+  const int row = static_cast<int>(i / n), column = static_cast<int>(i % n);
+  if (!is_finite(sum)) sum = plain_dot(a + row * lda, w + column * ldw, k);
+  c[row * ldc + column] = sum;
+}
+
+}  // namespace mxb
+
+using namespace mxb;
+
+// Into how many parts k is cut, so that few tiles still give every SM work: the fewest rounds of 148 blocks, each with a
+// start worth about two chunks and, with several parts, a pass that adds them up (worth about six).
+MXB_API int mxb_gemm_float_split_parts(int m, int n, int k) {
+  const long long tiles = static_cast<long long>(ceil_div(m, kSplitTile)) * ceil_div(n, kSplitTile);
+  const int chunks = ceil_div(k, kSplitChunk);
+  int best = 1;
+  long long least = 0;
+  for (int parts = 1; parts <= 8 && parts * 4 <= chunks; ++parts) {
+    const long long cost = (tiles * parts + 147) / 148 * (ceil_div(chunks, parts) + 2) + (parts > 1 ? 6 : 0);
+    if (parts == 1 || cost < least) least = cost, best = parts;
+  }
+  return best;
+}
+
+// c, a, w float32; k and the row strides of a and w multiples of 4, a and w on 16 bytes; scratch: parts * m * n float32 where
+// parts > 1.
+MXB_API int mxb_gemm_float_split(void* c, const void* a, const void* w, int m, int n, int k, long long lda, long long ldw,
+                                 long long ldc, int parts, float* scratch, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return 0;
+  if (k <= 0 || k % 4 != 0 || lda % 4 != 0 || ldw % 4 != 0 || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0 ||
+      parts < 1 || parts > ceil_div(k, kSplitChunk) || (parts > 1 && scratch == nullptr))
+    return static_cast<int>(cudaErrorInvalidValue);
+  const long long units = static_cast<long long>(ceil_div(m, kSplitTile)) * ceil_div(n, kSplitTile) * parts;
+  if (units > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
+  int device = 0, sms = 0;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaError_t e = cudaFuncSetAttribute(gemm_float_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSharedBytes);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  float* to = static_cast<float*>(c);
+  const float *x = static_cast<const float*>(a), *weight = static_cast<const float*>(w);
+  gemm_float_split_kernel<<<static_cast<int>(units < sms ? units : sms), kSplitThreads, kSplitSharedBytes, stream>>>(
+      to, x, weight, m, n, k, lda, ldw, ldc, parts, scratch, status);
+  e = cudaGetLastError();
+  if (e != cudaSuccess || parts == 1) return static_cast<int>(e);
+  const size_t all = static_cast<size_t>(m) * n;
+  gemm_float_parts_kernel<<<static_cast<unsigned>((all + 255) / 256), 256, 0, stream>>>(to, scratch, x, weight, m, n, k, lda, ldw, ldc, parts);
+  return static_cast<int>(cudaGetLastError());
+}

@@ -109,6 +109,8 @@ _SIGNATURES = {
     "mxb_flash_prefill_tcgen05_supported": [_I, _I, _I, _I, _I],
     "mxb_flash_prefill_tcgen05_tile": [],
     "mxb_gemm_simple": [_P, _I, _P, _P, _I, _I, _I, _I, _L, _L, _L, _P],
+    "mxb_gemm_float_split": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _P, _P, _P],
+    "mxb_gemm_float_split_parts": [_I, _I, _I],
     "mxb_gemm_skinny": [_P, _I, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _F, _P],
     "mxb_gemm_skinny_supported": [_I, _I, _I, _L, _L],
     "mxb_gemm_stream": [_P, _I, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _F, _P, _P],
@@ -1728,6 +1730,46 @@ def gemm_simple(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
     _call("mxb_gemm_simple", out.data_ptr(), _CODES[out_dtype], a.data_ptr(), w.data_ptr(),
           _CODES[a.dtype], m, n, k, a.stride(0), w.stride(0), out.stride(0), _stream())
     return out
+
+
+def gemm_float(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """a [m, k] times w [n, k] transposed of float32 operands on the tensor
+    cores: each number as three bfloat16 parts, sums of 64 products at a time
+    added up in float32 (closer to 64 bits than a float32 sum in ascending k)."""
+    _need(a.is_cuda and w.is_cuda, "operands must be on a CUDA device")
+    _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "shapes do not match a @ w.T")
+    _need(a.dtype == torch.float32 and w.dtype == torch.float32, "operands must be float32")
+    _need(gemm_float_supported(a, w), "k and the row strides must be multiples of 4, the operands on 16 bytes")
+    (m, k), n = a.shape, w.shape[0]
+    if out is None:
+        out = torch.empty((m, n), dtype=torch.float32, device=a.device)
+    _need(out.shape == (m, n) and out.dtype == torch.float32 and out.stride(1) == 1, "out does not fit")
+    parts = _fn("mxb_gemm_float_split_parts")(m, n, k)
+    scratch = torch.empty(parts * m * n, dtype=torch.float32, device=a.device) if parts > 1 else None
+    _call("mxb_gemm_float_split", out.data_ptr(), a.data_ptr(), w.data_ptr(), m, n, k, a.stride(0), w.stride(0),
+          out.stride(0), parts, _ptr(scratch), status_word(a.device).data_ptr(), _stream())
+    if parts > 1:
+        global _launches
+        _launches += 1   # the kernel that adds the parts up
+    return out
+
+
+# Rows of A from which float32 products of at least this many rows of W and values each go to the tensor cores, us against the
+# CUDA cores' kernels: 9 rows x 4096 x 1024 14.3 and 25.2, x 1024 x 2048 14.4 and 48.0, x 151936 x 1024 307 and 436; 917 rows 72 and
+# 212, 45 and 129; but 400 x 512 x 512 21 and 20, 256 x 1024 x 512 21 and 19.
+FLOAT_ROWS, FLOAT_SIDE = 9, 1024
+
+
+def gemm_float_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the tensor cores make this float32 product faster."""
+    return gemm_float_supported(a, w) and a.shape[0] >= FLOAT_ROWS and min(w.shape) >= FLOAT_SIDE
+
+
+def gemm_float_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the tensor-core product of float32 operands takes this call."""
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[0] > 0 and w.shape[0] > 0 and a.shape[1] > 0
+            and a.stride(1) == 1 and w.stride(1) == 1 and a.shape[1] % 4 == 0 and a.stride(0) % 4 == 0
+            and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 # Up to this many rows "auto" takes the weight-streaming kernel; beyond it every

@@ -412,6 +412,8 @@ class GQAttention:
         self.fused = norms_fuse and eps_agree and position_fuses and self.value_dim == self.head_dim
         self.split_decode = not self.general_only and ops.decode_attention_supported(
             self.head_dim, self.num_heads, self.num_kv_heads, self.dtype)
+        if self.split_decode and self.dtype == torch.float32:
+            runtime.ordered_sums = False
         # heads of 256 values: attend_cached asks whether the kernel takes the cache's pages
         self.flash = not self.general_only and (ops.flash_prefill_supported(
             self.head_dim, self.num_heads, self.num_kv_heads, self.dtype) or (self.split_decode and self.head_dim == 256))

@@ -43,6 +43,7 @@ class LinearHead:
             self.linear.out_features, self.linear.in_features = embedding.table.shape
             self.linear.dtype = runtime.dtype
             self.linear.backend = runtime.gemm_backend
+            self.linear.runtime = runtime
             weights.take(spec["weight"])
             self.tied = True
         else:

@@ -24,6 +24,7 @@ class Linear:
         self.out_features, self.in_features = self.weight.shape
         self.dtype = runtime.dtype
         self.backend = runtime.gemm_backend
+        self.runtime = runtime   # a part that is built later may change what it says of sums
 
     @classmethod
     def stacked(cls, weights: Sequence[torch.Tensor], runtime: Runtime) -> "Linear":
@@ -35,6 +36,8 @@ class Linear:
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
         out_dtype = out_dtype or self.dtype
         if self.dtype == torch.float32:
+            if not self.runtime.ordered_sums and ops.gemm_float_takes(x, self.weight):
+                return ops.gemm_float(x, self.weight, out=out)
             return ops.gemm_simple(x, self.weight, out_dtype=torch.float32, out=out)
         return ops.gemm_bf16(x, self.weight, out_dtype=out_dtype, backend=self.backend, out=out)
 

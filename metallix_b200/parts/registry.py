@@ -57,6 +57,9 @@ class Runtime:
     # Read-only tensors that parts built from equal parameters may share
     # (tables of a position encoding, say), by a key of those parameters.
     shared: Dict[tuple, object] = field(default_factory=dict)
+    # Whether float32 sums have one order however a step is cut, so that every cut gives the same bits. An attention whose
+    # single tokens and portions run on kernels of different orders says no; then large products may take the tensor cores.
+    ordered_sums: bool = True
 
 
 class WeightStore:

@@ -1097,6 +1097,21 @@ def test_float32_products_have_one_order_of_additions(ops, m, n, k):
     assert float((out - ref).norm() / ref.norm()) < 1e-6
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1, 4), (128, 128, 64), (129, 257, 100), (33, 77, 1028), (300, 1030, 2048), (200, 384, 3072)])
+def test_float32_products_on_the_tensor_cores(ops, m, n, k):
+    """Tiles with remainders, one part of k and several: no further from 64 bits than the sum in ascending k, and what is not
+    finite, or nearly not, where that has it too."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, w = (torch.randn(rows, k, generator=gen, device="cuda") for rows in (m, n))
+    out, plain_out, ref = ops.gemm_float(a, w), ops.gemm_simple(a, w), a.double() @ w.double().t()
+    ops.check_status("cuda")
+    assert float((out - ref).norm()) <= max(float((plain_out - ref).norm()), 2.0 ** -24 * float(ref.norm()))
+    a[m // 2, k - 1], w[n // 3, 0], a[0, k // 2] = float("inf"), float("nan"), 3.4e38
+    out, plain_out = ops.gemm_float(a, w), ops.gemm_simple(a, w)
+    odd = ~plain_out.isfinite()
+    assert torch.equal(odd, ~out.isfinite()) and torch.equal(out[odd].nan_to_num(1.0), plain_out[odd].nan_to_num(1.0))
+
+
 def test_float32_products_of_two_threads(ops):
     """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
     import threading
