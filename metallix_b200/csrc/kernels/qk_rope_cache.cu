@@ -125,8 +125,11 @@ template <typename T, int V> struct alignas(sizeof(T) * V) Pack { T v[V]; };
 // same of the upper half, so the rotation partner of element i (i +- head_dim
 // / 2) sits in the same lane; head_dim / (2 V) lanes make up a head, a warp
 // takes 32 / that many heads at once, and the sum of squares runs over a
-// head's lanes only.
-template <typename T, int HD>
+// head's lanes only. Bound by its loads and stores: a head's rotation and norm
+// weights are as many bytes again as what it reads and writes, so in steps of
+// many tokens a lane takes EACH neighbouring heads of a token with one set of
+// them, all their loads under way at once.
+template <typename T, int HD, int EACH>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_cache_warp_kernel(
     const T* __restrict__ q_in, const T* __restrict__ k_in, const T* __restrict__ v_in,
@@ -147,7 +150,7 @@ qk_norm_rope_cache_warp_kernel(
   // Up to chain_wait(): only the step's integers, the norm weights and the
   // cos/sin tables, none of which a kernel of this step writes.
   const int lane = threadIdx.x & 31, sub = lane % LANES;
-  const int per_token = heads + 2 * kv_heads;
+  const int per_token = (heads + 2 * kv_heads) / EACH;
   // The launcher keeps tokens * per_token below 2^31: 32-bit division, which
   // is a fraction of the instructions the 64-bit one takes.
   const unsigned total = static_cast<unsigned>(tokens) * static_cast<unsigned>(per_token);
@@ -155,7 +158,7 @@ qk_norm_rope_cache_warp_kernel(
   // Lanes without work stay to the end: the sums below shuffle within a head's lanes.
   bool active = item < total;
   const int t = active ? static_cast<int>(item / static_cast<unsigned>(per_token)) : 0;
-  const int h = active ? static_cast<int>(item - static_cast<unsigned>(t) * static_cast<unsigned>(per_token)) : 0;
+  const int h = active ? static_cast<int>(item - static_cast<unsigned>(t) * static_cast<unsigned>(per_token)) * EACH : 0;   // the first of EACH
   const bool is_q = h < heads;
   const bool is_k = !is_q && h < heads + kv_heads;
   const int kv = is_q ? 0 : (is_k ? h - heads : h - heads - kv_heads);
@@ -219,54 +222,64 @@ qk_norm_rope_cache_warp_kernel(
   const float factor = active && is_q ? query_factor(q_factors, factor_positions, positions[t], sub == 0, status) : 1.0f;
   chain_wait();
   src = behind_wait(src);  // written by the kernel ahead of this one
-  Values in_lo = {}, in_hi = {};
+  Values in_lo[EACH] = {}, in_hi[EACH] = {};
   if (active) {
-    in_lo = reinterpret_cast<const Values*>(src)[sub];
-    in_hi = reinterpret_cast<const Values*>(src + HALF)[sub];
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) {
+      in_lo[e] = reinterpret_cast<const Values*>(src + e * HD)[sub];
+      in_hi[e] = reinterpret_cast<const Values*>(src + e * HD + HALF)[sub];
+    }
   }
+  const size_t next_head = is_q ? HD : static_cast<size_t>(page_tokens) * HD;   // in the output
   if (plain_copy) {   // the same for every lane of a head; other heads of the warp go on below
     if (active) {
-      reinterpret_cast<Values*>(dst)[sub] = in_lo;
-      reinterpret_cast<Values*>(dst + HALF)[sub] = in_hi;
+#pragma unroll
+      for (int e = 0; e < EACH; ++e) {
+        reinterpret_cast<Values*>(dst + e * next_head)[sub] = in_lo[e];
+        reinterpret_cast<Values*>(dst + e * next_head + HALF)[sub] = in_hi[e];
+      }
     }
     active = false;
   }
   // A warp whose heads are all values (or past the end) has nothing left to do.
   if (__all_sync(0xffffffffu, !active)) return;
-  float x[2 * V];
-  float sum = 0.0f;
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    x[j] = to_float(in_lo.v[j]);
-    x[V + j] = to_float(in_hi.v[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < 2 * V; ++j) sum += x[j] * x[j];
-#pragma unroll
-  for (int offset = LANES / 2; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
-  if (weight != nullptr) {
-    const float scale = rsqrtf(sum / static_cast<float>(HD) + eps);
-#pragma unroll
-    for (int j = 0; j < 2 * V; ++j) x[j] = x[j] * scale * gain[j];
-  }
-  if (cos_table != nullptr) {
+  for (int e = 0; e < EACH; ++e) {
+    float x[2 * V];
+    float sum = 0.0f;
 #pragma unroll
     for (int j = 0; j < V; ++j) {
-      // element V sub + j (below HALF) and its partner HALF further, x[V + j]
-      const float lo = x[j], hi = x[V + j];
-      x[j] = lo * c[j] - hi * sn[j];
-      x[V + j] = hi * c[j] + lo * sn[j];
+      x[j] = to_float(in_lo[e].v[j]);
+      x[V + j] = to_float(in_hi[e].v[j]);
     }
-  }
-  if (!active) return;
-  Values out_lo, out_hi;
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    out_lo.v[j] = from_float<T>(x[j] * factor);
-    out_hi.v[j] = from_float<T>(x[V + j] * factor);
+    for (int j = 0; j < 2 * V; ++j) sum += x[j] * x[j];
+#pragma unroll
+    for (int offset = LANES / 2; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+    if (weight != nullptr) {
+      const float scale = rsqrtf(sum / static_cast<float>(HD) + eps);
+#pragma unroll
+      for (int j = 0; j < 2 * V; ++j) x[j] = x[j] * scale * gain[j];
+    }
+    if (cos_table != nullptr) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        // element V sub + j (below HALF) and its partner HALF further, x[V + j]
+        const float lo = x[j], hi = x[V + j];
+        x[j] = lo * c[j] - hi * sn[j];
+        x[V + j] = hi * c[j] + lo * sn[j];
+      }
+    }
+    if (!active) continue;
+    Values out_lo, out_hi;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      out_lo.v[j] = from_float<T>(x[j] * factor);
+      out_hi.v[j] = from_float<T>(x[V + j] * factor);
+    }
+    reinterpret_cast<Values*>(dst + e * next_head)[sub] = out_lo;
+    reinterpret_cast<Values*>(dst + e * next_head + HALF)[sub] = out_hi;
   }
-  reinterpret_cast<Values*>(dst)[sub] = out_lo;
-  reinterpret_cast<Values*>(dst + HALF)[sub] = out_hi;
 }
 
 // The same for rotations over part of a head or of neighbouring values: a lane holds V consecutive values of a head, so a
@@ -598,17 +611,24 @@ MXB_API int mxb_qk_norm_rope_cache(
     const long long items = static_cast<long long>(tokens) * (heads + 2 * kv_heads);
     if (items >= 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
     const int heads_per_warp = 32 / (head_dim / 2 / (16 / element));
-    const unsigned blocks = static_cast<unsigned>((items + 8 * heads_per_warp - 1) / (8 * heads_per_warp));
+    // Four heads a lane from the number of heads on that gives every SM several blocks either way. us with one and with four,
+    // bfloat16, heads of 128: 732 tokens of 32 / 8 heads 6.2 and 5.0, 2,048 13.9 and 12.3; 2,048 of 16 / 8 9.4 and 8.6, 732 5.2 and
+    // 5.2, 400 3.4 and 4.2. Heads of 64 lose throughout (2,048 tokens of 16 / 4 5.0 and 5.5).
+    const int each = head_dim >= 128 && heads % 4 == 0 && kv_heads % 4 == 0 && items >= 24576 ? 4 : 1;
+    const long long groups = items / each;
+    const unsigned blocks = static_cast<unsigned>((groups + 8 * heads_per_warp - 1) / (8 * heads_per_warp));
     cudaError_t launch_status = cudaSuccess;
-#define WARP_LAUNCH(T, HD) launch_status = launch_chained(qk_norm_rope_cache_warp_kernel<T, HD>, dim3(blocks), dim3(256), 0, stream, \
+#define WARP_KERNEL(T, HD, EACH) launch_status = launch_chained(qk_norm_rope_cache_warp_kernel<T, HD, EACH>, dim3(blocks), dim3(256), 0, stream, \
         static_cast<const T*>(q_in), static_cast<const T*>(k_in), static_cast<const T*>(v_in), q_stride, k_stride, \
         v_stride, static_cast<T*>(q_out), static_cast<T*>(cache), slots, positions, q_weight, k_weight, cos_table, \
         sin_table, table_positions, tokens, heads, kv_heads, page_tokens, num_pages, eps, q_factors, factor_positions, status)
+#define WARP_LAUNCH(T, HD) do { if (each == 4) WARP_KERNEL(T, HD, 4); else WARP_KERNEL(T, HD, 1); } while (0)
     if (dtype == kF32) {
-      if (head_dim == 64) WARP_LAUNCH(float, 64); else if (head_dim == 128) WARP_LAUNCH(float, 128); else WARP_LAUNCH(float, 256);
+      if (head_dim == 64) WARP_KERNEL(float, 64, 1); else if (head_dim == 128) WARP_LAUNCH(float, 128); else WARP_LAUNCH(float, 256);
     } else {
-      if (head_dim == 64) WARP_LAUNCH(__nv_bfloat16, 64); else if (head_dim == 128) WARP_LAUNCH(__nv_bfloat16, 128); else WARP_LAUNCH(__nv_bfloat16, 256);
+      if (head_dim == 64) WARP_KERNEL(__nv_bfloat16, 64, 1); else if (head_dim == 128) WARP_LAUNCH(__nv_bfloat16, 128); else WARP_LAUNCH(__nv_bfloat16, 256);
     }
+#undef WARP_KERNEL
 #undef WARP_LAUNCH
     return static_cast<int>(launch_status);
   }

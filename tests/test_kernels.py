@@ -165,6 +165,31 @@ def test_partly_turned_heads_by_lanes_and_by_blocks(ops, dtype, head_dim, rotary
     assert float(results[0][1].abs().max()) > 0.5
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, kv_heads, head_dim", [(16, 8, 128), (4, 4, 256), (12, 4, 128)])
+def test_several_heads_a_lane(ops, dtype, heads, kv_heads, head_dim):
+    """A step of many tokens, skipped ones among them, has the bits of the same step in portions of few."""
+    gen, width = torch.Generator(device="cuda").manual_seed(heads), heads + 2 * kv_heads
+    tokens = 24576 // width + 3
+    x = torch.randn(tokens, width * head_dim, generator=gen, device="cuda").to(dtype)
+    q, k, v = x.split([heads * head_dim, kv_heads * head_dim, kv_heads * head_dim], dim=1)
+    positions = torch.randint(0, 500, (tokens,), generator=gen, device="cuda").int()
+    slots = torch.randperm(tokens, generator=gen, device="cuda").int()
+    slots[::7] = -1
+    weights = [torch.rand(head_dim, generator=gen, device="cuda") + 0.5 for _ in range(2)]
+    tables = [torch.rand(500, head_dim // 2, generator=gen, device="cuda") for _ in range(2)]
+    results = []
+    for size in (tokens, 200):
+        out = torch.zeros(tokens, heads, head_dim, dtype=dtype, device="cuda")
+        cache = torch.zeros(-(-tokens // 16), 2, kv_heads, 16, head_dim, dtype=dtype, device="cuda")
+        for at in range(0, tokens, size):
+            cut = slice(at, at + size)
+            ops.qk_norm_rope_cache(q[cut], k[cut], v[cut], out[cut], cache, slots[cut], positions[cut], *weights, *tables, 1e-6)
+        results.append((out, cache))
+    ops.check_status("cuda")
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 def test_rotation_keeps_accuracy_at_far_positions(ops):
     """cos and sin come from a float64 table: at position 4000 a float32
     product of position and frequency would already be off by 1e-4."""
