@@ -116,6 +116,10 @@ class Engine:
         # state that a step advances is advanced once, like the pages it writes. (Three prompts of up to 1,201 tokens
         # through four Sadosun layers of 1,024 values, some 110 launches: 2,585 us launched one by one, 1,430 replayed.)
         self._step_graphs: Optional[Dict] = {} if self.graphs is not None else None
+        # How often a shape has to have come. A capture takes 60 to 100 ms; models with state, whose steps gain some 1 ms from
+        # it, wait until a shape has come more often than a prompt cut into a few portions brings it.
+        stateless = not any(need is not None and need.has_state() for need in self.cache.needs)
+        self._sightings = 1 if stateless else 4
         self.replay_general_steps = True   # False: general steps are launched kernel by kernel (measurements)
         values = self.model.weight_bytes() / torch.empty((), dtype=self.dtype).element_size()
         self.step_graph_tokens = int(min(STEP_GRAPH_TOKENS, max(256, STEP_GRAPH_SECONDS * DEVICE_FLOPS / (2.0 * values))))
@@ -408,7 +412,7 @@ class Engine:
         bound = self.context_bucket(longest)
         shape_key = (tuple(counts), len(wanted), bound, tuple(p.graph_key for p in prepared.values()))
         graphed = tap is None and self._step_graphs is not None and self.replay_general_steps and total <= self.step_graph_tokens and (
-            shape_key in self._step_graphs or self._shapes_seen.get(shape_key, 0) >= 1)
+            shape_key in self._step_graphs or self._shapes_seen.get(shape_key, 0) >= self._sightings)
         if graphed:   # the parts' integers and bounds for every step of this shape
             plan = StepPlan(counts, starts, rows, bound, replayable=True)
             prepared = {key: part.prepare_step(plan) for key, part in self._preparers.items()}

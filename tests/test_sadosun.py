@@ -1095,17 +1095,17 @@ def test_trace_program_and_command_line(folders, tmp_path):
 @gpu
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_steps_of_a_shape_seen_before_replay_with_their_state(folders, dtype):
-    """Portions of two prompts beside a decoded token, the same shape five times: launched, captured, then replayed. Each
-    advances the requests' state once, as an engine does that launches every step."""
+    """Portions of two prompts beside a decoded token, the same shape seven times: launched four times, captured, then
+    replayed. Each advances the requests' state once, as an engine does that launches every step."""
     from metallix_b200.engine import StepEntry
     name, seen = next(iter(MODELS)), {}
     requests = some_requests(name, 60, [60, 45, 12])
     for graphs in (True, False):
         engine = make_engine(folders, name, dtype, cuda_graphs=graphs)
         a, b, c = (list(ids) for ids in requests.values())
-        engine.step([StepEntry("c", c[:7], [])])
-        seen[graphs] = [engine.step([StepEntry("a", a[12 * n:12 * n + 12], [11]), StepEntry("c", c[7 + n:8 + n], [0]),
-                                     StepEntry("b", b[9 * n:9 * n + 9], [0, 8])]).clone() for n in range(5)]
+        engine.step([StepEntry("c", c[:4], [])])
+        seen[graphs] = [engine.step([StepEntry("a", a[8 * n:8 * n + 8], [7]), StepEntry("c", c[4 + n:5 + n], [0]),
+                                     StepEntry("b", b[6 * n:6 * n + 6], [0, 5])]).clone() for n in range(7)]
         engine.check()
         assert not graphs or len(engine._step_graphs) == 1
     assert all(torch.equal(x, y) for x, y in zip(seen[True], seen[False]))
