@@ -10,10 +10,10 @@
 //
 // What bounds it: the tensor core, 6 x 64 cycles per 16 k of a 128 x 128 tile. The operands are read as float32 and
 // split by eight warps (5.5 instructions a value) on their way to shared memory: no pass over W beforehand and no room for
-// it. 917 rows (us, against the CUDA cores' kernel): 4096 x 1024 72 and 212, 6144 x 1024 109 and 261, 1024 x 2048 45 and 129, 1024 x
-// 3072 63 and 188: 106 TFLOP/s of float32, 640 of the tensor core's. Without the splitters' arithmetic it took 50 us for the
-// first of these, without their loads 55: a load has one step to arrive in, and they are volatile because the compiler moved
-// them down to their use (100 us).
+// it. 917 rows (us, against the CUDA cores' kernel): 4096 x 1024 70 and 213, 6144 x 1024 105 and 261, 1024 x 2048 43 and 129, 1024 x
+// 3072 58 and 189, 4096 x 12288 664 and 2,465: 110 to 139 TFLOP/s of float32, 660 to 830 of the tensor core's. Without the
+// splitters' arithmetic the first of these took 50 us, without their loads 55: a load has two steps to arrive in (with one
+// 72 us), and they are volatile because the compiler moved them down to their use (100 us).
 //
 // A number that is not finite, or too near the largest, has no such parts (infinity minus infinity), and leaves an output that is
 // not finite: such outputs are made again by one thread each, in float32 and ascending k, as the general product makes them.
@@ -201,13 +201,12 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
     if (!ok) failed = 1;
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");
-    // ---- splitters: float32 from memory, a step ahead in registers, to three bfloat16 tiles each in shared memory
+    // ---- splitters: float32 from memory, two steps ahead in registers, to three bfloat16 tiles each in shared memory
     const int t = threadIdx.x - 32 * (4 + kSplitAdders);
     // Eight lanes bring a row's 128 bytes. A half-warp's two rows are four apart, so that the swizzle puts their 64 bytes a
     // part into different banks.
     const int quad = t & 7, eight = t >> 3;
     const int row_in = (eight & ~7) | ((eight & 1) << 2) | ((eight >> 1) & 3);   // of 32 rows a pass
-    float4 next[8];
     const float* rows[8];   // of A and of W that this thread brings; rows behind the last one bring that one again
     int unit = blockIdx.x, at = 0, last = 0;   // the step that is fetched next
     auto open = [&]() {
@@ -226,30 +225,45 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(from));
       return v;
     };
-    bool more = unit < units;
-    if (more) {
-      open();
-#pragma unroll
-      for (int i = 0; i < 8; ++i) next[i] = fetch(i);
-    }
-    int step = 0;
-    bool ok = true;
-    while (more && ok && !failed) {
-      const bool beyond = at * kSplitStep + quad * 4 >= k;   // what was fetched lies behind the end of k
+    bool more = unit < units;   // a step is left to be fetched
+    if (more) open();
+    auto advance = [&]() {
       if (++at == last) {
         unit += gridDim.x;
         more = unit < units;
         if (more) open();
       }
+    };
+    struct Fetched {
+      float4 four[8];
+      bool held, beyond;   // there is one; it lies behind the end of k
+    } first, second;       // two steps under way
+    auto fill = [&](Fetched& f) {
+      f.held = more;
+      if (!more) return;
+      f.beyond = at * kSplitStep + quad * 4 >= k;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f.four[i] = fetch(i);
+      advance();
+    };
+    fill(first);
+    fill(second);
+    int step = 0;
+    bool ok = true;
+    auto split_step = [&](Fetched& f) {
+      if (!f.held) return false;
       const int slot = step % kSplitSlots;
       ok = barrier_wait(&step_empty[slot], ((step / kSplitSlots) & 1) ^ 1, status);
-      if (!ok) break;
+      if (!ok || failed) return false;
       unsigned char* stage = stages + (slot >> 1) * kSplitStageBytes;
       const int piece = (slot & 1) * 4 + (quad >> 1);   // of 16 bytes in the row of 128
+      const bool beyond = f.beyond;
+      f.held = more;
+      f.beyond = at * kSplitStep + quad * 4 >= k;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        float4 now = next[i];
-        if (more) next[i] = fetch(i);   // has this step's time to arrive
+        float4 now = f.four[i];
+        if (more) f.four[i] = fetch(i);   // has two steps' time to arrive
         if (beyond) now = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const int row = (i & 3) * 32 + row_in;
         unsigned char* to = stage + (i < 4 ? 0 : 3) * kSplitPlaneBytes + row * 128 + ((piece ^ (row & 7)) << 4) + (quad & 1) * 8;
@@ -259,10 +273,14 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
           *reinterpret_cast<uint2*>(to + part * kSplitPlaneBytes) = make_uint2(low, high);
         }
       }
+      if (more) advance();
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // before the tensor core reads them
       __syncwarp();
       if (lane == 0) barrier_arrive(&step_full[slot]);
       ++step;
+      return true;
+    };
+    while (split_step(first) && split_step(second)) {
     }
     if (!ok) failed = 1;
   }

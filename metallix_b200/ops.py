@@ -1755,8 +1755,8 @@ def gemm_float(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
 
 
 # Rows of A from which float32 products of at least this many rows of W and values each go to the tensor cores, us against the
-# CUDA cores' kernels: 9 rows x 4096 x 1024 14.3 and 25.2, x 1024 x 2048 14.4 and 48.0, x 151936 x 1024 307 and 436; 917 rows 72 and
-# 212, 45 and 129; but 400 x 512 x 512 21 and 20, 256 x 1024 x 512 21 and 19.
+# CUDA cores' kernels: 9 rows x 4096 x 1024 14.3 and 25.2, x 1024 x 2048 14.4 and 48.0, x 151936 x 1024 307 and 436; 917 rows 70 and
+# 213, 43 and 129; but 400 x 512 x 512 21 and 20, 256 x 1024 x 512 21 and 19.
 FLOAT_ROWS, FLOAT_SIDE = 9, 1024
 
 
