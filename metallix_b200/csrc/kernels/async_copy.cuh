@@ -69,4 +69,9 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity,
   return false;
 }
 
+// The same for a warp that is there as a whole and goes on together: where a lane's wait ran out, the warp's did.
+__device__ __forceinline__ bool barrier_wait_warp(uint64_t* barrier, uint32_t parity, int* status) {
+  return __all_sync(0xffffffffu, barrier_wait(barrier, parity, status));
+}
+
 }  // namespace mxb

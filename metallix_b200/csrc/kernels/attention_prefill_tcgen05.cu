@@ -267,9 +267,9 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     const uint64_t v_desc = tc_smem_descriptor_mn(shared_address(v_tiles), kFaHalfBytes);
     int k_stage = 0, v_stage = 0;
     uint32_t k_parity = 0, v_parity = 0;
-    bool ok = barrier_wait(q_full, 0, status);
+    bool ok = barrier_wait_warp(q_full, 0, status);
     auto scores = [&](int i) {  // S_i = Q K_i^T
-      if (!barrier_wait(&k_full[k_stage], k_parity, status)) return false;
+      if (!barrier_wait_warp(&k_full[k_stage], k_parity, status)) return false;
       tc_fence_after_sync();
       if (elect_one()) {
         const uint64_t k_at = k_desc + k_stage * (Config::kKeyBytes >> 4);
@@ -287,10 +287,10 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     };
     auto outputs = [&](int i) {  // O_tile_i = P_i V_i
       const int buffer = i & 1;
-      if (!barrier_wait(&v_full[v_stage], v_parity, status)) return false;
+      if (!barrier_wait_warp(&v_full[v_stage], v_parity, status)) return false;
       // The output buffer is free: every softmax thread took tile i - 2 out of
       // it before it arrived for P of tile i - 1, let alone of tile i.
-      if (!barrier_wait(&p_full[buffer], (i >> 1) & 1, status)) return false;
+      if (!barrier_wait_warp(&p_full[buffer], (i >> 1) & 1, status)) return false;
       tc_fence_after_sync();
       if (elect_one()) {
         const uint64_t v_at = v_desc + v_stage * (Config::kValueBytes >> 4);

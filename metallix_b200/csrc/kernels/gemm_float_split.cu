@@ -106,15 +106,15 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
         const int split = unit / m_tiles % splits;
         const int begin = first_chunk(split), end = first_chunk(split + 1);
         const uint32_t tmem_small = tmem_base + 2 * kSplitTile + (local & 1) * kSplitTile;
-        ok = barrier_wait(&small_empty[local & 1], ((local >> 1) & 1) ^ 1, status);
+        ok = barrier_wait_warp(&small_empty[local & 1], ((local >> 1) & 1) ^ 1, status);
         for (int chunk = begin; chunk < end && ok; ++chunk, ++chunk_count) {
           const int buffer = chunk_count & 1;
-          ok = barrier_wait(&large_empty[buffer], ((chunk_count >> 1) & 1) ^ 1, status);
+          ok = barrier_wait_warp(&large_empty[buffer], ((chunk_count >> 1) & 1) ^ 1, status);
           const uint32_t tmem_large = tmem_base + buffer * kSplitTile;
 #pragma unroll
           for (int half = 0; half < 2; ++half, ++step) {
             const int slot = step % kSplitSlots;
-            ok = ok && barrier_wait(&step_full[slot], (step / kSplitSlots) & 1, status);
+            ok = ok && barrier_wait_warp(&step_full[slot], (step / kSplitSlots) & 1, status);
             if (!ok) break;
             tc_fence_after_sync();
             if (elect_one()) {
@@ -253,7 +253,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
     auto split_step = [&](Fetched& f) {
       if (!f.held) return false;
       const int slot = step % kSplitSlots;
-      ok = barrier_wait(&step_empty[slot], ((step / kSplitSlots) & 1) ^ 1, status);
+      ok = barrier_wait_warp(&step_empty[slot], ((step / kSplitSlots) & 1) ^ 1, status);
       if (!ok || failed) return false;
       unsigned char* stage = stages + (slot >> 1) * kSplitStageBytes;
       const int piece = (slot & 1) * 4 + (quad >> 1);   // of 16 bytes in the row of 128

@@ -142,7 +142,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         n0 += group * group_rows;   // the rows of this group's matrix
       }
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!barrier_wait(&empty_barrier[stage], parity, status)) { failed = 1; break; }
+        if (!barrier_wait_warp(&empty_barrier[stage], parity, status)) { failed = 1; break; }
         if (elect_one()) {
           unsigned char* a_tile = tiles + stage * Config::kStageBytes;
           unsigned char* b_tile = a_tile + kTcM * kTcK * 2;
@@ -170,11 +170,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
       const int buffer = local & 1;
       // The epilogue must have drained this accumulator (two tiles ago).
-      if (!barrier_wait(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
+      if (!barrier_wait_warp(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
       tc_fence_after_sync();
       const uint32_t tmem_d = tmem_base + buffer * BN;
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!barrier_wait(&full_barrier[stage], parity, status)) { failed = 1; break; }
+        if (!barrier_wait_warp(&full_barrier[stage], parity, status)) { failed = 1; break; }
         tc_fence_after_sync();
         if (elect_one()) {
           const uint64_t a_stage = a_desc + stage * (Config::kStageBytes >> 4), b_stage = a_stage + (kTcM * kTcK * 2 >> 4);

@@ -79,7 +79,7 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         n0 += group * group_rows;   // the rows of this group's matrix
       }
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!barrier_wait(&empty_barrier[stage], parity, status)) { failed = 1; break; }
+        if (!barrier_wait_warp(&empty_barrier[stage], parity, status)) { failed = 1; break; }
         if (elect_one()) {
           unsigned char *a_tile = a_tiles + stage * 2 * a_half, *w_tile = w_tiles + stage * 2 * w_half;
           barrier_arrive_expect(&full_barrier[stage], 2 * (a_half + w_half));
@@ -107,11 +107,11 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
       if (tile_group != nullptr && tile_group[tile / n_tiles] < 0) continue;
       const int buffer = local & 1;
-      if (!barrier_wait(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
+      if (!barrier_wait_warp(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
       tc_fence_after_sync();
       const uint32_t tmem_d = tmem_base + buffer * kRowsColumns;
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!barrier_wait(&full_barrier[stage], parity, status)) { failed = 1; break; }
+        if (!barrier_wait_warp(&full_barrier[stage], parity, status)) { failed = 1; break; }
         tc_fence_after_sync();
         if (elect_one()) {
           const uint64_t a_at = a_desc + stage * 2 * a_step, w_at = w_desc + stage * 2 * w_step;
