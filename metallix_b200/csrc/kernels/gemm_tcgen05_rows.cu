@@ -6,8 +6,8 @@
 // is its few rows only (the instruction reads 128 rows from there on: what it finds behind them makes accumulator rows
 // that nobody stores), and W's rows are dealt out so that one round of 148 blocks, or several full ones, takes them all.
 // An instruction takes 40 cycles however narrow its tile is, so a block of 128 k takes some 450: tiles of a few rows of W
-// are bound by that (4096 x 4096 at 8 rows 15.8 us, 12.3 in the load-based kernel), tall matrices by W (ops.TALL_ROWS has
-// both sides), and so are experts: 16 tokens over 13 of 6144 x 4096 136 -> 117 us (5.6 TB/s), 3 tokens over 1536 x 1024 18.4 ->
+// are bound by that (4096 x 4096 at 8 rows 15.8 us, 12.3 in the load-based kernel), tall matrices by W, and so are
+// experts: 16 tokens over 13 of 6144 x 4096 136 -> 117 us (5.6 TB/s), 3 tokens over 1536 x 1024 18.4 ->
 // 10.3, where tiles of 128 rows and 256 columns leave SMs idle in the last round.
 //
 // Warp 0 feeds the stages, warp 1 issues the MMAs, warps 2..9 run the epilogues of gemm_tcgen05_kernel (the accumulators'

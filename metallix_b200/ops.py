@@ -1826,23 +1826,6 @@ def gemm_skinny_takes(a: torch.Tensor, w: torch.Tensor, swiglu: bool = False) ->
 GATE_ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "clamped": 2}
 
 
-# From this many rows of W on (a vocabulary, gate and up of a wide layer) few rows of A take the tensor-core kernel that
-# streams W (csrc/kernels/gemm_tcgen05_rows.cu): each of its 148 blocks then has a hundred rows of W and more to fetch. us
-# against the load-based kernel and the library: 32768 x 4096, 8 rows 46.0, 50.6, 47.1; 32 rows 46.6, -, 47.8; 64 rows 49.3, -,
-# 48.8; 151936 x 1024, 2 rows 52.3, 49.1, 54.5; 8 rows 53.3, 55.6, 55.7; gate and up 24576 x 4096 with the activation, 2 rows 36.7,
-# 40.9, 37.2; 8 rows 36.8, 43.0, 37.4; 64 rows 38.2, -, 41.5; but 8192 x 4096, 8 rows 18.1, 16.2, 13.9.
-TALL_ROWS = 16384
-
-
-def gemm_rows_takes(a: torch.Tensor, w: torch.Tensor, swiglu: bool = False) -> bool:
-    """Whether few rows of ``a`` times a tall ``w`` go to the tensor-core kernel
-    for few rows; with short rows of W only from five rows of ``a`` on."""
-    rows, k = a.shape
-    if w.shape[0] < TALL_ROWS or (swiglu and k <= STREAM_K):
-        return False
-    return (1 if k > STREAM_K else 5) <= rows <= (64 if swiglu else 32)
-
-
 def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
                 swiglu: bool = False, out: Optional[torch.Tensor] = None, kernel: str = "auto",
                 activation: str = "silu", limit: float = 0.0) -> torch.Tensor:
@@ -1904,10 +1887,6 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.b
     few = SKINNY_ROWS if a.shape[1] <= STREAM_K else SKINNY_ROWS // 2
     if a.shape[1] > STREAM_K and LOAD_COLUMNS < w.shape[0] <= STREAM_COLUMNS:
         few = 0   # long rows and a middling width: the library reads these faster at any row count
-    if backend == "auto" and gemm_rows_takes(a, w):
-        from . import tensor_core
-        if tensor_core.supports(a, w, out_dtype):
-            return tensor_core.gemm(a, w, out_dtype=out_dtype, out=out)
     if (backend == "skinny" or (backend == "auto" and a.shape[0] <= few)) and gemm_skinny_takes(a, w):
         return gemm_skinny(a, w, out_dtype=out_dtype, out=out)
     _need(backend != "skinny", "the weight-streaming kernel does not take this shape")

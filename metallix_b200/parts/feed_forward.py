@@ -58,11 +58,6 @@ class SwiGLU:
             raise ValueError("the clamped activation needs a positive limit")
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        if self.gate_up.dtype == torch.bfloat16 and self.gate_up.backend == "auto" and ops.gemm_rows_takes(x, self.gate_up.weight, swiglu=True):
-            from .. import tensor_core
-            if tensor_core.supports(x, self.gate_up.weight, torch.bfloat16):
-                # A decode step of wide layers: gate, up and the activation in one pass over the weights on the tensor cores.
-                return self.down.forward(tensor_core.gemm_swiglu(x, self.gate_up.weight, activation=self.activation, limit=self.limit))
         few = ops.SKINNY_ROWS if x.shape[1] <= ops.STREAM_K else ops.SKINNY_ROWS // 2   # as ops.gemm_bf16
         if (x.shape[0] <= few and self.gate_up.backend in ("auto", "skinny")
                 and ops.gemm_skinny_takes(x, self.gate_up.weight, swiglu=True)):

@@ -1290,6 +1290,17 @@ def test_products_of_few_rows_on_the_tensor_cores(ops, m, n, k):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("m, n, k", [(8, 32768, 4096), (5, 40000, 1024), (16, 16384, 2048)])
+def test_few_rows_of_wide_matrices_add_up_in_float32(ops, m, n, k):
+    """A decode step's logits and gates: no further from 64 bits than a float32 sum in ascending k. (Sums inside the tensor
+    core over all of k are cut off where they are aligned and stray 2 to 4 times as far.)"""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    x, w = torch.randn(m, k, generator=gen, device="cuda").bfloat16(), torch.randn(n, k, generator=gen, device="cuda").bfloat16()
+    ref = x.double() @ w.double().t()
+    off = lambda out: float((out - ref).norm())
+    assert off(ops.gemm_bf16(x, w, out_dtype=torch.float32)) <= off(ops.gemm_simple(x, w, out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("counts, n, k", [([3, 0, 1, 64, 1, 29], 512, 128), ([7] * 13, 40, 256), ([0, 5, 0], 300, 72)])
 def test_few_rows_of_many_experts(ops, counts, n, k):
     """Tiles of which some rows are in use, the others not even loaded: the bits of the product that takes all of them."""
