@@ -69,9 +69,13 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity,
   return false;
 }
 
-// The same for a warp that is there as a whole and goes on together: where a lane's wait ran out, the warp's did.
+// The same for a warp that is there as a whole and goes on together: where a lane's wait ran out, the warp's did. Instructions
+// that a warp executes as one (tensor-memory loads and stores, elections, votes) need waits of this kind ahead of them.
 __device__ __forceinline__ bool barrier_wait_warp(uint64_t* barrier, uint32_t parity, int* status) {
   return __all_sync(0xffffffffu, barrier_wait(barrier, parity, status));
 }
+
+// Whether a block's `failed` is set, the same for the whole warp: its lanes may read it at different times.
+__device__ __forceinline__ bool given_up(const volatile int& failed) { return __any_sync(0xffffffffu, failed != 0); }
 
 }  // namespace mxb

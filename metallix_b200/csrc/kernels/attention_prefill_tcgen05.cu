@@ -218,7 +218,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       return kNoPage;
     };
     int page = page_of(0);
-    for (int i = 0; i < key_tiles && !failed; ++i) {
+    for (int i = 0; i < key_tiles && !given_up(failed); ++i) {
       const int stage = i % stages;
       const int upcoming = page_of(i + 1);   // in flight while this tile's requests go out
       if (page != kNoPage && (page < 0 || page >= num_pages)) {
@@ -234,14 +234,14 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       const bool tail = values && key_tile == all_end && zero_from < zero_to;
       uint64_t* landing = tail ? v_tail : &full[stage];
       // K as soon as the scores that read this stage last are done, V when the P V product is.
-      if (!barrier_wait(&empty[stage], ((i / stages) & 1) ^ 1, status)) { failed = 1; break; }
+      if (!barrier_wait_warp(&empty[stage], ((i / stages) & 1) ^ 1, status)) { failed = 1; break; }
       if (lane == 0) barrier_arrive_expect(landing, tile_bytes);
       __syncwarp();
       unsigned char* stage_tile = tiles + stage * tile_bytes;
       if (lane < copies)
         tma_load_2d(stage_tile + offset, &map_cache, column, box_row, landing);
       if (tail) {
-        if (!barrier_wait(v_tail, 0, status)) { failed = 1; break; }
+        if (!barrier_wait_warp(v_tail, 0, status)) { failed = 1; break; }
         // a key's 64 values of one half are 128 bytes, swizzled among themselves
         for (int c = lane; c < (zero_to - zero_from) * Config::kValueHalves * 8; c += 32)
           *reinterpret_cast<uint4*>(stage_tile + ((c >> 3) % Config::kValueHalves) * kFaHalfBytes +
@@ -312,7 +312,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       return true;
     };
     ok = ok && (key_tiles == 0 || scores(0));
-    for (int i = 0; i < key_tiles && ok && !failed; ++i) {
+    for (int i = 0; i < key_tiles && ok && !given_up(failed); ++i) {
       if (i + 1 < key_tiles) ok = scores(i + 1);
       ok = ok && outputs(i);
     }
@@ -343,7 +343,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
 
     auto accumulate = [&](int i, float alpha) {  // acc = acc * alpha + O_tile_i
       const int buffer = i & 1;
-      if (!barrier_wait(&o_full[buffer], (i >> 1) & 1, status)) return false;
+      if (!barrier_wait_warp(&o_full[buffer], (i >> 1) & 1, status)) return false;
       tc_fence_after_sync();
       uint32_t o[PART_HD];
       tc_load(tmem_lane + Config::kOutputBase + buffer * HDV + part * PART_HD, o);
@@ -356,7 +356,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     for (int i = 0; i < key_tiles; ++i) {
       const int buffer = i & 1;
       const int key0 = walk.tile(step_begin + i) * kFaKeys + part * PART_KEYS;  // first key of this thread's share
-      if (!barrier_wait(&s_full[buffer], (i >> 1) & 1, status) || failed) { ok = false; break; }
+      if (!barrier_wait_warp(&s_full[buffer], (i >> 1) & 1, status) || given_up(failed)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t tmem_s = tmem_lane + buffer * Config::kScoreColumns + part * PART_KEYS;
       const bool all_seen = (key0 >= key_lo || key0 + PART_KEYS <= keep) && key0 + PART_KEYS - 1 <= key_hi;
@@ -395,7 +395,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       for (int j = 0; j < PART_KEYS; ++j) max4[j & 3] = fmaxf(max4[j & 3], s[j]);
       row_max[buffer][part][row] = fmaxf(fmaxf(max4[0], max4[1]), fmaxf(max4[2], max4[3]));
       barrier_arrive(meet);
-      if (!barrier_wait(meet, i & 1, status)) { ok = false; break; }
+      if (!barrier_wait_warp(meet, i & 1, status)) { ok = false; break; }
       const float tile_max = fmaxf(fmaxf(row_max[buffer][0][row], row_max[buffer][1][row]),
                                    fmaxf(row_max[buffer][2][row], row_max[buffer][3][row]));
       const float m_new = fmaxf(m, tile_max * scale_log2);
@@ -425,14 +425,14 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
       if (i > 0 && !accumulate(i - 1, alpha_pending)) { ok = false; break; }
       alpha_pending = alpha;
     }
-    if (ok && !failed && key_tiles > 0) ok = accumulate(key_tiles - 1, alpha_pending);
+    if (ok && !given_up(failed) && key_tiles > 0) ok = accumulate(key_tiles - 1, alpha_pending);
     if (!ok) failed = 1;
     // The row's sum: this thread's keys plus its partners' (all scaled to the
     // same final maximum). The buffer of this parity was last read two
     // exchanges ago.
     row_max[key_tiles & 1][part][row] = l;
     barrier_arrive(meet);
-    if (ok && !barrier_wait(meet, key_tiles & 1, status)) ok = false;
+    if (ok && !barrier_wait_warp(meet, key_tiles & 1, status)) ok = false;
     l = (row_max[key_tiles & 1][0][row] + row_max[key_tiles & 1][1][row]) +
         (row_max[key_tiles & 1][2][row] + row_max[key_tiles & 1][3][row]);
     if (!ok) failed = 1;

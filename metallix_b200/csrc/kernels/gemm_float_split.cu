@@ -102,7 +102,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       const uint64_t desc = tc_smem_descriptor(shared_address(stages));
       int step = 0, chunk_count = 0, local = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < units && ok && !failed; unit += gridDim.x, ++local) {
+      for (int unit = blockIdx.x; unit < units && ok && !given_up(failed); unit += gridDim.x, ++local) {
         const int split = unit / m_tiles % splits;
         const int begin = first_chunk(split), end = first_chunk(split + 1);
         const uint32_t tmem_small = tmem_base + 2 * kSplitTile + (local & 1) * kSplitTile;
@@ -153,7 +153,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
       for (int chunk = begin; chunk < end; ++chunk, ++chunk_count) {
         const int buffer = chunk_count & 1;
-        if (!barrier_wait(&large_full[buffer], (chunk_count >> 1) & 1, status) || failed) { ok = false; break; }
+        if (!barrier_wait_warp(&large_full[buffer], (chunk_count >> 1) & 1, status) || given_up(failed)) { ok = false; break; }
         tc_fence_after_sync();
 #pragma unroll
         for (int part = 0; part < 4; ++part) {
@@ -179,24 +179,26 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       if (lane == 0) barrier_arrive(&small_empty[local & 1]);
       const int row = unit % m_tiles * kSplitTile + lane_base + lane;
       const int column = unit / m_tiles / splits * kSplitTile + columns;
-      if (row >= m) continue;
-      float* to = splits > 1 ? scratch + (static_cast<long long>(split) * m + row) * n + column : c + row * ldc + column;
-      if (column + 64 <= n && (reinterpret_cast<uintptr_t>(to) & 15) == 0) {
+      if (row < m) {
+        float* to = splits > 1 ? scratch + (static_cast<long long>(split) * m + row) * n + column : c + row * ldc + column;
+        if (column + 64 <= n && (reinterpret_cast<uintptr_t>(to) & 15) == 0) {
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-      } else {
+          for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (column + i < n) to[i] = acc[i];
+          for (int i = 0; i < 64; ++i)
+            if (column + i < n) to[i] = acc[i];
+        }
+        if (splits == 1) {
+          float worst = 0.0f;   // stays finite, or becomes NaN
+#pragma unroll
+          for (int i = 0; i < 64; ++i) worst += 0.0f * acc[i];
+          if (worst != 0.0f)
+            for (int i = 0; i < 64 && column + i < n; ++i)
+              if (!is_finite(to[i])) to[i] = plain_dot(a + row * lda, w + (column + i) * ldw, k);
+        }
       }
-      if (splits == 1) {
-        float worst = 0.0f;   // stays finite, or becomes NaN
-#pragma unroll
-        for (int i = 0; i < 64; ++i) worst += 0.0f * acc[i];
-        if (worst != 0.0f)
-          for (int i = 0; i < 64 && column + i < n; ++i)
-            if (!is_finite(to[i])) to[i] = plain_dot(a + row * lda, w + (column + i) * ldw, k);
-      }
+      __syncwarp();   // rows behind the last one are here first; the next unit's loads take the warp as a whole
     }
     if (!ok) failed = 1;
   } else {
@@ -254,7 +256,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       if (!f.held) return false;
       const int slot = step % kSplitSlots;
       ok = barrier_wait_warp(&step_empty[slot], ((step / kSplitSlots) & 1) ^ 1, status);
-      if (!ok || failed) return false;
+      if (!ok || given_up(failed)) return false;
       unsigned char* stage = stages + (slot >> 1) * kSplitStageBytes;
       const int piece = (slot & 1) * 4 + (quad >> 1);   // of 16 bytes in the row of 128
       const bool beyond = f.beyond;
@@ -286,6 +288,12 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
   }
 
   tc_fence_before_sync();
+  __syncthreads();
+  if (failed && threadIdx.x == 0) {
+    // A wait ran out somewhere. Give products that may still be under way a
+    // millisecond before the block's memory goes back.
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  }
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kSplitTmemColumns) : "memory");

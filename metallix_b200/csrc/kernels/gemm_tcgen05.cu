@@ -66,7 +66,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __shared__ __align__(8) uint64_t accumulator_full[2];
   __shared__ __align__(8) uint64_t accumulator_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int failed;
+  __shared__ int failed_slot;
+  volatile int& failed = failed_slot;
   __shared__ uint16_t run_start[kTcListed], run_length[kTcListed];   // grouped: per row tile the first one of its run of one group; by that, how many
 
   unsigned char* tiles = tc_shared_raw + ((1024 - (shared_address(tc_shared_raw) & 1023)) & 1023);
@@ -131,7 +132,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // ---- producer: TMA loads of the A and B tiles of every k block of every tile
     int stage = 0;
     uint32_t parity = 1;
-    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < total_tiles && !given_up(failed); tile += gridDim.x) {
       int m_tile, n_tile;
       place(tile, m_tile, n_tile);
       const int m0 = m_tile * kTcM;
@@ -164,7 +165,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const uint64_t a_desc = tc_smem_descriptor(shared_address(tiles));
     int stage = 0, local = 0;
     uint32_t parity = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < total_tiles && !given_up(failed); tile += gridDim.x) {
       int m_tile, n_tile;
       place(tile, m_tile, n_tile);
       if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
@@ -198,8 +199,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
       const int buffer = local & 1;
       const int m0 = m_tile * kTcM, n0 = n_tile * OUT_COLUMNS;
-      if (!barrier_wait(&accumulator_full[buffer], (local >> 1) & 1, status)) { failed = 1; break; }
-      if (failed) break;
+      if (!barrier_wait_warp(&accumulator_full[buffer], (local >> 1) & 1, status)) { failed = 1; break; }
+      if (given_up(failed)) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const int row = m0 + lane_base + lane;
       const float scale = EPI == kTcGelu && row_scale != nullptr && row < m ? row_scale[row] : 1.0f;

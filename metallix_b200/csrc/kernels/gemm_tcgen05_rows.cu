@@ -34,7 +34,8 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   __shared__ __align__(8) uint64_t full_barrier[kRowsStages], empty_barrier[kRowsStages];
   __shared__ __align__(8) uint64_t accumulator_full[2], accumulator_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int failed;
+  __shared__ int failed_slot;
+  volatile int& failed = failed_slot;
   const int out_columns = tc_gated(EPI) ? w_rows / 2 : w_rows;
   // A's stages ahead of W's: the 128 rows that an instruction reads end within the stages either way.
   const int a_half = a_rows * 128, w_half = w_rows * 128;   // bytes of a box of 64 k
@@ -70,7 +71,7 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (warp == 0) {
     int stage = 0;
     uint32_t parity = 1;
-    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < total_tiles && !given_up(failed); tile += gridDim.x) {
       const int m_tile = tile / n_tiles;
       int n0 = tile % n_tiles * out_columns;
       if (tile_group != nullptr) {
@@ -104,7 +105,7 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t a_step = a_half >> 4, w_step = w_half >> 4;
     int stage = 0, local = 0;
     uint32_t parity = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < total_tiles && !given_up(failed); tile += gridDim.x) {
       if (tile_group != nullptr && tile_group[tile / n_tiles] < 0) continue;
       const int buffer = local & 1;
       if (!barrier_wait_warp(&accumulator_empty[buffer], ((local >> 1) & 1) ^ 1, status)) { failed = 1; break; }
@@ -132,8 +133,8 @@ gemm_tcgen05_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int m_tile = tile / n_tiles, n0 = tile % n_tiles * out_columns;
       if (tile_group != nullptr && tile_group[m_tile] < 0) continue;
       const int buffer = local & 1;
-      if (!barrier_wait(&accumulator_full[buffer], (local >> 1) & 1, status)) { failed = 1; break; }
-      if (failed) break;
+      if (!barrier_wait_warp(&accumulator_full[buffer], (local >> 1) & 1, status)) { failed = 1; break; }
+      if (given_up(failed)) break;
       tc_fence_after_sync();
       if (lane_base < tile_rows) {
         const int row = m_tile * tile_stride + lane_base + lane;

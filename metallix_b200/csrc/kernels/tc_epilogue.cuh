@@ -16,6 +16,7 @@ template <int EPI, int WIDE>
 __device__ __forceinline__ void tc_epilogue(uint32_t taddr, uint32_t taddr_up, void* out, int row, bool stored, int column,
                                             int n, long long ldo, float limit, float scale) {
   uint32_t acc[WIDE];
+  __syncwarp();   // lanes that stored nothing of the columns before are back ahead of the others
   tc_load(taddr, acc);
   float values[WIDE];
   if (tc_gated(EPI)) {

@@ -1,0 +1,29 @@
+"""What no run shows, read in the kernels' sources (no GPU)."""
+import os
+import re
+
+import pytest
+
+KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "metallix_b200", "csrc", "kernels")
+
+
+@pytest.mark.parametrize("name", ["gemm_tcgen05.cu", "gemm_tcgen05_rows.cu", "gemm_float_split.cu", "attention_prefill_tcgen05.cu"])
+def test_warps_that_use_tensor_memory_wait_and_give_up_as_a_whole(name):
+    """A warp takes loads and stores of tensor memory, elections and votes as one: no lane may end a wait, or see that its
+    block has given up, by itself."""
+    with open(os.path.join(KERNELS, name)) as handle:
+        text = re.sub(r"//[^\n]*", "", handle.read())
+    assert not re.findall(r"\bbarrier_wait\(", text)
+    reads = [line.strip() for line in text.split("\n") if re.search(r"\bfailed\b", line)
+             and not re.search(r"given_up\(failed\)|failed = |failed_slot|if \(failed && threadIdx\.x == 0\)", line)]
+    assert reads == []
+
+
+def test_lanes_without_rows_are_back_before_tensor_memory_is_loaded():
+    """Lanes whose row does not exist store nothing and are ahead of the others: the warp meets before the next load."""
+    with open(os.path.join(KERNELS, "tc_epilogue.cuh")) as handle:
+        epilogue = handle.read()
+    assert re.search(r"__syncwarp\(\);[^\n]*\n\s*tc_load\(taddr, acc\);", epilogue)
+    with open(os.path.join(KERNELS, "gemm_float_split.cu")) as handle:
+        adders = handle.read().split("// ---- adders")[1].split("// ---- splitters")[0]
+    assert "continue;" not in adders and re.search(r"__syncwarp\(\);[^\n]*\n    }\n", adders)

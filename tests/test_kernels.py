@@ -1137,6 +1137,23 @@ def test_float32_products_on_the_tensor_cores(ops, m, n, k):
     assert torch.equal(odd, ~out.isfinite()) and torch.equal(out[odd].nan_to_num(1.0), plain_out[odd].nan_to_num(1.0))
 
 
+@pytest.mark.parametrize("m, n, k", [(130, 40000, 68), (917, 4096, 256), (257, 20100, 72)])
+def test_float32_products_of_several_tiles_a_block(ops, m, n, k):
+    """Blocks that go on to another tile behind one whose last rows or columns do not exist; operands and result inside wider
+    rows. Every output as far from 64 bits as the sum in ascending k at most, over all of them."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    wide = [torch.randn(rows, k + extra, generator=gen, device="cuda") for rows, extra in ((m, 8), (n, 4))]
+    a, w, out = wide[0][:, 4:k + 4], wide[1][:, :k], torch.full((m, n + 3), 7.0, device="cuda")
+    ops.gemm_float(a, w, out=out[:, 1:n + 1])
+    ops.check_status("cuda")
+    plain_out, ref = ops.gemm_simple(a, w), a.double() @ w.double().t()
+    off, plain_off = (out[:, 1:n + 1] - ref).abs(), (plain_out - ref).abs()
+    assert float(off.norm()) <= max(float(plain_off.norm()), 2.0 ** -24 * float(ref.norm()))
+    # 2^-24 for the last addition, 2^-22 of the absolute products for what is left out and the sums inside the tensor core
+    assert bool((off <= 2.0 ** -24 * ref.abs() + 2.0 ** -22 * (a.double().abs() @ w.double().abs().t())).all())
+    assert bool((out[:, 0] == 7.0).all()) and bool((out[:, n + 1:] == 7.0).all())
+
+
 def test_float32_products_of_two_threads(ops):
     """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
     import threading
