@@ -1154,6 +1154,24 @@ def test_float32_products_of_several_tiles_a_block(ops, m, n, k):
     assert bool((out[:, 0] == 7.0).all()) and bool((out[:, n + 1:] == 7.0).all())
 
 
+@pytest.mark.parametrize("m, n, k", [(300, 19300, 260), (257, 1030, 3076), (140, 5000, 12288), (5, 1100, 1024)])
+def test_float32_products_of_rows_that_are_not_finite(ops, m, n, k):
+    """Whole rows and columns, and a tile of nothing else, in blocks with more tiles to come: every wait ends in time, what is
+    not finite has the general product's bits and the rest is untouched by it."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, w = (torch.randn(rows, k, generator=gen, device="cuda") for rows in (m, n))
+    clean = ops.gemm_float(a, w)
+    a[m // 2:m // 2 + max(1, m // 5)], w[n // 3, 3], a[0, k - 1], a[m - 1, 0] = float("nan"), float("inf"), float("-inf"), 3.3e38
+    out, plain_out = ops.gemm_float(a, w), ops.gemm_simple(a, w)
+    ops.check_status("cuda")
+    odd = ~plain_out.isfinite()
+    assert torch.equal(odd, ~out.isfinite()) and torch.equal(out[odd].nan_to_num(1.0), plain_out[odd].nan_to_num(1.0))
+    same = torch.ones(m, dtype=torch.bool, device="cuda")
+    same[0] = same[m - 1] = same[m // 2:m // 2 + max(1, m // 5)] = False
+    columns = torch.arange(n, device="cuda") != n // 3
+    assert torch.equal(out[same][:, columns], clean[same][:, columns])
+
+
 def test_float32_products_of_two_threads(ops):
     """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
     import threading
