@@ -10,15 +10,20 @@
 //
 // What bounds it: the tensor core, 6 x 64 cycles per 16 k of a 128 x 128 tile. The operands are read as float32 and
 // split by eight warps (5.5 instructions a value) on their way to shared memory: no pass over W beforehand and no room for
-// it. 917 rows (us, against the CUDA cores' kernel): 4096 x 1024 70 and 213, 6144 x 1024 105 and 261, 1024 x 2048 43 and 129, 1024 x
-// 3072 58 and 189, 4096 x 12288 664 and 2,465: 110 to 139 TFLOP/s of float32, 660 to 830 of the tensor core's. Without the
-// splitters' arithmetic the first of these took 50 us, without their loads 55: a load has two steps to arrive in (with one
+// it. 917 rows (us, against the CUDA cores' kernel): 4096 x 1024 77 and 213, 6144 x 1024 110 and 261, 1024 x 2048 50 and 128, 1024 x
+// 3072 65 and 188, 4096 x 12288 745 and 2,465: 77 to 124 TFLOP/s of float32, 460 to 740 of the tensor core's. Without the
+// splitters' arithmetic the first of these took 50 us of 70, without their loads 55: a load has two steps to arrive in (with one
 // 72 us), and they are volatile because the compiler moved them down to their use (100 us).
+//
+// A row's bits do not depend on what other rows there are: how the sums over k are grouped follows from n and k alone. Few
+// rows give each group to a block of its own and add the groups up in a second kernel; with many, a tile's block takes
+// its groups one after the other, and their sum stays in tensor memory, in the same order. (With as many parts of k as the
+// rows left room for, 917 rows took 70, 105, 43 and 58 us of the first four.)
 //
 // A number that is not finite, or too near the largest, has no such parts (infinity minus infinity), and leaves an output that is
 // not finite: such outputs are made again in float32 and ascending k, with the general product's bits, tile by tile, by the
-// adders of a block once it has walked all of its tiles (nobody waits for them any more), or by the kernel that adds the parts up.
-// 917 rows x 4096 x 1024: 73 us, 161 with a row of NaN, 746 with nothing else (the CUDA cores' kernel 213).
+// adders of a block once it has walked all of its tiles (nobody waits for them any more), or by the kernel that adds the groups up.
+// 917 rows x 4096 x 1024: 77 us, some 90 more with a row of NaN, 680 more with nothing else (the CUDA cores' kernel 213).
 //
 // Every wait on a barrier is bounded: if it runs out, the status word gets a bit and the block stops, frees its tensor
 // memory and leaves.
@@ -34,10 +39,12 @@ constexpr int kSplitChunk = 64;          // k that the tensor core sums up
 constexpr int kSplitSlots = 4;           // steps in shared memory: two stages of 64 k, each in halves
 constexpr int kSplitPlaneBytes = kSplitTile * kSplitChunk * 2;
 constexpr int kSplitStageBytes = 6 * kSplitPlaneBytes;   // three parts of A, three of W
-constexpr int kSplitSharedBytes = 2 * kSplitStageBytes + 1024;
 constexpr int kSplitAdders = 8, kSplitSplitters = 8;     // warps
+constexpr int kSplitPutPitch = 20;       // floats: eight rows' 16 bytes in different banks
+constexpr int kSplitPutBytes = kSplitAdders * 32 * kSplitPutPitch * 4;   // where the adders turn their results around
+constexpr int kSplitSharedBytes = 2 * kSplitStageBytes + kSplitPutBytes + 1024;
 constexpr int kSplitThreads = 32 * (4 + kSplitAdders + kSplitSplitters);   // warpgroups: one that issues, two and two
-constexpr int kSplitTmemColumns = 512;   // large sums twice, then small sums twice
+constexpr int kSplitTmemColumns = 512;   // large sums twice, then small sums twice, or once and the sum of the groups so far
 
 __device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= FLT_MAX; }
 
@@ -120,7 +127,7 @@ __device__ __forceinline__ bool make_again(float (&v)[2][8], float* shared, int 
 
 __global__ void __launch_bounds__(kSplitThreads, 1)
 gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w, int m, int n, int k,
-                        long long lda, long long ldw, long long ldc, int splits, float* __restrict__ scratch, int* status) {
+                        long long lda, long long ldw, long long ldc, int groups, int slices, float* __restrict__ scratch, int* status) {
   extern __shared__ unsigned char split_shared_raw[];
   __shared__ __align__(8) uint64_t step_full[kSplitSlots], step_empty[kSplitSlots];
   __shared__ __align__(8) uint64_t large_full[2], large_empty[2], small_empty[2];
@@ -131,7 +138,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = ceil_div(m, kSplitTile), n_tiles = ceil_div(n, kSplitTile);
   const int chunks = ceil_div(k, kSplitChunk);
-  const int units = m_tiles * n_tiles * splits;   // (tile, part of k), the row tile fastest
+  const int units = m_tiles * n_tiles * slices;   // (tile, slice: some groups of k side by side), the row tile fastest
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSplitSlots; ++s) {
@@ -155,7 +162,13 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
-  auto first_chunk = [&](int split) { return static_cast<int>(static_cast<long long>(split) * chunks / splits); };
+  auto first_group = [&](int unit, int after) { return (unit / m_tiles % slices + after) * groups / slices; };   // after 1: of the next slice
+  // All groups of a tile one after the other in one block: their sum lies in tensor memory meanwhile, where else the second
+  // accumulator of small sums is.
+  const bool chained = slices == 1 && groups > 1;
+  auto small_of = [&](int local) { return chained ? 0 : local & 1; };
+  auto small_turn = [&](int local) { return static_cast<uint32_t>(chained ? local & 1 : (local >> 1) & 1); };
+  auto first_chunk = [&](int group) { return static_cast<int>(static_cast<long long>(group) * chunks / groups); };
 
   // 640 threads start with 96 registers each; the adders' 64 sums want more and the issuing warps need few.
   if (warp < 4) {
@@ -166,36 +179,37 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
       const uint64_t desc = tc_smem_descriptor(shared_address(stages));
       int step = 0, chunk_count = 0, local = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < units && ok && !given_up(failed); unit += gridDim.x, ++local) {
-        const int split = unit / m_tiles % splits;
-        const int begin = first_chunk(split), end = first_chunk(split + 1);
-        const uint32_t tmem_small = tmem_base + 2 * kSplitTile + (local & 1) * kSplitTile;
-        ok = barrier_wait_warp(&small_empty[local & 1], ((local >> 1) & 1) ^ 1, status);
-        for (int chunk = begin; chunk < end && ok; ++chunk, ++chunk_count) {
-          const int buffer = chunk_count & 1;
-          ok = barrier_wait_warp(&large_empty[buffer], ((chunk_count >> 1) & 1) ^ 1, status);
-          const uint32_t tmem_large = tmem_base + buffer * kSplitTile;
+      for (int unit = blockIdx.x; unit < units && ok && !given_up(failed); unit += gridDim.x) {
+        for (int group = first_group(unit, 0), last = first_group(unit, 1); group < last && ok; ++group, ++local) {
+          const int begin = first_chunk(group), end = first_chunk(group + 1);
+          const uint32_t tmem_small = tmem_base + (2 + small_of(local)) * kSplitTile;
+          ok = barrier_wait_warp(&small_empty[small_of(local)], small_turn(local) ^ 1, status);
+          for (int chunk = begin; chunk < end && ok; ++chunk, ++chunk_count) {
+            const int buffer = chunk_count & 1;
+            ok = barrier_wait_warp(&large_empty[buffer], ((chunk_count >> 1) & 1) ^ 1, status);
+            const uint32_t tmem_large = tmem_base + buffer * kSplitTile;
 #pragma unroll
-          for (int half = 0; half < 2; ++half, ++step) {
-            const int slot = step % kSplitSlots;
-            ok = ok && barrier_wait_warp(&step_full[slot], (step / kSplitSlots) & 1, status);
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (elect_one()) {
-              const uint64_t at = desc + (((slot >> 1) * kSplitStageBytes + half * kSplitStep * 2) >> 4);
-              constexpr uint64_t plane = kSplitPlaneBytes >> 4;
+            for (int half = 0; half < 2; ++half, ++step) {
+              const int slot = step % kSplitSlots;
+              ok = ok && barrier_wait_warp(&step_full[slot], (step / kSplitSlots) & 1, status);
+              if (!ok) break;
+              tc_fence_after_sync();
+              if (elect_one()) {
+                const uint64_t at = desc + (((slot >> 1) * kSplitStageBytes + half * kSplitStep * 2) >> 4);
+                constexpr uint64_t plane = kSplitPlaneBytes >> 4;
 #pragma unroll
-              for (int kk = 0; kk < kSplitStep / 16; ++kk) {
-                const uint64_t x = at + kk * 2, y = x + 3 * plane;
-                tc_mma(tmem_small, x, y + 2 * plane, idesc, chunk > begin || half > 0 || kk > 0 ? 1u : 0u);
-                tc_mma(tmem_small, x + 2 * plane, y, idesc, 1u);
-                tc_mma(tmem_small, x + plane, y + plane, idesc, 1u);
-                tc_mma(tmem_small, x, y + plane, idesc, 1u);
-                tc_mma(tmem_small, x + plane, y, idesc, 1u);
-                tc_mma(tmem_large, x, y, idesc, half > 0 || kk > 0 ? 1u : 0u);
+                for (int kk = 0; kk < kSplitStep / 16; ++kk) {
+                  const uint64_t x = at + kk * 2, y = x + 3 * plane;
+                  tc_mma(tmem_small, x, y + 2 * plane, idesc, chunk > begin || half > 0 || kk > 0 ? 1u : 0u);
+                  tc_mma(tmem_small, x + 2 * plane, y, idesc, 1u);
+                  tc_mma(tmem_small, x + plane, y + plane, idesc, 1u);
+                  tc_mma(tmem_small, x, y + plane, idesc, 1u);
+                  tc_mma(tmem_small, x + plane, y, idesc, 1u);
+                  tc_mma(tmem_large, x, y, idesc, half > 0 || kk > 0 ? 1u : 0u);
+                }
+                tc_commit(&step_empty[slot]);
+                if (half == 1) tc_commit(&large_full[buffer]);   // the last one of a tile covers its small sums too
               }
-              tc_commit(&step_empty[slot]);
-              if (half == 1) tc_commit(&large_full[buffer]);   // the last one of a tile covers its small sums too
             }
           }
         }
@@ -207,62 +221,100 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
     // ---- adders: two warps per 32 rows, 64 columns each
     const int lane_base = (warp & 3) * 32, columns = ((warp - 4) >> 2) * 64;
     const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + columns;
+    float* turned = reinterpret_cast<float*>(stages + 2 * kSplitStageBytes) + (warp - 4) * 32 * kSplitPutPitch;
     int chunk_count = 0, local = 0;
     bool ok = true, odd = false;
-    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local) {
-      const int split = unit / m_tiles % splits;
-      const int begin = first_chunk(split), end = first_chunk(split + 1);
-      float acc[64];
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      for (int group = first_group(unit, 0), last = first_group(unit, 1); group < last; ++group, ++local) {
+        const int begin = first_chunk(group), end = first_chunk(group + 1);
+        float acc[64];
 #pragma unroll
-      for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
-      for (int chunk = begin; chunk < end; ++chunk, ++chunk_count) {
-        const int buffer = chunk_count & 1;
-        if (!barrier_wait_warp(&large_full[buffer], (chunk_count >> 1) & 1, status) || given_up(failed)) { ok = false; break; }
-        tc_fence_after_sync();
+        for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
+        for (int chunk = begin; chunk < end; ++chunk, ++chunk_count) {
+          const int buffer = chunk_count & 1;
+          if (!barrier_wait_warp(&large_full[buffer], (chunk_count >> 1) & 1, status) || given_up(failed)) { ok = false; break; }
+          tc_fence_after_sync();
+#pragma unroll
+          for (int part = 0; part < 4; ++part) {
+            uint32_t sum[16];
+            tc_load_16(tmem_lane + buffer * kSplitTile + part * 16, sum);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(sum[i]);
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) barrier_arrive(&large_empty[buffer]);
+        }
+        if (!ok) break;
 #pragma unroll
         for (int part = 0; part < 4; ++part) {
           uint32_t sum[16];
-          tc_load_16(tmem_lane + buffer * kSplitTile + part * 16, sum);
+          tc_load_16(tmem_lane + (2 + small_of(local)) * kSplitTile + part * 16, sum);
 #pragma unroll
           for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(sum[i]);
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) barrier_arrive(&large_empty[buffer]);
-      }
-      if (!ok) break;
+        if (lane == 0) barrier_arrive(&small_empty[small_of(local)]);
+        if (chained && group > 0) {   // eight columns at a time: sixteen did not leave the other roles their registers
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        uint32_t sum[16];
-        tc_load_16(tmem_lane + 2 * kSplitTile + (local & 1) * kSplitTile + part * 16, sum);
+          for (int part = 0; part < 64; part += 8) {
+            uint32_t sum[8];
+            tc_load_8(tmem_lane + 3 * kSplitTile + part, sum);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(sum[i]);
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) barrier_arrive(&small_empty[local & 1]);
-      const int row = unit % m_tiles * kSplitTile + lane_base + lane;
-      const int column = unit / m_tiles / splits * kSplitTile + columns;
-      if (row < m) {
-        float* to = splits > 1 ? scratch + (static_cast<long long>(split) * m + row) * n + column : c + row * ldc + column;
-        if (column + 64 <= n && (reinterpret_cast<uintptr_t>(to) & 15) == 0) {
-#pragma unroll
-          for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (column + i < n) to[i] = acc[i];
+            for (int i = 0; i < 8; ++i) acc[part + i] += __uint_as_float(sum[i]);
+          }
         }
-        float worst = 0.0f;   // stays finite, or becomes NaN
+        if (chained && group + 1 < last) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) worst += 0.0f * acc[i];
-        odd = odd || worst != 0.0f;
+          for (int part = 0; part < 64; part += 8) {
+            uint32_t sum[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sum[i] = __float_as_uint(acc[part + i]);
+            tc_store_8(tmem_lane + 3 * kSplitTile + part, sum);
+          }
+          tc_store_wait();
+        } else {
+          const int row0 = unit % m_tiles * kSplitTile + lane_base, column0 = unit / m_tiles / slices * kSplitTile + columns;
+          float* to = slices > 1 ? scratch + static_cast<long long>(group) * m * n : c;
+          const long long ld = slices > 1 ? n : ldc;
+          const bool quads = (reinterpret_cast<uintptr_t>(to) & 15) == 0 && ld % 4 == 0;
+          float worst = 0.0f;   // stays finite, or becomes NaN
+          // 16 columns at a time by way of shared memory, so that a store takes 64 bytes of eight rows and not 16 of all 32,
+          // which kept the adders some 4 us a tile.
+#pragma unroll
+          for (int part = 0; part < 4; ++part) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+              *reinterpret_cast<float4*>(turned + lane * kSplitPutPitch + i) =
+                  make_float4(acc[part * 16 + i], acc[part * 16 + i + 1], acc[part * 16 + i + 2], acc[part * 16 + i + 3]);
+            __syncwarp();
+            const int column = column0 + part * 16 + (lane & 3) * 4;
+#pragma unroll 1
+            for (int r = lane >> 2; r < 32; r += 8) {
+              const float4 x = *reinterpret_cast<const float4*>(turned + r * kSplitPutPitch + (lane & 3) * 4);
+              if (row0 + r < m) {
+                worst += 0.0f * x.x + 0.0f * x.y + 0.0f * x.z + 0.0f * x.w;
+                float* at = to + (row0 + r) * ld + column;
+                if (quads && column + 4 <= n) {
+                  *reinterpret_cast<float4*>(at) = x;
+                } else {
+                  if (column < n) at[0] = x.x;
+                  if (column + 1 < n) at[1] = x.y;
+                  if (column + 2 < n) at[2] = x.z;
+                  if (column + 3 < n) at[3] = x.w;
+                }
+              }
+            }
+            __syncwarp();   // the next 16 columns go where these were; tensor memory is loaded by the warp as a whole
+          }
+          odd = odd || worst != 0.0f;
+        }
       }
-      __syncwarp();   // rows behind the last one are here first; the next unit's loads take the warp as a whole
     }
     if (!ok) failed = 1;
     // Every product of the block's is finished where all of these waits ended: nothing reads or writes the stages any more.
-    if (splits == 1 && again_any(odd) && !again_any(!ok)) {
+    if (slices == 1 && again_any(odd) && !again_any(!ok)) {
       const int t = threadIdx.x - 4 * 32;
       for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
         const int col0 = unit / m_tiles * kSplitTile;
@@ -297,9 +349,8 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
     const float* rows[8];   // of A and of W that this thread brings; rows behind the last one bring that one again
     int unit = blockIdx.x, at = 0, last = 0;   // the step that is fetched next
     auto open = [&]() {
-      const int split = unit / m_tiles % splits;
-      at = first_chunk(split) * 2, last = first_chunk(split + 1) * 2;
-      const int rows_a = unit % m_tiles * kSplitTile + row_in, rows_w = unit / m_tiles / splits * kSplitTile + row_in;
+      at = first_chunk(first_group(unit, 0)) * 2, last = first_chunk(first_group(unit, 1)) * 2;
+      const int rows_a = unit % m_tiles * kSplitTile + row_in, rows_w = unit / m_tiles / slices * kSplitTile + row_in;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         rows[i] = a + min(rows_a + i * 32, m - 1) * lda;
@@ -384,17 +435,17 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kSplitTmemColumns) : "memory");
 }
 
-// The parts of k, in order: a block a tile of 32 x 128.
+// The groups of k, in order: a block a tile of 32 x 128.
 __global__ void __launch_bounds__(kAgainThreads)
-gemm_float_parts_kernel(float* __restrict__ c, const float* __restrict__ scratch, const float* __restrict__ a,
-                        const float* __restrict__ w, int m, int n, int k, long long lda, long long ldw, long long ldc, int splits) {
+gemm_float_groups_kernel(float* __restrict__ c, const float* __restrict__ scratch, const float* __restrict__ a,
+                        const float* __restrict__ w, int m, int n, int k, long long lda, long long ldw, long long ldc, int groups) {
   __shared__ __align__(16) float shared[kAgainShared];
   const int t = threadIdx.x, row0 = blockIdx.x * kAgainRows, col0 = blockIdx.y * kAgainColumns;
   const size_t all = static_cast<size_t>(m) * n;
   const bool quads = n % 4 == 0;
   float v[2][8] = {};
 #pragma unroll 4
-  for (int s = 0; s < splits; ++s)   // the loads of several parts are under way at once
+  for (int s = 0; s < groups; ++s)   // the loads of several groups are under way at once
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -431,29 +482,42 @@ gemm_float_parts_kernel(float* __restrict__ c, const float* __restrict__ scratch
 
 using namespace mxb;
 
-// Into how many parts k is cut, so that few tiles still give every SM work: the fewest rounds of 148 blocks, each with a
-// start worth about two chunks and, with several parts, a pass that adds them up (worth about six).
-MXB_API int mxb_gemm_float_split_parts(int m, int n, int k) {
+// Into how many groups the sums over k are cut: by n and k alone, so that a row of A has the same bits whatever else is in the
+// batch. As many as one round of 148 blocks takes where there is one tile of rows, none shorter than four chunks.
+MXB_API int mxb_gemm_float_split_groups(int n, int k) {
+  const int chunks = ceil_div(k, kSplitChunk), fitting = 148 / ceil_div(n, kSplitTile);
+  const int most = chunks / 4 < 8 ? chunks / 4 : 8;
+  const int groups = fitting < most ? fitting : most;
+  return groups > 1 ? groups : 1;
+}
+
+// How the groups are dealt out: all to the block of their tile, which adds them up as it goes (1), or in slices to several
+// blocks, which leave each group's sums in scratch for a second kernel. The fewest rounds of 148 blocks, each with a start
+// worth about two chunks (a chunk is 2.1 us); with several slices the second kernel (worth three) and the sums' way through
+// memory, 30 MB a chunk. us with one slice and with the best number: 917 rows x 1024 x 2048 74 and 50 (2 slices), x 1024 x 3072
+// 104 and 65 (2), x 4096 x 1024 77 and 77 (1); 8 rows 75 and 20 (8), 106 and 24 (8), 42 and 19 (4).
+MXB_API int mxb_gemm_float_split_slices(int m, int n, int k) {
   const long long tiles = static_cast<long long>(ceil_div(m, kSplitTile)) * ceil_div(n, kSplitTile);
-  const int chunks = ceil_div(k, kSplitChunk);
+  const int chunks = ceil_div(k, kSplitChunk), groups = mxb_gemm_float_split_groups(n, k);
   int best = 1;
   long long least = 0;
-  for (int parts = 1; parts <= 8 && parts * 4 <= chunks; ++parts) {
-    const long long cost = (tiles * parts + 147) / 148 * (ceil_div(chunks, parts) + 2) + (parts > 1 ? 6 : 0);
-    if (parts == 1 || cost < least) least = cost, best = parts;
+  for (int slices = 1; slices <= groups; ++slices) {
+    const long long through_memory = slices > 1 ? 3 + 8LL * groups * m * n / 30000000 : 0;
+    const long long cost = (tiles * slices + 147) / 148 * (ceil_div(ceil_div(groups, slices) * chunks, groups) + 2) + through_memory;
+    if (slices == 1 || cost < least) least = cost, best = slices;
   }
   return best;
 }
 
-// c, a, w float32; k and the row strides of a and w multiples of 4, a and w on 16 bytes; scratch: parts * m * n float32 where
-// parts > 1.
+// c, a, w float32; k and the row strides of a and w multiples of 4, a and w on 16 bytes; scratch: groups * m * n float32 where
+// slices > 1.
 MXB_API int mxb_gemm_float_split(void* c, const void* a, const void* w, int m, int n, int k, long long lda, long long ldw,
-                                 long long ldc, int parts, float* scratch, int* status, cudaStream_t stream) {
+                                 long long ldc, int groups, int slices, float* scratch, int* status, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (k <= 0 || k % 4 != 0 || lda % 4 != 0 || ldw % 4 != 0 || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0 ||
-      parts < 1 || parts > ceil_div(k, kSplitChunk) || (parts > 1 && scratch == nullptr))
+      groups < 1 || groups > ceil_div(k, kSplitChunk) || slices < 1 || slices > groups || (slices > 1 && scratch == nullptr))
     return static_cast<int>(cudaErrorInvalidValue);
-  const long long units = static_cast<long long>(ceil_div(m, kSplitTile)) * ceil_div(n, kSplitTile) * parts;
+  const long long units = static_cast<long long>(ceil_div(m, kSplitTile)) * ceil_div(n, kSplitTile) * slices;
   if (units > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   int device = 0, sms = 0;
   cudaGetDevice(&device);
@@ -463,10 +527,10 @@ MXB_API int mxb_gemm_float_split(void* c, const void* a, const void* w, int m, i
   float* to = static_cast<float*>(c);
   const float *x = static_cast<const float*>(a), *weight = static_cast<const float*>(w);
   gemm_float_split_kernel<<<static_cast<int>(units < sms ? units : sms), kSplitThreads, kSplitSharedBytes, stream>>>(
-      to, x, weight, m, n, k, lda, ldw, ldc, parts, scratch, status);
+      to, x, weight, m, n, k, lda, ldw, ldc, groups, slices, scratch, status);
   e = cudaGetLastError();
-  if (e != cudaSuccess || parts == 1) return static_cast<int>(e);
-  gemm_float_parts_kernel<<<dim3(ceil_div(m, kAgainRows), ceil_div(n, kAgainColumns)), kAgainThreads, 0, stream>>>(
-      to, scratch, x, weight, m, n, k, lda, ldw, ldc, parts);
+  if (e != cudaSuccess || slices == 1) return static_cast<int>(e);
+  gemm_float_groups_kernel<<<dim3(ceil_div(m, kAgainRows), ceil_div(n, kAgainColumns)), kAgainThreads, 0, stream>>>(
+      to, scratch, x, weight, m, n, k, lda, ldw, ldc, groups);
   return static_cast<int>(cudaGetLastError());
 }

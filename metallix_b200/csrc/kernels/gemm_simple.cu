@@ -1,9 +1,9 @@
 // C[M, N] = A[M, K] * W[N, K]^T on CUDA cores with float32 accumulation.
 //
-// This is the 32-bit matrix product of the float32 path where sums keep one
-// order or matrices are small (large products of models whose attention has no
-// such order go to gemm_float_split.cu) and the plain twin of the tensor-core
-// kernels. Every output element sums its K products in ascending k, in the
+// This is the 32-bit matrix product of the float32 path, but for the large
+// products of portions of prompts in models whose attention adds these up in
+// another order than single tokens (gemm_float_split.cu), and the plain twin of
+// the tensor-core kernels. Every output element sums its K products in ascending k, in the
 // same order whatever M is, so a row's result does not depend on what else is
 // in the batch. W is [out, in] row-major and applied as x W^T, as in the
 // reference's projection (crates/models/qwen/src/forward/projection.rs:257-265).

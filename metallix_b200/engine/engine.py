@@ -24,7 +24,7 @@ import torch
 from .. import ops
 from ..cache import PagedCache
 from ..config import read_config
-from ..parts.registry import Runtime, StepContext, StepPlan, step_preparers
+from ..parts.registry import Runtime, StepContext, StepPlan, row_runs, step_preparers
 from ..weights import load_tensors, random_tensors
 from .model import DecoderModel
 
@@ -466,7 +466,8 @@ class Engine:
                 positions=d_positions, token_request=d_token_request, request_slots=d_request_slots,
                 # inside a graph the host's view of one step would be baked in for all
                 request_offsets=None if graphed else [int(v) for v in offsets],
-                request_positions=None if graphed else starts, extras=extras)
+                request_positions=None if graphed else starts, extras=extras,
+                runs=None if self.runtime.ordered_sums or self.dtype != torch.float32 else row_runs(counts))
             return self.model.forward(
                 d_ids, ctx, lambda entry, write: cache.view(entry, write, tables, slots),
                 d_wanted if wanted else None, tap=tap)

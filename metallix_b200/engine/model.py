@@ -82,15 +82,19 @@ class DecoderModel:
         if self.joins:
             first = residual if self.order[0].join is not None else residual.clone()
         pending = None
-        for index, run in enumerate(self.order):
-            block = self.blocks[run.layer]
-            if run.join is not None:
-                residual, pending = self.joins[run.join].forward(residual, pending, first, run.turn)
-            pending = block.forward(residual, pending, ctx, views(run.cache_entry(), run.write_cache))
-            if tap is not None:
-                settle(residual, pending)
-                pending = None
-                tap(index, sum_of_streams(residual) if streams else residual)
+        self.runtime.runs = ctx.runs   # through the layers, whose products are of the step's rows; the head's are not
+        try:
+            for index, run in enumerate(self.order):
+                block = self.blocks[run.layer]
+                if run.join is not None:
+                    residual, pending = self.joins[run.join].forward(residual, pending, first, run.turn)
+                pending = block.forward(residual, pending, ctx, views(run.cache_entry(), run.write_cache))
+                if tap is not None:
+                    settle(residual, pending)
+                    pending = None
+                    tap(index, sum_of_streams(residual) if streams else residual)
+        finally:
+            self.runtime.runs = None
         if wanted_rows is None or wanted_rows.numel() == 0:
             return None
         if streams:   # what is pending joins, the streams are summed and normed, on the wanted rows only

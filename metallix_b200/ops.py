@@ -109,8 +109,9 @@ _SIGNATURES = {
     "mxb_flash_prefill_tcgen05_supported": [_I, _I, _I, _I, _I],
     "mxb_flash_prefill_tcgen05_tile": [],
     "mxb_gemm_simple": [_P, _I, _P, _P, _I, _I, _I, _I, _L, _L, _L, _P],
-    "mxb_gemm_float_split": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _P, _P, _P],
-    "mxb_gemm_float_split_parts": [_I, _I, _I],
+    "mxb_gemm_float_split": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _P, _P, _P],
+    "mxb_gemm_float_split_groups": [_I, _I],
+    "mxb_gemm_float_split_slices": [_I, _I, _I],
     "mxb_gemm_skinny": [_P, _I, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _F, _P],
     "mxb_gemm_skinny_supported": [_I, _I, _I, _L, _L],
     "mxb_gemm_stream": [_P, _I, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _F, _P, _P],
@@ -1735,7 +1736,8 @@ def gemm_simple(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
 def gemm_float(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a [m, k] times w [n, k] transposed of float32 operands on the tensor
     cores: each number as three bfloat16 parts, sums of 64 products at a time
-    added up in float32 (closer to 64 bits than a float32 sum in ascending k)."""
+    added up in float32 (closer to 64 bits than a float32 sum in ascending k).
+    A row's bits do not depend on the other rows."""
     _need(a.is_cuda and w.is_cuda, "operands must be on a CUDA device")
     _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "shapes do not match a @ w.T")
     _need(a.dtype == torch.float32 and w.dtype == torch.float32, "operands must be float32")
@@ -1744,25 +1746,26 @@ def gemm_float(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
     if out is None:
         out = torch.empty((m, n), dtype=torch.float32, device=a.device)
     _need(out.shape == (m, n) and out.dtype == torch.float32 and out.stride(1) == 1, "out does not fit")
-    parts = _fn("mxb_gemm_float_split_parts")(m, n, k)
-    scratch = torch.empty(parts * m * n, dtype=torch.float32, device=a.device) if parts > 1 else None
+    groups, slices = _fn("mxb_gemm_float_split_groups")(n, k), _fn("mxb_gemm_float_split_slices")(m, n, k)
+    scratch = torch.empty(groups * m * n, dtype=torch.float32, device=a.device) if slices > 1 else None
     _call("mxb_gemm_float_split", out.data_ptr(), a.data_ptr(), w.data_ptr(), m, n, k, a.stride(0), w.stride(0),
-          out.stride(0), parts, _ptr(scratch), status_word(a.device).data_ptr(), _stream())
-    if parts > 1:
+          out.stride(0), groups, slices, _ptr(scratch), status_word(a.device).data_ptr(), _stream())
+    if slices > 1:
         global _launches
-        _launches += 1   # the kernel that adds the parts up
+        _launches += 1   # the kernel that adds the groups up
     return out
 
 
-# Rows of A from which float32 products of at least this many rows of W and values each go to the tensor cores, us against the
-# CUDA cores' kernels: 9 rows x 4096 x 1024 14.3 and 25.2, x 1024 x 2048 14.4 and 48.0, x 151936 x 1024 307 and 436; 917 rows 70 and
-# 213, 43 and 129; but 400 x 512 x 512 21 and 20, 256 x 1024 x 512 21 and 19.
-FLOAT_ROWS, FLOAT_SIDE = 9, 1024
+# Float32 products with at least this many rows of W and values each go to the tensor cores where they are of a prompt's
+# rows, us against the CUDA cores' kernels: 917 rows x 4096 x 1024 77 and 213, x 1024 x 2048 50 and 128; 16 rows 19 and 48, 20
+# and 97; but 8 rows 19 and 17, 20 and 12, and 400 x 512 x 1024 19 and 39, 64 x 768 x 768 17 and 31, 8 x 768 x 768 15 and 5. The
+# number of rows has no say: a row's bits would depend on what else is in the step.
+FLOAT_SIDE = 1024
 
 
 def gemm_float_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the tensor cores make this float32 product faster."""
-    return gemm_float_supported(a, w) and a.shape[0] >= FLOAT_ROWS and min(w.shape) >= FLOAT_SIDE
+    """Whether float32 products of a prompt's rows with ``w`` go to the tensor cores."""
+    return min(w.shape) >= FLOAT_SIDE and gemm_float_supported(a, w)
 
 
 def gemm_float_supported(a: torch.Tensor, w: torch.Tensor) -> bool:

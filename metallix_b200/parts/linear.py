@@ -1,7 +1,9 @@
 """x @ W^T for a weight ``[out, in]`` (the reference's one path from a weight
 name to a matmul, crates/models/qwen/src/forward/projection.rs:257-265).
 
-float32 runs on the hand-written CUDA-core kernel (true 32-bit, fixed order).
+float32 runs on the hand-written CUDA-core kernel (true 32-bit, fixed order),
+or, for large products of a prompt's rows, on the tensor cores in three
+bfloat16 parts a number (``Runtime.ordered_sums``).
 bfloat16 runs on the hand-written tcgen05 kernel where its shape rules hold,
 else on the library product (the reference itself calls a library matmul
 here), or on the plain CUDA-core kernel when asked.
@@ -24,7 +26,7 @@ class Linear:
         self.out_features, self.in_features = self.weight.shape
         self.dtype = runtime.dtype
         self.backend = runtime.gemm_backend
-        self.runtime = runtime   # a part that is built later may change what it says of sums
+        self.runtime = runtime   # a part that is built later may change what it says of sums, a step what it says of rows
 
     @classmethod
     def stacked(cls, weights: Sequence[torch.Tensor], runtime: Runtime) -> "Linear":
@@ -36,10 +38,21 @@ class Linear:
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
         out_dtype = out_dtype or self.dtype
         if self.dtype == torch.float32:
-            if not self.runtime.ordered_sums and ops.gemm_float_takes(x, self.weight):
-                return ops.gemm_float(x, self.weight, out=out)
-            return ops.gemm_simple(x, self.weight, out_dtype=torch.float32, out=out)
+            return self._float32(x, out)
         return ops.gemm_bf16(x, self.weight, out_dtype=out_dtype, backend=self.backend, out=out)
+
+    def _float32(self, x: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:
+        """Single tokens in ascending order; rows of portions, where large enough matrices make that faster, on the tensor
+        cores. Both give a row the same bits whatever other rows come with it, so a request's do not depend on what else a
+        step holds, nor on how its prompt was cut into portions of several tokens."""
+        runs = self.runtime.runs
+        if runs is None or runs[-1][1] != x.shape[0] or not ops.gemm_float_takes(x, self.weight):
+            return ops.gemm_simple(x, self.weight, out_dtype=torch.float32, out=out)
+        if out is None:
+            out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)
+        for begin, end, several in runs:
+            (ops.gemm_float if several else ops.gemm_simple)(x[begin:end], self.weight, out=out[begin:end])
+        return out
 
     def rows_are_short(self) -> bool:
         """Whether this is a weight of the kind whose decode-step products are

@@ -58,8 +58,12 @@ class Runtime:
     # (tables of a position encoding, say), by a key of those parameters.
     shared: Dict[tuple, object] = field(default_factory=dict)
     # Whether float32 sums have one order however a step is cut, so that every cut gives the same bits. An attention whose
-    # single tokens and portions run on kernels of different orders says no; then large products may take the tensor cores.
+    # single tokens and portions run on kernels of different orders says no; then large products of portions take the tensor
+    # cores, in an order that what else is in the step does not change.
     ordered_sums: bool = True
+    # During a step through the layers, where ordered_sums is False: the step's packed rows as runs (first row, row behind the
+    # last, whether they are of portions of several tokens). A row's kernel follows from its own request's portion alone.
+    runs: Optional[Sequence[Tuple[int, int, bool]]] = None
 
 
 class WeightStore:
@@ -200,6 +204,18 @@ class StepContext:
     request_positions: Optional[List[int]]  # host, first position of each row's tokens
     extras: Dict[str, object] = field(default_factory=dict)
     token_ids: Optional[torch.Tensor] = None   # int32 [tokens]: the step's token ids, for a part that reads a table by them
+    runs: Optional[List[Tuple[int, int, bool]]] = None   # host: as Runtime.runs
+
+
+def row_runs(counts: Sequence[int]) -> List[Tuple[int, int, bool]]:
+    """The packed rows of requests that bring ``counts`` tokens, as runs of rows of one kind: (first row, row behind the last
+    one, whether they belong to portions of several tokens)."""
+    runs, begin = [], 0
+    for count in counts:
+        first = runs.pop()[0] if runs and runs[-1][2] == (count > 1) else begin
+        begin += count
+        runs.append((first, begin, count > 1))
+    return runs
 
 
 def step_preparers(blocks) -> Dict[str, object]:

@@ -1172,6 +1172,17 @@ def test_float32_products_of_rows_that_are_not_finite(ops, m, n, k):
     assert torch.equal(out[same][:, columns], clean[same][:, columns])
 
 
+@pytest.mark.parametrize("n, k", [(1024, 2048), (1030, 3076), (4096, 1024), (6144, 1028), (20000, 72)])
+def test_float32_products_keep_a_rows_bits_among_others(ops, n, k):
+    """One tile of rows with its groups of k in many blocks, several with them in few, in one and in the tiles' own."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x, w = torch.randn(1300, k, generator=gen, device="cuda"), torch.randn(n, k, generator=gen, device="cuda")
+    every = ops.gemm_float(x, w)
+    for begin, end in ((0, 1), (5, 7), (3, 12), (100, 228), (1, 300), (200, 840), (0, 917)):
+        assert torch.equal(ops.gemm_float(x[begin:end], w), every[begin:end]), (begin, end)
+    ops.check_status("cuda")
+
+
 def test_float32_products_of_two_threads(ops):
     """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
     import threading

@@ -106,6 +106,80 @@ def test_a_mixed_step_replays_a_graph(model_folders, name, dtype):
     assert drift < cut_limit
 
 
+# Matrices large enough for the float32 products on the tensor cores, heads of the split-key decode kernel.
+WIDE = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_act="silu", num_hidden_layers=2, hidden_size=1024,
+            num_attention_heads=16, num_key_value_heads=8, head_dim=64, intermediate_size=1100, vocab_size=500,
+            rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True, max_position_embeddings=512)
+
+
+def wide_engine(**options):
+    from metallix_b200 import Qwen3Config
+    from metallix_b200.engine import Engine
+    return Engine.from_random(Qwen3Config.from_dict(WIDE), 5, dtype="float32", max_tokens=8192, **options)
+
+
+def test_float32_bits_do_not_depend_on_the_batch_or_the_portions(monkeypatch):
+    """Heads whose single tokens have a kernel of their own: a prompt's logits are the same in portions of several tokens,
+    beside decoded tokens of others and alone; a decoded token's alone, among eleven others and beside portions."""
+    from metallix_b200 import ops
+    from metallix_b200.engine import StepEntry
+    launched, product = [], ops.gemm_float
+    monkeypatch.setattr(ops, "gemm_float", lambda *a, **k: (launched.append(1), product(*a, **k))[1])
+    engine = wide_engine(cuda_graphs=False)
+    ids = [random_ids(40 + i, 150, 500) for i in range(12)]
+
+    def in_portions(sizes, beside=()):
+        seen, at = [], 0
+        for size in sizes:
+            entries = [StepEntry(name, [t], []) for name, t in beside[:1]]
+            entries += [StepEntry("p", ids[0][at:at + size], list(range(size)))]
+            entries += [StepEntry(name, [t], []) for name, t in beside[1:]]
+            seen.append(engine.step(entries).clone())
+            at += size
+        engine.release("p")
+        return torch.cat(seen)
+
+    whole = in_portions([150])
+    assert launched
+    assert torch.equal(whole, in_portions([128, 22])) and torch.equal(whole, in_portions([2, 7, 9, 3, 129]))
+    contexts = {f"r{i}": ids[i][:100] for i in range(12)}
+    for name, tokens in contexts.items():
+        engine.step([StepEntry(name, tokens, [])])
+    assert torch.equal(whole, in_portions([90, 60], [(f"r{i}", 7) for i in range(11)]))
+    for name in contexts:
+        engine.release(name)
+
+    def decoded(names, beside=None):
+        for name in names:
+            engine.step([StepEntry(name, contexts[name], [])])
+        out = []
+        for step in range(3):
+            entries = [StepEntry(name, [ids[int(name[1:])][100 + step]], [0]) for name in names]
+            if beside is not None:
+                entries.insert(1, StepEntry("p", ids[11][20 * step:20 * step + 20], []))
+            out.append(engine.step(entries)[0].clone())
+        engine.release_all()
+        return torch.stack(out)
+
+    alone = decoded(["r0"])
+    for among in (decoded(list(contexts)), decoded(["r0", "r5"]), decoded(["r0", "r5", "r6"], beside=True)):
+        assert torch.equal(alone, among)
+    engine.check()
+
+
+def test_float32_bits_are_the_same_in_captured_steps():
+    from metallix_b200.engine import StepEntry
+    ids, seen = [random_ids(60 + i, 200, 500) for i in range(3)], {}
+    for graphs in (True, False):
+        engine = wide_engine(cuda_graphs=graphs)
+        engine.step([StepEntry("a", ids[0][:30], [])])
+        seen[graphs] = [engine.step([StepEntry("a", [ids[0][30 + n]], [0]), StepEntry("b", ids[1][16 * n:16 * n + 16], [15]),
+                                     StepEntry("c", ids[2][5 * n:5 * n + 5], [4])]).clone() for n in range(5)]
+        engine.check()
+        assert not graphs or len(engine._step_graphs) == 1
+    assert all(torch.equal(x, y) for x, y in zip(seen[True], seen[False]))
+
+
 def test_more_shapes_than_graphs_are_kept(model_folders):
     """Ten shapes, each stepped twice (the second time captures), then the
     first shape again: its graph has made room meanwhile and is captured
