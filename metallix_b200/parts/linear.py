@@ -46,7 +46,7 @@ class Linear:
         cores. Both give a row the same bits whatever other rows come with it, so a request's do not depend on what else a
         step holds, nor on how its prompt was cut into portions of several tokens."""
         runs = self.runtime.runs
-        if runs is None or runs[-1][1] != x.shape[0] or not ops.gemm_float_takes(x, self.weight):
+        if runs is None or runs[-1][1] != x.shape[0] or self.backend != "auto" or not ops.gemm_float_takes(x, self.weight):
             return ops.gemm_simple(x, self.weight, out_dtype=torch.float32, out=out)
         if out is None:
             out = torch.empty((x.shape[0], self.out_features), dtype=torch.float32, device=x.device)

@@ -53,13 +53,15 @@ class Runtime:
     device: torch.device
     dtype: torch.dtype          # compute dtype: torch.bfloat16 or torch.float32
     max_positions: int          # longest context the engine will run
-    gemm_backend: str = "auto"  # how bfloat16 matrix products run: auto | tcgen05 | cublas | simple
+    # How bfloat16 matrix products run: auto | tcgen05 | cublas | simple. In float32 anything but auto means the general
+    # product in ascending order throughout.
+    gemm_backend: str = "auto"
     # Read-only tensors that parts built from equal parameters may share
     # (tables of a position encoding, say), by a key of those parameters.
     shared: Dict[tuple, object] = field(default_factory=dict)
     # Whether float32 sums have one order however a step is cut, so that every cut gives the same bits. An attention whose
     # single tokens and portions run on kernels of different orders says no; then large products of portions take the tensor
-    # cores, in an order that what else is in the step does not change.
+    # cores (with gemm_backend "auto"), in an order that what else is in the step does not change.
     ordered_sums: bool = True
     # During a step through the layers, where ordered_sums is False: the step's packed rows as runs (first row, row behind the
     # last, whether they are of portions of several tokens). A row's kernel follows from its own request's portion alone.

@@ -167,6 +167,19 @@ def test_float32_bits_do_not_depend_on_the_batch_or_the_portions(monkeypatch):
     engine.check()
 
 
+def test_a_caller_who_asks_for_the_general_product_gets_it_in_float32(monkeypatch):
+    """What checks the other kernels (``--verify-cache``) must not run on them."""
+    from metallix_b200 import ops
+    from metallix_b200.engine import StepEntry
+    ids = random_ids(77, 40, 500)
+    fast = wide_engine().step([StepEntry("a", ids, list(range(40)))]).clone()
+    monkeypatch.setattr(ops, "gemm_float", lambda *a, **k: pytest.fail("not the general product"))
+    engine = wide_engine(gemm_backend="simple")
+    general = engine.step([StepEntry("a", ids, list(range(40)))])
+    engine.check()
+    assert not torch.equal(fast, general) and float((fast - general).abs().max()) < TOL_F32
+
+
 def test_float32_bits_are_the_same_in_captured_steps():
     from metallix_b200.engine import StepEntry
     ids, seen = [random_ids(60 + i, 200, 500) for i in range(3)], {}
