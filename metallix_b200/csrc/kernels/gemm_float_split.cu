@@ -21,7 +21,9 @@
 // rows left room for, 917 rows took 70, 105, 43 and 58 us of the first four.)
 //
 // A number that is not finite, or too near the largest, has no such parts (infinity minus infinity), and leaves an output that is
-// not finite: such outputs are made again in float32 and ascending k, with the general product's bits, tile by tile, by the
+// not finite. A number below 2^-102 has parts that bfloat16 holds with fewer bits or not at all, which leaves up to 2^-126 of it
+// out: 2^-24 of an output from 2^-60 on, as long as the other operands add up to no more than 2^42. Outputs that are not finite, or nearer 0 but
+// not 0, are made again in float32 and ascending k, with the general product's bits, tile by tile, by the
 // adders of a block once it has walked all of its tiles (nobody waits for them any more), or by the kernel that adds the groups up.
 // 917 rows x 4096 x 1024: 77 us, some 90 more with a row of NaN, 680 more with nothing else (the CUDA cores' kernel 213).
 //
@@ -46,7 +48,11 @@ constexpr int kSplitSharedBytes = 2 * kSplitStageBytes + kSplitPutBytes + 1024;
 constexpr int kSplitThreads = 32 * (4 + kSplitAdders + kSplitSplitters);   // warpgroups: one that issues, two and two
 constexpr int kSplitTmemColumns = 512;   // large sums twice, then small sums twice, or once and the sum of the groups so far
 
-__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= FLT_MAX; }
+constexpr float kSplitLeast = 8.67361738e-19f;   // 2^-60
+
+// An output that the parts cannot be trusted with: not finite, or so near 0 (but not 0, which rows of zeros give) that it may
+// be made of numbers whose smallest parts bfloat16 does not reach.
+__device__ __forceinline__ bool is_doubtful(float x) { return !(fabsf(x) <= FLT_MAX) || (fabsf(x) < kSplitLeast && x != 0.0f); }
 
 // Two numbers' leading bfloat16 parts, packed; the numbers become what that left.
 __device__ __forceinline__ uint32_t split_pair(float& x, float& y) {
@@ -78,14 +84,14 @@ __device__ __forceinline__ bool again_any(bool mine) {
 __device__ __forceinline__ int again_row(int t, int i) { return (t >> 4) * 2 + i; }
 __device__ __forceinline__ int again_column(int t, int j) { return (t & 15) * 4 + (j >> 2) * 64 + (j & 3); }
 
-// The tile's outputs that are not finite, as sums in ascending k; v are this thread's. False where there are none.
+// The tile's doubtful outputs, as sums in ascending k; v are this thread's. False where there are none.
 __device__ __forceinline__ bool make_again(float (&v)[2][8], float* shared, int t, int row0, int col0, const float* __restrict__ a,
                                            const float* __restrict__ w, int m, int n, int k, long long lda, long long ldw) {
   bool odd = false;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) odd = odd || !is_finite(v[i][j]);
+    for (int j = 0; j < 8; ++j) odd = odd || is_doubtful(v[i][j]);
   if (!again_any(odd)) return false;
   float* sA = shared;                                  // [kAgainK][kAgainRows + 4]
   float* sW = shared + kAgainK * (kAgainRows + 4);     // [kAgainK][kAgainColumns + 4]
@@ -121,7 +127,7 @@ __device__ __forceinline__ bool make_again(float (&v)[2][8], float* shared, int 
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (!is_finite(v[i][j])) v[i][j] = acc[i][j];
+      if (is_doubtful(v[i][j])) v[i][j] = acc[i][j];
   return true;
 }
 
@@ -279,7 +285,6 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
           float* to = slices > 1 ? scratch + static_cast<long long>(group) * m * n : c;
           const long long ld = slices > 1 ? n : ldc;
           const bool quads = (reinterpret_cast<uintptr_t>(to) & 15) == 0 && ld % 4 == 0;
-          float worst = 0.0f;   // stays finite, or becomes NaN
           // 16 columns at a time by way of shared memory, so that a store takes 64 bytes of eight rows and not 16 of all 32,
           // which kept the adders some 4 us a tile.
 #pragma unroll
@@ -294,7 +299,7 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
             for (int r = lane >> 2; r < 32; r += 8) {
               const float4 x = *reinterpret_cast<const float4*>(turned + r * kSplitPutPitch + (lane & 3) * 4);
               if (row0 + r < m) {
-                worst += 0.0f * x.x + 0.0f * x.y + 0.0f * x.z + 0.0f * x.w;
+                odd = odd || is_doubtful(x.x) || is_doubtful(x.y) || is_doubtful(x.z) || is_doubtful(x.w);
                 float* at = to + (row0 + r) * ld + column;
                 if (quads && column + 4 <= n) {
                   *reinterpret_cast<float4*>(at) = x;
@@ -308,7 +313,6 @@ gemm_float_split_kernel(float* __restrict__ c, const float* __restrict__ a, cons
             }
             __syncwarp();   // the next 16 columns go where these were; tensor memory is loaded by the warp as a whole
           }
-          odd = odd || worst != 0.0f;
         }
       }
     }

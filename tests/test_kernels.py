@@ -1183,6 +1183,25 @@ def test_float32_products_keep_a_rows_bits_among_others(ops, n, k):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("m, n, k", [(140, 20000, 256), (9, 1100, 1024)])
+def test_float32_products_of_numbers_near_nothing(ops, m, n, k):
+    """Operands whose third, second or first part lies below what bfloat16 reaches, beside rows of ordinary ones and of zeros:
+    the bits of the sum in ascending k, or its error against 64 bits."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, w = (torch.randn(rows, k, generator=gen, device="cuda") for rows in (m, n))
+    scales = torch.tensor([0.0, -30.0, -105.0, -112.0, -118.0, -126.0, -132.0, 0.0, 0.0], device="cuda").repeat(m // 9 + 1)[:m]
+    a = (a.double() * 2.0 ** scales.double()[:, None]).float()
+    a[8::9] = 0.0
+    w[::3] = (w[::3].double() * 2.0 ** 20).float()
+    out, plain_out, ref = ops.gemm_float(a, w), ops.gemm_simple(a, w), a.double() @ w.double().t()
+    ops.check_status("cuda")
+    for row in range(min(m, 9)):
+        if scales[row] < -100.0 or row == 8:
+            assert torch.equal(out[row::9], plain_out[row::9]), row
+        else:
+            assert float((out[row::9] - ref[row::9]).norm()) <= float((plain_out[row::9] - ref[row::9]).norm()), row
+
+
 def test_float32_products_of_two_threads(ops):
     """Two host threads whose products want different amounts of shared memory: neither's launch meets the other's limit."""
     import threading
