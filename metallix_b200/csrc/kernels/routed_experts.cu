@@ -45,6 +45,17 @@ enum ExpertForm : int { kExpertReluSquared = 0, kExpertGated = 1, kExpertGelu = 
 enum RouteScores : int { kScoreSoftmax = 0, kScoreSigmoid = 1, kScoreChosen = 2 };
 constexpr int kRouteThreads = 128;   // four tokens a block, a warp each
 
+// The first output that is not among a token's first `count` choices: a token takes an expert once at most, which the
+// products rest on that are told how many rows of a tile are in use.
+__device__ __forceinline__ int first_not_taken(const int* taken, int count, int outputs) {
+  for (int r = 0; r < outputs; ++r) {
+    bool is_taken = false;
+    for (int i = 0; i < count; ++i) is_taken = is_taken || taken[i] == r;
+    if (!is_taken) return r;
+  }
+  return 0;
+}
+
 __global__ void __launch_bounds__(kRouteThreads)
 route_kernel(const float* __restrict__ logits, const float* __restrict__ correction, int* __restrict__ chosen,
              float* __restrict__ weights, float* __restrict__ dense, float* __restrict__ identity_weight,
@@ -145,7 +156,7 @@ route_kernel(const float* __restrict__ logits, const float* __restrict__ correct
       const int other_where = __shfl_xor_sync(0xffffffffu, where, offset);
       if (other > best || (other == best && other_where < where)) { best = other; where = other_where; }
     }
-    if (where >= outputs) where = k < outputs ? k : 0;   // nothing comparable left (non-finite logits)
+    if (where >= outputs) where = first_not_taken(chosen + static_cast<size_t>(t) * choices, k, outputs);   // nothing comparable left
     if (lane == 0) {
       chosen[static_cast<size_t>(t) * choices + k] = where;
       choice[where] = -INFINITY;

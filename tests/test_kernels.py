@@ -1383,6 +1383,28 @@ def test_few_rows_of_many_experts(ops, counts, n, k):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("scores, groups", [("chosen", None), ("softmax", None), ("sigmoid", (4, 2)), ("softmax", (3, 1))])
+def test_a_token_takes_an_expert_once(ops, scores, groups):
+    """Routers with fewer usable outputs than choices (minus infinities, infinities, NaN): the choices still differ, and no
+    expert has more rows than there are tokens, which the products of few rows are told."""
+    rng = np.random.default_rng(5)
+    outputs, top = 12, 4
+    logits = rng.normal(size=(40, outputs))
+    for t in range(1, 40):
+        usable = rng.permutation(outputs)[:rng.integers(0, top)]
+        row = np.full(outputs, [-np.inf, np.nan][t % 2] if scores != "softmax" else np.nan)
+        row[usable] = rng.normal(size=len(usable))
+        logits[t] = row
+    logits[5], logits[6, 3] = np.inf, np.inf
+    correction = dev(np.where(np.arange(outputs) % 5 == 4, -np.inf, 0.0))
+    chosen = ops.route_experts(dev(logits), correction, outputs, top, scores=scores, groups=groups)[0]
+    assert bool(((chosen >= 0) & (chosen < outputs)).all())
+    assert int(torch.tensor([row.unique().numel() for row in chosen]).min()) == top
+    position, tile_group, _ = ops.expert_rows(chosen, outputs)
+    assert int((position % ops.expert_rows_tile()).max()) < 40
+    ops.check_status("cuda")
+
+
 def test_tcgen05_refuses_what_it_cannot_take(ops):
     from metallix_b200 import tensor_core
     a, w = dev(np.zeros((4, 100)), torch.bfloat16), dev(np.zeros((8, 100)), torch.bfloat16)
