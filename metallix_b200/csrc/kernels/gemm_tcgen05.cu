@@ -356,7 +356,7 @@ MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, co
   if (w_rows > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   if (epilogue == kTcSwiGLU && group_rows != 2 * n) return static_cast<int>(cudaErrorInvalidValue);
   if (tile_rows < 1 || tile_rows > kTcM) return static_cast<int>(cudaErrorInvalidValue);
-  if (tile_rows <= tc_rows_limit() && !(tc_gated(epilogue) && epilogue != kTcSwiGLU))
+  if (tile_rows <= tc_rows_limit() && (!tc_gated(epilogue) || (epilogue == kTcSwiGLU && n < kTcFewGatedColumns)))
     return launch_tc_rows({out, a, w, m, n, k, static_cast<int>(w_rows), lda, ldw, ldo, tile_group, group_rows, tile_rows, 0.0f, row_scale,
                            status}, epilogue, stream);
   // a gated tile of width bn holds bn / 2 gate and bn / 2 up rows

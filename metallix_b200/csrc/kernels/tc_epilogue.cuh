@@ -89,6 +89,12 @@ struct TcProduct {
 
 // Products of few rows, bound by reading W (gemm_tcgen05_rows.cu).
 constexpr int kTcFewRows = 64;
+// Gated experts only up to here: a tile holds 32 gate and 32 up rows, and wide ones fill the SMs in tiles of 128 and 128 anyway. us in
+// few rows and in whole tiles, 12 experts, two or three a token: 4096 x 4096 with 16 tokens 174 and 146, 4 tokens 94 and 86; 2048 x 4096
+// 83 and 86, but 65 and 49 with 3 tokens; 1536 x 1024 23 and 27; 768 x 2048 19 and 23. Not gated: 6144 x 4096, 3, 16 and 64 tokens
+// 59 and 63, 120 and 139, 129 and 138; 1024 x 3072 15 and 29, 26 and 33, 27 and 33; the exceptions are counts whose narrow
+// tiles just open another round (7 experts of 4096 x 4096 57 and 53).
+constexpr int kTcFewGatedColumns = 2048;
 int launch_tc_rows(const TcProduct& p, int epilogue, cudaStream_t stream);
 
 }  // namespace mxb
