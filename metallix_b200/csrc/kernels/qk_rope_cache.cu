@@ -611,10 +611,13 @@ MXB_API int mxb_qk_norm_rope_cache(
     const long long items = static_cast<long long>(tokens) * (heads + 2 * kv_heads);
     if (items >= 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
     const int heads_per_warp = 32 / (head_dim / 2 / (16 / element));
-    // Four heads a lane from the number of heads on that gives every SM several blocks either way. us with one and with four,
+    // Four heads a lane from the number of heads on that gives every SM several blocks either way. us with one and with four:
     // bfloat16, heads of 128: 732 tokens of 32 / 8 heads 6.2 and 5.0, 2,048 13.9 and 12.3; 2,048 of 16 / 8 9.4 and 8.6, 732 5.2 and
-    // 5.2, 400 3.4 and 4.2. Heads of 64 lose throughout (2,048 tokens of 16 / 4 5.0 and 5.5).
-    const int each = head_dim >= 128 && heads % 4 == 0 && kv_heads % 4 == 0 && items >= 24576 ? 4 : 1;
+    // 5.2, 400 3.4 and 4.2; heads of 256: 800 of 16 / 8 8.1 and 6.9, 2,048 16.7 and 12.9; float32: 2,048 of 16 / 8 heads of 128 11.2 and
+    // 8.4, of 256 26.2 and 21.0. Heads of 64 lose throughout (2,048 tokens of 16 / 4 5.0 and 5.5), and so do bfloat16 heads of 128
+    // where a third of the lanes only copies values (4,096 tokens of 4 / 4 7.2 and 7.9).
+    const bool gains = head_dim == 256 || (head_dim == 128 && (dtype == kF32 || heads > kv_heads));
+    const int each = gains && heads % 4 == 0 && kv_heads % 4 == 0 && items >= 24576 ? 4 : 1;
     const long long groups = items / each;
     const unsigned blocks = static_cast<unsigned>((groups + 8 * heads_per_warp - 1) / (8 * heads_per_warp));
     cudaError_t launch_status = cudaSuccess;
