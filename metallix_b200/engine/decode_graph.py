@@ -55,6 +55,30 @@ def capture_quietly(graph: torch.cuda.CUDAGraph, pool):
             gc.enable()
 
 
+@contextlib.contextmanager
+def capture_beside(graph: torch.cuda.CUDAGraph, pool, stream: torch.cuda.Stream):
+    """Captures into ``graph`` on ``stream``. Nothing is collected and the
+    allocator's blocks are not given back beforehand, as ``capture_quietly``
+    does: these took 30 and 5 to 50 ms of a step's 45 to 85, the capture itself
+    takes 6. Other threads may go on using the device meanwhile."""
+    collecting = gc.isenabled()
+    gc.disable()   # freeing another engine's graph or device memory in the middle would invalidate the capture
+    try:
+        stream.wait_stream(torch.cuda.current_stream(stream.device))
+        with torch.cuda.stream(stream):
+            graph.capture_begin(**({} if pool is None else {"pool": pool}), capture_error_mode="thread_local")
+            try:
+                yield
+            except BaseException:
+                with contextlib.suppress(RuntimeError):
+                    graph.capture_end()
+                raise
+            graph.capture_end()
+    finally:
+        if collecting:
+            gc.enable()
+
+
 class _Bucket:
     def __init__(self, size: int, bound: int, table_width: int):
         self.size, self.bound, self.table_width = size, bound, table_width

@@ -14,6 +14,7 @@ failure after the reservation rolls every entry of the step back.
 """
 from __future__ import annotations
 
+import gc
 import os
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Optional, Sequence
@@ -27,6 +28,7 @@ from ..config import read_config
 from ..parts.registry import Runtime, StepContext, StepPlan, row_runs, step_preparers
 from ..weights import load_tensors, random_tensors
 from .model import DecoderModel
+from .step_shapes import StepShapes
 
 _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32,
            "fp32": torch.float32, torch.bfloat16: torch.bfloat16, torch.float32: torch.float32}
@@ -116,14 +118,14 @@ class Engine:
         # state that a step advances is advanced once, like the pages it writes. (Three prompts of up to 1,201 tokens
         # through four Sadosun layers of 1,024 values, some 110 launches: 2,585 us launched one by one, 1,430 replayed.)
         self._step_graphs: Optional[Dict] = {} if self.graphs is not None else None
-        # How often a shape has to have come. A capture takes 60 to 100 ms; models with state, whose steps gain some 1 ms from
+        # How often a shape has to have come. A capture takes some 6 ms; models with state, whose steps gain some 1 ms from
         # it, wait until a shape has come more often than a prompt cut into a few portions brings it.
         stateless = not any(need is not None and need.has_state() for need in self.cache.needs)
-        self._sightings = 1 if stateless else 4
+        self._shapes = StepShapes(STEP_GRAPHS, 1 if stateless else 4)
+        self._capture_stream: Optional[torch.cuda.Stream] = None
         self.replay_general_steps = True   # False: general steps are launched kernel by kernel (measurements)
         values = self.model.weight_bytes() / torch.empty((), dtype=self.dtype).element_size()
         self.step_graph_tokens = int(min(STEP_GRAPH_TOKENS, max(256, STEP_GRAPH_SECONDS * DEVICE_FLOPS / (2.0 * values))))
-        self._shapes_seen: Dict = {}
         self._ids: Dict[Hashable, int] = {}   # request name -> manager id
         self._next_id = 1 << 40               # above any id a scheduler hands out
         self.steps = 0
@@ -366,7 +368,7 @@ class Engine:
             bound *= 2
         return min(bound, self.max_context)
 
-    def _run(self, entries: List[StepEntry], tap=None) -> Optional[torch.Tensor]:
+    def _run(self, entries: List[StepEntry], tap=None, graphs: bool = True) -> Optional[torch.Tensor]:
         """A general step: any mix of portions of prompts and decoded tokens.
 
         The step's integers (token ids, positions, block tables, slots, and
@@ -411,8 +413,8 @@ class Engine:
         # contexts inside the bucket are.
         bound = self.context_bucket(longest)
         shape_key = (tuple(counts), len(wanted), bound, tuple(p.graph_key for p in prepared.values()))
-        graphed = tap is None and self._step_graphs is not None and self.replay_general_steps and total <= self.step_graph_tokens and (
-            shape_key in self._step_graphs or self._shapes_seen.get(shape_key, 0) >= self._sightings)
+        graphed = (graphs and tap is None and self._step_graphs is not None and self.replay_general_steps
+                   and total <= self.step_graph_tokens and self._shapes.came(shape_key, self._step_graphs))
         if graphed:   # the parts' integers and bounds for every step of this shape
             plan = StepPlan(counts, starts, rows, bound, replayable=True)
             prepared = {key: part.prepare_step(plan) for key, part in self._preparers.items()}
@@ -473,35 +475,54 @@ class Engine:
                 d_wanted if wanted else None, tap=tap)
 
         if not graphed:
-            if tap is None and self._step_graphs is not None and self.replay_general_steps:
-                self._shapes_seen[shape_key] = self._shapes_seen.get(shape_key, 0) + 1
-                if len(self._shapes_seen) > 4096:
-                    self._shapes_seen.clear()
             return forward(packed.to(self.device, non_blocking=True))
-        return self._replay_step(shape_key, packed, forward)
+        if shape_key not in self._step_graphs and not self._capture_step(shape_key, packed, forward):
+            return self._run(entries, graphs=False)
+        return self._replay_step(shape_key, packed)
 
-    def _replay_step(self, shape_key, packed: torch.Tensor, forward) -> Optional[torch.Tensor]:
-        """Replays (after capturing it, the first time) the graph of a general
-        step of this shape with the integers in ``packed``."""
-        from .decode_graph import capture_quietly
-        held = self._step_graphs.get(shape_key)
-        if held is None:
-            # A step of this shape has run before, kernel by kernel: libraries
-            # and lazily loaded kernels have settled, the capture needs no
-            # warm-up run of its own.
-            static = packed.to(self.device)
-            torch.cuda.synchronize(self.device)
-            graph = torch.cuda.CUDAGraph()
-            before = ops.launch_count()
-            pool = self.graphs.pool if self.graphs is not None else None
-            with capture_quietly(graph, pool):
-                logits = forward(static)
-            if self.graphs is not None and self.graphs.pool is None:
-                self.graphs.pool = graph.pool()
-            held = {"graph": graph, "static": static, "logits": logits, "kernels": ops.launch_count() - before}
-            if len(self._step_graphs) >= STEP_GRAPHS:
-                self._step_graphs.pop(next(iter(self._step_graphs)))   # the oldest shape makes room
-            self._step_graphs[shape_key] = held
+    def _capture_step(self, shape_key, packed: torch.Tensor, forward) -> bool:
+        """Captures the graph of a general step of this shape, which executes
+        nothing. False where that fails: a graph holds the step's activations
+        a second time, and memory may be short."""
+        from . import decode_graph
+        if len(self._step_graphs) >= STEP_GRAPHS:
+            least = self._shapes.least(self._step_graphs)
+            del self._step_graphs[least]
+            self._shapes.evicted(least)
+        if self._capture_stream is None:
+            self._capture_stream = torch.cuda.Stream(self.device)   # the same for all: graphs of one stream share their memory
+        for last_try in (False, True):
+            before, graph = ops.launch_count(), torch.cuda.CUDAGraph()
+            out_of_memory = None
+            try:
+                # A step of this shape has run before, kernel by kernel: libraries
+                # and lazily loaded kernels have settled, the capture needs no
+                # warm-up run of its own.
+                static = packed.to(self.device)
+                with decode_graph.capture_beside(graph, self.graphs.pool, self._capture_stream):
+                    logits = forward(static)
+            except torch.OutOfMemoryError:
+                out_of_memory = True
+            except RuntimeError:   # whatever it is shows again where the step is launched kernel by kernel
+                out_of_memory = False
+            if out_of_memory is None:
+                if self.graphs.pool is None:
+                    self.graphs.pool = graph.pool()
+                self._step_graphs[shape_key] = {"graph": graph, "static": static, "logits": logits,
+                                                "kernels": ops.launch_count() - before}
+                return True
+            del graph
+            if last_try or not out_of_memory:
+                break
+            gc.collect()
+            torch.cuda.empty_cache()   # blocks that the allocator keeps for launched steps
+        self._shapes.failed(shape_key)
+        return False
+
+    def _replay_step(self, shape_key, packed: torch.Tensor) -> Optional[torch.Tensor]:
+        """Replays the graph of a general step of this shape with the integers
+        in ``packed``."""
+        held = self._step_graphs[shape_key]
         held["static"].copy_(packed, non_blocking=True)
         held["graph"].replay()
         ops.count_launches(held["kernels"])
