@@ -293,7 +293,7 @@ walk_kernel(WalkArgs a) {
       T value[kEight];
 #pragma unroll
       for (int t = 0; t < kEight; ++t) value[t] = next[t];
-      if (!barrier_wait(&full[stage], (r / kWalkStages) & 1, a.status)) { ok = false; break; }
+      if (!barrier_wait_warp(&full[stage], (r / kWalkStages) & 1, a.status)) { ok = false; break; }
       fetch((r + 1) * kEight);   // on their way while this stage is walked
       const float* record = stages + stage * RECORD;
       auto vector = [&](int index, Pair (&into)[PAIRS]) {

@@ -531,6 +531,10 @@ using namespace mxb;
 //   sixteen of 128                          1,017 and 486                 365 and 204                 108 and 112
 //   eight of 64                               265 and 167                 110 and 104                  33 and  99
 //   four of 64, 300 single tokens           2,169 and 2,692               872 and 843                 222 and 509
+// The second figures are those of products that read one value at a time, when the lines were drawn. Since they read four,
+// what is taken costs, walk first again: one row of 192 99 and 62; of 256 131 and 64, 90 and 47, 90 and 46; of 2,048 1,011 and 296,
+// 688 and 120, 684 and 61; 512 beside 127 single tokens 1,235 and 1,009, 519 and 327, 243 and 172; four of 128 260 and 93; sixteen
+// of 128 941 and 336, 312 and 124.
 MXB_API int mxb_mlstm_chunks_scratch(long long tokens, int rows, int longest, int heads, int dim, int vdim) {
   const bool much = tokens * heads * dim * vdim > 1ll << 26;
   const bool few_beside_long = (longest >= 256 || (longest >= 192 && much)) && 3ll * rows <= longest - 128;

@@ -19,6 +19,13 @@ def test_warps_that_use_tensor_memory_wait_and_give_up_as_a_whole(name):
     assert reads == []
 
 
+def test_warps_that_exchange_values_wait_as_a_whole():
+    """The delta rule's walkers exchange sums by shuffles of the whole warp; only its fetching lane waits alone."""
+    with open(os.path.join(KERNELS, "delta_prompt.cu")) as handle:
+        text = handle.read()
+    assert text.count("= barrier_wait(&empty[stage]") == 1 and len(re.findall(r"\bbarrier_wait\(", text)) == 1
+
+
 def test_lanes_without_rows_are_back_before_tensor_memory_is_loaded():
     """Lanes whose row does not exist store nothing and are ahead of the others: the warp meets before the next load."""
     with open(os.path.join(KERNELS, "tc_epilogue.cuh")) as handle:
