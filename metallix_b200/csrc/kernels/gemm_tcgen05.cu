@@ -229,16 +229,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ------------------------------------------------------------------ host side
-int g_tc_bn = 0, g_tc_deep = -1;  // tuning overrides: tile width, deep (1) or shallow (0) pipeline
-int g_tc_rows = -1;               // rows up to which the kernel for few rows is taken, -1: kTcFewRows
-static int tc_rows_limit() { return g_tc_rows < 0 ? kTcFewRows : g_tc_rows; }
-
-template <int BN, int EPI, int STAGES_>
-static int launch_tc_staged(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n, int k,
-                            long long ldo, const int* tile_group, int group_rows, float limit, const float* row_scale,
-                            int* status, cudaStream_t stream) {
-  using Config = TcConfig<BN, STAGES_>;
-  auto kernel = gemm_tcgen05_kernel<BN, EPI, STAGES_>;
+// The whole shared memory is pipeline: a block owns its SM, and tensor memory holds two accumulators.
+template <int BN, int EPI>
+static int launch_tc(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n, int k,
+                     long long ldo, int* status, cudaStream_t stream, const int* tile_group = nullptr,
+                     int group_rows = 0, float limit = 0.0f, const float* row_scale = nullptr) {
+  constexpr int stages = BN >= 256 ? 4 : (BN >= 128 ? 6 : 8);
+  using Config = TcConfig<BN, stages>;
+  auto kernel = gemm_tcgen05_kernel<BN, EPI, stages>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Config::kSharedBytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   constexpr int out_columns = tc_gated(EPI) ? BN / 2 : BN;
@@ -253,19 +251,6 @@ static int launch_tc_staged(const CUtensorMap& map_a, const CUtensorMap& map_b, 
   kernel<<<grid, kTcThreads, Config::kSharedBytes, stream>>>(map_a, map_b, out, m, n, k, ldo, tile_group, group_rows,
                                                              limit, row_scale, status);
   return static_cast<int>(cudaGetLastError());
-}
-
-// Deep: the whole shared memory as pipeline (the default; a block owns its SM
-// and tensor memory holds two accumulators). Shallow: half the stages.
-template <int BN, int EPI>
-static int launch_tc(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n, int k,
-                     long long ldo, int* status, cudaStream_t stream, const int* tile_group = nullptr,
-                     int group_rows = 0, float limit = 0.0f, const float* row_scale = nullptr) {
-  constexpr int deep = BN >= 256 ? 4 : (BN >= 128 ? 6 : 8);
-  const bool shallow = g_tc_deep == 0;
-  if (shallow)
-    return launch_tc_staged<BN, EPI, deep / 2>(map_a, map_b, out, m, n, k, ldo, tile_group, group_rows, limit, row_scale, status, stream);
-  return launch_tc_staged<BN, EPI, deep>(map_a, map_b, out, m, n, k, ldo, tile_group, group_rows, limit, row_scale, status, stream);
 }
 
 }  // namespace mxb
@@ -287,14 +272,15 @@ MXB_API int mxb_gemm_tcgen05(void* out, const void* a, const void* w, int m, int
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return static_cast<int>(cudaErrorInvalidValue);
   const int w_rows = tc_gated(epilogue) ? 2 * n : n;
   if (epilogue == kTcReluSquared) return static_cast<int>(cudaErrorInvalidValue);   // of grouped products
-  if (g_tc_bn == 0 && m <= tc_rows_limit())
+  if (m <= kTcFewRows)
     return launch_tc_rows({out, a, w, m, n, k, w_rows, lda, ldw, ldo, nullptr, 0, m, limit, nullptr, status}, epilogue, stream);
   // Narrow outputs take narrower tiles so that the grid still covers the GPU.
   const int m_tiles = (m + kTcM - 1) / kTcM;
   int bn = 256;
   if (tc_gated(epilogue)) {
     // A SwiGLU tile of width bn holds bn / 2 gate and bn / 2 up rows. Timed
-    // on [m, 1024] x [6144, 1024]: up to 128 rows 64 is fastest (10 against 14
+    // on [m, 1024] x [6144, 1024]: up to 128 rows (from 65 on, fewer went to the
+    // kernel for few rows above) 64 is fastest (10 against 14
     // us), at 256 rows 128 (12 against 15), from 512 rows on 256.
     bn = m <= 128 ? 64 : (m <= 256 ? 128 : 256);
   } else {
@@ -302,7 +288,6 @@ MXB_API int mxb_gemm_tcgen05(void* out, const void* a, const void* w, int m, int
     if (m_tiles * ((n + 255) / 256) < 118) bn = 128;
     if (bn == 128 && m_tiles * ((n + 127) / 128) < 118) bn = 64;
   }
-  if (g_tc_bn != 0) bn = g_tc_bn;
   CUtensorMap map_a, map_b;
   const int b_box = tc_gated(epilogue) ? bn / 2 : bn;
   if (!make_map(&map_a, a, m, k, lda, kTcM) || !make_map(&map_b, w, w_rows, k, ldw, b_box))
@@ -356,7 +341,7 @@ MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, co
   if (w_rows > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   if (epilogue == kTcSwiGLU && group_rows != 2 * n) return static_cast<int>(cudaErrorInvalidValue);
   if (tile_rows < 1 || tile_rows > kTcM) return static_cast<int>(cudaErrorInvalidValue);
-  if (tile_rows <= tc_rows_limit() && (!tc_gated(epilogue) || (epilogue == kTcSwiGLU && n < kTcFewGatedColumns)))
+  if (tile_rows <= kTcFewRows && (!tc_gated(epilogue) || (epilogue == kTcSwiGLU && n < kTcFewGatedColumns)))
     return launch_tc_rows({out, a, w, m, n, k, static_cast<int>(w_rows), lda, ldw, ldo, tile_group, group_rows, tile_rows, 0.0f, row_scale,
                            status}, epilogue, stream);
   // a gated tile of width bn holds bn / 2 gate and bn / 2 up rows
@@ -376,12 +361,4 @@ MXB_API int mxb_gemm_tcgen05_grouped(void* out, const void* a, const void* w, co
   if (epilogue == kTcSwiGLU) { GROUPED(kTcSwiGLU) }
 #undef GROUPED
   return static_cast<int>(cudaErrorInvalidValue);
-}
-
-// Tuning hook: force the tile width (64, 128, 256; 0 = choose) and the
-// pipeline depth (1 deep, 0 shallow, -1 = choose).
-MXB_API void mxb_gemm_tcgen05_tune_rows(int rows) { mxb::g_tc_rows = rows; }
-MXB_API void mxb_gemm_tcgen05_tune(int bn, int deep) {
-  mxb::g_tc_bn = bn;
-  mxb::g_tc_deep = deep;
 }

@@ -34,3 +34,18 @@ def test_lanes_without_rows_are_back_before_tensor_memory_is_loaded():
     with open(os.path.join(KERNELS, "gemm_float_split.cu")) as handle:
         adders = handle.read().split("// ---- adders")[1].split("// ---- splitters")[0]
     assert "continue;" not in adders.split("again_any")[0] and re.search(r"__syncwarp\(\);[^\n]*\n *}\n", adders)
+
+
+def test_every_exported_function_is_reached():
+    """What the shared library exports, the Python side binds, or a C program links against."""
+    from metallix_b200 import ops
+    exported = set()
+    for name in os.listdir(KERNELS):
+        if name.endswith(".cu"):
+            with open(os.path.join(KERNELS, name)) as handle:
+                exported |= set(re.findall(r"MXB_API\s+[\w ]+?\b(mxb_\w+)\(", handle.read()))
+    with open(ops.__file__) as handle:
+        by_hand = set(re.findall(r"\.(mxb_\w+)", handle.read()))
+    with open(os.path.join(KERNELS, "attention_decode_noalloc.h")) as handle:
+        linked = set(re.findall(r"\b(mxb_\w+)\(", handle.read()))
+    assert len(exported) > 60 and exported - set(ops._SIGNATURES) - by_hand - linked == set()
