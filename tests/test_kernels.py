@@ -1383,6 +1383,40 @@ def test_few_rows_of_many_experts(ops, counts, n, k):
     ops.check_status("cuda")
 
 
+def test_grouped_products_of_several_tiles_a_block(ops):
+    """Blocks that go on from tile to tile, over runs, bands and tiles that are left out in the middle of their walk: each
+    group's rows have the bits of its own product."""
+    from metallix_b200 import tensor_core
+    gen, n, k = torch.Generator(device="cuda").manual_seed(3), 6100, 136
+    tiles = [0, 0, 0, -1, 1, 1, 1, -1, -1, 1, 2] + [3] * 18 + [-1]
+    a = torch.randn(128 * len(tiles), k, generator=gen, device="cuda").bfloat16()
+    w = torch.randn(4 * n, k, generator=gen, device="cuda").bfloat16()
+    out = tensor_core.gemm_grouped(a, w, dev(tiles, torch.int32), 4, tensor_core.STORE_F32)
+    for tile, group in enumerate(tiles):
+        if group >= 0:
+            rows = slice(128 * tile, 128 * tile + 128)
+            assert torch.equal(out[rows], tensor_core.gemm(a[rows], w[group * n:(group + 1) * n], torch.float32)), tile
+    ops.check_status("cuda")
+
+
+@pytest.mark.parametrize("epilogue, n, k", [("STORE_F32", 4100, 136), ("GELU", 2500, 264), ("SWIGLU", 1100, 520), ("SWIGLU", 2100, 72)])
+def test_few_rows_of_experts_over_several_tiles_a_block(ops, epilogue, n, k):
+    """Thirteen experts, more tiles than three rounds of blocks hold, some left out between others."""
+    from metallix_b200 import tensor_core
+    gen, epilogue = torch.Generator(device="cuda").manual_seed(n), getattr(tensor_core, epilogue)
+    tiles = [0, 1, 2, -1, 3, 4, -1, -1, 5, 6, 7, 8, 9, 10, 11, -1, 12]
+    per = 2 * n if epilogue == tensor_core.SWIGLU else n
+    used = (torch.arange(17) + torch.arange(len(tiles))[:, None] * 128).reshape(-1).cuda()
+    live = torch.tensor([tile >= 0 for tile in tiles]).repeat_interleave(17).cuda()
+    a = torch.randn(128 * len(tiles), k, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(13 * per, k, generator=gen, device="cuda") * k ** -0.5).bfloat16()
+    scale = torch.rand(a.shape[0], generator=gen, device="cuda") if epilogue == tensor_core.GELU else None
+    few = tensor_core.gemm_grouped(a, w, dev(tiles, torch.int32), 13, epilogue, row_scale=scale, tile_rows=17)
+    every = tensor_core.gemm_grouped(a, w, dev(tiles, torch.int32), 13, epilogue, row_scale=scale)
+    assert torch.equal(few[used[live]], every[used[live]])
+    ops.check_status("cuda")
+
+
 @pytest.mark.parametrize("scores, groups", [("chosen", None), ("softmax", None), ("sigmoid", (4, 2)), ("softmax", (3, 1))])
 def test_a_token_takes_an_expert_once(ops, scores, groups):
     """Routers with fewer usable outputs than choices (minus infinities, infinities, NaN): the choices still differ, and no
