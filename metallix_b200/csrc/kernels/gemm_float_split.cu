@@ -1,7 +1,8 @@
 // C[M, N] = A[M, K] * W[N, K]^T of float32 operands on the fifth-generation tensor cores, with float32's precision.
 //
 // A float32 number is the sum of three bfloat16 numbers, x = x1 + x2 + x3, each the rounding of what the ones before
-// left: 8 bits each, 24 together. Of the nine products of two such numbers six are made: x1 y1, x1 y2, x2 y1, x2 y2, x1 y3
+// left: 8 bits each, 24 together (Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for
+// higher-precision computations", ARITH 2019). Of the nine products of two such numbers six are made: x1 y1, x1 y2, x2 y1, x2 y2, x1 y3
 // and x3 y1; what is left out is at most 2^-24 of |x y|, and 2^-27 on average. Products of bfloat16 are exact; what
 // limits the result is how they are added up. The tensor core cuts sums off where it aligns them, so x1 y1 is summed
 // over 64 k at a time and these sums are added up in registers, rounded to nearest; the five small products have an

@@ -413,6 +413,11 @@ class Engine:
         # contexts inside the bucket are.
         bound = self.context_bucket(longest)
         shape_key = (tuple(counts), len(wanted), bound, tuple(p.graph_key for p in prepared.values()))
+        runs = wanted_runs = None
+        if self.dtype == torch.float32 and not self.runtime.ordered_sums:
+            runs, wanted_runs = row_runs(counts, counts), row_runs(counts, [len(e.want) for e in entries])
+            if len(runs) > 1:   # which of the wanted rows are of portions decides their kernel
+                shape_key += (tuple(wanted_runs or ()),)
         graphed = (graphs and tap is None and self._step_graphs is not None and self.replay_general_steps
                    and total <= self.step_graph_tokens and self._shapes.came(shape_key, self._step_graphs))
         if graphed:   # the parts' integers and bounds for every step of this shape
@@ -469,7 +474,7 @@ class Engine:
                 # inside a graph the host's view of one step would be baked in for all
                 request_offsets=None if graphed else [int(v) for v in offsets],
                 request_positions=None if graphed else starts, extras=extras,
-                runs=None if self.runtime.ordered_sums or self.dtype != torch.float32 else row_runs(counts))
+                runs=runs, wanted_runs=wanted_runs)
             return self.model.forward(
                 d_ids, ctx, lambda entry, write: cache.view(entry, write, tables, slots),
                 d_wanted if wanted else None, tap=tap)

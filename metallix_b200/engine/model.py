@@ -82,7 +82,7 @@ class DecoderModel:
         if self.joins:
             first = residual if self.order[0].join is not None else residual.clone()
         pending = None
-        self.runtime.runs = ctx.runs   # through the layers, whose products are of the step's rows; the head's are not
+        self.runtime.runs = ctx.runs
         try:
             for index, run in enumerate(self.order):
                 block = self.blocks[run.layer]
@@ -93,13 +93,14 @@ class DecoderModel:
                     settle(residual, pending)
                     pending = None
                     tap(index, sum_of_streams(residual) if streams else residual)
+            if wanted_rows is None or wanted_rows.numel() == 0:
+                return None
+            self.runtime.runs = ctx.wanted_runs
+            if streams:   # what is pending joins, the streams are summed and normed, on the wanted rows only
+                return self.head.forward(read_streams(residual, pending, None, self.final_norm, self.runtime.dtype,
+                                                      rows_index=wanted_rows, keep_streams=False))
+            settle(residual, pending)
+            normed = self.final_norm.forward(residual, self.runtime.dtype, rows_index=wanted_rows)
+            return self.head.forward(normed)
         finally:
             self.runtime.runs = None
-        if wanted_rows is None or wanted_rows.numel() == 0:
-            return None
-        if streams:   # what is pending joins, the streams are summed and normed, on the wanted rows only
-            return self.head.forward(read_streams(residual, pending, None, self.final_norm, self.runtime.dtype,
-                                                  rows_index=wanted_rows, keep_streams=False))
-        settle(residual, pending)
-        normed = self.final_norm.forward(residual, self.runtime.dtype, rows_index=wanted_rows)
-        return self.head.forward(normed)

@@ -63,8 +63,9 @@ class Runtime:
     # single tokens and portions run on kernels of different orders says no; then large products of portions take the tensor
     # cores (with gemm_backend "auto"), in an order that what else is in the step does not change.
     ordered_sums: bool = True
-    # During a step through the layers, where ordered_sums is False: the step's packed rows as runs (first row, row behind the
-    # last, whether they are of portions of several tokens). A row's kernel follows from its own request's portion alone.
+    # During a step, where ordered_sums is False: the rows that pass through the layers, and then those that pass through the
+    # head, as runs (first row, row behind the last, whether they are of portions of several tokens). A row's kernel follows
+    # from its own request's portion alone.
     runs: Optional[Sequence[Tuple[int, int, bool]]] = None
 
 
@@ -206,18 +207,20 @@ class StepContext:
     request_positions: Optional[List[int]]  # host, first position of each row's tokens
     extras: Dict[str, object] = field(default_factory=dict)
     token_ids: Optional[torch.Tensor] = None   # int32 [tokens]: the step's token ids, for a part that reads a table by them
-    runs: Optional[List[Tuple[int, int, bool]]] = None   # host: as Runtime.runs
+    runs: Optional[List[Tuple[int, int, bool]]] = None         # host: as Runtime.runs, of the packed tokens
+    wanted_runs: Optional[List[Tuple[int, int, bool]]] = None  # host: of the rows whose logits are wanted
 
 
-def row_runs(counts: Sequence[int]) -> List[Tuple[int, int, bool]]:
-    """The packed rows of requests that bring ``counts`` tokens, as runs of rows of one kind: (first row, row behind the last
-    one, whether they belong to portions of several tokens)."""
+def row_runs(counts: Sequence[int], rows: Sequence[int]) -> Optional[List[Tuple[int, int, bool]]]:
+    """``rows[r]`` rows each of requests that bring ``counts[r]`` tokens, one after another, as runs of rows of one kind:
+    (first row, row behind the last one, whether they belong to portions of several tokens). None for no rows."""
     runs, begin = [], 0
-    for count in counts:
-        first = runs.pop()[0] if runs and runs[-1][2] == (count > 1) else begin
-        begin += count
-        runs.append((first, begin, count > 1))
-    return runs
+    for count, size in zip(counts, rows):
+        if size:
+            first = runs.pop()[0] if runs and runs[-1][2] == (count > 1) else begin
+            begin += size
+            runs.append((first, begin, count > 1))
+    return runs or None
 
 
 def step_preparers(blocks) -> Dict[str, object]:

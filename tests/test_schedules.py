@@ -108,7 +108,7 @@ def test_a_mixed_step_replays_a_graph(model_folders, name, dtype):
 
 # Matrices large enough for the float32 products on the tensor cores, heads of the split-key decode kernel.
 WIDE = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_act="silu", num_hidden_layers=2, hidden_size=1024,
-            num_attention_heads=16, num_key_value_heads=8, head_dim=64, intermediate_size=1100, vocab_size=500,
+            num_attention_heads=16, num_key_value_heads=8, head_dim=64, intermediate_size=1100, vocab_size=1100,
             rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True, max_position_embeddings=512)
 
 
@@ -186,10 +186,13 @@ def test_float32_bits_are_the_same_in_captured_steps():
     for graphs in (True, False):
         engine = wide_engine(cuda_graphs=graphs)
         engine.step([StepEntry("a", ids[0][:30], [])])
-        seen[graphs] = [engine.step([StepEntry("a", [ids[0][30 + n]], [0]), StepEntry("b", ids[1][16 * n:16 * n + 16], [15]),
-                                     StepEntry("c", ids[2][5 * n:5 * n + 5], [4])]).clone() for n in range(5)]
+        seen[graphs] = []
+        for n in range(8):   # two wanted rows, now of the decoded token and a portion, now of the portions
+            mine = n % 2
+            seen[graphs].append(engine.step([StepEntry("a", [ids[0][30 + n]], [0] * mine), StepEntry("b", ids[1][16 * n:16 * n + 16], [15]),
+                                             StepEntry("c", ids[2][5 * n:5 * n + 5], [4] * (1 - mine))]).clone())
         engine.check()
-        assert not graphs or len(engine._step_graphs) == 1
+        assert not graphs or len(engine._step_graphs) == 2
     assert all(torch.equal(x, y) for x, y in zip(seen[True], seen[False]))
 
 
