@@ -1759,8 +1759,8 @@ def gemm_float(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
 # Float32 products with at least this many rows of W and values each go to the tensor cores where they are of a prompt's
 # rows, us against the CUDA cores' kernels: 917 rows x 4096 x 1024 77 and 213, x 1024 x 2048 50 and 128; 16 rows 19 and 48, 20
 # and 97; but 8 rows 19 and 17, 20 and 12, and 400 x 512 x 1024 19 and 39, 64 x 768 x 768 17 and 31, 8 x 768 x 768 15 and 5; logits
-# (151936 x 1024) of 32 rows 338 and 439, of one 332 and 156. The
-# number of rows has no say: a row's bits would depend on what else is in the step.
+# (151936 x 1024) of 32 rows 338 and 439, of one 332 and 156. The number of rows has no say: a row's bits would depend on what
+# else is in the step.
 FLOAT_SIDE = 1024
 
 
