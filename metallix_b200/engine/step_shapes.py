@@ -1,14 +1,15 @@
 """Which shapes of general steps are worth a captured graph.
 
 A capture takes 3 to 8 ms, two or three launched steps, and pays by the
-millisecond or so that each replay saves, so a shape has to come again before it gets one, and room for a
-graph is limited. Where more shapes come again and again than there is room
-for, graphs that make room for each other all the time would cost more than
-they save (40 shapes picked evenly, 32 graphs, the oldest making room: one step
-in five a capture; by the rule below one in forty, with as many replays. 40
-shapes of three prompts through four Sadosun layers: 1.84 ms a step, 2.5 launched). So a
-graph makes room only for a shape that comes as often of late as its own, and
-that came again within a sixteenth of the time that the graph has not been used.
+millisecond or so that each replay saves, so a shape has to come again before
+it gets one, and room for a graph is limited. Where more shapes come again and
+again than there is room for, graphs that make room for each other all the time
+would cost more than they save (40 shapes picked evenly, 32 graphs, the oldest
+making room: one step in five a capture; by the rule below one in forty, with as
+many replays. 40 shapes of three prompts through four Sadosun layers: 1.8 ms a
+step, some 2.5 launched). So a graph makes room only for a shape that comes as
+often of late as its own, and that came again within a sixteenth of the time
+that the graph has not been used.
 """
 from __future__ import annotations
 
